@@ -88,28 +88,84 @@ struct StepParams {
     int fixed_axes;         // bit a: the two faces of axis a are Fixed (frozen, not evolved)
 };
 
-// The mixed form's per-site constants in float, precomputed on the host and
-// passed by value, so the step's FP32 arithmetic takes them as constant
-// operands (no double-to-float conversion or FP64 arithmetic per site, no
-// registers held for them; measured 2-3 % on the SM step).
+// The per-site constants of the throughput forms in their compute type,
+// precomputed on the host and passed by value, so the step takes them as constant
+// operands (no conversion or product of parameters per site, no registers held for
+// them).  Everything that enters a force carries its factor dt^2, and the couplings
+// the currents' 1/4 (site_step), which saves a multiply per force component.
+template <class C>
+struct KConst {
+    C ldt[3];          // dt^2 / dx_a^2
+    C diag;            // -2 dt^2 (1/dx^2 + 1/dy^2 + 1/dz^2)
+    C keep;            // 1 - damping_step
+    C cY, cI, cH;      // dt^2 g'^2 / 4, dt^2 g^2 / 4, dt^2 g''^2 / 4
+    C lambda, eta_sqr; // dt^2 lambda; eta^2
+    // Double_SO_N dV/dphi coefficients (Potentials/Source/Double_SO_N.cpp:244-341), times dt^2
+    C diag1, diag2;                          // diag + 2 m1, diag + 2 m2
+    C l1x4, l2x4, l3x2;                      // 4 l1, 4 l2, 2 l3
+    C m12r, l4p5x2, l6r, l7r, l6rx2, l7rx2;  // m12r, 2 l4p5, l6r, l7r, 2 l6r, 2 l7r
+    C m12i, l4m5x2, l5ix2, l6i, l7i, l6ix2, l7ix2;
+    // logging-step energy weights
+    C e_plaq[3];       // 4 lap_i lap_j for the planes (0,1), (0,2), (1,2)
+    C e_grad[3];       // 0.5 / dx_a^2
+    C e_elec[3];       // 4 lap_d / dt^2
+    C inv_g_sqr, inv_gp_sqr, inv_gpp_sqr;
+};
+
+template <class C>
+__host__ __device__ inline KConst<C> make_kconst(const StepParams& P)
+{
+    KConst<C> F;
+    const double d2 = P.dt2, dg = -2.0 * (P.lap[0] + P.lap[1] + P.lap[2]);
+    for (int a = 0; a < 3; a++) F.ldt[a] = (C)(d2 * P.lap[a]);
+    F.diag = (C)(d2 * dg);
+    F.keep = (C)(1.0 - P.damping_step);
+    F.cY = (C)(0.25 * d2 * P.gsq[0]);
+    F.cI = (C)(0.25 * d2 * P.gsq[1]);
+    F.cH = (C)(0.25 * d2 * P.gsq_hf);
+    F.lambda = (C)(d2 * P.lambda);
+    F.eta_sqr = (C)P.eta_sqr;
+    F.diag1 = (C)(d2 * (dg + 2.0 * P.m1));
+    F.diag2 = (C)(d2 * (dg + 2.0 * P.m2));
+    F.l1x4 = (C)(4.0 * d2 * P.l1);
+    F.l2x4 = (C)(4.0 * d2 * P.l2);
+    F.l3x2 = (C)(2.0 * d2 * P.l3);
+    F.m12r = (C)(d2 * P.m12r);
+    F.l4p5x2 = (C)(2.0 * d2 * P.l4p5);
+    F.l6r = (C)(d2 * P.l6r);
+    F.l7r = (C)(d2 * P.l7r);
+    F.l6rx2 = (C)(2.0 * d2 * P.l6r);
+    F.l7rx2 = (C)(2.0 * d2 * P.l7r);
+    F.m12i = (C)(d2 * P.m12i);
+    F.l4m5x2 = (C)(2.0 * d2 * P.l4m5);
+    F.l5ix2 = (C)(2.0 * d2 * P.l5i);
+    F.l6i = (C)(d2 * P.l6i);
+    F.l7i = (C)(d2 * P.l7i);
+    F.l6ix2 = (C)(2.0 * d2 * P.l6i);
+    F.l7ix2 = (C)(2.0 * d2 * P.l7i);
+    const int pi[3] = {0, 0, 1}, pj[3] = {1, 2, 2};
+    for (int pl = 0; pl < 3; pl++) F.e_plaq[pl] = (C)(4.0 * P.lap[pi[pl]] * P.lap[pj[pl]]);
+    for (int a = 0; a < 3; a++) {
+        F.e_grad[a] = (C)(0.5 * P.inv_dx[a] * P.inv_dx[a]);
+        F.e_elec[a] = (C)(4.0 * P.lap[a] * P.inv_sqr_dt);
+    }
+    F.inv_g_sqr = (C)P.inv_g_sqr;
+    F.inv_gp_sqr = (C)P.inv_gp_sqr;
+    F.inv_gpp_sqr = (C)P.inv_gpp_sqr;
+    return F;
+}
+
+// The same for the SM plain steps with two sites per thread and with each site
+// split between two threads (gft_pair_body.cuh, gft_split_body.cuh).
 struct FConst {
     float lap[3];      // 1/dx_a^2
     float diag;        // -2 (1/dx^2 + 1/dy^2 + 1/dz^2)
     float dt2, keep;   // dt^2, 1 - damping_step
     float gY, gI;      // g'^2, g^2 as the couplings of the link equations
     float lambda, eta_sqr;
-    // Double_SO_N dV/dphi coefficients (Potentials/Source/Double_SO_N.cpp:244-341)
-    float m1x2n, l1x4, l3x2, m2x2n, l2x4;        // -2 m1, 4 l1, 2 l3, -2 m2, 4 l2
-    float m12rn, l4p5x2, l6r, l7r, l6rx2, l7rx2;  // -m12r, 2 l4p5, l6r, l7r, 2 l6r, 2 l7r
-    float m12i, l4m5x2, l5ix2, l6i, l7i, l6ix2, l7ix2;
-    // logging-step energy weights (the float values of the FP64 products they replace)
-    float e_plaq[3];   // 4 lap_i lap_j for the planes (0,1), (0,2), (1,2)
-    float e_grad[3];   // 0.5 / dx_a^2
-    float e_elec[3];   // 4 lap_d / dt^2
-    float inv_g_sqr, inv_gp_sqr, inv_gpp_sqr;
 };
 
-__host__ __device__ inline FConst make_fconst(const StepParams& P)
+inline FConst make_fconst(const StepParams& P)
 {
     FConst F;
     for (int a = 0; a < 3; a++) F.lap[a] = (float)P.lap[a];
@@ -120,33 +176,6 @@ __host__ __device__ inline FConst make_fconst(const StepParams& P)
     F.gI = (float)P.gsq[1];
     F.lambda = (float)P.lambda;
     F.eta_sqr = (float)P.eta_sqr;
-    F.m1x2n = (float)(-2.0 * P.m1);
-    F.l1x4 = (float)(4.0 * P.l1);
-    F.l3x2 = (float)(2.0 * P.l3);
-    F.m2x2n = (float)(-2.0 * P.m2);
-    F.l2x4 = (float)(4.0 * P.l2);
-    F.m12rn = (float)(-P.m12r);
-    F.l4p5x2 = (float)(2.0 * P.l4p5);
-    F.l6r = (float)P.l6r;
-    F.l7r = (float)P.l7r;
-    F.l6rx2 = (float)(2.0 * P.l6r);
-    F.l7rx2 = (float)(2.0 * P.l7r);
-    F.m12i = (float)P.m12i;
-    F.l4m5x2 = (float)(2.0 * P.l4m5);
-    F.l5ix2 = (float)(2.0 * P.l5i);
-    F.l6i = (float)P.l6i;
-    F.l7i = (float)P.l7i;
-    F.l6ix2 = (float)(2.0 * P.l6i);
-    F.l7ix2 = (float)(2.0 * P.l7i);
-    const int pi[3] = {0, 0, 1}, pj[3] = {1, 2, 2};
-    for (int pl = 0; pl < 3; pl++) F.e_plaq[pl] = (float)(4.0 * P.lap[pi[pl]] * P.lap[pj[pl]]);
-    for (int a = 0; a < 3; a++) {
-        F.e_grad[a] = (float)(0.5 * P.inv_dx[a] * P.inv_dx[a]);
-        F.e_elec[a] = (float)(4.0 * P.lap[a] * P.inv_sqr_dt);
-    }
-    F.inv_g_sqr = (float)P.inv_g_sqr;
-    F.inv_gp_sqr = (float)P.inv_gp_sqr;
-    F.inv_gpp_sqr = (float)P.inv_gpp_sqr;
     return F;
 }
 

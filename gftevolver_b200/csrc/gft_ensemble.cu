@@ -62,7 +62,7 @@ struct EnsParams {
     // as by-value kernel parameters (constant operands) instead of through the
     // member index.
     StepParams common;
-    FConst fcommon;
+    KConst<float> fcommon;
 };
 // Kernel parameter space (sm_70 and later, CUDA 12.1+): 32,764 bytes; the kernel's
 // other parameters take 48.
@@ -164,9 +164,9 @@ __global__ void __launch_bounds__(TY * TZ, 512 / (TY * TZ))
             Pu.fixed_axes = Pm.fixed_axes;
         }
         const StepParams& P = UNIFORM ? Pu : ep.P[m];
-        FConst Fm;
-        if constexpr (!UNIFORM) Fm = make_fconst(P);
-        const FConst& F = UNIFORM ? ep.fcommon : Fm;
+        KConst<float> Fm;
+        if constexpr (!UNIFORM) Fm = make_kconst<float>(P);
+        const KConst<float>& F = UNIFORM ? ep.fcommon : Fm;
         const bool ok = run_tile<float, MODEL, TY, TZ, ENERGY, EnsLevel, ens_stage<MODEL, TY, TZ, ENERGY>()>(
             mp.tm[tn], mp.tp[1 - tn], P, F, ep.lv[m][tn], ep.lv[m][1 - tn], w.y, w.z, w.w, min(lx, P.nx - w.w), smem,
             bars, ring, &s_abort, obs, warn, smem + HaloStage<float, TY, TZ, ND>::OFFSET);
@@ -476,7 +476,7 @@ bool fill_params(const gft_batch* b, int g, int ti, bool energy, EnsParams* ep)
         ep->lv[j][1] = b->lv[m][1];
         if (j == 0) {
             ep->common = ep->P[0];
-            ep->fcommon = make_fconst(ep->P[0]);
+            ep->fcommon = make_kconst<float>(ep->P[0]);
         }
         else if (!same_physics(ep->P[j], ep->common))
             uniform = false;

@@ -45,7 +45,7 @@ struct GlobalAcc {
 
 // One thread per site; the kernel below instantiates it with its launch bounds.
 template <class S, int MODEL, int HF, bool ENERGY>
-__device__ __forceinline__ void fast_step_body(StepParams P, FConst F, LevelPtrs<S> now, LevelPtrs<S> past,
+__device__ __forceinline__ void fast_step_body(StepParams P, KConst<S> F, LevelPtrs<S> now, LevelPtrs<S> past,
                                                unsigned* status, double* partials)
 {
     const int z = blockIdx.x * blockDim.x + threadIdx.x;
@@ -83,29 +83,27 @@ __device__ __forceinline__ void fast_step_body(StepParams P, FConst F, LevelPtrs
     if (warn) atomicOr(status, warn);
 }
 
-template <class S, int MODEL, int HF, bool ENERGY>
-__global__ void __launch_bounds__(128) fast_step_kernel(StepParams P, FConst F, LevelPtrs<S> now, LevelPtrs<S> past,
-                                                        unsigned* status, double* partials)
+// Resident blocks per SM the launch bounds of an instance ask for: as many as its
+// registers take with no or a few spilled words, since the warps hide the
+// neighbour loads' latency (us per step on a B200, unbounded / bounded):
+//   FP64 SM 256^3: 8 warps per SM 3410, three blocks (168 registers) 2637; four
+//     blocks spill 288 bytes and were 5 % slower than three;
+//   float 2HDM 192^3: 132 registers, three blocks 689; four blocks (128) 576;
+//   float 2HDM with the family SU(2) 96 x 96 x 192: three blocks (168) 243;
+//   float SM: 86-100 registers, five blocks either way.
+template <class S, int MODEL, int HF>
+constexpr int fast_min_blocks()
 {
-    fast_step_body<S, MODEL, HF, ENERGY>(P, F, now, past, status, partials);
+    if (sizeof(S) == 8) return MODEL == kModelSM ? 3 : 2;
+    if (MODEL == kModelSM) return 5;
+    return HF == kHfSU2 ? 3 : 4;
 }
 
-// The FP64 SM step: left to itself the compiler takes 176 registers (two blocks,
-// 8 warps per SM); capped at three blocks it fits 168 with no spills in the plain
-// step, and the extra warps hide more of its load latency (2.68 against 3.41 ms
-// per step at 256^3).  The other instances run fastest unbounded, a minimum of one
-// block included.
-template <>
-__global__ void __launch_bounds__(128, 3) fast_step_kernel<double, kModelSM, kHfNone, false>(
-    StepParams P, FConst F, LevelPtrs<double> now, LevelPtrs<double> past, unsigned* status, double* partials)
+template <class S, int MODEL, int HF, bool ENERGY>
+__global__ void __launch_bounds__(128, fast_min_blocks<S, MODEL, HF>())
+    fast_step_kernel(StepParams P, KConst<S> F, LevelPtrs<S> now, LevelPtrs<S> past, unsigned* status, double* partials)
 {
-    fast_step_body<double, kModelSM, kHfNone, false>(P, F, now, past, status, partials);
-}
-template <>
-__global__ void __launch_bounds__(128, 3) fast_step_kernel<double, kModelSM, kHfNone, true>(
-    StepParams P, FConst F, LevelPtrs<double> now, LevelPtrs<double> past, unsigned* status, double* partials)
-{
-    fast_step_body<double, kModelSM, kHfNone, true>(P, F, now, past, status, partials);
+    fast_step_body<S, MODEL, HF, ENERGY>(P, F, now, past, status, partials);
 }
 
 // Gauss-law residual after a step (gauss_site in gft_step_body.cuh), one
@@ -138,9 +136,9 @@ void fast_step_launch(const StepParams& P, const LevelPtrs<S>& now, const LevelP
     const dim3 block(32, 4, 1);
     const dim3 grid((P.nz + 31) / 32, (P.ny + 3) / 4, P.nx);
     if (energy)
-        fast_step_kernel<S, MODEL, HF, true><<<grid, block, 0, stream>>>(P, make_fconst(P), now, past, status, partials);
+        fast_step_kernel<S, MODEL, HF, true><<<grid, block, 0, stream>>>(P, make_kconst<S>(P), now, past, status, partials);
     else
-        fast_step_kernel<S, MODEL, HF, false><<<grid, block, 0, stream>>>(P, make_fconst(P), now, past, status, partials);
+        fast_step_kernel<S, MODEL, HF, false><<<grid, block, 0, stream>>>(P, make_kconst<S>(P), now, past, status, partials);
 }
 
 template <class S, int MODEL, int HF>

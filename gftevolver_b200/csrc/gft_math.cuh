@@ -122,11 +122,32 @@ static __device__ __noinline__ double gasin_wide(double x) { return asin(x); }
 static __device__ __noinline__ float sqrt1m_wide(float c) { return -c / (1.0f + sqrtf(1.0f - c)); }
 static __device__ __noinline__ double sqrt1m_wide(double c) { return -c / (1.0 + sqrt(1.0 - c)); }
 
-__device__ __forceinline__ float gasin(float x)
+// Where the series below serve, per compute type.
+template <class C>
+struct AsinSeries;
+template <>
+struct AsinSeries<float> {
+    static constexpr float limit = 0.25f;
+};
+template <>
+struct AsinSeries<double> {
+    static constexpr double limit = 0.125;
+};
+template <class C>
+struct Sqrt1mSeries;
+template <>
+struct Sqrt1mSeries<float> {
+    static constexpr float limit = 0.015625f;
+};
+template <>
+struct Sqrt1mSeries<double> {
+    static constexpr double limit = 0.0001220703125;
+};
+
+// asin x = sum_n C(2n,n) / (4^n (2n+1)) x^(2n+1); through n = 6 the first
+// omitted term is < 1e-9 relative at |x| = 1/4
+__device__ __forceinline__ float asin_series(float x)
 {
-    if (fabsf(x) > 0.25f) return gasin_wide(x);
-    // asin x = sum_n C(2n,n) / (4^n (2n+1)) x^(2n+1); through n = 6 the first
-    // omitted term is < 1e-9 relative at |x| = 1/4
     const float x2 = x * x;
     float p = 924.0f / 53248.0f;           // n = 6
     p = fmaf(p, x2, 252.0f / 11264.0f);    // n = 5
@@ -135,6 +156,10 @@ __device__ __forceinline__ float gasin(float x)
     p = fmaf(p, x2, 6.0f / 80.0f);         // n = 2
     p = fmaf(p, x2, 2.0f / 12.0f);         // n = 1
     return fmaf(p * x2, x, x);
+}
+__device__ __forceinline__ float gasin(float x)
+{
+    return fabsf(x) > AsinSeries<float>::limit ? gasin_wide(x) : asin_series(x);
 }
 
 // ---- double ----------------------------------------------------------------
@@ -214,10 +239,9 @@ __device__ __forceinline__ void gsincos(double x, double& s, double& c)
     c = __longlong_as_double(__double_as_longlong(c) ^ (long long)sg);
 }
 
-__device__ __forceinline__ double gasin(double x)
+// through n = 9 the first omitted term is < 1e-20 relative at |x| = 1/8
+__device__ __forceinline__ double asin_series(double x)
 {
-    if (fabs(x) > 0.125) return gasin_wide(x);
-    // through n = 9 the first omitted term is < 1e-20 relative at |x| = 1/8
     const double x2 = x * x;
     double p = 48620.0 / 4980736.0;            // n = 9
     p = fma(p, x2, 12870.0 / 1114112.0);        // n = 8
@@ -230,21 +254,27 @@ __device__ __forceinline__ double gasin(double x)
     p = fma(p, x2, 2.0 / 12.0);                 // n = 1
     return fma(p * x2, x, x);
 }
+__device__ __forceinline__ double gasin(double x)
+{
+    return fabs(x) > AsinSeries<double>::limit ? gasin_wide(x) : asin_series(x);
+}
 
 // sqrt(1 - c) - 1 for the link update's |c|^2 = c (tiny in practice):
 // -c/2 - c^2/8 - c^3/16 - 5c^4/128 when c < 1/64 (float: the first omitted
 // term is 7c^4/128 < 4e-9 relative) or c < 1/8192 (double: < 2e-17), else the
 // exact -c / (1 + sqrt(1 - c)).
-__device__ __forceinline__ float sqrt1m_minus1(float c)
+__device__ __forceinline__ float sqrt1m_series(float c)
 {
-    if (c < 0.015625f) return c * fmaf(c, fmaf(c, fmaf(c, -5.0f / 128.0f, -1.0f / 16.0f), -1.0f / 8.0f), -0.5f);
-    return sqrt1m_wide(c);
+    return c * fmaf(c, fmaf(c, fmaf(c, -5.0f / 128.0f, -1.0f / 16.0f), -1.0f / 8.0f), -0.5f);
 }
-
-__device__ __forceinline__ double sqrt1m_minus1(double c)
+__device__ __forceinline__ double sqrt1m_series(double c)
 {
-    if (c < 0.0001220703125) return c * fma(c, fma(c, fma(c, -5.0 / 128.0, -1.0 / 16.0), -1.0 / 8.0), -0.5);
-    return sqrt1m_wide(c);
+    return c * fma(c, fma(c, fma(c, -5.0 / 128.0, -1.0 / 16.0), -1.0 / 8.0), -0.5);
+}
+template <class C>
+__device__ __forceinline__ C sqrt1m_minus1(C c)
+{
+    return c < Sqrt1mSeries<C>::limit ? sqrt1m_series(c) : sqrt1m_wide(c);
 }
 
 // 1/sqrt(s) and 1/d for arguments of order one: the hardware approximations

@@ -10,12 +10,14 @@
 //   * the reference builds, for every link i and plane j, the loops
 //       P1 = U_j(x+i)^dag U_i(x+j) U_j(x) U_i(x)^dag,
 //       P2 = U_i(x) U_j(x-j) U_i(x-j)^dag U_j(x+i-j)^dag,
-//     renormalising intermediate products.  Here the staples are summed first,
-//       SA_i = sum_j w_j U_j(x+i)^dag U_i(x+j) U_j(x),   SB_i = sum_j w_j U_j(x-j) U_i(x-j)^dag U_j(x+i-j)^dag,
-//     and vec(P1) - vec(P2) summed over j becomes vec(SA_i U_i^dag) - vec(U_i SB_i)
-//     (the vector part is linear).  C_ij = U_j(x+i)^dag U_i(x+j) is shared by
-//     the staples of links i and j.  Intermediate renormalisation is dropped:
-//     it changes products of unit quaternions only at the rounding level.
+//     renormalising intermediate products.  Here the upper loops of both links of a
+//     plane come from two products (plaq_forces); the lower ones are summed as
+//       SB_i = sum_j w_j U_j(x-j) U_i(x-j)^dag U_j(x+i-j)^dag
+//     before the product with U_i (the vector part is linear), and in an x-march those
+//     of the planes with x are the x-1 site's upper loops, turned:
+//       P2 of link i in plane x = U_i(x) (P1 of link 0 at x-e_0 in plane i)^dag U_i(x)^dag.
+//     Intermediate renormalisation is dropped: it changes products of unit quaternions
+//     only at the rounding level.
 //   * the U(1) plaquette angle of plane (i,j) is computed once for both links.
 //   * sin, cos and asin are the range-reduced series of gft_math.cuh.
 // Precision of the mixed form (C = float): operations that would lose
@@ -32,15 +34,6 @@
 namespace gft {
 
 __device__ __forceinline__ float sqrt_(float x) { return sqrtf(x); }
-// A parameter in the compute type: the precomputed float copy, or the double.
-template <class C>
-__device__ __forceinline__ C pf(float f, double d)
-{
-    if constexpr (sizeof(C) == 4)
-        return f;
-    else
-        return d;
-}
 __device__ __forceinline__ double sqrt_(double x) { return sqrt(x); }
 
 // Doublet phi rotated by the hypercharge phase (cos, sin) then acted on by the
@@ -58,6 +51,13 @@ __device__ __forceinline__ Q<C> transport(Q<C> u, C cs, C sn, Q<C> f)
     t.y = -u.y * h0 - u.x * h1 + u.w * h2 + u.z * h3;
     t.z = u.x * h0 - u.y * h1 - u.z * h2 + u.w * h3;
     return t;
+}
+
+// The inverse transport: acted on by the conjugate link, phase rotated back.
+template <class C>
+__device__ __forceinline__ Q<C> transport_back(Q<C> u, C cs, C sn, Q<C> f)
+{
+    return transport(qconj(u), cs, -sn, f);
 }
 
 // The isospin action alone (the 4x4 above on an already phase-rotated h); the
@@ -99,27 +99,44 @@ __device__ __forceinline__ void hf_act(Q<C>& t1, Q<C>& t2, C hc, C hs, Q<C> hu)
     }
 }
 
-// Leapfrog update of one SU(2) link from the vector part (R1, R2, R3) of
-// u = U(t+dt) U(t)^dag (WilsonLoops/Source/StandardModel.cpp:478-504), written as
-// U + correction (see site_step); returns the new link, adds to `check`.
-template <class C>
-__device__ __forceinline__ Q<C> su2_advance(Q<C> Un, C R1, C R2, C R3, unsigned& warn, C& check)
+// Leapfrog update of a site's three SU(2) links from the vector parts R[d] of
+// u = U(t+dt) U(t)^dag (WilsonLoops/Source/StandardModel.cpp:478-504), stored to
+// out[d][s] and added to `check`.  U(t+dt) = normalise(u U(t)) is written as U + correction:
+//   dU = (u - 1) U with u0 - 1 = sqrt(1 - |R|^2) - 1,
+//   |U + dU|^2 - 1 = (|U|^2 - 1) + 2 U.dU + |dU|^2 =: e,  1/sqrt(1+e) - 1 = -e/2 + 3e^2/8.
+// The series of u0 - 1 serves where all three |R|^2 are small; one test for the three.
+template <class C, class S>
+__device__ __forceinline__ void su2_advance3(const Q<C> (&U)[3], const C (&R)[3][3], S* const (&out)[3], int s,
+                                             unsigned& warn, C& check)
 {
-    const C cm = R1 * R1 + R2 * R2 + R3 * R3;
-    if (cm > (C)1) warn |= kWarnSqrt;
-    const C u0m1 = sqrt1m_minus1(cm);
-    const Q<C> dU = qmul(Q<C>{u0m1, R1, R2, R3}, Un);
-    C e = fma(Un.w, Un.w, (C)-1);
-    e = fma(Un.x, Un.x, e);
-    e = fma(Un.y, Un.y, e);
-    e = fma(Un.z, Un.z, e);
-    const C udu = Un.w * dU.w + Un.x * dU.x + Un.y * dU.y + Un.z * dU.z;
-    const C dd = dU.w * dU.w + dU.x * dU.x + dU.y * dU.y + dU.z * dU.z;
-    e += (C)2 * udu + dd;
-    const C fm1 = e * ((C)0.375 * e - (C)0.5);
-    check += e;
-    return {Un.w + (dU.w + fm1 * (Un.w + dU.w)), Un.x + (dU.x + fm1 * (Un.x + dU.x)),
-            Un.y + (dU.y + fm1 * (Un.y + dU.y)), Un.z + (dU.z + fm1 * (Un.z + dU.z))};
+    C cm[3], u0m1[3];
+#pragma unroll
+    for (int d = 0; d < 3; d++) cm[d] = R[d][0] * R[d][0] + R[d][1] * R[d][1] + R[d][2] * R[d][2];
+    const C m = fmax(fmax(cm[0], cm[1]), cm[2]);
+    if (m >= Sqrt1mSeries<C>::limit) {
+        if (m > (C)1) warn |= kWarnSqrt;
+#pragma unroll
+        for (int d = 0; d < 3; d++) u0m1[d] = sqrt1m_minus1(cm[d]);
+    } else {
+#pragma unroll
+        for (int d = 0; d < 3; d++) u0m1[d] = sqrt1m_series(cm[d]);
+    }
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        const Q<C> Un = U[d];
+        const Q<C> dU = qmul(Q<C>{u0m1[d], R[d][0], R[d][1], R[d][2]}, Un);
+        C e = fma(Un.w, Un.w, (C)-1);
+        e = fma(Un.x, Un.x, e);
+        e = fma(Un.y, Un.y, e);
+        e = fma(Un.z, Un.z, e);
+        const C udu = Un.w * dU.w + Un.x * dU.x + Un.y * dU.y + Un.z * dU.z;
+        const C dd = dU.w * dU.w + dU.x * dU.x + dU.y * dU.y + dU.z * dU.z;
+        e += (C)2 * udu + dd;
+        const C fm1 = e * ((C)0.375 * e - (C)0.5);
+        check += e;
+        st4(out[d], s, Un.w + (dU.w + fm1 * (Un.w + dU.w)), Un.x + (dU.x + fm1 * (Un.x + dU.x)),
+            Un.y + (dU.y + fm1 * (Un.y + dU.y)), Un.z + (dU.z + fm1 * (Un.z + dU.z)));
+    }
 }
 
 // 1 - a0/|a| in the compute type without cancellation: |vec a|^2 / (|a| (|a| + a0))
@@ -154,12 +171,16 @@ struct Stencil {
 
 // Values a site computes that its +x neighbour needs, carried along an x-march:
 // the sines of the (0,1) and (0,2) plaquette angles, which are the x+e_0
-// site's lower U(1) loop angles, and the doublet transported along the x link,
-// U_0(x) R(theta_0(x)) phi(x), which is the x+e_0 site's D- term.
+// site's lower U(1) loop angles; the vector parts of the x link's (0,1) and (0,2)
+// plaquettes, which turned by U_1 and U_2 are the x+e_0 site's lower loops of the
+// links 1 and 2; and the doublet transported along the x link, U_0(x) R(theta_0(x))
+// phi(x), which is the x+e_0 site's D- term.  With them a site reads nothing of
+// the plane x - 1.
 template <class C, int ND>
 struct XCarry {
     bool valid;
     C s01, s02;
+    C v01[3], v02[3];
     Q<C> t0[ND];
 };
 
@@ -179,22 +200,141 @@ __device__ __forceinline__ void energy_total(double (&obs)[kObsCount])
     obs[kObsEnergy] = obs[kObsPotential] + obs[kObsGradient] + obs[kObsKinetic] + obs[kObsMagnetic] + obs[kObsElectric];
 }
 
+// Both SU(2) plaquette forces of a plane (i, j) from its four links: with
+// C = U_j(x+i)^dag U_i(x+j) and D = U_j(x) U_i(x)^dag the loop of link i is C D and
+// that of link j is (D C)^dag, so the vector parts are vi = s - k and vj = s + k of
+// s = c_0 d + d_0 c and k = c x d (the force on link j is -vj).  Returns the scalar
+// part of C D (the plaquette trace; the same for both loops).
+template <class C>
+__device__ __forceinline__ C plaq_forces(Q<C> Uj_pi, Q<C> Ui_pj, Q<C> Ui, Q<C> Uj, C (&vi)[3], C (&vj)[3])
+{
+    const Q<C> c = qmul(qconj(Uj_pi), Ui_pj);
+    const Q<C> d = qmul(Uj, qconj(Ui));
+    const C s1 = c.w * d.x + d.w * c.x, s2 = c.w * d.y + d.w * c.y, s3 = c.w * d.z + d.w * c.z;
+    const C k1 = c.y * d.z - c.z * d.y, k2 = c.z * d.x - c.x * d.z, k3 = c.x * d.y - c.y * d.x;
+    vi[0] = s1 - k1;
+    vi[1] = s2 - k2;
+    vi[2] = s3 - k3;
+    vj[0] = s1 + k1;
+    vj[1] = s2 + k2;
+    vj[2] = s3 + k3;
+    return c.w * d.w - c.x * d.x - c.y * d.y - c.z * d.z;
+}
+
+// m += s vec(u v u^dag) for a unit quaternion u and a vector part v:
+// u v u^dag = v + 2 (u x t - u_0 t) with t = u x v.
+template <class C>
+__device__ __forceinline__ void add_turned(C (&m)[3], C s, Q<C> u, const C (&v)[3])
+{
+    const C t1 = u.y * v[2] - u.z * v[1], t2 = u.z * v[0] - u.x * v[2], t3 = u.x * v[1] - u.y * v[0];
+    const C r1 = u.y * t3 - u.z * t2 - u.w * t1;
+    const C r2 = u.z * t1 - u.x * t3 - u.w * t2;
+    const C r3 = u.x * t2 - u.y * t1 - u.w * t3;
+    const C s2 = s + s;
+    m[0] += s * v[0] + s2 * r1;
+    m[1] += s * v[1] + s2 * r2;
+    m[2] += s * v[2] + s2 * r3;
+}
+
+// The SU(2) magnetic force on the three links of a site, sum_j l_j (vec P1 - vec P2)
+// (the loops at the head of this file), from link accessor q(d, R).  CARRY: the
+// lower loops in the planes with x come from the x - 1 site's plaquettes w01, w02,
+// which this site's replace.  trace(plane, scalar part, vector part) receives the
+// upper plaquettes where the caller wants their energy.
+template <bool CARRY, class C, class R, class QA, class Trace>
+__device__ __forceinline__ void su2_force(QA&& q, const Stencil<R>& n, const Q<C> (&U)[3], const C (&l)[3], C (&w01)[3],
+                                          C (&w02)[3], C (&Mg)[3][3], Trace&& trace)
+{
+#pragma unroll
+    for (int i = 0; i < 3; i++) Mg[i][0] = Mg[i][1] = Mg[i][2] = (C)0;
+    if constexpr (CARRY) {
+        add_turned(Mg[1], l[0], U[1], w01);
+        add_turned(Mg[2], l[0], U[2], w02);
+    }
+#pragma unroll
+    for (int pl = 0; pl < 3; pl++) {
+        const int i = (pl == 2) ? 1 : 0;
+        const int j = (pl == 0) ? 1 : 2;
+        C vi[3], vj[3];
+        const C w = plaq_forces(q(j, n.p[i]), q(i, n.p[j]), U[i], U[j], vi, vj);
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            Mg[i][k] += l[j] * vi[k];
+            Mg[j][k] -= l[i] * vj[k];
+            if constexpr (CARRY) {
+                if (pl == 0) w01[k] = vi[k];
+                if (pl == 1) w02[k] = vi[k];
+            }
+        }
+        trace(pl, Q<C>{w, vi[0], vi[1], vi[2]});
+    }
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        Q<C> SB = {(C)0, (C)0, (C)0, (C)0};
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            if (j == i || (CARRY && j == 0)) continue;
+            const Q<C> B = qmul(qmul(q(j, n.m[j]), qconj(q(i, n.m[j]))), qconj(q(j, n.dg(i, j))));
+            SB = qadd_scaled(SB, l[j], B);
+        }
+        C b1, b2, b3;
+        qmul_vec(U[i], SB, b1, b2, b3);
+        Mg[i][0] -= b1;
+        Mg[i][1] -= b2;
+        Mg[i][2] -= b3;
+    }
+}
+
+// What the site at n.c hands to its +x neighbour (XCarry), without evolving it:
+// the start of an x-march, and sites on Fixed x faces.  Reads the planes x and x + 1.
+template <class C, int ND, class A, class R>
+__device__ __forceinline__ void site_carry(const A& acc, const Stencil<R>& n, XCarry<C, ND>& carry)
+{
+    const Q<C> U0 = acc.q(0, n.c);
+    const C th0 = acc.th(0, n.c);
+    C vj[3];
+    plaq_forces(acc.q(1, n.p[0]), acc.q(0, n.p[1]), U0, acc.q(1, n.c), carry.v01, vj);
+    plaq_forces(acc.q(2, n.p[0]), acc.q(0, n.p[2]), U0, acc.q(2, n.c), carry.v02, vj);
+    carry.s01 = gsin(th0 + acc.th(1, n.p[0]) - acc.th(0, n.p[1]) - acc.th(1, n.c));
+    carry.s02 = gsin(th0 + acc.th(2, n.p[0]) - acc.th(0, n.p[2]) - acc.th(2, n.c));
+    C sn, cs;
+    gsincos(th0, sn, cs);
+#pragma unroll
+    for (int db = 0; db < ND; db++) carry.t0[db] = transport(U0, cs, sn, acc.ph(db, n.c));
+    carry.valid = true;
+}
+
+// asin of the three U(1) increments: the series where all are small, which
+// the link update's increments are; one test for the three.
+template <class C>
+__device__ __forceinline__ void asin3(const C (&r)[3], C (&a)[3], unsigned& warn)
+{
+    const C m = fmax(fmax(fabs(r[0]), fabs(r[1])), fabs(r[2]));
+    if (m > AsinSeries<C>::limit) {
+        if (m > (C)1) warn |= kWarnAsin;
+#pragma unroll
+        for (int d = 0; d < 3; d++) a[d] = gasin(r[d]);
+    } else {
+#pragma unroll
+        for (int d = 0; d < 3; d++) a[d] = asin_series(r[d]);
+    }
+}
+
 // The per-site update.  A provides q(d, R) -> Q<C>, th(d, R) -> C, ph(k, R) -> Q<C>
 // for the "now" level (and hth / hq for a 2HDM Higgs-family field, HF != 0).
 // obs receives the energy-step observables except the total (energy_total after
 // the last site) and warn the warning bits, both only when `count` (the site is
-// not on a ghost plane).  With HF != 0 the x-carry is not used (the caller passes
-// an invalid one).  STEADY: the caller guarantees a valid x-carry (a site of a
-// march after one that was evolved), so the recomputation of the carried values
-// is not compiled in; the general instance keeps both and the compiler
-// evaluates the recomputation alongside the carry where it predicates the
-// choice, which costs the x-march kernels 4 % of their step time.
-template <class S, int MODEL, bool ENERGY, int HF = kHfNone, bool STEADY = false, class A, class R, class LV>
-__device__ __forceinline__ void site_step(const StepParams& P, const FConst& F, const A& acc, const Stencil<R>& n,
+// not on a ghost plane).  CARRY (HF == 0 only): `carry` holds the x - 1 site's
+// values (site_step or site_carry of that site) and receives this site's; nothing
+// of the plane x - 1 is read.  Forces are formed already multiplied by dt^2 (the
+// constants of KConst).
+template <class S, int MODEL, bool ENERGY, int HF = kHfNone, bool CARRY = false, class A, class R, class LV>
+__device__ __forceinline__ void site_step(const StepParams& P, const KConst<S>& F, const A& acc, const Stencil<R>& n,
                                           PastSite<S, LV> ps,
                                           XCarry<S, (MODEL == kModelSM) ? 1 : 2>& carry, double (&obs)[kObsCount],
                                           unsigned& warn, bool count = true)
 {
+    static_assert(!CARRY || HF == kHfNone, "the x-carry holds no Higgs-family values");
     const unsigned warn_in = warn;
     using C = S;  // FP64 form -> double, mixed form -> float
     constexpr int ND = (MODEL == kModelSM) ? 1 : 2;
@@ -212,8 +352,7 @@ __device__ __forceinline__ void site_step(const StepParams& P, const FConst& F, 
             pst_t[d] = ld1<C>(ps.L.th[d], ps.s);
         }
     }
-    const bool have = STEADY || carry.valid;
-    const C lap[3] = {pf<C>(F.lap[0], P.lap[0]), pf<C>(F.lap[1], P.lap[1]), pf<C>(F.lap[2], P.lap[2])};
+    const C l[3] = {F.ldt[0], F.ldt[1], F.ldt[2]};  // dt^2 / dx_a^2
 
     Q<C> U[3];
     C th[3];
@@ -223,48 +362,34 @@ __device__ __forceinline__ void site_step(const StepParams& P, const FConst& F, 
         th[a] = acc.th(a, n.c);
     }
 
-    // ---- magnetic term: U(1) sines and SU(2) staple sums ----
-    C MgY[3] = {(C)0, (C)0, (C)0};
-    // lower U(1) loops of the links 1 and 2 in the planes with x: the x-1 site's (0,1), (0,2) angles
-    const C prev01 = carry.s01, prev02 = carry.s02;
-    Q<C> SA[3], SB[3];
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-        SA[a] = {(C)0, (C)0, (C)0, (C)0};
-        SB[a] = {(C)0, (C)0, (C)0, (C)0};
-    }
+    // ---- magnetic term: U(1) sines and SU(2) loops ----
     // logging-step terms: per-site partial sums in the form's arithmetic (a few
     // cancellation-free terms each), added to the FP64 block sums once per site
     C mag_e = (C)0, plaq2 = (C)0, plaq1 = (C)0;
+    C MgY[3] = {(C)0, (C)0, (C)0};
+    if constexpr (CARRY) {
+        MgY[1] = -l[0] * carry.s01;
+        MgY[2] = -l[0] * carry.s02;
+    }
 #pragma unroll
     for (int pl = 0; pl < 3; pl++) {
         const int i = (pl == 2) ? 1 : 0;
         const int j = (pl == 0) ? 1 : 2;
-        const Q<C> Uj_pi = acc.q(j, n.p[i]);
-        const Q<C> Ui_pj = acc.q(i, n.p[j]);
         // F_ij(x) = theta_i(x) + theta_j(x+i) - theta_i(x+j) - theta_j(x); the reference's
         // local angle is -F for link i and +F for link j (StandardModel.cpp:348-353).
         const C Fa = th[i] + acc.th(j, n.p[i]) - acc.th(i, n.p[j]) - th[j];
         const C sF = gsin(Fa);
-        MgY[i] -= sF * lap[j];
-        MgY[j] += sF * lap[i];
-        if (pl == 0) carry.s01 = sF;
-        if (pl == 1) carry.s02 = sF;
-        const Q<C> Cij = qmul(qconj(Uj_pi), Ui_pj);
-        const Q<C> Aij = qmul(Cij, U[j]);
-        const Q<C> Aji = qmul(qconj(Cij), U[i]);
-        SA[i] = qadd_scaled(SA[i], lap[j], Aij);
-        SA[j] = qadd_scaled(SA[j], lap[i], Aji);
+        MgY[i] -= sF * l[j];
+        MgY[j] += sF * l[i];
+        if constexpr (CARRY) {
+            if (pl == 0) carry.s01 = sF;
+            if (pl == 1) carry.s02 = sF;
+        }
         if (ENERGY) {
-            // plaquette P1 = Aij U_i^dag: both orientations have the same trace;
             // 1 - cos F = 2 sin^2(F/2) (no cancellation for small F)
-            const Q<C> P1 = qmul(Aij, qconj(U[i]));
-            const C omt = one_minus_trace(P1);
             const C hF = gsin((C)0.5 * Fa);
             const C omc = (C)2 * hF * hF;
-            mag_e += pf<C>(F.e_plaq[pl], 4.0 * P.lap[i] * P.lap[j]) *
-                     (pf<C>(F.inv_g_sqr, P.inv_g_sqr) * omt + pf<C>(F.inv_gp_sqr, P.inv_gp_sqr) * omc);
-            plaq2 += (C)1 - omt;
+            mag_e += F.e_plaq[pl] * (F.inv_gp_sqr * omc);
             plaq1 += (C)1 - omc;
         }
     }
@@ -272,22 +397,21 @@ __device__ __forceinline__ void site_step(const StepParams& P, const FConst& F, 
     for (int i = 0; i < 3; i++) {
 #pragma unroll
         for (int j = 0; j < 3; j++) {
-            if (j == i) continue;
+            if (j == i || (CARRY && j == 0)) continue;
             const R mj = n.m[j];
-            const R dg = n.dg(i, j);
-            const Q<C> Uj_mj = acc.q(j, mj);
-            const Q<C> Ui_mj = acc.q(i, mj);
-            const Q<C> Uj_dg = acc.q(j, dg);
-            if (j == 0 && have) {
-                MgY[i] -= ((i == 1) ? prev01 : prev02) * lap[0];
-            } else {
-                const C neigh = -acc.th(j, dg) - acc.th(i, mj) + acc.th(j, mj) + th[i];
-                MgY[i] -= gsin(neigh) * lap[j];
-            }
-            const Q<C> B = qmul(qmul(Uj_mj, qconj(Ui_mj)), qconj(Uj_dg));
-            SB[i] = qadd_scaled(SB[i], lap[j], B);
+            const C neigh = -acc.th(j, n.dg(i, j)) - acc.th(i, mj) + acc.th(j, mj) + th[i];
+            MgY[i] -= gsin(neigh) * l[j];
         }
     }
+    C Mg[3][3];
+    su2_force<CARRY>([&](int d, const R& r) { return acc.q(d, r); }, n, U, l, carry.v01, carry.v02, Mg,
+                     [&](int pl, Q<C> p) {
+                         if (ENERGY) {
+                             const C omt = one_minus_trace(p);
+                             mag_e += F.e_plaq[pl] * (F.inv_g_sqr * omt);
+                             plaq2 += (C)1 - omt;
+                         }
+                     });
     // ---- Higgs-family magnetic term (WilsonLoops/Source/TwoHDM.cpp:484-551): the same
     //      loops on theta_H (U(1)) or the family quaternion (SU(2)), coupling g'' ----
     C MgH[3][3];
@@ -303,12 +427,11 @@ __device__ __forceinline__ void site_step(const StepParams& P, const FConst& F, 
             const int j = (pl == 0) ? 1 : 2;
             const C Fa = hc[i] + acc.hth(j, n.p[i]) - acc.hth(i, n.p[j]) - hc[j];
             const C sF = gsin(Fa);
-            MgH[i][0] -= sF * lap[j];
-            MgH[j][0] += sF * lap[i];
+            MgH[i][0] -= sF * l[j];
+            MgH[j][0] += sF * l[i];
             if (ENERGY) {
                 const C hF = gsin((C)0.5 * Fa);
-                mag_e += pf<C>(F.e_plaq[pl], 4.0 * P.lap[i] * P.lap[j]) * pf<C>(F.inv_gpp_sqr, P.inv_gpp_sqr) *
-                         ((C)2 * hF * hF);
+                mag_e += F.e_plaq[pl] * F.inv_gpp_sqr * ((C)2 * hF * hF);
             }
         }
 #pragma unroll
@@ -317,120 +440,151 @@ __device__ __forceinline__ void site_step(const StepParams& P, const FConst& F, 
             for (int j = 0; j < 3; j++) {
                 if (j == i) continue;
                 const C neigh = -acc.hth(j, n.dg(i, j)) - acc.hth(i, n.m[j]) + acc.hth(j, n.m[j]) + hc[i];
-                MgH[i][0] -= gsin(neigh) * lap[j];
+                MgH[i][0] -= gsin(neigh) * l[j];
             }
         }
     } else if constexpr (HF == kHfSU2) {
-        Q<C> UH[3], SAH[3], SBH[3];
+        Q<C> UH[3];
 #pragma unroll
-        for (int a = 0; a < 3; a++) {
-            UH[a] = acc.hq(a, n.c);
-            SAH[a] = {(C)0, (C)0, (C)0, (C)0};
-            SBH[a] = {(C)0, (C)0, (C)0, (C)0};
-        }
-#pragma unroll
-        for (int pl = 0; pl < 3; pl++) {
-            const int i = (pl == 2) ? 1 : 0;
-            const int j = (pl == 0) ? 1 : 2;
-            const Q<C> Cij = qmul(qconj(acc.hq(j, n.p[i])), acc.hq(i, n.p[j]));
-            const Q<C> Aij = qmul(Cij, UH[j]);
-            const Q<C> Aji = qmul(qconj(Cij), UH[i]);
-            SAH[i] = qadd_scaled(SAH[i], lap[j], Aij);
-            SAH[j] = qadd_scaled(SAH[j], lap[i], Aji);
-            if (ENERGY)
-                mag_e += pf<C>(F.e_plaq[pl], 4.0 * P.lap[i] * P.lap[j]) * pf<C>(F.inv_gpp_sqr, P.inv_gpp_sqr) *
-                         one_minus_trace(qmul(Aij, qconj(UH[i])));
-        }
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-#pragma unroll
-            for (int j = 0; j < 3; j++) {
-                if (j == i) continue;
-                const Q<C> Bq = qmul(qmul(acc.hq(j, n.m[j]), qconj(acc.hq(i, n.m[j]))), qconj(acc.hq(j, n.dg(i, j))));
-                SBH[i] = qadd_scaled(SBH[i], lap[j], Bq);
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-            C a1, a2, a3, b1, b2, b3;
-            qmul_vec(SAH[i], qconj(UH[i]), a1, a2, a3);
-            qmul_vec(UH[i], SBH[i], b1, b2, b3);
-            MgH[i][0] = a1 - b1;
-            MgH[i][1] = a2 - b2;
-            MgH[i][2] = a3 - b3;
-        }
+        for (int a = 0; a < 3; a++) UH[a] = acc.hq(a, n.c);
+        su2_force<false>([&](int d, const R& r) { return acc.hq(d, r); }, n, UH, l, carry.v01, carry.v02, MgH,
+                         [&](int pl, Q<C> p) {
+                             if (ENERGY) mag_e += F.e_plaq[pl] * F.inv_gpp_sqr * one_minus_trace(p);
+                         });
     }
 
-    C Mg[3][3];
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-        C a1, a2, a3, b1, b2, b3;
-        qmul_vec(SA[i], qconj(U[i]), a1, a2, a3);
-        qmul_vec(U[i], SB[i], b1, b2, b3);
-        Mg[i][0] = a1 - b1;
-        Mg[i][1] = a2 - b2;
-        Mg[i][2] = a3 - b3;
-    }
-
-    // ---- scalar sector: covariant Laplacian D and currents J ----
+    // ---- potential dV/dphi: D starts as dt^2 times the own-site terms, the Laplacian's
+    //      diagonal minus dV/dphi (both multiples of the doublets) ----
     Q<C> fc[ND];
 #pragma unroll
     for (int db = 0; db < ND; db++) fc[db] = acc.ph(db, n.c);
     Q<C> D[ND];
+    double pot_e = 0.0;
+    if (MODEL == kModelSM) {
+        const C fsq = fc[0].w * fc[0].w + fc[0].x * fc[0].x + fc[0].y * fc[0].y + fc[0].z * fc[0].z;
+        const C k = F.diag - F.lambda * (fsq - F.eta_sqr);
+        D[0] = {k * fc[0].w, k * fc[0].x, k * fc[0].y, k * fc[0].z};
+        if (ENERGY) {
+            const double t = (double)fsq - P.eta_sqr;
+            pot_e = 0.25 * P.lambda * t * t;
+        }
+    } else {
+        const Q<C> f1 = fc[0], f2 = fc[ND - 1];
+        const C s1 = f1.w * f1.w + f1.x * f1.x + f1.y * f1.y + f1.z * f1.z;
+        const C s2 = f2.w * f2.w + f2.x * f2.x + f2.y * f2.y + f2.z * f2.z;
+        const C dot = P.break_son ? f1.w * f2.w + f1.x * f2.x + f1.y * f2.y + f1.z * f2.z : (C)0;
+        const C anti = (P.break_son && P.break_uhalfn) ? f1.w * f2.x - f1.x * f2.w + f1.y * f2.z - f1.z * f2.y : (C)0;
+        C a1 = F.diag1 - F.l1x4 * s1 - F.l3x2 * s2;
+        C a2 = F.diag2 - F.l2x4 * s2 - F.l3x2 * s1;
+        const C f1v[4] = {f1.w, f1.x, f1.y, f1.z};
+        const C f2v[4] = {f2.w, f2.x, f2.y, f2.z};
+        C v1[4], v2[4];
+        if (P.break_son) {
+            // single SO(N): (-m12r + 2 l4p5 dot + l6r s1 + l7r s2) f_other + 2 l6r|l7r dot f_self
+            const C bs = F.m12r - F.l4p5x2 * dot - F.l6r * s1 - F.l7r * s2;
+            a1 -= F.l6rx2 * dot;
+            a2 -= F.l7rx2 * dot;
+            if (P.break_uhalfn) {
+                // U(N/2): (m12i + 2 l4m5 anti - 2 l5i dot - l6i s1 - l7i s2) J f_other - 2 l5i anti f_other
+                // - 2 l6i|l7i anti f_self
+                const C cu = F.l5ix2 * dot + F.l6i * s1 + F.l7i * s2 - F.m12i - F.l4m5x2 * anti;
+                const C bo = bs + F.l5ix2 * anti;
+                a1 += F.l6ix2 * anti;
+                a2 += F.l7ix2 * anti;
 #pragma unroll
-    for (int db = 0; db < ND; db++) {
-        const C w = pf<C>(F.diag, -2.0 * (P.lap[0] + P.lap[1] + P.lap[2]));
-        D[db] = {w * fc[db].w, w * fc[db].x, w * fc[db].y, w * fc[db].z};
+                for (int k = 0; k < 4; k++) {
+                    const int alt = 1 - 2 * (k % 2);
+                    v1[k] = a1 * f1v[k] + bo * f2v[k] + cu * (C)alt * f2v[k + alt];
+                    v2[k] = a2 * f2v[k] + bo * f1v[k] - cu * (C)alt * f1v[k + alt];
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    v1[k] = a1 * f1v[k] + bs * f2v[k];
+                    v2[k] = a2 * f2v[k] + bs * f1v[k];
+                }
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                v1[k] = a1 * f1v[k];
+                v2[k] = a2 * f2v[k];
+            }
+        }
+        D[0] = {v1[0], v1[1], v1[2], v1[3]};
+        D[ND - 1] = {v2[0], v2[1], v2[2], v2[3]};
+        if (ENERGY) {
+            const double d1 = s1, d2 = s2, dd = dot, da = anti;
+            double v = -P.m1 * d1 - P.m2 * d2 + P.l1 * d1 * d1 + P.l2 * d2 * d2 + P.l3 * d1 * d2;
+            if (P.break_son) {
+                v += -P.m12r * dd + P.l4p5 * dd * dd + P.l6r * d1 * dd + P.l7r * d2 * dd;
+                if (P.break_uhalfn)
+                    v += P.m12i * da + P.l4m5 * da * da - 2.0 * P.l5i * dd * da - P.l6i * d1 * da - P.l7i * d2 * da;
+            }
+            if (P.apply_norm) v += P.energy_offset;
+            pot_e = v;
+        }
     }
+
+    // ---- scalar sector: covariant Laplacian D and currents J (four times the reference's, whose
+    //      1/4 is in the constants cY, cI and cH) ----
     C J[3][4];
     C JH[3][3];  // Higgs-family currents (Gradients/Source/TwoHDM.cpp:465-485)
     C grad_e = (C)0;
-    if constexpr (HF != kHfNone) {
 #pragma unroll
-        for (int a = 0; a < 3; a++) {
-            C sn, cs, smm, cmm;
-            gsincos(th[a], sn, cs);
-            gsincos(acc.th(a, n.m[a]), smm, cmm);
-            const Q<C> Um = acc.q(a, n.m[a]);
-            C hcs = (C)1, hsn = (C)0, hcm = (C)1, hsm = (C)0;
-            Q<C> uh = {(C)1, (C)0, (C)0, (C)0}, uhm = {(C)1, (C)0, (C)0, (C)0};
-            if constexpr (HF == kHfU1) {
-                gsincos(acc.hth(a, n.c), hsn, hcs);
-                gsincos(acc.hth(a, n.m[a]), hsm, hcm);
-            } else {
-                uh = acc.hq(a, n.c);
-                uhm = acc.hq(a, n.m[a]);
-            }
-            Q<C> tm[2], tp[2], t[2], fp[2];
+    for (int a = 0; a < 3; a++) {
+        C sn, cs;
+        gsincos(th[a], sn, cs);
+        const bool back = !(CARRY && a == 0);  // the x - e_0 transport is carried
+        C sm = (C)0, cm = (C)1;
+        Q<C> Um = {(C)1, (C)0, (C)0, (C)0};
+        if (back) {
+            gsincos(acc.th(a, n.m[a]), sm, cm);
+            Um = acc.q(a, n.m[a]);
+        }
+        Q<C> tm[ND], tp[ND], t[ND], fp[ND];
 #pragma unroll
-            for (int db = 0; db < 2; db++) {
-                fp[db] = acc.ph(db, n.p[a]);
-                tm[db] = transport(Um, cmm, smm, acc.ph(db, n.m[a]));
-                tp[db] = transport(qconj(U[a]), cs, -sn, fp[db]);
-                t[db] = transport(U[a], cs, sn, fc[db]);
-            }
-            hf_act<HF>(tm[0], tm[1], hcm, hsm, uhm);
-            hf_act<HF>(tp[0], tp[1], hcs, -hsn, qconj(uh));
-            hf_act<HF>(t[0], t[1], hcs, hsn, uh);
-            C j0 = 0, j1 = 0, j2 = 0, j3 = 0;
+        for (int db = 0; db < ND; db++) {
+            fp[db] = acc.ph(db, n.p[a]);
+            // D: U_a(x-a) phi(x-a) + U_a(x)^dag phi(x+a); the first is the x-1 site's transported doublet
+            tm[db] = back ? transport(Um, cm, sm, acc.ph(db, n.m[a])) : carry.t0[db];
+            tp[db] = transport_back(U[a], cs, sn, fp[db]);
+            // J: Im of (U_a(x) phi(x))^dag sigma phi(x+a)
+            t[db] = transport(U[a], cs, sn, fc[db]);
+            if (CARRY && a == 0) carry.t0[db] = t[db];
+        }
+        if constexpr (HF == kHfU1) {
+            C hsn, hcs, hsm, hcm;
+            gsincos(acc.hth(a, n.c), hsn, hcs);
+            gsincos(acc.hth(a, n.m[a]), hsm, hcm);
+            const Q<C> one = {(C)1, (C)0, (C)0, (C)0};
+            hf_act<HF>(tm[0], tm[1], hcm, hsm, one);
+            hf_act<HF>(tp[0], tp[1], hcs, -hsn, one);
+            hf_act<HF>(t[0], t[1], hcs, hsn, one);
+        } else if constexpr (HF == kHfSU2) {
+            const Q<C> uh = acc.hq(a, n.c), uhm = acc.hq(a, n.m[a]);
+            hf_act<HF>(tm[0], tm[1], (C)1, (C)0, uhm);
+            hf_act<HF>(tp[0], tp[1], (C)1, (C)0, qconj(uh));
+            hf_act<HF>(t[0], t[1], (C)1, (C)0, uh);
+        }
 #pragma unroll
-            for (int db = 0; db < 2; db++) {
-                D[db] = qadd_scaled(D[db], lap[a], tm[db]);
-                D[db] = qadd_scaled(D[db], lap[a], tp[db]);
-                const Q<C> u = t[db], f = fp[db];
-                j0 += u.w * f.x - u.x * f.w + u.y * f.z - u.z * f.y;
-                j1 += u.w * f.z - u.x * f.y + u.y * f.x - u.z * f.w;
-                j2 += -u.w * f.y - u.x * f.z + u.y * f.w + u.z * f.x;
-                j3 += u.w * f.x - u.x * f.w - u.y * f.z + u.z * f.y;
-                if (ENERGY) {
-                    const C e0 = f.w - u.w, e1 = f.x - u.x, e2 = f.y - u.y, e3 = f.z - u.z;
-                    grad_e += pf<C>(F.e_grad[a], 0.5 * P.inv_dx[a] * P.inv_dx[a]) * (e0 * e0 + e1 * e1 + e2 * e2 + e3 * e3);
-                }
+        for (int db = 0; db < ND; db++) {
+            D[db] = qadd_scaled(D[db], l[a], tm[db]);
+            D[db] = qadd_scaled(D[db], l[a], tp[db]);
+            const Q<C> u = t[db], f = fp[db];
+            const C up = u.w * f.x - u.x * f.w, lo = u.y * f.z - u.z * f.y;
+            const C j1 = u.w * f.z - u.x * f.y + u.y * f.x - u.z * f.w;
+            const C j2 = -u.w * f.y - u.x * f.z + u.y * f.w + u.z * f.x;
+            J[a][0] = (db ? J[a][0] : (C)0) + (up + lo);
+            J[a][1] = (db ? J[a][1] : (C)0) + j1;
+            J[a][2] = (db ? J[a][2] : (C)0) + j2;
+            J[a][3] = (db ? J[a][3] : (C)0) + (up - lo);
+            if (ENERGY) {
+                const C e0 = f.w - u.w, e1 = f.x - u.x, e2 = f.y - u.y, e3 = f.z - u.z;
+                grad_e += F.e_grad[a] * (e0 * e0 + e1 * e1 + e2 * e2 + e3 * e3);
             }
-            J[a][0] = (C)0.25 * j0;
-            J[a][1] = (C)0.25 * j1;
-            J[a][2] = (C)0.25 * j2;
-            J[a][3] = (C)0.25 * j3;
+        }
+        if constexpr (HF != kHfNone) {
             // family pairs: components (i, i+1) of doublet 1 and of doublet 2, i = 0 (upper) and 2 (lower)
             const C t8[8] = {t[0].w, t[0].x, t[0].y, t[0].z, t[1].w, t[1].x, t[1].y, t[1].z};
             const C n8[8] = {fp[0].w, fp[0].x, fp[0].y, fp[0].z, fp[1].w, fp[1].x, fp[1].y, fp[1].z};
@@ -445,112 +599,9 @@ __device__ __forceinline__ void site_step(const StepParams& P, const FConst& F, 
                     h6 += t8[i] * n8[i + 1] - t8[i + 1] * n8[i] - t8[i + 4] * n8[i + 5] + t8[i + 5] * n8[i + 4];
                 }
             }
-            JH[a][0] = (C)0.25 * h4;
-            JH[a][1] = (C)0.25 * h5;
-            JH[a][2] = (C)0.25 * h6;
-        }
-    } else {
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-        C sn, cs;
-        gsincos(th[a], sn, cs);
-        const Q<C> Uc = qconj(U[a]);
-        C j0 = 0, j1 = 0, j2 = 0, j3 = 0;
-        const bool from_carry = (a == 0) && have;
-        C sm = (C)0, cm = (C)1;
-        Q<C> Um = {(C)1, (C)0, (C)0, (C)0};
-        if (!from_carry) {
-            gsincos(acc.th(a, n.m[a]), sm, cm);
-            Um = acc.q(a, n.m[a]);
-        }
-#pragma unroll
-        for (int db = 0; db < ND; db++) {
-            const Q<C> fp = acc.ph(db, n.p[a]);
-            // D: U_a(x-a) phi(x-a) + U_a(x)^dag phi(x+a); the first is the x-1 site's transported doublet
-            const Q<C> tm = from_carry ? carry.t0[db] : transport(Um, cm, sm, acc.ph(db, n.m[a]));
-            const Q<C> tp = transport(Uc, cs, -sn, fp);
-            D[db] = qadd_scaled(D[db], lap[a], tm);
-            D[db] = qadd_scaled(D[db], lap[a], tp);
-            // J: Im of (U_a(x) phi(x))^dag sigma phi(x+a)
-            const Q<C> t = transport(U[a], cs, sn, fc[db]);
-            if (a == 0) carry.t0[db] = t;
-            j0 += t.w * fp.x - t.x * fp.w + t.y * fp.z - t.z * fp.y;
-            j1 += t.w * fp.z - t.x * fp.y + t.y * fp.x - t.z * fp.w;
-            j2 += -t.w * fp.y - t.x * fp.z + t.y * fp.w + t.z * fp.x;
-            j3 += t.w * fp.x - t.x * fp.w - t.y * fp.z + t.z * fp.y;
-            if (ENERGY) {
-                const C e0 = fp.w - t.w, e1 = fp.x - t.x, e2 = fp.y - t.y, e3 = fp.z - t.z;
-                grad_e += pf<C>(F.e_grad[a], 0.5 * P.inv_dx[a] * P.inv_dx[a]) * (e0 * e0 + e1 * e1 + e2 * e2 + e3 * e3);
-            }
-        }
-        J[a][0] = (C)0.25 * j0;
-        J[a][1] = (C)0.25 * j1;
-        J[a][2] = (C)0.25 * j2;
-        J[a][3] = (C)0.25 * j3;
-    }
-    }
-
-    // ---- potential dV/dphi ----
-    C Pot[ND][4];
-    double pot_e = 0.0;
-    if (MODEL == kModelSM) {
-        const C fsq = fc[0].w * fc[0].w + fc[0].x * fc[0].x + fc[0].y * fc[0].y + fc[0].z * fc[0].z;
-        const C k = pf<C>(F.lambda, P.lambda) * (fsq - pf<C>(F.eta_sqr, P.eta_sqr));
-        Pot[0][0] = k * fc[0].w;
-        Pot[0][1] = k * fc[0].x;
-        Pot[0][2] = k * fc[0].y;
-        Pot[0][3] = k * fc[0].z;
-        if (ENERGY) {
-            const double t = (double)fsq - P.eta_sqr;
-            pot_e = 0.25 * P.lambda * t * t;
-        }
-    } else {
-        const Q<C> f1 = fc[0], f2 = fc[ND - 1];
-        const C s1 = f1.w * f1.w + f1.x * f1.x + f1.y * f1.y + f1.z * f1.z;
-        const C s2 = f2.w * f2.w + f2.x * f2.x + f2.y * f2.y + f2.z * f2.z;
-        const C dot = P.break_son ? f1.w * f2.w + f1.x * f2.x + f1.y * f2.y + f1.z * f2.z : (C)0;
-        const C anti = (P.break_son && P.break_uhalfn) ? f1.w * f2.x - f1.x * f2.w + f1.y * f2.z - f1.z * f2.y : (C)0;
-        const C l3x2 = pf<C>(F.l3x2, 2.0 * P.l3);
-        const C a1 = pf<C>(F.m1x2n, -2.0 * P.m1) + pf<C>(F.l1x4, 4.0 * P.l1) * s1 + l3x2 * s2;
-        const C a2 = pf<C>(F.m2x2n, -2.0 * P.m2) + pf<C>(F.l2x4, 4.0 * P.l2) * s2 + l3x2 * s1;
-        // single SO(N): (-m12r + 2 l4p5 dot + l6r s1 + l7r s2) f_other + 2 l6r|l7r dot f_self
-        const C bs = pf<C>(F.m12rn, -P.m12r) + pf<C>(F.l4p5x2, 2.0 * P.l4p5) * dot + pf<C>(F.l6r, P.l6r) * s1 +
-                     pf<C>(F.l7r, P.l7r) * s2;
-        const C b1 = pf<C>(F.l6rx2, 2.0 * P.l6r) * dot, b2 = pf<C>(F.l7rx2, 2.0 * P.l7r) * dot;
-        // U(N/2): (m12i + 2 l4m5 anti - 2 l5i dot - l6i s1 - l7i s2) J f_other - 2 l5i anti f_other - 2 l6i|l7i anti f_self
-        const C l5ix2 = pf<C>(F.l5ix2, 2.0 * P.l5i);
-        const C cu = pf<C>(F.m12i, P.m12i) + pf<C>(F.l4m5x2, 2.0 * P.l4m5) * anti - l5ix2 * dot -
-                     pf<C>(F.l6i, P.l6i) * s1 - pf<C>(F.l7i, P.l7i) * s2;
-        const C c5 = l5ix2 * anti;
-        const C c1 = pf<C>(F.l6ix2, 2.0 * P.l6i) * anti, c2 = pf<C>(F.l7ix2, 2.0 * P.l7i) * anti;
-        const C f1v[4] = {f1.w, f1.x, f1.y, f1.z};
-        const C f2v[4] = {f2.w, f2.x, f2.y, f2.z};
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const int alt = 1 - 2 * (k % 2);
-            C v1 = a1 * f1v[k];
-            C v2 = a2 * f2v[k];
-            if (P.break_son) {
-                v1 += bs * f2v[k] + b1 * f1v[k];
-                v2 += bs * f1v[k] + b2 * f2v[k];
-                if (P.break_uhalfn) {
-                    v1 += cu * (C)alt * f2v[k + alt] - c5 * f2v[k] - c1 * f1v[k];
-                    v2 += -cu * (C)alt * f1v[k + alt] - c5 * f1v[k] - c2 * f2v[k];
-                }
-            }
-            Pot[0][k] = v1;
-            Pot[ND - 1][k] = v2;
-        }
-        if (ENERGY) {
-            const double d1 = s1, d2 = s2, dd = dot, da = anti;
-            double v = -P.m1 * d1 - P.m2 * d2 + P.l1 * d1 * d1 + P.l2 * d2 * d2 + P.l3 * d1 * d2;
-            if (P.break_son) {
-                v += -P.m12r * dd + P.l4p5 * dd * dd + P.l6r * d1 * dd + P.l7r * d2 * dd;
-                if (P.break_uhalfn)
-                    v += P.m12i * da + P.l4m5 * da * da - 2.0 * P.l5i * dd * da - P.l6i * d1 * da - P.l7i * d2 * da;
-            }
-            if (P.apply_norm) v += P.energy_offset;
-            pot_e = v;
+            JH[a][0] = h4;
+            JH[a][1] = h5;
+            JH[a][2] = h6;
         }
     }
 
@@ -558,8 +609,7 @@ __device__ __forceinline__ void site_step(const StepParams& P, const FConst& F, 
     //      phi(t+dt) = phi + [(phi - phi_past)(1 - damping) + dt^2 (D - dV)], one rounding at the end
     C kin_e = (C)0, phisq = (C)0;
     C check = (C)0;  // sum of every new value: non-finite iff one of them is
-    const C dt2 = pf<C>(F.dt2, P.dt2);
-    const C keep = pf<C>(F.keep, 1.0 - P.damping_step);
+    const C keep = F.keep;
 #pragma unroll
     for (int db = 0; db < ND; db++) {
         const Q<C> fpast = ENERGY ? ld4<C>(ps.L.ph[db], ps.s) : pst_f[db];
@@ -570,7 +620,7 @@ __device__ __forceinline__ void site_step(const StepParams& P, const FConst& F, 
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             const C vel = fn[k] - fo[k];
-            out[k] = fn[k] + (keep * vel + dt2 * (dd[k] - Pot[db][k]));
+            out[k] = fn[k] + (keep * vel + dd[k]);
             check += out[k];
             if (ENERGY) {
                 kin_e += vel * vel;  // x 0.5 / dt^2 below
@@ -581,90 +631,91 @@ __device__ __forceinline__ void site_step(const StepParams& P, const FConst& F, 
     }
 
     // ---- link update (WilsonLoops/Source/StandardModel.cpp:456-514) ----
+    // theta(t+dt) = theta(t) + asin(RHS_Y)
     C elec_e = (C)0;
-    const C gY = pf<C>(F.gY, P.gsq[0]), gI = pf<C>(F.gI, P.gsq[1]);
+    C R0[3], inc[3];
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        const C dth = th[d] - (ENERGY ? ld1<C>(ps.L.th[d], ps.s) : pst_t[d]);
+        R0[d] = keep * gsin(dth) + (MgY[d] + F.cY * J[d][0]);
+        if (ENERGY) {  // 1 - cos(dtheta) = 2 sin^2(dtheta/2)
+            const C h = gsin((C)0.5 * dth);
+            elec_e += F.e_elec[d] * (F.inv_gp_sqr * (C)2 * h * h);
+        }
+    }
+    if (fmax(fmax(fabs(th[0]), fabs(th[1])), fabs(th[2])) > (C)1e4) warn |= kWarnRange;
+    asin3(R0, inc, warn);
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        const C thn = th[d] + inc[d];
+        check += thn;
+        ps.L.th[d][ps.s] = thn;
+    }
+    // u = (sqrt(1-|c|^2), c); U(t+dt) = normalise(u U(t)) (su2_advance3)
+    C W[3][3];
 #pragma unroll
     for (int d = 0; d < 3; d++) {
         const Q<C> Un = U[d];
         const Q<C> Up = ENERGY ? ld4<C>(ps.L.q[d], ps.s) : pst_u[d];
-        const C thp = ENERGY ? ld1<C>(ps.L.th[d], ps.s) : pst_t[d];
         // link momentum vec(U_now U_past^dag) = vec((U_now - U_past) U_past^dag)
         const Q<C> dlt = {Un.w - Up.w, Un.x - Up.x, Un.y - Up.y, Un.z - Up.z};
         C E1, E2, E3;
         qmul_vec(dlt, qconj(Up), E1, E2, E3);
-        const C dth = th[d] - thp;
-        const C R0 = keep * gsin(dth) + dt2 * (MgY[d] + gY * J[d][0]);
-        const C R1 = keep * E1 + dt2 * (Mg[d][0] + gI * J[d][1]);
-        const C R2 = keep * E2 + dt2 * (Mg[d][1] + gI * J[d][2]);
-        const C R3 = keep * E3 + dt2 * (Mg[d][2] + gI * J[d][3]);
+        W[d][0] = keep * E1 + (Mg[d][0] + F.cI * J[d][1]);
+        W[d][1] = keep * E2 + (Mg[d][1] + F.cI * J[d][2]);
+        W[d][2] = keep * E3 + (Mg[d][2] + F.cI * J[d][3]);
         if (ENERGY) {
-            // 1 - (U_now U_past^dag)_0 / |U_now U_past^dag| and 1 - cos(dtheta) = 2 sin^2(dtheta/2)
+            // 1 - (U_now U_past^dag)_0 / |U_now U_past^dag|
             const Q<C> Ed = {Un.w * Up.w + Un.x * Up.x + Un.y * Up.y + Un.z * Up.z, E1, E2, E3};
-            const C h = gsin((C)0.5 * dth);
-            elec_e += pf<C>(F.e_elec[d], 4.0 * P.lap[d] * P.inv_sqr_dt) *
-                      (pf<C>(F.inv_g_sqr, P.inv_g_sqr) * one_minus_trace(Ed) + pf<C>(F.inv_gp_sqr, P.inv_gp_sqr) * (C)2 * h * h);
+            elec_e += F.e_elec[d] * (F.inv_g_sqr * one_minus_trace(Ed));
         }
-        if (R0 * R0 > (C)1) warn |= kWarnAsin;
-        if (fabs(th[d]) > (C)1e4) warn |= kWarnRange;
-        // theta(t+dt) = theta(t) + asin(RHS_Y)
-        const C thn = th[d] + gasin(R0);
-        // u = (sqrt(1-|c|^2), c); U(t+dt) = normalise(u U(t)), written as U + correction:
-        //   dU = (u - 1) U with u0 - 1 = -|c|^2 / (1 + sqrt(1 - |c|^2)),
-        //   |U + dU|^2 - 1 = (|U|^2 - 1) + 2 U.dU + |dU|^2 =: e,  1/sqrt(1+e) - 1 = -e/2 + 3e^2/8
-        const C cm = R1 * R1 + R2 * R2 + R3 * R3;
-        if (cm > (C)1) warn |= kWarnSqrt;
-        const C u0m1 = sqrt1m_minus1(cm);
-        const Q<C> dU = qmul(Q<C>{u0m1, R1, R2, R3}, Un);
-        C e = fma(Un.w, Un.w, (C)-1);
-        e = fma(Un.x, Un.x, e);
-        e = fma(Un.y, Un.y, e);
-        e = fma(Un.z, Un.z, e);
-        const C udu = Un.w * dU.w + Un.x * dU.x + Un.y * dU.y + Un.z * dU.z;
-        const C dd = dU.w * dU.w + dU.x * dU.x + dU.y * dU.y + dU.z * dU.z;
-        e += (C)2 * udu + dd;
-        const C fm1 = e * ((C)0.375 * e - (C)0.5);
-        const Q<C> Unew = {Un.w + (dU.w + fm1 * (Un.w + dU.w)), Un.x + (dU.x + fm1 * (Un.x + dU.x)),
-                           Un.y + (dU.y + fm1 * (Un.y + dU.y)), Un.z + (dU.z + fm1 * (Un.z + dU.z))};
-        check += thn + e;
-        ps.L.th[d][ps.s] = thn;
-        st4(ps.L.q[d], ps.s, Unew.w, Unew.x, Unew.y, Unew.z);
+    }
+    su2_advance3(U, W, ps.L.q, ps.s, warn, check);
 
-        // Higgs-family link (WilsonLoops/Source/TwoHDM.cpp:601-633, 702-745), coupling g''
-        if constexpr (HF == kHfU1) {
-            const C gH = (C)P.gsq_hf;
-            const C hn = acc.hth(d, n.c);
-            const C dh = hn - ld1<C>(ps.L.hth[d], ps.s);
-            const C RH = keep * gsin(dh) + dt2 * (MgH[d][0] + gH * JH[d][0]);
+    // Higgs-family links (WilsonLoops/Source/TwoHDM.cpp:601-633, 702-745), coupling g''
+    if constexpr (HF == kHfU1) {
+        C RH[3], hinc[3], hn[3];
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            hn[d] = acc.hth(d, n.c);
+            const C dh = hn[d] - ld1<C>(ps.L.hth[d], ps.s);
+            RH[d] = keep * gsin(dh) + (MgH[d][0] + F.cH * JH[d][0]);
             if (ENERGY) {
                 const C h = gsin((C)0.5 * dh);
-                elec_e += pf<C>(F.e_elec[d], 4.0 * P.lap[d] * P.inv_sqr_dt) * pf<C>(F.inv_gpp_sqr, P.inv_gpp_sqr) * ((C)2 * h * h);
+                elec_e += F.e_elec[d] * F.inv_gpp_sqr * ((C)2 * h * h);
             }
-            if (RH * RH > (C)1) warn |= kWarnAsin;
-            if (fabs(hn) > (C)1e4) warn |= kWarnRange;
-            const C hnew = hn + gasin(RH);
+        }
+        if (fmax(fmax(fabs(hn[0]), fabs(hn[1])), fabs(hn[2])) > (C)1e4) warn |= kWarnRange;
+        asin3(RH, hinc, warn);
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            const C hnew = hn[d] + hinc[d];
             check += hnew;
             ps.L.hth[d][ps.s] = hnew;
-        } else if constexpr (HF == kHfSU2) {
-            const C gH = (C)P.gsq_hf;
+        }
+    } else if constexpr (HF == kHfSU2) {
+        Q<C> H[3];
+        C RH[3][3];
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
             const Q<C> Hn = acc.hq(d, n.c);
+            H[d] = Hn;
             const Q<C> Hp = ld4<C>(ps.L.hq[d], ps.s);
             const Q<C> dH = {Hn.w - Hp.w, Hn.x - Hp.x, Hn.y - Hp.y, Hn.z - Hp.z};
             C F1, F2, F3;
             qmul_vec(dH, qconj(Hp), F1, F2, F3);
-            const C H1 = keep * F1 + dt2 * (MgH[d][0] + gH * JH[d][0]);
-            const C H2 = keep * F2 + dt2 * (MgH[d][1] + gH * JH[d][1]);
-            const C H3 = keep * F3 + dt2 * (MgH[d][2] + gH * JH[d][2]);
+            RH[d][0] = keep * F1 + (MgH[d][0] + F.cH * JH[d][0]);
+            RH[d][1] = keep * F2 + (MgH[d][1] + F.cH * JH[d][1]);
+            RH[d][2] = keep * F3 + (MgH[d][2] + F.cH * JH[d][2]);
             if (ENERGY) {
                 const Q<C> Ed = {Hn.w * Hp.w + Hn.x * Hp.x + Hn.y * Hp.y + Hn.z * Hp.z, F1, F2, F3};
-                elec_e += pf<C>(F.e_elec[d], 4.0 * P.lap[d] * P.inv_sqr_dt) * pf<C>(F.inv_gpp_sqr, P.inv_gpp_sqr) *
-                          one_minus_trace(Ed);
+                elec_e += F.e_elec[d] * F.inv_gpp_sqr * one_minus_trace(Ed);
             }
-            const Q<C> Hnew = su2_advance(Hn, H1, H2, H3, warn, check);
-            st4(ps.L.hq[d], ps.s, Hnew.w, Hnew.x, Hnew.y, Hnew.z);
         }
+        su2_advance3(H, RH, ps.L.hq, ps.s, warn, check);
     }
     if (!isfinite(check)) warn |= kWarnNonFinite;
-    carry.valid = true;
+    if constexpr (CARRY) carry.valid = true;
     if (!count) {
         warn = warn_in;
         return;

@@ -33,7 +33,7 @@ constexpr int tiled_min_blocks()
 template <class S, int MODEL, int TY, int TZ, bool ENERGY>
 __global__ void __launch_bounds__(TY * TZ, tiled_min_blocks<S, MODEL, TY, TZ>()) tiled_step_kernel(const __grid_constant__ TMaps maps,
                                                              const __grid_constant__ TMaps pmaps, StepParams P,
-                                                             FConst F, LevelPtrs<S> now, LevelPtrs<S> past, int lx,
+                                                             KConst<S> F, LevelPtrs<S> now, LevelPtrs<S> past, int lx,
                                                              int xa, int xn, unsigned* status, double* partials)
 {
     constexpr int ND = (MODEL == kModelSM) ? 1 : 2;
@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(TY * TZ, tiled_min_blocks<S, MODEL, TY, TZ>())
 // the cell TY/2 rows further (site B), as (A, B) pairs.
 template <int TY, int TZ>
 struct PairAcc {
-    using G = Geom<float, TY, TZ, 1>;
+    using G = Geom<float, TY, TZ, 1, 4>;
     static constexpr int DQ = (TY / 2) * G::QP, DH = (TY / 2) * G::HP;
     __device__ __forceinline__ static pair::Q2 ld2(const unsigned char* base, int cell)
     {
@@ -104,8 +104,8 @@ __global__ void __launch_bounds__(TY * TZ / 2, 2) tiled_pair_kernel(const __grid
                                                                    LevelPtrs<float> past, int lx, int xa, int xn,
                                                                    unsigned* status)
 {
-    using G = Geom<float, TY, TZ, 1>;
-    using H = HaloStage<float, TY, TZ, 1>;
+    using G = Geom<float, TY, TZ, 1, 4>;
+    using H = HaloStage<float, TY, TZ, 1, 4>;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem =
         reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~(uintptr_t)127);
@@ -130,8 +130,9 @@ __global__ void __launch_bounds__(TY * TZ / 2, 2) tiled_pair_kernel(const __grid
     carry.valid = false;
     unsigned warn = 0;
     RingPhase ring = {0u};
-    const bool ok = run_ring<float, TY, TZ, 1, LevelPtrs<float>, H::kUse>(
+    const bool ok = run_ring<float, TY, TZ, 1, LevelPtrs<float>, H::kUse, true>(
         maps, pmaps, P, now, y0, z0, x0, min(lx, xa + xn - x0), smem, bars, ring, &s_abort, smem + H::OFFSET, tid,
+        [](const unsigned char*, const unsigned char*) {},
         [&](int i, const unsigned char* bm, const unsigned char* bc, const unsigned char* bp) {
             const Stencil<TRef> n = plane_stencil<G::QP, G::HP>(bm, bc, bp, cq0, ch0);
             const int x = x0 + i;
@@ -146,8 +147,8 @@ __global__ void __launch_bounds__(TY * TZ / 2, 2) tiled_pair_kernel(const __grid
 // staging (when it fits) and the scalars-to-links handoff.
 template <int TY, int TZ>
 struct SplitLayout {
-    using G = Geom<float, TY, TZ, 1>;
-    using H = HaloStage<float, TY, TZ, 1>;
+    using G = Geom<float, TY, TZ, 1, 4>;
+    using H = HaloStage<float, TY, TZ, 1, 4>;
     using HO = split::Handoff<TY * TZ>;
     static constexpr bool kStage = H::kUse;
     static constexpr int OFF_HO = kStage ? (H::OFFSET + H::BYTES + 15) / 16 * 16 : G::NBUF * G::BUF + 64;
@@ -177,7 +178,7 @@ __global__ void __launch_bounds__(2 * TY * TZ, 3) tiled_split_kernel(const __gri
                                                                     LevelPtrs<float> past, int lx, int xa, int xn,
                                                                     unsigned* status)
 {
-    using G = Geom<float, TY, TZ, 1>;
+    using G = Geom<float, TY, TZ, 1, 4>;
     using L = SplitLayout<TY, TZ>;
     constexpr int NT = TY * TZ;  // sites of the tile = threads per role
     static_assert(NT % 32 == 0, "each role is whole warps");
@@ -208,9 +209,9 @@ __global__ void __launch_bounds__(2 * TY * TZ, 3) tiled_split_kernel(const __gri
     carry.valid = false;
     unsigned warn = 0;
     RingPhase ring = {0u};
-    const bool ok = run_ring<float, TY, TZ, 1, LevelPtrs<float>, L::kStage>(
+    const bool ok = run_ring<float, TY, TZ, 1, LevelPtrs<float>, L::kStage, true>(
         maps, pmaps, P, now, y0, z0, x0, min(lx, xa + xn - x0), smem, bars, ring, &s_abort,
-        smem + HaloStage<float, TY, TZ, 1>::OFFSET, tid,
+        smem + HaloStage<float, TY, TZ, 1, 4>::OFFSET, tid, [](const unsigned char*, const unsigned char*) {},
         [&](int i, const unsigned char* bm, const unsigned char* bc, const unsigned char* bp) {
             const Stencil<TRef> n = plane_stencil<G::QP, G::HP>(bm, bc, bp, cq0, ch0);
             const int x = x0 + i;
@@ -329,13 +330,13 @@ static cudaError_t launch_tiled_t(const TMaps& maps, const TMaps& pmaps, const S
     if (energy) {
         auto k = tiled_step_kernel<S, MODEL, TY, TZ, true>;
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM);
-        k<<<grid, block, G::SMEM, stream>>>(maps, pmaps, P, make_fconst(P), now, past, lx, xa, xn, status, partials);
+        k<<<grid, block, G::SMEM, stream>>>(maps, pmaps, P, make_kconst<S>(P), now, past, lx, xa, xn, status, partials);
     } else {
         using H = HaloStage<S, TY, TZ, ND>;
         constexpr int SMEM = H::kUse ? H::SMEM : G::SMEM;  // plain steps stage their wrapped halo cells
         auto k = tiled_step_kernel<S, MODEL, TY, TZ, false>;
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-        k<<<grid, block, SMEM, stream>>>(maps, pmaps, P, make_fconst(P), now, past, lx, xa, xn, status, partials);
+        k<<<grid, block, SMEM, stream>>>(maps, pmaps, P, make_kconst<S>(P), now, past, lx, xa, xn, status, partials);
     }
     return cudaGetLastError();
 }
@@ -359,8 +360,8 @@ static cudaError_t launch_pair_t(const TMaps& maps, const TMaps& pmaps, const St
                                  const LevelPtrs<float>& now, const LevelPtrs<float>& past, int lx, int xa, int xn,
                                  unsigned* status, cudaStream_t stream)
 {
-    using G = Geom<float, TY, TZ, 1>;
-    using H = HaloStage<float, TY, TZ, 1>;
+    using G = Geom<float, TY, TZ, 1, 4>;
+    using H = HaloStage<float, TY, TZ, 1, 4>;
     constexpr int SMEM = H::kUse ? H::SMEM : G::SMEM;
     const dim3 block(TZ, TY / 2, 1);
     const dim3 grid(P.nz / TZ, P.ny / TY, (xn + lx - 1) / lx);

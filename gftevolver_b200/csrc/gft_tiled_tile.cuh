@@ -7,8 +7,9 @@
 // the stencil touches is brought into shared memory once, by the Tensor Memory
 // Accelerator: one cp.async.bulk.tensor per field array per plane, a
 // (TY+2) x (TZ+2) box including the one-site halo, completing on an mbarrier.
-// Four plane buffers form a ring: while plane x is computed from planes x-1, x
-// and x+1, the copy of plane x+2 is in flight.  Halo cells that wrap around
+// The plane buffers form a ring: while plane x is computed from planes x and
+// x+1 (what the site needs of plane x-1 it holds from its own last site, XCarry),
+// the copy of plane x+2 is in flight.  Halo cells that wrap around
 // the periodic boundary (tiles on the lattice faces) are outside the tensor
 // and arrive zero-filled; the CTA overwrites them with plain loads of the
 // wrapped sites.  The own-site past level is read and written directly
@@ -148,8 +149,9 @@ __device__ __forceinline__ void prefetch_past(const TMaps& pm, int X, int y0, in
     for (int k = 0; k < ND; k++) tma_prefetch_l2_4d(&pm.ph[k], 0, z0, y0, X);
 }
 
-// Shared-memory plane geometry.
-template <class S, int TY, int TZ, int ND>
+// Shared-memory plane geometry of a ring of NB planes: three (x, x + 1 and the one
+// in flight), four for the bodies that also read plane x - 1.
+template <class S, int TY, int TZ, int ND, int NB = 3>
 struct Geom {
     static constexpr int TP = 16 / (int)sizeof(S);  // theta box starts TP columns left (16-byte aligned)
     static constexpr int ROWS = TY + 2;
@@ -162,7 +164,7 @@ struct Geom {
     static constexpr int OFF_TH = 3 * QB;
     static constexpr int OFF_PH = 3 * QB + 3 * HB;
     static constexpr int BUF = 3 * QB + 3 * HB + ND * QB;
-    static constexpr int NBUF = 4;
+    static constexpr int NBUF = NB;
     static constexpr unsigned TX = 3 * QBOX + 3 * HBOX + ND * QBOX;  // bytes per plane copy
     static constexpr int SMEM = NBUF * BUF + 128 + 64;             // + alignment slack + barriers
 };
@@ -171,9 +173,9 @@ struct Geom {
 // tiled kernel): one slot per halo cell (the halo_cell numbering), quaternion
 // records [3 + ND][NH] then phases [3][NH], placed after the plane barriers.
 // FP32 only (the tiled kernel serves the mixed form).
-template <class S, int TY, int TZ, int ND>
+template <class S, int TY, int TZ, int ND, int NB = 3>
 struct HaloStage {
-    using G = Geom<S, TY, TZ, ND>;
+    using G = Geom<S, TY, TZ, ND, NB>;
     static constexpr int NH = 2 * G::QP + 2 * TY;
     static constexpr int OFF_H = (3 + ND) * NH * 16;
     static constexpr int BYTES = OFF_H + 3 * NH * 4;
@@ -354,7 +356,7 @@ __device__ __forceinline__ void patch_from_stage(const StepParams& P, unsigned c
     for (int k = 0; k < ND; k++) reinterpret_cast<float4*>(buf + G::OFF_PH + k * G::QB)[cq] = sq[(3 + k) * H::NH + tid];
 }
 
-// Parity of the completed phases of the NBUF plane barriers (bit b for
+// Parity of the completed phases of the plane barriers (bit b for
 // barrier b), carried from tile to tile by a persistent CTA (every thread
 // holds the same value).
 struct RingPhase {
@@ -364,7 +366,9 @@ struct RingPhase {
 // The plane ring of one tile (planes x0 .. x0+nloc-1 of columns y0.., z0..):
 // TMA copies, waits, wrapped-halo patches and one CTA barrier per plane.
 // body(i, bm, bc, bp) evolves the tile's sites of plane x0 + i from the staged
-// planes bm (x - 1), bc (x) and bp (x + 1).  tid: the thread's index in the CTA
+// planes bc (x) and bp (x + 1), and with BACK also bm (x - 1).  Without BACK,
+// start(bc, bp) is called first, on the planes x0 - 1 and x0: what the first sites
+// need of the plane before them.  tid: the thread's index in the CTA
 // (the halo cells and the copy issue are divided by it).  smem: NBUF plane
 // buffers followed by NBUF initialised mbarriers; s_abort: a shared flag that
 // is 0 on entry.  Returns false (on every thread) if a wait gave up; the ring
@@ -373,20 +377,27 @@ struct RingPhase {
 // STAGE: the wrapped halo cells of plane i+4 are copied by cp.async into
 // `stage` (HaloStage) while plane i+1 is computed, instead of prefetched into L2
 // and loaded after the plane's wait.
-template <class S, int TY, int TZ, int ND, class LV, bool STAGE, class Body>
+template <class S, int TY, int TZ, int ND, class LV, bool STAGE, bool BACK, class Start, class Body>
 __device__ __forceinline__ bool run_ring(const TMaps& maps, const TMaps& pmaps, const StepParams& P, const LV& now,
                                          int y0, int z0, int x0, int nloc, unsigned char* smem,
                                          unsigned long long* bars, RingPhase& ring, int* s_abort,
-                                         unsigned char* stage, int tid, Body&& body)
+                                         unsigned char* stage, int tid, Start&& start, Body&& body)
 {
-    using G = Geom<S, TY, TZ, ND>;
+    using G = Geom<S, TY, TZ, ND, BACK ? 4 : 3>;
+    // the plane whose buffer is free once plane i has been computed: i + FREE (relative planes)
+    constexpr int FREE = BACK ? 0 : 1;
     const int nplanes = nloc + 2;  // planes x0-1 .. x0+nloc
     const bool wraps = (y0 == 0) || (y0 + TY == P.ny) || (z0 == 0) || (z0 + TZ == P.nz);
     auto plane_x = [&](int p) {  // global x of relative plane p (p = 0 is x0 - 1)
         int X = x0 - 1 + p;
         return (X < 0) ? X + P.nx : (X >= P.nx ? X - P.nx : X);
     };
-    auto parity = [&](int p) { return ((ring.bits >> (p % G::NBUF)) ^ (unsigned)(p / G::NBUF)) & 1u; };
+    // buffer of relative plane p and the parity of its phase
+    auto slot = [&](int p) { return p % G::NBUF; };
+    auto parity = [&](int p) { return ((ring.bits >> slot(p)) ^ (unsigned)(p / G::NBUF)) & 1u; };
+    auto issue = [&](int p) {
+        issue_plane<S, TY, TZ, ND>(maps, smem + slot(p) * G::BUF, &bars[slot(p)], plane_x(p), y0, z0);
+    };
     // Tiles without wrapped halo cells in the FP64 form march without a CTA
     // barrier per plane (below): its warps wait on long FP64 latencies, and the
     // FP64 step (one CTA of 8 warps per SM) measured 2 % faster at 256^3.  The
@@ -394,14 +405,13 @@ __device__ __forceinline__ bool run_ring(const TMaps& maps, const TMaps& pmaps, 
     // 3 % slower at 256^3 and the 2HDM step (one CTA per SM) 4 % slower at
     // 192^3, their warps waiting on copies and past-level loads instead.
     constexpr bool kFree = sizeof(S) == 8;
-    // After the barriers: per buffer, the warps that have computed the plane in
+    // After the barriers: per buffer, the warps that are done with the plane in
     // it (tiles without wrapped halo); then the number of planes issued.
     unsigned* ctr = reinterpret_cast<unsigned*>(bars + G::NBUF);
     const unsigned nwarps = (blockDim.x * blockDim.y * blockDim.z) >> 5;
 
     if (tid == 0) {
-        for (int p = 0; p < min(G::NBUF, nplanes); p++)
-            issue_plane<S, TY, TZ, ND>(maps, smem + p * G::BUF, &bars[p], plane_x(p), y0, z0);
+        for (int p = 0; p < min(G::NBUF, nplanes); p++) issue(p);
         if constexpr (kFree) {
             for (int b = 0; b < G::NBUF; b++) ctr[b] = 0u;
             ctr[G::NBUF] = (unsigned)min(G::NBUF, nplanes);
@@ -421,8 +431,8 @@ __device__ __forceinline__ bool run_ring(const TMaps& maps, const TMaps& pmaps, 
     // planes 0, 1, 2 (x0-1, x0, x0+1) resident and patched before the first site
     bool ok = true;
     for (int p = 0; p < 3; p++) {  // nplanes >= 3
-        ok = ok && mbar_wait_bounded(&bars[p], parity(p), P.wait_limit_ns);
-        if (ok && wraps) patch_wrapped_halo<S, TY, TZ, ND>(P, now, smem + p * G::BUF, plane_x(p), y0, z0, tid);
+        ok = ok && mbar_wait_bounded(&bars[slot(p)], parity(p), P.wait_limit_ns);
+        if (ok && wraps) patch_wrapped_halo<S, TY, TZ, ND>(P, now, smem + slot(p) * G::BUF, plane_x(p), y0, z0, tid);
     }
     if (!ok) *s_abort = 1;
     __syncthreads();
@@ -430,29 +440,38 @@ __device__ __forceinline__ bool run_ring(const TMaps& maps, const TMaps& pmaps, 
     int drain0 = 0, drain1 = min(G::NBUF, nplanes);
     bool aborted = *s_abort != 0;
 
+    if constexpr (!BACK) {
+        if (!aborted) {
+            start(smem, smem + G::BUF);
+            __syncthreads();  // plane 0's buffer is free
+            if (tid == 0 && G::NBUF < nplanes) {
+                issue(G::NBUF);
+                if constexpr (kFree) ctr[G::NBUF] = (unsigned)(G::NBUF + 1);
+            }
+        }
+    }
+
     // Tiles with wrapped halo cells: one CTA barrier per plane: after computing
     // plane i the threads wait for (and patch) plane i+3, which the next site
     // needs, then synchronise once; that barrier both publishes the patches and
-    // frees plane i's buffer for the copy of plane i+4.
+    // frees a plane's buffer for the next copy.
     for (int i = 0; i < nloc && !aborted; i++) {
-        body(i, smem + (i % G::NBUF) * G::BUF, smem + ((i + 1) % G::NBUF) * G::BUF,
-             smem + ((i + 2) % G::NBUF) * G::BUF);
+        body(i, smem + slot(i) * G::BUF, smem + slot(i + 1) * G::BUF, smem + slot(i + 2) * G::BUF);
 
+        const int nxt = i + FREE + G::NBUF;  // the plane copied into the buffer freed by this one
         if (kFree && !wraps) {
-            // No patches to publish: plane i's buffer is free once every warp has
-            // computed plane i, and the last warp to finish it issues the copy of
-            // plane i+4 there (release by each warp's count, acquire by the last),
+            // No patches to publish: the buffer is free once every warp has
+            // computed plane i, and the last warp to finish it issues the next copy
+            // there (release by each warp's count, acquire by the last),
             // so a warp waits only for the copy of the plane it needs next and may
             // run up to a plane ahead of the slowest.
             __syncwarp();
-            if ((tid & 31) == 0 && i + G::NBUF < nplanes &&
-                atom_add_acq_rel(&ctr[i % G::NBUF], 1u) % nwarps == nwarps - 1) {
-                issue_plane<S, TY, TZ, ND>(maps, smem + (i % G::NBUF) * G::BUF, &bars[i % G::NBUF],
-                                           plane_x(i + G::NBUF), y0, z0);
-                *reinterpret_cast<volatile unsigned*>(&ctr[G::NBUF]) = (unsigned)(i + G::NBUF + 1);
+            if ((tid & 31) == 0 && nxt < nplanes && atom_add_acq_rel(&ctr[slot(nxt)], 1u) % nwarps == nwarps - 1) {
+                issue(nxt);
+                *reinterpret_cast<volatile unsigned*>(&ctr[G::NBUF]) = (unsigned)(nxt + 1);
             }
             if (tid == 32 % (TY * TZ) && i + 3 <= nloc) prefetch_past<ND>(pmaps, plane_x(i + 3), y0, z0);
-            if (i + 3 < nplanes && !mbar_wait_bounded(&bars[(i + 3) % G::NBUF], parity(i + 3), P.wait_limit_ns))
+            if (i + 3 < nplanes && !mbar_wait_bounded(&bars[slot(i + 3)], parity(i + 3), P.wait_limit_ns))
                 *reinterpret_cast<volatile int*>(s_abort) = 1;
             // leave the march warp by warp (the next __syncwarp needs every lane)
             if (__any_sync(0xffffffffu, *reinterpret_cast<volatile int*>(s_abort) != 0)) break;
@@ -462,21 +481,21 @@ __device__ __forceinline__ bool run_ring(const TMaps& maps, const TMaps& pmaps, 
         // plane i+3 (x+2) for the next site; its copy was issued one plane ago
         bool okn = true;
         if (i + 3 < nplanes) {
-            okn = mbar_wait_bounded(&bars[(i + 3) % G::NBUF], parity(i + 3), P.wait_limit_ns);
+            okn = mbar_wait_bounded(&bars[slot(i + 3)], parity(i + 3), P.wait_limit_ns);
             if (okn && wraps) {
                 if constexpr (STAGE)
-                    patch_from_stage<S, TY, TZ, ND>(P, smem + ((i + 3) % G::NBUF) * G::BUF, y0, z0, tid, stage);
+                    patch_from_stage<S, TY, TZ, ND>(P, smem + slot(i + 3) * G::BUF, y0, z0, tid, stage);
                 else
-                    patch_wrapped_halo<S, TY, TZ, ND>(P, now, smem + ((i + 3) % G::NBUF) * G::BUF, plane_x(i + 3), y0,
-                                                      z0, tid);
+                    patch_wrapped_halo<S, TY, TZ, ND>(P, now, smem + slot(i + 3) * G::BUF, plane_x(i + 3), y0, z0,
+                                                      tid);
             }
         }
         if (!okn) *s_abort = 1;
         __syncthreads();
-        if (*s_abort) {  // planes 0 .. i+2 were waited; the last copy issued was plane i+3
+        if (*s_abort) {  // planes 0 .. i+2 were waited; the last copy issued was plane nxt-1 <= i+3
             aborted = true;
             drain0 = i + 3;
-            drain1 = min(nplanes, i + 4);
+            drain1 = min(nplanes, nxt);
             break;
         }
         if (tid == 32 % (TY * TZ) && i + 3 <= nloc) prefetch_past<ND>(pmaps, plane_x(i + 3), y0, z0);
@@ -486,9 +505,7 @@ __device__ __forceinline__ bool run_ring(const TMaps& maps, const TMaps& pmaps, 
             else
                 prefetch_wrapped_halo<S, TY, TZ, ND>(P, now, plane_x(i + 4), y0, z0, tid);
         }
-        if (tid == 0 && i + G::NBUF < nplanes)
-            issue_plane<S, TY, TZ, ND>(maps, smem + (i % G::NBUF) * G::BUF, &bars[i % G::NBUF],
-                                       plane_x(i + G::NBUF), y0, z0);
+        if (tid == 0 && nxt < nplanes) issue(nxt);
     }
     if constexpr (STAGE) cp_async_wait_all();  // a staged plane not patched (abort) is still in flight
     if (kFree && !wraps) {
@@ -504,7 +521,7 @@ __device__ __forceinline__ bool run_ring(const TMaps& maps, const TMaps& pmaps, 
     if (aborted) {
         // drain: wait (bounded) for the copies still in flight into this CTA's buffers
         if (tid == 0)
-            for (int p = drain0; p < drain1; p++) mbar_wait_bounded(&bars[p % G::NBUF], parity(p));
+            for (int p = drain0; p < drain1; p++) mbar_wait_bounded(&bars[slot(p)], parity(p));
         __syncthreads();
         return false;
     }
@@ -538,7 +555,7 @@ __device__ __forceinline__ Stencil<TRef> plane_stencil(const unsigned char* bm, 
 
 // Evolves one tile by one step, one site per thread (threads TZ x TY).
 template <class S, int MODEL, int TY, int TZ, bool ENERGY, class LV, bool STAGE = false>
-__device__ __forceinline__ bool run_tile(const TMaps& maps, const TMaps& pmaps, const StepParams& P, const FConst& F,
+__device__ __forceinline__ bool run_tile(const TMaps& maps, const TMaps& pmaps, const StepParams& P, const KConst<S>& F,
                                          const LV& now, const LV& past, int y0, int z0, int x0,
                                          int nloc, unsigned char* smem, unsigned long long* bars, RingPhase& ring,
                                          int* s_abort, double (&obs)[kObsCount], unsigned& warn,
@@ -554,20 +571,24 @@ __device__ __forceinline__ bool run_tile(const TMaps& maps, const TMaps& pmaps, 
     const int y = y0 + ty, z = z0 + tz;
     XCarry<S, ND> carry;
     carry.valid = false;
-    return run_ring<S, TY, TZ, ND, LV, STAGE>(
+    // Fixed y and z faces freeze whole columns, Fixed x faces the ends of a march
+    const bool column_frozen = ((P.fixed_axes & 2) && (y == 0 || y == P.ny - 1)) ||
+                               ((P.fixed_axes & 4) && (z == 0 || z == P.nz - 1));
+    return run_ring<S, TY, TZ, ND, LV, STAGE, false>(
         maps, pmaps, P, now, y0, z0, x0, nloc, smem, bars, ring, s_abort, stage, tid,
-        [&](int i, const unsigned char* bm, const unsigned char* bc, const unsigned char* bp) {
-            const Stencil<TRef> n = plane_stencil<G::QP, G::HP>(bm, bc, bp, cq0, ch0);
+        [&](const unsigned char* bc, const unsigned char* bp) {
+            site_carry<S, ND>(TileAcc<S, TY, TZ, ND>{}, plane_stencil<G::QP, G::HP>(bc, bc, bp, cq0, ch0), carry);
+        },
+        [&](int i, const unsigned char*, const unsigned char* bc, const unsigned char* bp) {
+            const Stencil<TRef> n = plane_stencil<G::QP, G::HP>(bc, bc, bp, cq0, ch0);
             const int x = x0 + i;
             const int s = (x * P.ny + y) * P.nz + z;
-            if (frozen(P, x, y, z))  // Fixed faces: not evolved, and the next site recomputes what it carries
-                carry.valid = false;
-            else if (carry.valid)  // every site of the march after the first (uniform without Fixed faces)
+            if (column_frozen) return;
+            if ((P.fixed_axes & 1) && (x == 0 || x == P.nx - 1))
+                site_carry<S, ND>(TileAcc<S, TY, TZ, ND>{}, n, carry);  // not evolved; the next site needs its loops
+            else
                 site_step<S, MODEL, ENERGY, kHfNone, true>(P, F, TileAcc<S, TY, TZ, ND>{}, n,
                                                            PastSite<S, LV>{past, s}, carry, obs, warn, counts(P, x));
-            else
-                site_step<S, MODEL, ENERGY>(P, F, TileAcc<S, TY, TZ, ND>{}, n, PastSite<S, LV>{past, s}, carry, obs,
-                                            warn, counts(P, x));
         });
 }
 

@@ -1,0 +1,36 @@
+"""The x-march's carried loops at the ends of marches (GPU).
+
+A tile's site reads nothing of the plane x - 1: the lower loops of that plane
+come from the site before it in the march, or, at the start of a march, from the
+values of the plane before it (site_carry).  The cases are the shortest lattices
+and marches (every site starts a march, marches of one and two planes left over,
+rings with fewer planes than buffers), with and without Fixed x faces, whose
+frozen sites hand their loops on unevolved.  Bars: the FP64 form 1e-12 relative
+to the FP64 oracle after 6 steps, the mixed form 6e-6 absolute.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("fixed", [0, 1], ids=["periodic", "fixed_x"])
+@pytest.mark.parametrize("form,model", [("fp64", 1), ("mixed", 1), ("mixed", 2)])
+@pytest.mark.parametrize("nx,march", [(1, 1), (2, 1), (2, 8), (3, 2), (4, 3), (5, 4), (7, 3)])
+def test_march_ends_match_oracle(oracle_mod, form, model, nx, march, fixed):
+    from gftevolver_b200 import Evolver, LatticeParams
+    op = oracle_mod.Params(model=model, nx=nx, ny=24, nz=96, energy_every=3, fixed_axes=fixed)
+    ic = oracle_mod.ICSpec(seed=17, mean=[1.0 if model == 1 else 0.7] * 8, sigma=[0.1] * 8, theta_sigma=0.1,
+                           eps_sigma=0.1)
+    sc, ve = oracle_mod.init_fields(op, ic, np.float64)
+    with Evolver(LatticeParams(**op.__dict__), form=form) as ev:
+        ev.set_kernel(2, 0, march)
+        assert ev.step_kernel_name == "tiled_step_kernel"
+        ev.upload(sc, ve, 0)
+        ev.evolve(6)
+        assert ev.last_warnings == 0
+        g_sc, g_ve = ev.download()
+    oracle_mod.evolve(op, sc, ve, 6)
+    for a, b in ((g_sc, sc), (g_ve, ve)):
+        err = np.max(np.abs(a.astype(np.float64) - b))
+        assert err <= (1e-12 * np.max(np.abs(b)) if form == "fp64" else 6e-6)
