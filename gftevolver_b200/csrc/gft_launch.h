@@ -31,7 +31,7 @@ int fast_launch_blocks(const StepParams& P, int variant);
 int fast_gauss_blocks(const StepParams& P);
 
 // Tiled throughput kernel (gft_tiled_kernels.cu): TMA-staged planes, x-march.
-// Tensor maps of the "now" level: quaternions and doublets as {4, nz, ny, nx},
+// Tensor maps of the "now" level: quaternions and doublets as {4 nz, ny, nx},
 // hypercharge phases as {nz, ny, nx}.
 struct TMaps {
     CUtensorMap q[3];

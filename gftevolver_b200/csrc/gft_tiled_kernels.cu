@@ -260,39 +260,32 @@ bool tiled_encode_maps(const StepParams& P, const LevelPtrs<S>& L, int nd, int t
     const CUtensorMapDataType dt = (sizeof(S) == 4) ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64;
     const cuuint64_t es = sizeof(S);
     const int tp = 16 / (int)sizeof(S);
-    const cuuint32_t estr[4] = {1, 1, 1, 1};
-    // quaternion / doublet arrays: dims {4, nz, ny, nx}
-    const cuuint64_t qdim[4] = {4, (cuuint64_t)P.nz, (cuuint64_t)P.ny, (cuuint64_t)P.nx};
-    const cuuint64_t qstr[3] = {4 * es, 4 * es * P.nz, 4 * es * P.nz * P.ny};
-    const int hz = halo ? 2 : 0, hy = halo ? 2 : 0, hp = halo ? 2 * tp : 0;
-    const cuuint32_t qbox[4] = {4, (cuuint32_t)(tz + hz), (cuuint32_t)(ty + hy), 1};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    // quaternion / doublet arrays: dims {4 nz, ny, nx}, the four words of a site and the sites of
+    // a z row in one dimension.  A box row is then one run of 16-byte records; with the words as a
+    // dimension of their own ({4, nz, ny, nx}) the copy engine takes a record at a time and the
+    // copies were what the step waited for (us per step: SM mixed 256^3 1020 against 930, FP64
+    // 2390 against 2370, 2HDM mixed 192^3 593 against 531).
     // theta arrays: dims {nz, ny, nx}
-    const cuuint64_t hdim[3] = {(cuuint64_t)P.nz, (cuuint64_t)P.ny, (cuuint64_t)P.nx};
-    const cuuint64_t hstr[2] = {es * P.nz, es * P.nz * P.ny};
-    const cuuint32_t hbox[3] = {(cuuint32_t)(tz + hp), (cuuint32_t)(ty + hy), 1};
-    for (int d = 0; d < 3; d++) {
-        if (enc(&out->q[d], dt, 4, L.q[d], qdim, qstr, qbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) !=
-            CUDA_SUCCESS)
-            return false;
-        if (enc(&out->th[d], dt, 3, L.th[d], hdim, hstr, hbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) !=
-            CUDA_SUCCESS)
-            return false;
-    }
+    const int hz = halo ? 2 : 0, hy = halo ? 2 : 0, hp = halo ? 2 * tp : 0;
+    auto encode = [&](CUtensorMap* map, S* mem, int words, int cols) {
+        const cuuint64_t row = (cuuint64_t)words * P.nz;
+        const cuuint64_t dim[3] = {row, (cuuint64_t)P.ny, (cuuint64_t)P.nx};
+        const cuuint64_t str[2] = {es * row, es * row * P.ny};
+        const cuuint32_t box[3] = {(cuuint32_t)(words * cols), (cuuint32_t)(ty + hy), 1};
+        return enc(map, dt, 3, mem, dim, str, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
+    for (int d = 0; d < 3; d++)
+        if (!encode(&out->q[d], L.q[d], 4, tz + hz) || !encode(&out->th[d], L.th[d], 1, tz + hp)) return false;
     for (int k = 0; k < 2; k++) {
-        if (k >= nd) {
+        if (k >= nd)
             out->ph[k] = out->ph[0];
-            continue;
-        }
-        if (enc(&out->ph[k], dt, 4, L.ph[k], qdim, qstr, qbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) !=
-            CUDA_SUCCESS)
+        else if (!encode(&out->ph[k], L.ph[k], 4, tz + hz))
             return false;
     }
     return true;
 }
-
 
 bool tiled_supported(const StepParams& P, int variant)
 {

@@ -103,16 +103,6 @@ __device__ __forceinline__ bool mbar_wait_bounded(unsigned long long* bar, unsig
     }
 }
 
-__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, int c3,
-                                            unsigned long long* bar)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, "
-        "%5}], [%6];" ::"r"(smem_u32(dst)),
-        "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(bar))
-        : "memory");
-}
-
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int c0, int c1, int c2,
                                             unsigned long long* bar)
 {
@@ -121,13 +111,6 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
         "[%5];" ::"r"(smem_u32(dst)),
         "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar))
         : "memory");
-}
-
-__device__ __forceinline__ void tma_prefetch_l2_4d(const CUtensorMap* map, int c0, int c1, int c2, int c3)
-{
-    asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];" ::"l"(map), "r"(c0),
-                 "r"(c1), "r"(c2), "r"(c3)
-                 : "memory");
 }
 
 __device__ __forceinline__ void tma_prefetch_l2_3d(const CUtensorMap* map, int c0, int c1, int c2)
@@ -142,11 +125,11 @@ template <int ND>
 __device__ __forceinline__ void prefetch_past(const TMaps& pm, int X, int y0, int z0)
 {
 #pragma unroll
-    for (int d = 0; d < 3; d++) tma_prefetch_l2_4d(&pm.q[d], 0, z0, y0, X);
+    for (int d = 0; d < 3; d++) tma_prefetch_l2_3d(&pm.q[d], 4 * z0, y0, X);
 #pragma unroll
     for (int d = 0; d < 3; d++) tma_prefetch_l2_3d(&pm.th[d], z0, y0, X);
 #pragma unroll
-    for (int k = 0; k < ND; k++) tma_prefetch_l2_4d(&pm.ph[k], 0, z0, y0, X);
+    for (int k = 0; k < ND; k++) tma_prefetch_l2_3d(&pm.ph[k], 4 * z0, y0, X);
 }
 
 // Shared-memory plane geometry of a ring of NB planes: three (x, x + 1 and the one
@@ -224,11 +207,11 @@ __device__ __forceinline__ void issue_plane(const TMaps& maps, unsigned char* bu
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     mbar_expect_tx(bar, G::TX);
 #pragma unroll
-    for (int d = 0; d < 3; d++) tma_load_4d(buf + d * G::QB, &maps.q[d], 0, z0 - 1, y0 - 1, X, bar);
+    for (int d = 0; d < 3; d++) tma_load_3d(buf + d * G::QB, &maps.q[d], 4 * (z0 - 1), y0 - 1, X, bar);
 #pragma unroll
     for (int d = 0; d < 3; d++) tma_load_3d(buf + G::OFF_TH + d * G::HB, &maps.th[d], z0 - G::TP, y0 - 1, X, bar);
 #pragma unroll
-    for (int k = 0; k < ND; k++) tma_load_4d(buf + G::OFF_PH + k * G::QB, &maps.ph[k], 0, z0 - 1, y0 - 1, X, bar);
+    for (int k = 0; k < ND; k++) tma_load_3d(buf + G::OFF_PH + k * G::QB, &maps.ph[k], 4 * (z0 - 1), y0 - 1, X, bar);
 }
 
 // Halo cell handled by thread `tid` (2*QP + 2*TY cells: rows 0 and TY+1, then
