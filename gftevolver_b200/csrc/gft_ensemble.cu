@@ -95,13 +95,13 @@ __device__ __forceinline__ void tmap_acquire(const TMaps& m)
 // group, y0, z0, x0}; tile i's energy partials go to partials row i.  UNIFORM:
 // the members share ep.common but for their geometry (the per-member fields
 // copied below).
-// Plain steps stage the wrapped halo sites (run_tile's STAGE) where the staging
+// Steps stage the wrapped halo sites (run_tile's STAGE) where the staging
 // area leaves the resident CTAs per SM unchanged; the dynamic shared memory
 // then includes it.
 template <int MODEL, int TY, int TZ, bool ENERGY>
 constexpr bool ens_stage()
 {
-    return !ENERGY && HaloStage<float, TY, TZ, (MODEL == kModelSM) ? 1 : 2>::kUse;
+    return HaloStage<float, TY, TZ, (MODEL == kModelSM) ? 1 : 2>::use(ENERGY);
 }
 template <int MODEL, int TY, int TZ, bool ENERGY>
 constexpr int ens_smem()

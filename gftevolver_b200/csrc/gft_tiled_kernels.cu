@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(TY * TZ, tiled_min_blocks<S, MODEL, TY, TZ>())
     unsigned warn = 0;
     RingPhase ring = {0u};
     const int x0 = xa + blockIdx.z * lx;  // planes [xa, xa + xn) in chunks of lx
-    constexpr bool STAGE = !ENERGY && HaloStage<S, TY, TZ, ND>::kUse;
+    constexpr bool STAGE = HaloStage<S, TY, TZ, ND>::use(ENERGY);
     const bool ok = run_tile<S, MODEL, TY, TZ, ENERGY, LevelPtrs<S>, STAGE>(
         maps, pmaps, P, F, now, past, blockIdx.y * TY, blockIdx.x * TZ, x0, min(lx, xa + xn - x0), smem, bars, ring,
         &s_abort, obs, warn, smem + HaloStage<S, TY, TZ, ND>::OFFSET);
@@ -318,15 +318,18 @@ static cudaError_t launch_tiled_t(const TMaps& maps, const TMaps& pmaps, const S
 {
     constexpr int ND = (MODEL == kModelSM) ? 1 : 2;
     using G = Geom<S, TY, TZ, ND>;
+    using H = HaloStage<S, TY, TZ, ND>;
     const dim3 block(TZ, TY, 1);
     const dim3 grid(P.nz / TZ, P.ny / TY, (xn + lx - 1) / lx);
+    // both step kinds stage their wrapped halo cells where that costs no resident CTA (logging step,
+    // us at SM 256^3 / 2HDM 192^3: 1187 / 715 loading them after the plane's wait, 1161 / 687 staged)
     if (energy) {
+        constexpr int SMEM = H::use(true) ? H::SMEM : G::SMEM;
         auto k = tiled_step_kernel<S, MODEL, TY, TZ, true>;
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM);
-        k<<<grid, block, G::SMEM, stream>>>(maps, pmaps, P, make_kconst<S>(P), now, past, lx, xa, xn, status, partials);
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+        k<<<grid, block, SMEM, stream>>>(maps, pmaps, P, make_kconst<S>(P), now, past, lx, xa, xn, status, partials);
     } else {
-        using H = HaloStage<S, TY, TZ, ND>;
-        constexpr int SMEM = H::kUse ? H::SMEM : G::SMEM;  // plain steps stage their wrapped halo cells
+        constexpr int SMEM = H::use(false) ? H::SMEM : G::SMEM;
         auto k = tiled_step_kernel<S, MODEL, TY, TZ, false>;
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
         k<<<grid, block, SMEM, stream>>>(maps, pmaps, P, make_kconst<S>(P), now, past, lx, xa, xn, status, partials);

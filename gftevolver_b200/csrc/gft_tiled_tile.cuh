@@ -152,8 +152,7 @@ struct Geom {
     static constexpr int SMEM = NBUF * BUF + 128 + 64;             // + alignment slack + barriers
 };
 
-// Staging area for the wrapped halo cells of one plane (plain steps of the
-// tiled kernel): one slot per halo cell (the halo_cell numbering), quaternion
+// Staging area for the wrapped halo cells of one plane: one slot per halo cell (the halo_cell numbering), quaternion
 // records [3 + ND][NH] then phases [3][NH], placed after the plane barriers.
 // FP32 only (the tiled kernel serves the mixed form).
 template <class S, int TY, int TZ, int ND, int NB = 3>
@@ -165,9 +164,17 @@ struct HaloStage {
     static constexpr int OFFSET = G::NBUF * G::BUF + 64;  // 16-byte aligned (BUF is a multiple of 128)
     static constexpr int SMEM = OFFSET + BYTES + 128;      // + alignment slack of the dynamic base
     // Used only when it leaves the resident CTAs per SM unchanged: 228 KB of
-    // shared memory per SM, 1 KB reserved and 16 bytes static per CTA.
-    static constexpr int per_sm(int dyn) { return (228 * 1024) / (dyn + 16 + 1024); }
-    static constexpr bool kUse = sizeof(S) == 4 && SMEM <= 227 * 1024 && per_sm(SMEM) >= per_sm(G::SMEM);
+    // shared memory per SM, 1 KB reserved and 16 bytes static per CTA, and on
+    // logging steps the reduction's 32 rows of kObsCount doubles.
+    static constexpr int per_sm(int dyn, bool energy)
+    {
+        return (228 * 1024) / (dyn + 16 + (energy ? 32 * kObsCount * 8 : 0) + 1024);
+    }
+    static constexpr bool use(bool energy)
+    {
+        return sizeof(S) == 4 && SMEM <= 227 * 1024 - 16 && per_sm(SMEM, energy) >= per_sm(G::SMEM, energy);
+    }
+    static constexpr bool kUse = use(false);
 };
 
 // Reference to a site in a staged plane: buffer base, q/phi cell, theta cell.
