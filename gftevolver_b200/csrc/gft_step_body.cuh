@@ -102,8 +102,10 @@ __device__ __forceinline__ void hf_act(Q<C>& t1, Q<C>& t2, C hc, C hs, Q<C> hu)
 // Leapfrog update of a site's three SU(2) links from the vector parts R[d] of
 // u = U(t+dt) U(t)^dag (WilsonLoops/Source/StandardModel.cpp:478-504), stored to
 // out[d][s] and added to `check`.  U(t+dt) = normalise(u U(t)) is written as U + correction:
-//   dU = (u - 1) U with u0 - 1 = sqrt(1 - |R|^2) - 1,
-//   |U + dU|^2 - 1 = (|U|^2 - 1) + 2 U.dU + |dU|^2 =: e,  1/sqrt(1+e) - 1 = -e/2 + 3e^2/8.
+// u = (sqrt(1 - |R|^2), R) is a unit quaternion, so |u U|^2 - 1 = |U|^2 - 1 =: e, and with
+// f = 1/sqrt(1+e) - 1 = -e/2 + 3e^2/8
+//   U(t+dt) = U + (u0 - 1 + f, R) U      (f R U is below the rounding of R U),
+// one rounding at the end.
 // The series of u0 - 1 serves where all three |R|^2 are small; one test for the three.
 template <class C, class S>
 __device__ __forceinline__ void su2_advance3(const Q<C> (&U)[3], const C (&R)[3][3], S* const (&out)[3], int s,
@@ -124,18 +126,14 @@ __device__ __forceinline__ void su2_advance3(const Q<C> (&U)[3], const C (&R)[3]
 #pragma unroll
     for (int d = 0; d < 3; d++) {
         const Q<C> Un = U[d];
-        const Q<C> dU = qmul(Q<C>{u0m1[d], R[d][0], R[d][1], R[d][2]}, Un);
         C e = fma(Un.w, Un.w, (C)-1);
         e = fma(Un.x, Un.x, e);
         e = fma(Un.y, Un.y, e);
         e = fma(Un.z, Un.z, e);
-        const C udu = Un.w * dU.w + Un.x * dU.x + Un.y * dU.y + Un.z * dU.z;
-        const C dd = dU.w * dU.w + dU.x * dU.x + dU.y * dU.y + dU.z * dU.z;
-        e += (C)2 * udu + dd;
-        const C fm1 = e * ((C)0.375 * e - (C)0.5);
-        check += e;
-        st4(out[d], s, Un.w + (dU.w + fm1 * (Un.w + dU.w)), Un.x + (dU.x + fm1 * (Un.x + dU.x)),
-            Un.y + (dU.y + fm1 * (Un.y + dU.y)), Un.z + (dU.z + fm1 * (Un.z + dU.z)));
+        const C a = u0m1[d] + e * ((C)0.375 * e - (C)0.5);
+        const Q<C> dU = qmul(Q<C>{a, R[d][0], R[d][1], R[d][2]}, Un);
+        check += a;  // non-finite if a word of U or R is
+        st4(out[d], s, Un.w + dU.w, Un.x + dU.x, Un.y + dU.y, Un.z + dU.z);
     }
 }
 
