@@ -9,43 +9,38 @@
 //           relative error <= 6.1e-9; cos r = 1 + r^2 Q(r^2), degree 10, absolute
 //           error <= 2.5e-10 -- both below float's rounding, and two multiply-adds
 //           shorter each than the Taylor series of equal accuracy (degree 13 / 14);
-//   double: Taylor series, sin to r^23, cos to r^24 (omitted term <= 1e-19).
+//   double: the same forms by the same fit in extended precision, sin of degree 17
+//           (relative error <= 2.8e-19), cos of degree 16 (absolute error <= 4.2e-18):
+//           three and four multiply-adds shorter than the Taylor series of equal use.
 // The reduction uses the 1.5*2^p rounding constant (no conversion to integer):
 // it holds for |x| < 1.3e7 (float) / 1.4e15 (double); phases that large do not
 // occur in the evolution (the step kernels flag |theta| > 1e4).
-// asin: odd series x + x^3/6 + 3x^5/40 + ... for |x| <= 1/4 (float) or 1/8
-// (double) -- the link update's argument is dt * E ~ 1e-3 -- and CUDA's asin
-// otherwise.
+// asin: x + x^3 A(x^2), minimax for |x| <= 1/4 (float, relative error <= 5.5e-11)
+// or 1/8 (double, <= 4.5e-19) -- the link update's argument is dt * E ~ 1e-3 to
+// 1e-1 -- and CUDA's asin otherwise.
 #pragma once
 
 #include <cuda_runtime.h>
 
 namespace gft {
 
-// Taylor coefficients (-1)^n / (2n+1)!  and  (-1)^n / (2n)!
-#define GFT_S3 (-1.0 / 6.0)
-#define GFT_S5 (1.0 / 120.0)
-#define GFT_S7 (-1.0 / 5040.0)
-#define GFT_S9 (1.0 / 362880.0)
-#define GFT_S11 (-1.0 / 39916800.0)
-#define GFT_S13 (1.0 / 6227020800.0)
-#define GFT_S15 (-1.0 / 1307674368000.0)
-#define GFT_S17 (1.0 / 355687428096000.0)
-#define GFT_S19 (-1.0 / 121645100408832000.0)
-#define GFT_S21 (1.0 / 51090942171709440000.0)
-#define GFT_S23 (-1.0 / 25852016738884976640000.0)
-#define GFT_C2 (-1.0 / 2.0)
-#define GFT_C4 (1.0 / 24.0)
-#define GFT_C6 (-1.0 / 720.0)
-#define GFT_C8 (1.0 / 40320.0)
-#define GFT_C10 (-1.0 / 3628800.0)
-#define GFT_C12 (1.0 / 479001600.0)
-#define GFT_C14 (-1.0 / 87178291200.0)
-#define GFT_C16 (1.0 / 20922789888000.0)
-#define GFT_C18 (-1.0 / 6402373705728000.0)
-#define GFT_C20 (1.0 / 2432902008176640000.0)
-#define GFT_C22 (-1.0 / 1124000727777607680000.0)
-#define GFT_C24 (1.0 / 620448401733239439360000.0)
+// Double minimax coefficients on |r| <= pi/2 (gft_math_fit.py), sin r = r + r^3 P(r^2), cos r = 1 + r^2 Q(r^2).
+#define GFT_S3 (-1.66666666666666656e-1)
+#define GFT_S5 (8.33333333333319431e-3)
+#define GFT_S7 (-1.98412698412092192e-4)
+#define GFT_S9 (2.75573192111372807e-6)
+#define GFT_S11 (-2.5052106872802643e-8)
+#define GFT_S13 (1.6058939705911306e-10)
+#define GFT_S15 (-7.64299148958033802e-13)
+#define GFT_S17 (2.72117496446829863e-15)
+#define GFT_C2 (-4.99999999999999825e-1)
+#define GFT_C4 (4.16666666666643693e-2)
+#define GFT_C6 (-1.38888888887856523e-3)
+#define GFT_C8 (2.48015872791490212e-5)
+#define GFT_C10 (-2.75573165252276417e-7)
+#define GFT_C12 (2.08765677410145851e-9)
+#define GFT_C14 (-1.14630393689959251e-11)
+#define GFT_C16 (4.61029415573876858e-14)
 
 // Float minimax coefficients on |r| <= pi/2 (gft_math_fit.py): sin r = r + r^3 P(r^2), cos r = 1 + r^2 Q(r^2).
 #define GFT_FS3 (-0.16666659712791443f)
@@ -141,20 +136,16 @@ struct Sqrt1mSeries<float> {
 };
 template <>
 struct Sqrt1mSeries<double> {
-    static constexpr double limit = 0.0001220703125;
+    static constexpr double limit = 0.015625;
 };
 
-// asin x = sum_n C(2n,n) / (4^n (2n+1)) x^(2n+1); through n = 6 the first
-// omitted term is < 1e-9 relative at |x| = 1/4
 __device__ __forceinline__ float asin_series(float x)
 {
     const float x2 = x * x;
-    float p = 924.0f / 53248.0f;           // n = 6
-    p = fmaf(p, x2, 252.0f / 11264.0f);    // n = 5
-    p = fmaf(p, x2, 70.0f / 2304.0f);      // n = 4
-    p = fmaf(p, x2, 20.0f / 448.0f);       // n = 3
-    p = fmaf(p, x2, 6.0f / 80.0f);         // n = 2
-    p = fmaf(p, x2, 2.0f / 12.0f);         // n = 1
+    float p = 3.40801214445308396e-2f;
+    p = fmaf(p, x2, 4.4443265213162178e-2f);
+    p = fmaf(p, x2, 7.50041907289998445e-2f);
+    p = fmaf(p, x2, 1.6666663944730844e-1f);
     return fmaf(p * x2, x, x);
 }
 __device__ __forceinline__ float gasin(float x)
@@ -166,10 +157,7 @@ __device__ __forceinline__ float gasin(float x)
 __device__ __forceinline__ void sincos_poly(double r, double& s, double& c)
 {
     const double r2 = r * r;
-    double ps = GFT_S23;
-    ps = fma(ps, r2, GFT_S21);
-    ps = fma(ps, r2, GFT_S19);
-    ps = fma(ps, r2, GFT_S17);
+    double ps = GFT_S17;
     ps = fma(ps, r2, GFT_S15);
     ps = fma(ps, r2, GFT_S13);
     ps = fma(ps, r2, GFT_S11);
@@ -178,11 +166,7 @@ __device__ __forceinline__ void sincos_poly(double r, double& s, double& c)
     ps = fma(ps, r2, GFT_S5);
     ps = fma(ps, r2, GFT_S3);
     s = fma(ps * r2, r, r);
-    double pc = GFT_C24;
-    pc = fma(pc, r2, GFT_C22);
-    pc = fma(pc, r2, GFT_C20);
-    pc = fma(pc, r2, GFT_C18);
-    pc = fma(pc, r2, GFT_C16);
+    double pc = GFT_C16;
     pc = fma(pc, r2, GFT_C14);
     pc = fma(pc, r2, GFT_C12);
     pc = fma(pc, r2, GFT_C10);
@@ -196,10 +180,7 @@ __device__ __forceinline__ void sincos_poly(double r, double& s, double& c)
 __device__ __forceinline__ double sin_poly(double r)
 {
     const double r2 = r * r;
-    double ps = GFT_S23;
-    ps = fma(ps, r2, GFT_S21);
-    ps = fma(ps, r2, GFT_S19);
-    ps = fma(ps, r2, GFT_S17);
+    double ps = GFT_S17;
     ps = fma(ps, r2, GFT_S15);
     ps = fma(ps, r2, GFT_S13);
     ps = fma(ps, r2, GFT_S11);
@@ -211,16 +192,16 @@ __device__ __forceinline__ double sin_poly(double r)
 }
 
 // As for float, with t = x/pi + 1.5*2^52 (valid while |x| < 1.4e15) and
-// pi = PI_A + PI_B + PI_C, each the double nearest to the remainder; with FMA
+// pi = PI_A + PI_B, each the double nearest to the remainder (k times what is left,
+// 3e-33, is below r's rounding for any k the form holds); with FMA
 // each step rounds once, so r carries a relative error of ~1 ulp.
 __device__ __forceinline__ double reduce_pi(double x, unsigned long long& sign)
 {
     const double t = fma(x, 0.3183098861837907, 6755399441055744.0);
     const double kd = t - 6755399441055744.0;
     sign = (unsigned long long)__double_as_longlong(t) << 63;
-    double r = fma(-kd, 3.141592653589793, x);
-    r = fma(-kd, 1.2246467991473532e-16, r);
-    return fma(-kd, -2.9947698097183397e-33, r);
+    const double r = fma(-kd, 3.141592653589793, x);
+    return fma(-kd, 1.2246467991473532e-16, r);
 }
 
 __device__ __forceinline__ double gsin(double x)
@@ -239,19 +220,15 @@ __device__ __forceinline__ void gsincos(double x, double& s, double& c)
     c = __longlong_as_double(__double_as_longlong(c) ^ (long long)sg);
 }
 
-// through n = 9 the first omitted term is < 1e-20 relative at |x| = 1/8
 __device__ __forceinline__ double asin_series(double x)
 {
     const double x2 = x * x;
-    double p = 48620.0 / 4980736.0;            // n = 9
-    p = fma(p, x2, 12870.0 / 1114112.0);        // n = 8
-    p = fma(p, x2, 3432.0 / 245760.0);          // n = 7
-    p = fma(p, x2, 924.0 / 53248.0);            // n = 6
-    p = fma(p, x2, 252.0 / 11264.0);            // n = 5
-    p = fma(p, x2, 70.0 / 2304.0);              // n = 4
-    p = fma(p, x2, 20.0 / 448.0);               // n = 3
-    p = fma(p, x2, 6.0 / 80.0);                 // n = 2
-    p = fma(p, x2, 2.0 / 12.0);                 // n = 1
+    double p = 1.81280312314050132e-2;
+    p = fma(p, x2, 2.23556390763832123e-2);
+    p = fma(p, x2, 3.03821168203033322e-2);
+    p = fma(p, x2, 4.4642856235161617e-2);
+    p = fma(p, x2, 7.50000000021955577e-2);
+    p = fma(p, x2, 1.66666666666664899e-1);
     return fma(p * x2, x, x);
 }
 __device__ __forceinline__ double gasin(double x)
@@ -259,23 +236,48 @@ __device__ __forceinline__ double gasin(double x)
     return fabs(x) > AsinSeries<double>::limit ? gasin_wide(x) : asin_series(x);
 }
 
-// sqrt(1 - c) - 1 for the link update's |c|^2 = c (tiny in practice):
-// -c/2 - c^2/8 - c^3/16 - 5c^4/128 when c < 1/64 (float: the first omitted
-// term is 7c^4/128 < 4e-9 relative) or c < 1/8192 (double: < 2e-17), else the
-// exact -c / (1 + sqrt(1 - c)).
+// sqrt(1 - c) - 1 for the link update's |c|^2 = c (tiny in practice): c (-1/2 + c G(c)),
+// minimax for c <= 1/64 (relative error <= 1.2e-8 float, 2.7e-16 double: of a term that is
+// itself at most 1/128 of the link it is added to), else the exact -c / (1 + sqrt(1 - c)).
+// The limit covers links that turn by up to 0.125 a step; a double series to 1/8192 sent
+// fields at equilibrium (dt E ~ 0.015 per component) to the square root and division.
 __device__ __forceinline__ float sqrt1m_series(float c)
 {
-    return c * fmaf(c, fmaf(c, fmaf(c, -5.0f / 128.0f, -1.0f / 16.0f), -1.0f / 8.0f), -0.5f);
+    return c * fmaf(c, fmaf(c, -6.33604442620192054e-2f, -1.24995822362758278e-1f), -0.5f);
 }
 __device__ __forceinline__ double sqrt1m_series(double c)
 {
-    return c * fma(c, fma(c, fma(c, -5.0 / 128.0, -1.0 / 16.0), -1.0 / 8.0), -0.5);
+    double g = -2.12681029627174839e-2;
+    g = fma(g, c, -2.7330616486757293e-2);
+    g = fma(g, c, -3.90626025811028673e-2);
+    g = fma(g, c, -6.24999996508750068e-2);
+    g = fma(g, c, -1.25000000000385582e-1);
+    return c * fma(c, g, -0.5);
 }
 template <class C>
 __device__ __forceinline__ C sqrt1m_minus1(C c)
 {
     return c < Sqrt1mSeries<C>::limit ? sqrt1m_series(c) : sqrt1m_wide(c);
 }
+
+// The largest magnitude of several values against a limit.  In FP64 by the words that hold the
+// exponents, as integers: a comparison of doubles takes the FP64 pipe.  A NaN does not exceed
+// (float; the series pass it on) or does (double).
+template <class C>
+struct MaxAbs;
+template <>
+struct MaxAbs<float> {
+    float m = 0.0f;
+    __device__ __forceinline__ void add(float x) { m = fmaxf(m, fabsf(x)); }
+    __device__ __forceinline__ bool exceeds(float limit) const { return m > limit; }
+};
+template <>
+struct MaxAbs<double> {
+    unsigned m = 0u;
+    __device__ __forceinline__ void add(double x) { m = max(m, (unsigned)__double2hiint(x) & 0x7fffffffu); }
+    // true from the first value with the high word of `limit` on
+    __device__ __forceinline__ bool exceeds(double limit) const { return m >= (unsigned)__double2hiint(limit); }
+};
 
 // 1/sqrt(s) and 1/d for arguments of order one: the hardware approximations
 // (rsqrt.approx, rcp.approx; relative error below 2^-22) refined by one

@@ -1,83 +1,72 @@
-"""Regenerates the float minimax coefficients of gft_math.cuh (run: python gft_math_fit.py).
+"""Regenerates the minimax coefficients of gft_math.cuh (run: python gft_math_fit.py).
 
-Remez exchange (E. Ya. Remez, 1934) for the polynomial forms the kernels evaluate
-after the reduction to |r| <= pi/2 (s = r^2):
-  sin r = r + r^3 P(s),   P of degree 3 (sin of degree 9), weight r^3 / sin r: the
-                          relative error of sin;
-  cos r = 1 + s Q(s),     Q of degree 4 (cos of degree 10), weight s: the absolute
-                          error of cos.
-Prints the coefficients (lowest order first), the fit's own maximum error, and the
-maximum error of the float evaluation (coefficients rounded to float, Horner with
-single-rounding fused multiply-adds) against the double-precision function.
+Remez exchange (E. Ya. Remez, 1934) in 50-digit arithmetic for the polynomial forms
+the kernels evaluate (s = r^2):
+  sin r = r + r^3 P(s) on |r| <= pi/2, weighted to the relative error of sin;
+  cos r = 1 + s Q(s) on |r| <= pi/2, weighted to the absolute error of cos;
+  asin x = x + x^3 A(x^2) on |x| <= 1/4 (float), 1/8 (double), relative error;
+  sqrt(1 - c) - 1 = c (-1/2 + c G(c)) on 0 <= c <= 1/64, relative error.
+Prints each polynomial's maximum error and its coefficients, lowest order first.
 """
-import numpy as np
+from mpmath import lu_solve, matrix, mp, mpf, pi
 
-HALF_PI_SQ = (np.pi / 2) ** 2
+mp.dps = 50
 
 
-def remez(f, w, a, b, deg, iters=40, grid=200001):
+def remez(f, w, b, deg, iters=25, grid=4000):
+    """Coefficients of the polynomial of degree `deg` that minimises max |w (f - p)| on [0, b], and that maximum."""
     n = deg + 2
-    k = np.arange(n)
-    s = (a + b) / 2 + (b - a) / 2 * np.cos(np.pi * k[::-1] / (n - 1))
-    xs = np.linspace(a, b, grid)
+    xs = [b / 2 * (1 - mp.cos(pi * k / grid)) for k in range(grid + 1)]
+    fx, wx = [f(x) for x in xs], [w(x) for x in xs]
+    s = [b / 2 * (1 - mp.cos(pi * k / (n - 1))) for k in range(n)]
+    last = None
     for _ in range(iters):
-        A = np.zeros((n, n))
+        lhs, rhs = matrix(n, n), matrix(n, 1)
         for i in range(n):
-            A[i, :deg + 1] = s[i] ** np.arange(deg + 1)
-            A[i, deg + 1] = (-1) ** i / w(s[i])
-        sol = np.linalg.solve(A, f(s))
-        c = sol[:deg + 1]
-        err = w(xs) * (f(xs) - np.polyval(c[::-1], xs))
-        ext = [0] + [i for i in range(1, grid - 1) if (err[i] - err[i - 1]) * (err[i + 1] - err[i]) <= 0] + [grid - 1]
+            for j in range(deg + 1):
+                lhs[i, j] = s[i] ** j
+            lhs[i, deg + 1] = (-1) ** i / w(s[i])
+            rhs[i] = f(s[i])
+        sol = lu_solve(lhs, rhs)
+        c = [sol[j] for j in range(deg + 1)]
+        err = [wx[k] * (fx[k] - mp.polyval(c[::-1], xs[k])) for k in range(grid + 1)]
         pts = []
-        for i in sorted(ext):
-            if pts and np.sign(err[i]) == np.sign(err[pts[-1]]):
-                if abs(err[i]) > abs(err[pts[-1]]):
-                    pts[-1] = i
-            else:
-                pts.append(i)
+        for i in range(grid + 1):
+            if i in (0, grid) or (err[i] - err[i - 1]) * (err[i + 1] - err[i]) <= 0:
+                if pts and (err[i] > 0) == (err[pts[-1]] > 0):
+                    if abs(err[i]) > abs(err[pts[-1]]):
+                        pts[-1] = i
+                else:
+                    pts.append(i)
         while len(pts) > n:
             pts.pop(0 if abs(err[pts[0]]) < abs(err[pts[-1]]) else -1)
-        if len(pts) < n:
+        worst = max(abs(e) for e in err)
+        if len(pts) < n or (last is not None and abs(worst - last) < worst * mpf(10) ** -6):
             break
-        s = xs[pts]
-    return c, float(np.max(np.abs(err)))
+        last, s = worst, [xs[k] for k in pts]
+    return c, worst
 
 
-def sin_p(s):
-    r = np.sqrt(s)
-    small = s < 1e-6
-    return np.where(small, -1 / 6 + s / 120 - s * s / 5040, (np.sin(r) - r) / np.where(small, 1.0, r ** 3))
+def power(coef):
+    return lambda s: mp.polyval(coef[::-1], s)
 
 
-def sin_w(s):
-    r = np.sqrt(np.maximum(s, 1e-30))
-    return np.maximum(r ** 3 / np.sin(r), 1e-30)
-
-
-def cos_q(s):
-    small = s < 1e-6
-    return np.where(small, -0.5 + s / 24 - s * s / 720, (np.cos(np.sqrt(s)) - 1) / np.where(small, 1.0, s))
-
-
-def horner_f32(c, r, sin):
-    f32 = np.float32
-    r = f32(r)
-    r2 = f32(r * r)
-    p = f32(c[-1])
-    for k in c[-2::-1]:
-        p = f32(np.float64(p) * np.float64(r2) + np.float64(f32(k)))
-    if sin:
-        return float(f32(np.float64(f32(p * r2)) * np.float64(r) + np.float64(r)))
-    return float(f32(np.float64(p) * np.float64(r2) + 1.0))
-
+TINY = mpf(10) ** -30
+SIN = power([mpf((-1) ** (k + 1)) / mp.factorial(2 * k + 3) for k in range(30)])
+COS = power([mpf((-1) ** (k + 1)) / mp.factorial(2 * k + 2) for k in range(30)])
+ASIN = power([mp.binomial(2 * n, n) / (mpf(4) ** n * (2 * n + 1)) for n in range(1, 40)])
+SQRT = power([mp.binomial(mpf(1) / 2, k) * (-1) ** k for k in range(2, 45)])
+HALF_PI_SQ = (pi / 2) ** 2 * mpf("1.0000001")
 
 if __name__ == "__main__":
-    cs, es = remez(sin_p, sin_w, 0.0, HALF_PI_SQ, 3)
-    cc, ec = remez(cos_q, lambda s: np.maximum(s, 1e-10), 0.0, HALF_PI_SQ, 4)
-    rs = np.linspace(-np.pi / 2, np.pi / 2, 100001)
-    es32 = max(abs(horner_f32(cs, r, True) - np.sin(np.float32(r))) / max(abs(np.sin(np.float32(r))), 1e-30)
-               for r in rs if r != 0)
-    ec32 = max(abs(horner_f32(cc, r, False) - np.cos(np.float32(r))) for r in rs)
-    print("sin r = r + r^3 P(r^2): P =", [float(np.float32(v)) for v in cs], "fit rel", es, "float eval rel", es32)
-    print("cos r = 1 + r^2 Q(r^2): Q =", [float(np.float32(v)) for v in cc], "fit abs", ec, "float eval abs", ec32)
+    for name, f, w, b, deg in (
+            ("sin float", SIN, lambda s: s / (1 + s * SIN(s)), HALF_PI_SQ, 3),
+            ("cos float", COS, lambda s: s, HALF_PI_SQ, 4),
+            ("asin float", ASIN, lambda s: s / (1 + s * ASIN(s)), mpf(1) / 16, 3),
+            ("sqrt1m float", SQRT, lambda c: c / (mpf(1) / 2 - c * SQRT(c)), mpf(1) / 64, 1),
+            ("sin double", SIN, lambda s: s / (1 + s * SIN(s)), HALF_PI_SQ, 7),
+            ("cos double", COS, lambda s: s, HALF_PI_SQ, 7),
+            ("asin double", ASIN, lambda s: s / (1 + s * ASIN(s)), mpf(1) / 64, 5),
+            ("sqrt1m double", SQRT, lambda c: c / (mpf(1) / 2 - c * SQRT(c)), mpf(1) / 64, 4)):
+        c, e = remez(f, lambda s, w=w: max(w(s), TINY), b, deg)
+        print(f"{name}: error {mp.nstr(e, 3)}, coefficients {[mp.nstr(x, 18, min_fixed=0, max_fixed=0) for x in c]}")

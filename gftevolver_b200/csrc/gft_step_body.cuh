@@ -114,11 +114,15 @@ __device__ __forceinline__ void su2_advance3(const Q<C> (&U)[3], const C (&R)[3]
     C cm[3], u0m1[3];
 #pragma unroll
     for (int d = 0; d < 3; d++) cm[d] = R[d][0] * R[d][0] + R[d][1] * R[d][1] + R[d][2] * R[d][2];
-    const C m = fmax(fmax(cm[0], cm[1]), cm[2]);
-    if (m >= Sqrt1mSeries<C>::limit) {
-        if (m > (C)1) warn |= kWarnSqrt;
+    MaxAbs<C> m;
 #pragma unroll
-        for (int d = 0; d < 3; d++) u0m1[d] = sqrt1m_minus1(cm[d]);
+    for (int d = 0; d < 3; d++) m.add(cm[d]);
+    if (m.exceeds(Sqrt1mSeries<C>::limit)) {
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            if (cm[d] > (C)1) warn |= kWarnSqrt;
+            u0m1[d] = sqrt1m_minus1(cm[d]);
+        }
     } else {
 #pragma unroll
         for (int d = 0; d < 3; d++) u0m1[d] = sqrt1m_series(cm[d]);
@@ -307,14 +311,32 @@ __device__ __forceinline__ void site_carry(const A& acc, const Stencil<R>& n, XC
 template <class C>
 __device__ __forceinline__ void asin3(const C (&r)[3], C (&a)[3], unsigned& warn)
 {
-    const C m = fmax(fmax(fabs(r[0]), fabs(r[1])), fabs(r[2]));
-    if (m > AsinSeries<C>::limit) {
-        if (m > (C)1) warn |= kWarnAsin;
+    MaxAbs<C> m;
 #pragma unroll
-        for (int d = 0; d < 3; d++) a[d] = gasin(r[d]);
+    for (int d = 0; d < 3; d++) m.add(r[d]);
+    if (m.exceeds(AsinSeries<C>::limit)) {
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            if (r[d] * r[d] > (C)1) warn |= kWarnAsin;
+            a[d] = gasin(r[d]);
+        }
     } else {
 #pragma unroll
         for (int d = 0; d < 3; d++) a[d] = asin_series(r[d]);
+    }
+}
+
+// Phases beyond the reduction range of the elementary functions.
+template <class C>
+__device__ __forceinline__ void warn_range(const C (&th)[3], unsigned& warn)
+{
+    MaxAbs<C> m;
+#pragma unroll
+    for (int d = 0; d < 3; d++) m.add(th[d]);
+    if (m.exceeds((C)1e4)) {
+#pragma unroll
+        for (int d = 0; d < 3; d++)
+            if (fabs(th[d]) > (C)1e4) warn |= kWarnRange;
     }
 }
 
@@ -364,41 +386,60 @@ __device__ __forceinline__ void site_step(const StepParams& P, const KConst<S>& 
     // logging-step terms: per-site partial sums in the form's arithmetic (a few
     // cancellation-free terms each), added to the FP64 block sums once per site
     C mag_e = (C)0, plaq2 = (C)0, plaq1 = (C)0;
-    C MgY[3] = {(C)0, (C)0, (C)0};
-    if constexpr (CARRY) {
-        MgY[1] = -l[0] * carry.s01;
-        MgY[2] = -l[0] * carry.s02;
-    }
+    // F_ij(x) = theta_i(x) + theta_j(x+i) - theta_i(x+j) - theta_j(x) of the upper loops; the
+    // reference's local angle is -F for link i and +F for link j (StandardModel.cpp:348-353).
+    // Then the lower loops' angles, those of the planes with x carried as sines.
+    constexpr int NLOW = CARRY ? 4 : 6;
+    C Fa[3 + NLOW], sF[3 + NLOW];
 #pragma unroll
     for (int pl = 0; pl < 3; pl++) {
         const int i = (pl == 2) ? 1 : 0;
         const int j = (pl == 0) ? 1 : 2;
-        // F_ij(x) = theta_i(x) + theta_j(x+i) - theta_i(x+j) - theta_j(x); the reference's
-        // local angle is -F for link i and +F for link j (StandardModel.cpp:348-353).
-        const C Fa = th[i] + acc.th(j, n.p[i]) - acc.th(i, n.p[j]) - th[j];
-        const C sF = gsin(Fa);
-        MgY[i] -= sF * l[j];
-        MgY[j] += sF * l[i];
-        if constexpr (CARRY) {
-            if (pl == 0) carry.s01 = sF;
-            if (pl == 1) carry.s02 = sF;
-        }
-        if (ENERGY) {
-            // 1 - cos F = 2 sin^2(F/2) (no cancellation for small F)
-            const C hF = gsin((C)0.5 * Fa);
-            const C omc = (C)2 * hF * hF;
-            mag_e += F.e_plaq[pl] * (F.inv_gp_sqr * omc);
-            plaq1 += (C)1 - omc;
+        Fa[pl] = th[i] + acc.th(j, n.p[i]) - acc.th(i, n.p[j]) - th[j];
+    }
+    {
+        int k = 3;
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+#pragma unroll
+            for (int j = 0; j < 3; j++) {
+                if (j == i || (CARRY && j == 0)) continue;
+                const R mj = n.m[j];
+                Fa[k++] = -acc.th(j, n.dg(i, j)) - acc.th(i, mj) + acc.th(j, mj) + th[i];
+            }
         }
     }
 #pragma unroll
-    for (int i = 0; i < 3; i++) {
+    for (int k = 0; k < 3 + NLOW; k++) sF[k] = gsin(Fa[k]);
+    C MgY[3];
+    MgY[0] = -l[1] * sF[0] - l[2] * sF[1];
+    MgY[1] = l[0] * sF[0] - l[2] * sF[2];
+    MgY[2] = l[0] * sF[1] + l[1] * sF[2];
+    if constexpr (CARRY) {
+        MgY[1] -= l[0] * carry.s01;
+        MgY[2] -= l[0] * carry.s02;
+        carry.s01 = sF[0];
+        carry.s02 = sF[1];
+    }
+    {
+        int k = 3;
 #pragma unroll
-        for (int j = 0; j < 3; j++) {
-            if (j == i || (CARRY && j == 0)) continue;
-            const R mj = n.m[j];
-            const C neigh = -acc.th(j, n.dg(i, j)) - acc.th(i, mj) + acc.th(j, mj) + th[i];
-            MgY[i] -= gsin(neigh) * l[j];
+        for (int i = 0; i < 3; i++) {
+#pragma unroll
+            for (int j = 0; j < 3; j++) {
+                if (j == i || (CARRY && j == 0)) continue;
+                MgY[i] -= sF[k++] * l[j];
+            }
+        }
+    }
+    if (ENERGY) {
+#pragma unroll
+        for (int pl = 0; pl < 3; pl++) {
+            // 1 - cos F = 2 sin^2(F/2) (no cancellation for small F)
+            const C hF = gsin((C)0.5 * Fa[pl]);
+            const C omc = (C)2 * hF * hF;
+            mag_e += F.e_plaq[pl] * (F.inv_gp_sqr * omc);
+            plaq1 += (C)1 - omc;
         }
     }
     C Mg[3][3];
@@ -525,31 +566,36 @@ __device__ __forceinline__ void site_step(const StepParams& P, const KConst<S>& 
     }
 
     // ---- scalar sector: covariant Laplacian D and currents J (four times the reference's, whose
-    //      1/4 is in the constants cY, cI and cH) ----
-    C J[3][4];
+    //      1/4 is in the constants cY, cI and cH; the SU(2) currents join Mg) ----
+    C JY[3];
     C JH[3][3];  // Higgs-family currents (Gradients/Source/TwoHDM.cpp:465-485)
     C grad_e = (C)0;
+    constexpr int A0 = CARRY ? 1 : 0;  // directions whose backward transport is computed (x's is carried)
+    C ang[6 - A0], sn[6 - A0], cs[6 - A0];
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-        C sn, cs;
-        gsincos(th[a], sn, cs);
-        const bool back = !(CARRY && a == 0);  // the x - e_0 transport is carried
-        C sm = (C)0, cm = (C)1;
-        Q<C> Um = {(C)1, (C)0, (C)0, (C)0};
-        if (back) {
-            gsincos(acc.th(a, n.m[a]), sm, cm);
-            Um = acc.q(a, n.m[a]);
-        }
+        ang[a] = th[a];
+        if (a >= A0) ang[3 + a - A0] = acc.th(a, n.m[a]);
+    }
+#pragma unroll
+    for (int k = 0; k < 6 - A0; k++) gsincos(ang[k], sn[k], cs[k]);
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        const bool back = a >= A0;
+        // The doublet transported forward, U R phi: what the next site of a march and the family
+        // currents need.  Elsewhere the current is formed from phi and the transported-back
+        // neighbour and turned by the link.
+        const bool fwd = HF != kHfNone || !back;
         Q<C> tm[ND], tp[ND], t[ND], fp[ND];
 #pragma unroll
         for (int db = 0; db < ND; db++) {
             fp[db] = acc.ph(db, n.p[a]);
             // D: U_a(x-a) phi(x-a) + U_a(x)^dag phi(x+a); the first is the x-1 site's transported doublet
-            tm[db] = back ? transport(Um, cm, sm, acc.ph(db, n.m[a])) : carry.t0[db];
-            tp[db] = transport_back(U[a], cs, sn, fp[db]);
-            // J: Im of (U_a(x) phi(x))^dag sigma phi(x+a)
-            t[db] = transport(U[a], cs, sn, fc[db]);
-            if (CARRY && a == 0) carry.t0[db] = t[db];
+            tm[db] = back ? transport(acc.q(a, n.m[a]), cs[3 + a - A0], sn[3 + a - A0], acc.ph(db, n.m[a]))
+                          : carry.t0[db];
+            tp[db] = transport_back(U[a], cs[a], sn[a], fp[db]);
+            t[db] = fwd ? transport(U[a], cs[a], sn[a], fc[db]) : fc[db];
+            if (!back) carry.t0[db] = t[db];
         }
         if constexpr (HF == kHfU1) {
             C hsn, hcs, hsm, hcm;
@@ -565,22 +611,30 @@ __device__ __forceinline__ void site_step(const StepParams& P, const KConst<S>& 
             hf_act<HF>(tp[0], tp[1], (C)1, (C)0, qconj(uh));
             hf_act<HF>(t[0], t[1], (C)1, (C)0, uh);
         }
+        C J[3];
 #pragma unroll
         for (int db = 0; db < ND; db++) {
             D[db] = qadd_scaled(D[db], l[a], tm[db]);
             D[db] = qadd_scaled(D[db], l[a], tp[db]);
-            const Q<C> u = t[db], f = fp[db];
+            // J: Im of t^dag sigma f, with t = U phi and f = phi(x+a), or phi and U^dag phi(x+a)
+            const Q<C> u = t[db], f = fwd ? fp[db] : tp[db];
             const C up = u.w * f.x - u.x * f.w, lo = u.y * f.z - u.z * f.y;
             const C j1 = u.w * f.z - u.x * f.y + u.y * f.x - u.z * f.w;
             const C j2 = -u.w * f.y - u.x * f.z + u.y * f.w + u.z * f.x;
-            J[a][0] = (db ? J[a][0] : (C)0) + (up + lo);
-            J[a][1] = (db ? J[a][1] : (C)0) + j1;
-            J[a][2] = (db ? J[a][2] : (C)0) + j2;
-            J[a][3] = (db ? J[a][3] : (C)0) + (up - lo);
+            JY[a] = (db ? JY[a] : (C)0) + (up + lo);
+            J[0] = (db ? J[0] : (C)0) + j1;
+            J[1] = (db ? J[1] : (C)0) + j2;
+            J[2] = (db ? J[2] : (C)0) + (up - lo);
             if (ENERGY) {
                 const C e0 = f.w - u.w, e1 = f.x - u.x, e2 = f.y - u.y, e3 = f.z - u.z;
                 grad_e += F.e_grad[a] * (e0 * e0 + e1 * e1 + e2 * e2 + e3 * e3);
             }
+        }
+        if (fwd) {
+#pragma unroll
+            for (int k = 0; k < 3; k++) Mg[a][k] += F.cI * J[k];
+        } else {
+            add_turned(Mg[a], F.cI, U[a], J);
         }
         if constexpr (HF != kHfNone) {
             // family pairs: components (i, i+1) of doublet 1 and of doublet 2, i = 0 (upper) and 2 (lower)
@@ -635,13 +689,13 @@ __device__ __forceinline__ void site_step(const StepParams& P, const KConst<S>& 
 #pragma unroll
     for (int d = 0; d < 3; d++) {
         const C dth = th[d] - (ENERGY ? ld1<C>(ps.L.th[d], ps.s) : pst_t[d]);
-        R0[d] = keep * gsin(dth) + (MgY[d] + F.cY * J[d][0]);
+        R0[d] = keep * gsin(dth) + (MgY[d] + F.cY * JY[d]);
         if (ENERGY) {  // 1 - cos(dtheta) = 2 sin^2(dtheta/2)
             const C h = gsin((C)0.5 * dth);
             elec_e += F.e_elec[d] * (F.inv_gp_sqr * (C)2 * h * h);
         }
     }
-    if (fmax(fmax(fabs(th[0]), fabs(th[1])), fabs(th[2])) > (C)1e4) warn |= kWarnRange;
+    warn_range(th, warn);
     asin3(R0, inc, warn);
 #pragma unroll
     for (int d = 0; d < 3; d++) {
@@ -659,9 +713,9 @@ __device__ __forceinline__ void site_step(const StepParams& P, const KConst<S>& 
         const Q<C> dlt = {Un.w - Up.w, Un.x - Up.x, Un.y - Up.y, Un.z - Up.z};
         C E1, E2, E3;
         qmul_vec(dlt, qconj(Up), E1, E2, E3);
-        W[d][0] = keep * E1 + (Mg[d][0] + F.cI * J[d][1]);
-        W[d][1] = keep * E2 + (Mg[d][1] + F.cI * J[d][2]);
-        W[d][2] = keep * E3 + (Mg[d][2] + F.cI * J[d][3]);
+        W[d][0] = keep * E1 + Mg[d][0];
+        W[d][1] = keep * E2 + Mg[d][1];
+        W[d][2] = keep * E3 + Mg[d][2];
         if (ENERGY) {
             // 1 - (U_now U_past^dag)_0 / |U_now U_past^dag|
             const Q<C> Ed = {Un.w * Up.w + Un.x * Up.x + Un.y * Up.y + Un.z * Up.z, E1, E2, E3};
@@ -683,7 +737,7 @@ __device__ __forceinline__ void site_step(const StepParams& P, const KConst<S>& 
                 elec_e += F.e_elec[d] * F.inv_gpp_sqr * ((C)2 * h * h);
             }
         }
-        if (fmax(fmax(fabs(hn[0]), fabs(hn[1])), fabs(hn[2])) > (C)1e4) warn |= kWarnRange;
+        warn_range(hn, warn);
         asin3(RH, hinc, warn);
 #pragma unroll
         for (int d = 0; d < 3; d++) {
