@@ -654,12 +654,9 @@ int upload_impl(gft_handle* h, const H* sc, const H* ve, int time_iter, bool on_
         dsc = st;
         dve = st + nsc_w;
     }
-    for (int t = 0; t < 2 && e == cudaSuccess; t++) {
-        const H* s_t = dsc + (size_t)t * h->nsite * h->nsc;
-        const H* v_t = dve + (size_t)t * h->nsite * h->nve;
-        e = is_f64_storage(h) ? launch_aos_to_soa<double, H>(s_t, v_t, h->nsite, h->nsc, h->ld[t], h->stream, h->codec)
-                              : launch_aos_to_soa<float, H>(s_t, v_t, h->nsite, h->nsc, h->lf[t], h->stream, h->codec);
-    }
+    if (e == cudaSuccess)
+        e = is_f64_storage(h) ? launch_aos_to_soa<double, H>(dsc, dve, h->nsite, h->nsc, h->ld, h->stream, h->codec)
+                              : launch_aos_to_soa<float, H>(dsc, dve, h->nsite, h->nsc, h->lf, h->stream, h->codec);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) return h->cuda_fail(e, "gft_upload");
     h->time_iter = time_iter;
@@ -682,13 +679,9 @@ int download_impl(gft_handle* h, H* sc, H* ve, bool on_device = false)
         dsc = static_cast<H*>(h->d_stage);
         dve = dsc + nsc_w;
     }
-    cudaError_t e = cudaSuccess;
-    for (int t = 0; t < 2 && e == cudaSuccess; t++) {
-        H* s_t = dsc + (size_t)t * h->nsite * h->nsc;
-        H* v_t = dve + (size_t)t * h->nsite * h->nve;
-        e = is_f64_storage(h) ? launch_soa_to_aos<double, H>(h->ld[t], h->nsite, h->nsc, s_t, v_t, h->stream, h->codec)
-                              : launch_soa_to_aos<float, H>(h->lf[t], h->nsite, h->nsc, s_t, v_t, h->stream, h->codec);
-    }
+    cudaError_t e =
+        is_f64_storage(h) ? launch_soa_to_aos<double, H>(h->ld, h->nsite, h->nsc, dsc, dve, h->stream, h->codec)
+                          : launch_soa_to_aos<float, H>(h->lf, h->nsite, h->nsc, dsc, dve, h->stream, h->codec);
     if (!on_device) {
         if (e == cudaSuccess) e = cudaMemcpyAsync(sc, dsc, nsc_w * sizeof(H), cudaMemcpyDeviceToHost, h->stream);
         if (e == cudaSuccess) e = cudaMemcpyAsync(ve, dve, nve_w * sizeof(H), cudaMemcpyDeviceToHost, h->stream);

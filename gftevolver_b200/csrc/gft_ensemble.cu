@@ -958,10 +958,8 @@ int gft_batch_upload_f32(gft_batch* b, int member, const float* sc, const float*
     float* dve = dsc + nsc_w;
     cudaError_t e = cudaMemcpyAsync(dsc, sc, nsc_w * sizeof(float), cudaMemcpyHostToDevice, b->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(dve, ve, nve_w * sizeof(float), cudaMemcpyHostToDevice, b->stream);
-    for (int t = 0; t < 2 && e == cudaSuccess; t++)
-        e = launch_aos_to_soa<float, float>(dsc + (size_t)t * b->nsite[member] * b->nsc,
-                                            dve + (size_t)t * b->nsite[member] * b->nve, b->nsite[member], b->nsc,
-                                            b->lv[member][t], b->stream);
+    if (e == cudaSuccess)
+        e = launch_aos_to_soa<float, float>(dsc, dve, b->nsite[member], b->nsc, b->lv[member].data(), b->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
     if (e != cudaSuccess) return b->cuda_fail(e, "gft_batch_upload_f32");
     b->time_iter = time_iter;
@@ -979,11 +977,7 @@ int gft_batch_download_f32(gft_batch* b, int member, float* sc, float* ve)
     if (rc != GFT_OK) return rc;
     float* dsc = static_cast<float*>(b->d_stage);
     float* dve = dsc + nsc_w;
-    cudaError_t e = cudaSuccess;
-    for (int t = 0; t < 2 && e == cudaSuccess; t++)
-        e = launch_soa_to_aos<float, float>(b->lv[member][t], b->nsite[member], b->nsc,
-                                            dsc + (size_t)t * b->nsite[member] * b->nsc,
-                                            dve + (size_t)t * b->nsite[member] * b->nve, b->stream);
+    cudaError_t e = launch_soa_to_aos<float, float>(b->lv[member].data(), b->nsite[member], b->nsc, dsc, dve, b->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(sc, dsc, nsc_w * sizeof(float), cudaMemcpyDeviceToHost, b->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(ve, dve, nve_w * sizeof(float), cudaMemcpyDeviceToHost, b->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);

@@ -96,7 +96,7 @@ int slab_comm_wait(SlabComm* c, cudaStream_t stream, double seconds, std::string
 bool slab_comm_alive(const SlabComm* c);
 
 // Auxiliary kernels (gft_aux_kernels.cu).
-// The reference record has 3 x 5 link words per site, 3 x 6 with a Higgs-family
+// Both time levels lv[0], lv[1] at once.  The reference record has 3 x 5 link words per site, 3 x 6 with a Higgs-family
 // phase (lv.hth set) or 3 x 9 with a Higgs-family quaternion (lv.hq set); in the
 // generator representation 3 x 4, 3 x 5 or 3 x 7.
 struct LinkCodec {
@@ -105,10 +105,10 @@ struct LinkCodec {
     double tol = 0.0;  // divisionByZeroTolerance of the conversions
 };
 template <class S, class H>
-cudaError_t launch_aos_to_soa(const H* aos_sc, const H* aos_ve, int nsite, int nsc, LevelPtrs<S> lv, cudaStream_t s,
-                              LinkCodec codec = LinkCodec());
+cudaError_t launch_aos_to_soa(const H* aos_sc, const H* aos_ve, int nsite, int nsc, const LevelPtrs<S>* lv,
+                              cudaStream_t s, LinkCodec codec = LinkCodec());
 template <class S, class H>
-cudaError_t launch_soa_to_aos(LevelPtrs<S> lv, int nsite, int nsc, H* aos_sc, H* aos_ve, cudaStream_t s,
+cudaError_t launch_soa_to_aos(const LevelPtrs<S>* lv, int nsite, int nsc, H* aos_sc, H* aos_ve, cudaStream_t s,
                               LinkCodec codec = LinkCodec());
 
 struct ICParams {
