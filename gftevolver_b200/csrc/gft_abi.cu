@@ -821,16 +821,19 @@ cudaError_t issue_step(gft_handle* h, const LevelPtrs<S>* lv, int ti, double* ou
     } else {
         err = launch_step<S>(h, P, tn, lv[tn], lv[tp], e || el);
     }
-    h->launches += nstep + (e ? finalize_launches(step_blocks(h, P), true) : 0) + ((g || gl) ? 1 : 0) +
-                   (g ? finalize_launches(gauss_blocks(h, P), true) : 0);
+    // the row's reductions run together after the Gauss pass
+    FinJob jobs[2];
+    int njobs = 0;
+    if (e) jobs[njobs++] = {h->d_part_e, step_blocks(h, P), kObsCount, kObsCount, h->d_scale, out};
+    if (g)
+        jobs[njobs++] = {h->d_part_g, gauss_blocks(h, P), 2 * h->neq, h->neq, h->d_scale + kObsCount, out + kObsCount};
+    h->launches += nstep + ((g || gl) ? 1 : 0) + (njobs ? finalize_launches(jobs, njobs) : 0);
     if (prof) {
         cudaEventRecord(h->ev[2 * (size_t)h->ev_used + 1], h->stream);
         h->ev_steps[h->ev_used] = 1;
         h->ev_used++;
     }
     if (err != cudaSuccess) return err;
-    if (e) err = launch_finalize(h->d_part_e, step_blocks(h, P), kObsCount, kObsCount, h->d_scale, out, h->d_mid,
-                                 h->stream);
     if (h->comm && !split && err == cudaSuccess) {
         // logging steps (and forms without the split): the exchange after the whole step
         SlabPlanes pl;
@@ -847,12 +850,8 @@ cudaError_t issue_step(gft_handle* h, const LevelPtrs<S>* lv, int ti, double* ou
             return cudaSuccess;
         }
     }
-    if ((g || gl) && err == cudaSuccess) {
-        err = launch_gauss<S>(h, P, lv[tn], lv[tp]);
-        if (err == cudaSuccess && g)
-            err = launch_finalize(h->d_part_g, gauss_blocks(h, P), 2 * h->neq, h->neq, h->d_scale + kObsCount,
-                                  out + kObsCount, h->d_mid, h->stream);
-    }
+    if ((g || gl) && err == cudaSuccess) err = launch_gauss<S>(h, P, lv[tn], lv[tp]);
+    if (njobs && err == cudaSuccess) err = launch_finalize(jobs, njobs, h->d_mid, h->stream);
     return err;
 }
 
@@ -1103,8 +1102,8 @@ int gft_observe(gft_handle* h, gft_observables* row)
         }
     }
     // the step wrote into the copy; restore nothing (the levels are untouched)
-    if (e == cudaSuccess) e = launch_finalize(h->d_part_e, step_blocks(h, P), kObsCount, kObsCount, h->d_scale, h->d_rows,
-                                                  h->d_mid, h->stream);
+    const FinJob job = {h->d_part_e, step_blocks(h, P), kObsCount, kObsCount, h->d_scale, h->d_rows};
+    if (e == cudaSuccess) e = launch_finalize(&job, 1, h->d_mid, h->stream);
     std::vector<double> host(kRowSlots, 0.0);
     if (e == cudaSuccess) e = cudaMemcpyAsync(host.data(), h->d_rows, kObsCount * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(h->d_status, 0, sizeof(unsigned), h->stream);

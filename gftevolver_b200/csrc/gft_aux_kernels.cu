@@ -324,25 +324,29 @@ __global__ void init_fields_kernel(StepParams P, int nsc, ICParams ic, LevelPtrs
     }
 }
 
-// Reduces the per-block partials [nblocks][nslots] of a logging step (the
-// block reduction is reduce_rows_block, gft_reduce.cuh).  With a grid of G > 1
-// blocks, block g reduces rows [g * rows_per_cta, (g + 1) * rows_per_cta) and
-// writes one unscaled row out[g][nslots] (stage one of two); with G = 1 it
-// reduces all rows and writes out[k] = total * scale[k].
-constexpr int kFinMidRows = 512;  // most stage-one rows (the caller's mid buffer holds kFinMidRows x kMaxSlots)
-__global__ void __launch_bounds__(kFinThreads) finalize_kernel(const double* __restrict__ partials, int nblocks,
-                                                               int nslots, int max_from, const double* scale,
-                                                               double* out, int rows_per_cta)
+// One stage of a reduction of per-block partials [nblocks][nslots] (reduce_rows_block,
+// gft_reduce.cuh): block x reduces rows [x * rows_per_cta, (x + 1) * rows_per_cta) into row x
+// of out, scaled by scale[slot] in the last stage (null before it).
+struct FinStage {
+    const double* partials;
+    int nblocks, nslots, max_from;
+    const double* scale;
+    double* out;
+    int rows_per_cta;
+};
+constexpr int kFinMidRows = 512;  // most stage-one rows of a job
+static_assert(kFinMidCapacity >= 2 * kFinMidRows * kMaxSlots, "stage-one rows of two jobs");
+
+// A logging step's energy and Gauss rows (blockIdx.y) in one launch.
+__global__ void __launch_bounds__(kFinThreads) finalize_kernel(FinStage f0, FinStage f1)
 {
-    const int b0 = (int)blockIdx.x * rows_per_cta;
-    const int b1 = min(nblocks, b0 + rows_per_cta);
-    const double total = reduce_rows_block(partials, b0, b1, nslots, max_from);
-    if (threadIdx.x < (unsigned)nslots) {
+    const FinStage& f = blockIdx.y ? f1 : f0;
+    const int b0 = (int)blockIdx.x * f.rows_per_cta;
+    if (b0 >= f.nblocks) return;
+    const double total = reduce_rows_block(f.partials, b0, min(f.nblocks, b0 + f.rows_per_cta), f.nslots, f.max_from);
+    if (threadIdx.x < (unsigned)f.nslots) {
         const int k = threadIdx.x;
-        if (gridDim.x > 1)
-            out[(size_t)blockIdx.x * nslots + k] = total;
-        else
-            out[k] = total * scale[k];
+        f.out[(size_t)blockIdx.x * f.nslots + k] = f.scale ? total * f.scale[k] : total;
     }
 }
 
@@ -441,24 +445,46 @@ cudaError_t launch_init_fields(const StepParams& P, int nsc, const ICParams& ic,
     return cudaGetLastError();
 }
 
-cudaError_t launch_finalize(const double* partials, int nblocks, int nslots, int max_from, const double* scale_dev,
-                            double* out, double* mid, cudaStream_t s)
+// Rows one block reduces by itself; more go through stage-one rows in `mid`.
+constexpr int kFinOneStage = 2 * kFinThreads;
+
+cudaError_t launch_finalize(const FinJob* jobs, int njobs, double* mid, cudaStream_t s)
 {
-    if (nslots > kMaxSlots) return cudaErrorInvalidValue;
-    if (mid != nullptr && nblocks > 2 * kFinThreads) {
-        // two stages: at most kFinMidRows blocks of >= kFinThreads rows each, then one block
-        int rpc = (nblocks + kFinMidRows - 1) / kFinMidRows;
-        rpc = rpc < kFinThreads ? kFinThreads : rpc;
-        const int g = (nblocks + rpc - 1) / rpc;
-        finalize_kernel<<<g, kFinThreads, 0, s>>>(partials, nblocks, nslots, max_from, nullptr, mid, rpc);
-        finalize_kernel<<<1, kFinThreads, 0, s>>>(mid, g, nslots, max_from, scale_dev, out, g);
-        return cudaGetLastError();
+    FinStage st[2] = {};
+    bool two = false;
+    for (int j = 0; j < njobs; j++) {
+        const FinJob& f = jobs[j];
+        if (f.nslots > kMaxSlots) return cudaErrorInvalidValue;
+        st[j] = {f.partials, f.nblocks, f.nslots, f.max_from, f.scale, f.out, f.nblocks};
+        two = two || f.nblocks > kFinOneStage;
     }
-    finalize_kernel<<<1, kFinThreads, 0, s>>>(partials, nblocks, nslots, max_from, scale_dev, out, nblocks);
+    if (two) {
+        // at most kFinMidRows blocks of >= kFinThreads / 2 rows each, then one block
+        FinStage a[2] = {};
+        int g = 0;
+        for (int j = 0; j < njobs; j++) {
+            const int n = st[j].nblocks, even = (n + kFinMidRows - 1) / kFinMidRows;
+            const int rpc = even < kFinThreads / 2 ? kFinThreads / 2 : even, rows = (n + rpc - 1) / rpc;
+            a[j] = st[j];
+            a[j].scale = nullptr;
+            a[j].out = mid + (size_t)j * kFinMidRows * kMaxSlots;
+            a[j].rows_per_cta = rpc;
+            st[j].partials = a[j].out;
+            st[j].nblocks = st[j].rows_per_cta = rows;
+            g = rows > g ? rows : g;
+        }
+        finalize_kernel<<<dim3(g, njobs), kFinThreads, 0, s>>>(a[0], a[1]);
+    }
+    finalize_kernel<<<dim3(1, njobs), kFinThreads, 0, s>>>(st[0], st[1]);
     return cudaGetLastError();
 }
 
-int finalize_launches(int nblocks, bool have_mid) { return (have_mid && nblocks > 2 * kFinThreads) ? 2 : 1; }
+int finalize_launches(const FinJob* jobs, int njobs)
+{
+    for (int j = 0; j < njobs; j++)
+        if (jobs[j].nblocks > kFinOneStage) return 2;
+    return 1;
+}
 
 template cudaError_t launch_aos_to_soa<float, float>(const float*, const float*, int, int, const LevelPtrs<float>*, cudaStream_t,
                                                      LinkCodec);

@@ -620,16 +620,16 @@ cudaError_t issue_step_family(gft_batch* b, int ti, bool e, bool g, double* rows
         (*nlaunch)++;
         if (err == cudaSuccess && e) {
             const int nb = fast_launch_blocks(P, 0);
-            err = launch_finalize(b->d_part_f, nb, kObsCount, kObsCount, scale, row, b->d_mid, b->stream);
-            *nlaunch += finalize_launches(nb, true);
+            const FinJob job = {b->d_part_f, nb, kObsCount, kObsCount, scale, row};
+            err = launch_finalize(&job, 1, b->d_mid, b->stream);
+            *nlaunch += finalize_launches(&job, 1);
         }
         if (err == cudaSuccess && g) {
             const int nb = fast_gauss_blocks(P);
             err = launch_fast_gauss<float, kModel2HDM>(P, b->lv[m][tn], b->lv[m][tp], b->d_part_f, b->stream);
-            if (err == cudaSuccess)
-                err = launch_finalize(b->d_part_f, nb, 2 * b->neq, b->neq, scale + kObsCount, row + kObsCount,
-                                      b->d_mid, b->stream);
-            *nlaunch += 1 + finalize_launches(nb, true);
+            const FinJob job = {b->d_part_f, nb, 2 * b->neq, b->neq, scale + kObsCount, row + kObsCount};
+            if (err == cudaSuccess) err = launch_finalize(&job, 1, b->d_mid, b->stream);
+            *nlaunch += 1 + finalize_launches(&job, 1);
         }
     }
     return err;

@@ -126,16 +126,20 @@ template <class S>
 cudaError_t launch_init_fields(const StepParams& P, int nsc, const ICParams& ic, LevelPtrs<S> a, LevelPtrs<S> b,
                                cudaStream_t s);
 
-// Sum (slots < max_from, compensated) or max (slots >= max_from) the per-block
-// partials [nblocks][nslots] into out[nslots], scaled by scale[slot].
-// Deterministic FP64 reduction of per-block partials into one row (scaled by
-// scale[k]); `mid` (kFinMidRows x 16 doubles, may be null) enables a two-stage
-// reduction for large block counts.
-cudaError_t launch_finalize(const double* partials, int nblocks, int nslots, int max_from, const double* scale_dev,
-                            double* out, double* mid, cudaStream_t s);
-// Kernel launches launch_finalize makes for nblocks partial rows.
-int finalize_launches(int nblocks, bool have_mid);
-constexpr int kFinMidCapacity = 512 * 16;
+// Deterministic FP64 reduction of per-block partials [nblocks][nslots] into one row: the sum
+// (slots < max_from, compensated) or the maximum (slots >= max_from) times scale[slot].
+struct FinJob {
+    const double* partials;
+    int nblocks, nslots, max_from;
+    const double* scale;
+    double* out;
+};
+// One or two jobs together; `mid` (kFinMidCapacity doubles) holds the rows between the two stages
+// that large block counts take.
+cudaError_t launch_finalize(const FinJob* jobs, int njobs, double* mid, cudaStream_t s);
+// Kernel launches launch_finalize makes.
+int finalize_launches(const FinJob* jobs, int njobs);
+constexpr int kFinMidCapacity = 2 * 512 * 16;
 
 // Record the library-wide last error message (gft_last_error(NULL)).
 void set_last_error(const std::string& msg);
