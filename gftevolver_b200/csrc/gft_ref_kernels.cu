@@ -21,34 +21,49 @@ struct RefView {
     const LevelPtrs<S>& L;
     bool gen;    // links stored as generators (w1, w2, w3, unused)
     double tol;  // divisionByZeroTolerance
-    __device__ double th(int d, int s) const { return (double)L.th[d][s]; }
+    __device__ double th(int d, int s) const { return ld1<double>(L.th[d], s); }
+    // sin and cos of the phase together (the same bits as the two calls)
+    __device__ double2 trig(int d, int s) const
+    {
+        double2 t;
+        sincos(th(d, s), &t.x, &t.y);
+        return t;
+    }
+    __device__ double2 htrig(int d, int s) const
+    {
+        double2 t;
+        sincos(hth(d, s), &t.x, &t.y);
+        return t;
+    }
     // getSU2Representation (WilsonLoops/Source/StandardModel.cpp:76-112)
     __device__ void rep(int d, int s, bool conj, double c[4]) const { rep_of(L.q[d], s, conj, c); }
     // the same for the Higgs-family field (TwoHDM.cpp:94-126, 362-368)
-    __device__ double hth(int d, int s) const { return (double)L.hth[d][s]; }
+    __device__ double hth(int d, int s) const { return ld1<double>(L.hth[d], s); }
     __device__ void hrep(int d, int s, bool conj, double c[4]) const { rep_of(L.hq[d], s, conj, c); }
     __device__ void rep_of(const S* a, int s, bool conj, double c[4]) const
     {
-        const S* p = a + 4 * (size_t)s;
+        const Q<double> v = ld4<double>(a, s);  // one vector load: the record's words widened
+        const double p[4] = {v.w, v.x, v.y, v.z};
         if (gen) {
             // generator branch: c0 = cos|w|, c_a = conj * sin|w| * w_a / |w| (c1 = sin|w| when |w| <= tol)
             double wm = 0.0;
-            wm += (double)p[0] * (double)p[0];
-            wm += (double)p[1] * (double)p[1];
-            wm += (double)p[2] * (double)p[2];
+            wm += p[0] * p[0];
+            wm += p[1] * p[1];
+            wm += p[2] * p[2];
             wm = sqrt(wm);
             c[0] = cos(wm);
             c[1] = c[2] = c[3] = 0.0;
             if (wm > tol) {
                 const double cs = (double)(conj ? -1 : 1) * sin(wm);
-                for (int k = 1; k < 4; k++) c[k] = cs * (double)p[k - 1] / wm;
+                for (int k = 1; k < 4; k++) c[k] = cs * p[k - 1] / wm;
             } else {
                 c[1] = sin(wm);
             }
             return;
         }
-        c[0] = (double)p[0];
-        for (int k = 1; k < 4; k++) c[k] = conj ? -(double)p[k] : (double)p[k];
+        c[0] = p[0];
+#pragma unroll
+        for (int k = 1; k < 4; k++) c[k] = conj ? -p[k] : p[k];
     }
     // Store a link: the quaternion, or (generator representation) invertSU2Representation
     // (WilsonLoops/Source/StandardModel.cpp:114-158): phase = asin|c| (pi/2 when |c| > 1),
@@ -79,6 +94,17 @@ struct RefView {
     }
 };
 
+// a / b, correctly rounded, from inv = 1/b correctly rounded: the quotient estimate a inv
+// corrected once by its exact remainder (P. W. Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", 1990).  Four quotients by the same norm
+// then cost one reciprocal.  The same bits as the division outside subnormal remainders and
+// infinite norms.
+__device__ __forceinline__ double div_by(double a, double b, double inv)
+{
+    const double q = a * inv;
+    return fma(fma(-q, b, a), inv, q);
+}
+
 // SU2Product (WilsonLoops/Source/StandardModel.cpp:160-191).
 __device__ __forceinline__ void ref_su2_product(const double a[4], const double b[4], bool calc_trace, double out[4])
 {
@@ -93,10 +119,11 @@ __device__ __forceinline__ void ref_su2_product(const double a[4], const double 
         dot += a[3] * b[3];
         p0 = a[0] * b[0] - dot;
         double norm = sqrt(p0 * p0 + p1 * p1 + p2 * p2 + p3 * p3);
-        p0 = p0 / norm;
-        p1 = p1 / norm;
-        p2 = p2 / norm;
-        p3 = p3 / norm;
+        const double inv = __drcp_rn(norm);
+        p0 = div_by(p0, norm, inv);
+        p1 = div_by(p1, norm, inv);
+        p2 = div_by(p2, norm, inv);
+        p3 = div_by(p3, norm, inv);
     }
     out[0] = p0;
     out[1] = p1;
@@ -108,28 +135,29 @@ __device__ __forceinline__ void ref_su2_product(const double a[4], const double 
 // (Gradients/Source/StandardModel.cpp:72-100, TwoHDM.cpp:72-149): hypercharge
 // phase, isospin SU(2), then the Higgs-family U(1) (+theta_H on doublet 1,
 // -theta_H on doublet 2) or SU(2) (acting on doublet-1 / doublet-2 pairs).
+// tr, htr: (sin, cos) of the hypercharge phase and of the family phase of that link (sin(-x) is
+// -sin(x) to the bit, so a site's own links take them once for both directions).
 template <int NSC, class S>
 __device__ __forceinline__ void ref_transform_sm(const double* in, const RefView<S>& V, int d, int s, bool conj,
-                                                 double* out);
+                                                 double2 tr, double* out);
 
 template <int NSC, int HF, class S>
 __device__ __forceinline__ void ref_transform(const double* in, const RefView<S>& V, int d, int s, bool conj,
-                                              double* out)
+                                              double2 tr, double2 htr, double* out)
 {
     if (HF == kHfNone) {
-        ref_transform_sm<NSC>(in, V, d, s, conj, out);
+        ref_transform_sm<NSC>(in, V, d, s, conj, tr, out);
         return;
     }
     double sm[8];
-    ref_transform_sm<8>(in, V, d, s, conj, sm);
+    ref_transform_sm<8>(in, V, d, s, conj, tr, sm);
     const int conj_fac = conj ? -1 : 1;
     if (HF == kHfU1) {
-        const double th = V.hth(d, s);
 #pragma unroll
         for (int c = 0; c < 8; c++) {
             const int pm = -1 + 2 * (c % 2);
             const int pm4 = 1 - 2 * (c / 4);
-            out[c] = cos(th) * sm[c] + (double)pm * sin((double)(pm4 * conj_fac) * th) * sm[c - pm];
+            out[c] = htr.y * sm[c] + (double)pm * ((double)(pm4 * conj_fac) * htr.x) * sm[c - pm];
         }
     } else {
         double u[4];
@@ -147,11 +175,10 @@ __device__ __forceinline__ void ref_transform(const double* in, const RefView<S>
 
 template <int NSC, class S>
 __device__ __forceinline__ void ref_transform_sm(const double* in, const RefView<S>& V, int d, int s, bool conj,
-                                                 double* out)
+                                                 double2 tr, double* out)
 {
-    const double th = V.th(d, s);
-    const double sn = sin((conj ? -1.0 : 1.0) * th);
-    const double cs = cos(th);
+    const double sn = conj ? -tr.x : tr.x;
+    const double cs = tr.y;
     double h[NSC];
 #pragma unroll
     for (int c = 0; c < NSC; c++) {
@@ -175,9 +202,11 @@ __device__ __forceinline__ void ref_load_scalar(const LevelPtrs<S>& L, int s, do
 {
 #pragma unroll
     for (int db = 0; db < NSC / 4; db++) {
-        const S* p = L.ph[db] + 4 * (size_t)s;
-#pragma unroll
-        for (int k = 0; k < 4; k++) f[4 * db + k] = (double)p[k];
+        const Q<double> p = ld4<double>(L.ph[db], s);
+        f[4 * db] = p.w;
+        f[4 * db + 1] = p.x;
+        f[4 * db + 2] = p.y;
+        f[4 * db + 3] = p.z;
     }
 }
 
@@ -186,9 +215,11 @@ __device__ __forceinline__ void ref_load_scalar_S(const LevelPtrs<S>& L, int s, 
 {
 #pragma unroll
     for (int db = 0; db < NSC / 4; db++) {
-        const S* p = L.ph[db] + 4 * (size_t)s;
-#pragma unroll
-        for (int k = 0; k < 4; k++) f[4 * db + k] = p[k];
+        const Q<S> p = ld4<S>(L.ph[db], s);
+        f[4 * db] = p.w;
+        f[4 * db + 1] = p.x;
+        f[4 * db + 2] = p.y;
+        f[4 * db + 3] = p.z;
     }
 }
 
@@ -293,8 +324,20 @@ __device__ __forceinline__ S ref_potential_energy(const StepParams& P, const S* 
     }
 }
 
+// Resident blocks per SM the launch bounds ask for.  The kernel waits on FP64 and local-memory
+// latencies in rolled loops (unrolled, the code of six pairs of loops misses the instruction
+// cache: 163 -> 211 us per step at SM 64^3), so it runs faster with more warps and some spills
+// (us per step, SM 64^3 / 2HDM 64^3 / 2HDM with the family SU(2) 48^3: unbounded 144 / 190 /
+// 191, five blocks 152 / 176 / 206, seven 145 / 170 / 221, eight 148 / 175 / 175; logging steps
+// unbounded 210 / 258 / 227, seven 193 / 236 / 265, eight 196 / 242 / 210).
+template <int HF>
+constexpr int ref_min_blocks()
+{
+    return HF == kHfNone ? 7 : 8;
+}
+
 template <class S, int MODEL, int HF, bool ENERGY>
-__global__ void __launch_bounds__(128) ref_step_kernel(StepParams P, LevelPtrs<S> now, LevelPtrs<S> past,
+__global__ void __launch_bounds__(128, ref_min_blocks<HF>()) ref_step_kernel(StepParams P, LevelPtrs<S> now, LevelPtrs<S> past,
                                                        unsigned* status, double* partials)
 {
     constexpr int NSC = (MODEL == kModelSM) ? 4 : 8;
@@ -321,6 +364,12 @@ __global__ void __launch_bounds__(128) ref_step_kernel(StepParams P, LevelPtrs<S
         double Pot[NSC];
         ref_potential_derivs<MODEL>(P, f_now, Pot);
 
+        double2 tr[3], htr[3];  // the own links' phases
+        for (int a = 0; a < 3; a++) {
+            tr[a] = V.trig(a, n.c);
+            htr[a] = (HF == kHfU1) ? V.htrig(a, n.c) : make_double2(0.0, 1.0);
+        }
+
         // ---- calcDerivatives (Gradients/Source/StandardModel.cpp:272-320) ----
         double D[NSC];
 #pragma unroll
@@ -332,9 +381,10 @@ __global__ void __launch_bounds__(128) ref_step_kernel(StepParams P, LevelPtrs<S
                 ref_load_scalar<NSC>(now, s, f);
                 const double w = (st == 1) ? -2.0 * P.lap[a] : P.lap[a];
                 if (st == 0) {
-                    ref_transform<NSC, HF>(f, V, a, n.m[a], false, t);
+                    ref_transform<NSC, HF>(f, V, a, n.m[a], false, V.trig(a, n.m[a]),
+                                           (HF == kHfU1) ? V.htrig(a, n.m[a]) : make_double2(0.0, 1.0), t);
                 } else if (st == 2) {
-                    ref_transform<NSC, HF>(f, V, a, n.c, true, t);
+                    ref_transform<NSC, HF>(f, V, a, n.c, true, tr[a], htr[a], t);
                 } else {
 #pragma unroll
                     for (int c = 0; c < NSC; c++) t[c] = f[c];
@@ -350,7 +400,7 @@ __global__ void __launch_bounds__(128) ref_step_kernel(StepParams P, LevelPtrs<S
         for (int a = 0; a < 3; a++) {
             double f[NSC], t[NSC], nb[NSC];
             ref_load_scalar<NSC>(now, n.c, f);
-            ref_transform<NSC, HF>(f, V, a, n.c, false, t);
+            ref_transform<NSC, HF>(f, V, a, n.c, false, tr[a], htr[a], t);
             ref_load_scalar<NSC>(now, n.p[a], nb);
             double jj[NEQ];
 #pragma unroll
