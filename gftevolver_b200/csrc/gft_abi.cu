@@ -528,7 +528,11 @@ int gft_create(const gft_config* cfg, gft_handle** out)
         // default tile: the largest built shape the lattice divides
         h->tile_variant = 0;
         while (h->tile_variant < kTiledVariants && !tiled_supported(P, h->tile_variant)) h->tile_variant++;
-        h->tiled_ready = h->tile_variant < kTiledVariants && encode_tiled(h, P, h->tile_variant, h->tm, h->tp);
+        // FP64: two CTAs of four warps per SM, where an 8 x 32 tile's staged planes leave one of
+        // eight; its barriers stop half the warps (us per step, 256^3 / 192^3: 1936 / 823 against
+        // 2017 / 866; logging step 2928 against 2802)
+        if (cfg->form == GFT_FORM_FP64 && tiled_supported(P, kTileFP64)) h->tile_variant = kTileFP64;
+        h->tiled_ready = (h->tile_variant < kTiledVariants || h->tile_variant == kTileFP64) && encode_tiled(h, P, h->tile_variant, h->tm, h->tp);
     }
     int nb = std::max(fast_launch_blocks(P, 0), fast_gauss_blocks(P));
     nb = std::max(nb, ref_launch_blocks(P));

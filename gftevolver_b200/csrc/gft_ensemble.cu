@@ -101,17 +101,16 @@ __device__ __forceinline__ void tmap_acquire(const TMaps& m)
 template <int MODEL, int TY, int TZ, bool ENERGY>
 constexpr bool ens_stage()
 {
-    return HaloStage<float, TY, TZ, (MODEL == kModelSM) ? 1 : 2>::use(ENERGY);
+    return tile_stage<float, MODEL, TY, TZ, ENERGY>();
 }
 template <int MODEL, int TY, int TZ, bool ENERGY>
 constexpr int ens_smem()
 {
-    constexpr int ND = (MODEL == kModelSM) ? 1 : 2;
-    return ens_stage<MODEL, TY, TZ, ENERGY>() ? HaloStage<float, TY, TZ, ND>::SMEM : Geom<float, TY, TZ, ND>::SMEM;
+    return tile_smem<float, MODEL, TY, TZ, ENERGY>();
 }
 
 template <int MODEL, int TY, int TZ, bool ENERGY, bool UNIFORM>
-__global__ void __launch_bounds__(TY * TZ, 512 / (TY * TZ))
+__global__ void __launch_bounds__(TY * TZ, tile_ctas<float, MODEL, TY, TZ>())
     ensemble_step_kernel(const __grid_constant__ EnsParams ep, const EnsMaps* __restrict__ maps,
                          const int4* __restrict__ items, int nitems, const int* __restrict__ order,
                          const int* __restrict__ start, int nlist, int lx, int tn, unsigned* status,
@@ -169,7 +168,7 @@ __global__ void __launch_bounds__(TY * TZ, 512 / (TY * TZ))
         const KConst<float>& F = UNIFORM ? ep.fcommon : Fm;
         const bool ok = run_tile<float, MODEL, TY, TZ, ENERGY, EnsLevel, ens_stage<MODEL, TY, TZ, ENERGY>()>(
             mp.tm[tn], mp.tp[1 - tn], P, F, ep.lv[m][tn], ep.lv[m][1 - tn], w.y, w.z, w.w, min(lx, P.nx - w.w), smem,
-            bars, ring, &s_abort, obs, warn, smem + HaloStage<float, TY, TZ, ND>::OFFSET);
+            bars, ring, &s_abort, obs, warn);
         if (!ok) {
             if (tid == 0) atomicOr(status, kErrTimeout);
             break;

@@ -63,13 +63,15 @@ cudaError_t launch_tiled_split_step(const TMaps& maps, const TMaps& pmaps, const
                                     const LevelPtrs<float>& now, const LevelPtrs<float>& past, int lx,
                                     unsigned* status, cudaStream_t stream, int xa = 0, int xn = -1);
 constexpr int kTiledVariants = 4;  // 8x32, 4x32, 4x16, 16x16 (TY x TZ)
+// 8x16, the FP64 step's own choice: not among the shapes a caller picks
+constexpr int kTileFP64 = 4;
 // Tile shapes the two-sites-per-thread kernel is built for (8 x 32 and 16 x 16:
 // 128 threads per CTA, two CTAs per SM).
 inline bool tiled_pair_tile(int variant) { return variant == 0 || variant == 3; }
 inline void tiled_tile(int variant, int& ty, int& tz)
 {
-    static const int shapes[4][2] = {{8, 32}, {4, 32}, {4, 16}, {16, 16}};
-    const int v = (variant >= 0 && variant < 4) ? variant : 0;
+    static const int shapes[5][2] = {{8, 32}, {4, 32}, {4, 16}, {16, 16}, {8, 16}};
+    const int v = (variant >= 0 && variant < 5) ? variant : 0;
     ty = shapes[v][0];
     tz = shapes[v][1];
 }

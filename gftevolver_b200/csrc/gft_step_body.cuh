@@ -186,13 +186,35 @@ struct XCarry {
     Q<C> t0[ND];
 };
 
-// Own-site access to the past level (read, then overwritten with t + dt).  LV is
-// LevelPtrs<S>, or any struct with its q / th / ph members when no Higgs-family
-// field is evolved.
+// Own-site past level (read, then overwritten with t + dt).  LV is LevelPtrs<S>, or any
+// struct with its q / th / ph members when no Higgs-family field is evolved.
 template <class S, class LV = LevelPtrs<S>>
 struct PastSite {
     LV L;
     int s;
+};
+
+// Its values: EARLY, loaded together by load() so that their latency overlaps arithmetic
+// (plain steps); else each where it is used (logging steps have no registers to spare).
+template <class S, int ND, class LV, bool EARLY>
+struct PastValues {
+    PastSite<S, LV> at;
+    Q<S> f[ND], u[3];
+    S t[3];
+    __device__ __forceinline__ void load()
+    {
+        if (!EARLY) return;
+#pragma unroll
+        for (int db = 0; db < ND; db++) f[db] = ld4<S>(at.L.ph[db], at.s);
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            u[d] = ld4<S>(at.L.q[d], at.s);
+            t[d] = ld1<S>(at.L.th[d], at.s);
+        }
+    }
+    __device__ __forceinline__ Q<S> ph(int db) const { return EARLY ? f[db] : ld4<S>(at.L.ph[db], at.s); }
+    __device__ __forceinline__ Q<S> q(int d) const { return EARLY ? u[d] : ld4<S>(at.L.q[d], at.s); }
+    __device__ __forceinline__ S th(int d) const { return EARLY ? t[d] : ld1<S>(at.L.th[d], at.s); }
 };
 
 // A thread's total energy from its component sums, set once after its last site
@@ -340,6 +362,102 @@ __device__ __forceinline__ void warn_range(const C (&th)[3], unsigned& warn)
     }
 }
 
+// Scalar leapfrog (Model.cpp:347-356) of one doublet f, from D = dt^2 (Laplacian - dV/dphi):
+// phi(t+dt) = phi + [(phi - phi_past)(1 - damping) + D], one rounding at the end.
+template <bool ENERGY, class C, class S>
+__device__ __forceinline__ void leapfrog_doublet(const KConst<C>& F, Q<C> f, Q<C> fpast, Q<C> D, S* out, int s, C& kin_e,
+                                                 C& phisq, C& check)
+{
+    const C fn[4] = {f.w, f.x, f.y, f.z};
+    const C fo[4] = {fpast.w, fpast.x, fpast.y, fpast.z};
+    const C dd[4] = {D.w, D.x, D.y, D.z};
+    C o[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const C vel = fn[k] - fo[k];
+        o[k] = fn[k] + (F.keep * vel + dd[k]);
+        check += o[k];
+        if (ENERGY) {
+            kin_e += vel * vel;  // x 0.5 / dt^2 in record_energies
+            phisq += fn[k] * fn[k];
+        }
+    }
+    st4(out, s, o[0], o[1], o[2], o[3]);
+}
+
+// Link update (WilsonLoops/Source/StandardModel.cpp:456-514) from the forces dt^2 (magnetic + current).
+template <bool ENERGY, class C, class PV>
+__device__ __forceinline__ void leapfrog_links(const KConst<C>& F, const Q<C> (&U)[3], const C (&th)[3],
+                                               const C (&Mg)[3][3], const C (&MgY)[3], const PV& past, C& elec_e,
+                                               unsigned& warn, C& check)
+{
+    // theta(t+dt) = theta(t) + asin(RHS_Y)
+    C R0[3], inc[3];
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        const C dth = th[d] - past.th(d);
+        R0[d] = F.keep * gsin(dth) + MgY[d];
+        if (ENERGY) {  // 1 - cos(dtheta) = 2 sin^2(dtheta/2)
+            const C h = gsin((C)0.5 * dth);
+            elec_e += F.e_elec[d] * (F.inv_gp_sqr * (C)2 * h * h);
+        }
+    }
+    warn_range(th, warn);
+    asin3(R0, inc, warn);
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        const C thn = th[d] + inc[d];
+        check += thn;
+        past.at.L.th[d][past.at.s] = thn;
+    }
+    // u = (sqrt(1-|c|^2), c); U(t+dt) = normalise(u U(t)) (su2_advance3)
+    C W[3][3];
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        const Q<C> Un = U[d];
+        const Q<C> Up = past.q(d);
+        // link momentum vec(U_now U_past^dag) = vec((U_now - U_past) U_past^dag)
+        const Q<C> dlt = {Un.w - Up.w, Un.x - Up.x, Un.y - Up.y, Un.z - Up.z};
+        C E1, E2, E3;
+        qmul_vec(dlt, qconj(Up), E1, E2, E3);
+        W[d][0] = F.keep * E1 + Mg[d][0];
+        W[d][1] = F.keep * E2 + Mg[d][1];
+        W[d][2] = F.keep * E3 + Mg[d][2];
+        if (ENERGY) {
+            // 1 - (U_now U_past^dag)_0 / |U_now U_past^dag|
+            const Q<C> Ed = {Un.w * Up.w + Un.x * Up.x + Un.y * Up.y + Un.z * Up.z, E1, E2, E3};
+            elec_e += F.e_elec[d] * (F.inv_g_sqr * one_minus_trace(Ed));
+        }
+    }
+    su2_advance3(U, W, past.at.L.q, past.at.s, warn, check);
+}
+
+// A site's energy densities into the thread's sums, and into the local output where it is asked for.
+template <class C>
+__device__ __forceinline__ void record_energies(const StepParams& P, int s, double pot_e, C grad_e, C kin_e, C mag_e,
+                                                C elec_e, C plaq2, C plaq1, C phisq, double (&obs)[kObsCount])
+{
+    const double ge = (double)grad_e, ke = 0.5 * P.inv_sqr_dt * (double)kin_e;
+    const double me = (double)mag_e, ee = (double)elec_e;
+    if (P.loc_energy) {  // Energy's local densities (Analysers/Source/Energy.cpp:137-143)
+        float* o = P.loc_energy + 6 * (size_t)s;
+        o[0] = (float)(pot_e + ge + ke + me + ee);
+        o[1] = (float)pot_e;
+        o[2] = (float)ge;
+        o[3] = (float)ke;
+        o[4] = (float)me;
+        o[5] = (float)ee;
+    }
+    obs[kObsPotential] += pot_e;
+    obs[kObsGradient] += ge;
+    obs[kObsKinetic] += ke;
+    obs[kObsMagnetic] += me;
+    obs[kObsElectric] += ee;
+    obs[kObsPlaqSU2] += (double)plaq2;
+    obs[kObsPlaqU1] += (double)plaq1;
+    obs[kObsPhiSq] += (double)phisq;
+}
+
 // The per-site update.  A provides q(d, R) -> Q<C>, th(d, R) -> C, ph(k, R) -> Q<C>
 // for the "now" level (and hth / hq for a 2HDM Higgs-family field, HF != 0).
 // obs receives the energy-step observables except the total (energy_total after
@@ -358,20 +476,8 @@ __device__ __forceinline__ void site_step(const StepParams& P, const KConst<S>& 
     const unsigned warn_in = warn;
     using C = S;  // FP64 form -> double, mixed form -> float
     constexpr int ND = (MODEL == kModelSM) ? 1 : 2;
-    // Own-site past level: on non-logging steps loaded here, so that the
-    // memory latency overlaps the force arithmetic below (the logging-step
-    // variant has no registers to spare and loads it where it is used).
-    Q<C> pst_f[ND], pst_u[3];
-    C pst_t[3];
-    if (!ENERGY) {
-#pragma unroll
-        for (int db = 0; db < ND; db++) pst_f[db] = ld4<C>(ps.L.ph[db], ps.s);
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-            pst_u[d] = ld4<C>(ps.L.q[d], ps.s);
-            pst_t[d] = ld1<C>(ps.L.th[d], ps.s);
-        }
-    }
+    PastValues<S, ND, LV, !ENERGY> past = {ps};
+    past.load();
     const C l[3] = {F.ldt[0], F.ldt[1], F.ldt[2]};  // dt^2 / dx_a^2
 
     Q<C> U[3];
@@ -657,72 +763,15 @@ __device__ __forceinline__ void site_step(const StepParams& P, const KConst<S>& 
         }
     }
 
-    // ---- scalar leapfrog (Model.cpp:347-356):
-    //      phi(t+dt) = phi + [(phi - phi_past)(1 - damping) + dt^2 (D - dV)], one rounding at the end
-    C kin_e = (C)0, phisq = (C)0;
+    C kin_e = (C)0, phisq = (C)0, elec_e = (C)0;
     C check = (C)0;  // sum of every new value: non-finite iff one of them is
     const C keep = F.keep;
 #pragma unroll
-    for (int db = 0; db < ND; db++) {
-        const Q<C> fpast = ENERGY ? ld4<C>(ps.L.ph[db], ps.s) : pst_f[db];
-        const C fn[4] = {fc[db].w, fc[db].x, fc[db].y, fc[db].z};
-        const C fo[4] = {fpast.w, fpast.x, fpast.y, fpast.z};
-        const C dd[4] = {D[db].w, D[db].x, D[db].y, D[db].z};
-        C out[4];
+    for (int db = 0; db < ND; db++)
+        leapfrog_doublet<ENERGY>(F, fc[db], past.ph(db), D[db], ps.L.ph[db], ps.s, kin_e, phisq, check);
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const C vel = fn[k] - fo[k];
-            out[k] = fn[k] + (keep * vel + dd[k]);
-            check += out[k];
-            if (ENERGY) {
-                kin_e += vel * vel;  // x 0.5 / dt^2 below
-                phisq += fn[k] * fn[k];
-            }
-        }
-        st4(ps.L.ph[db], ps.s, out[0], out[1], out[2], out[3]);
-    }
-
-    // ---- link update (WilsonLoops/Source/StandardModel.cpp:456-514) ----
-    // theta(t+dt) = theta(t) + asin(RHS_Y)
-    C elec_e = (C)0;
-    C R0[3], inc[3];
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-        const C dth = th[d] - (ENERGY ? ld1<C>(ps.L.th[d], ps.s) : pst_t[d]);
-        R0[d] = keep * gsin(dth) + (MgY[d] + F.cY * JY[d]);
-        if (ENERGY) {  // 1 - cos(dtheta) = 2 sin^2(dtheta/2)
-            const C h = gsin((C)0.5 * dth);
-            elec_e += F.e_elec[d] * (F.inv_gp_sqr * (C)2 * h * h);
-        }
-    }
-    warn_range(th, warn);
-    asin3(R0, inc, warn);
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-        const C thn = th[d] + inc[d];
-        check += thn;
-        ps.L.th[d][ps.s] = thn;
-    }
-    // u = (sqrt(1-|c|^2), c); U(t+dt) = normalise(u U(t)) (su2_advance3)
-    C W[3][3];
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-        const Q<C> Un = U[d];
-        const Q<C> Up = ENERGY ? ld4<C>(ps.L.q[d], ps.s) : pst_u[d];
-        // link momentum vec(U_now U_past^dag) = vec((U_now - U_past) U_past^dag)
-        const Q<C> dlt = {Un.w - Up.w, Un.x - Up.x, Un.y - Up.y, Un.z - Up.z};
-        C E1, E2, E3;
-        qmul_vec(dlt, qconj(Up), E1, E2, E3);
-        W[d][0] = keep * E1 + Mg[d][0];
-        W[d][1] = keep * E2 + Mg[d][1];
-        W[d][2] = keep * E3 + Mg[d][2];
-        if (ENERGY) {
-            // 1 - (U_now U_past^dag)_0 / |U_now U_past^dag|
-            const Q<C> Ed = {Un.w * Up.w + Un.x * Up.x + Un.y * Up.y + Un.z * Up.z, E1, E2, E3};
-            elec_e += F.e_elec[d] * (F.inv_g_sqr * one_minus_trace(Ed));
-        }
-    }
-    su2_advance3(U, W, ps.L.q, ps.s, warn, check);
+    for (int d = 0; d < 3; d++) MgY[d] += F.cY * JY[d];
+    leapfrog_links<ENERGY>(F, U, th, Mg, MgY, past, elec_e, warn, check);
 
     // Higgs-family links (WilsonLoops/Source/TwoHDM.cpp:601-633, 702-745), coupling g''
     if constexpr (HF == kHfU1) {
@@ -773,27 +822,7 @@ __device__ __forceinline__ void site_step(const StepParams& P, const KConst<S>& 
         return;
     }
 
-    if (ENERGY) {
-        const double ge = (double)grad_e, ke = 0.5 * P.inv_sqr_dt * (double)kin_e;
-        const double me = (double)mag_e, ee = (double)elec_e;
-        if (P.loc_energy) {  // Energy's local densities (Analysers/Source/Energy.cpp:137-143)
-            float* o = P.loc_energy + 6 * (size_t)ps.s;
-            o[0] = (float)(pot_e + ge + ke + me + ee);
-            o[1] = (float)pot_e;
-            o[2] = (float)ge;
-            o[3] = (float)ke;
-            o[4] = (float)me;
-            o[5] = (float)ee;
-        }
-        obs[kObsPotential] += pot_e;
-        obs[kObsGradient] += ge;
-        obs[kObsKinetic] += ke;
-        obs[kObsMagnetic] += me;
-        obs[kObsElectric] += ee;
-        obs[kObsPlaqSU2] += (double)plaq2;
-        obs[kObsPlaqU1] += (double)plaq1;
-        obs[kObsPhiSq] += (double)phisq;
-    }
+    if (ENERGY) record_energies(P, ps.s, pot_e, grad_e, kin_e, mag_e, elec_e, plaq2, plaq1, phisq, obs);
 }
 
 // Gauss-law residual at site c after a step (Analysers/Source/GaugeCondition.cpp:117-165,

@@ -15,26 +15,10 @@ namespace {
 
 using namespace tiled;
 
-// CTAs per SM the launch bounds ask for: as many as shared memory admits, at
-// most 512 threads per SM.  For the SM model in float with 8 x 32 or 16 x 16
-// tiles that is two, which caps registers at 128 per thread (the logging-step
-// variant would otherwise exceed it); where the staged planes admit one CTA
-// (FP64, the 2HDM model's two doublets) the registers are left uncapped.
-template <class S, int MODEL, int TY, int TZ>
-constexpr int tiled_min_blocks()
-{
-    using G = Geom<S, TY, TZ, (MODEL == kModelSM) ? 1 : 2>;
-    constexpr int by_smem = (228 * 1024) / (G::SMEM + 16 + 1024);
-    constexpr int by_threads = 512 / (TY * TZ);
-    constexpr int b = by_smem < by_threads ? by_smem : by_threads;
-    return b < 1 ? 1 : b;
-}
-
 template <class S, int MODEL, int TY, int TZ, bool ENERGY>
-__global__ void __launch_bounds__(TY * TZ, tiled_min_blocks<S, MODEL, TY, TZ>()) tiled_step_kernel(const __grid_constant__ TMaps maps,
-                                                             const __grid_constant__ TMaps pmaps, StepParams P,
-                                                             KConst<S> F, LevelPtrs<S> now, LevelPtrs<S> past, int lx,
-                                                             int xa, int xn, unsigned* status, double* partials)
+__global__ void __launch_bounds__(TY * TZ, tile_ctas<S, MODEL, TY, TZ>())
+    tiled_step_kernel(const __grid_constant__ TMaps maps, const __grid_constant__ TMaps pmaps, StepParams P, KConst<S> F,
+                      LevelPtrs<S> now, LevelPtrs<S> past, int lx, int xa, int xn, unsigned* status, double* partials)
 {
     constexpr int ND = (MODEL == kModelSM) ? 1 : 2;
     using G = Geom<S, TY, TZ, ND>;
@@ -58,10 +42,10 @@ __global__ void __launch_bounds__(TY * TZ, tiled_min_blocks<S, MODEL, TY, TZ>())
     unsigned warn = 0;
     RingPhase ring = {0u};
     const int x0 = xa + blockIdx.z * lx;  // planes [xa, xa + xn) in chunks of lx
-    constexpr bool STAGE = HaloStage<S, TY, TZ, ND>::use(ENERGY);
+    constexpr bool STAGE = tile_stage<S, MODEL, TY, TZ, ENERGY>();
     const bool ok = run_tile<S, MODEL, TY, TZ, ENERGY, LevelPtrs<S>, STAGE>(
         maps, pmaps, P, F, now, past, blockIdx.y * TY, blockIdx.x * TZ, x0, min(lx, xa + xn - x0), smem, bars, ring,
-        &s_abort, obs, warn, smem + HaloStage<S, TY, TZ, ND>::OFFSET);
+        &s_abort, obs, warn);
     if (!ok && tid == 0) atomicOr(status, kErrTimeout);
 
     if (ENERGY) {
@@ -138,7 +122,8 @@ __global__ void __launch_bounds__(TY * TZ / 2, 2) tiled_pair_kernel(const __grid
             const int x = x0 + i;
             const int sa = (x * P.ny + y) * P.nz + z;
             pair::site_step2(F, PairAcc<TY, TZ>{}, n, past, sa, sa + sb_off, carry, warn, counts(P, x));
-        });
+        },
+        [](int) {});
     if (!ok && tid == 0) atomicOr(status, kErrTimeout);
     if (warn) atomicOr(status, warn);
 }
@@ -225,7 +210,8 @@ __global__ void __launch_bounds__(2 * TY * TZ, 3) tiled_split_kernel(const __gri
                                   [&] { named_sync(pair_bar, 64); }, warn);
             }
             if (!counts(P, x)) warn = warn_in;  // ghost planes of an x-slab
-        });
+        },
+        [](int) {});
     if (!ok && tid == 0) atomicOr(status, kErrTimeout);
     if (warn) atomicOr(status, warn);
 }
@@ -297,10 +283,11 @@ bool tiled_supported(const StepParams& P, int variant)
 int tiled_ctas_per_sm(int variant, bool fp64)
 {
     switch (variant) {
-    case 0: return fp64 ? tiled_min_blocks<double, kModelSM, 8, 32>() : tiled_min_blocks<float, kModelSM, 8, 32>();
-    case 1: return fp64 ? tiled_min_blocks<double, kModelSM, 4, 32>() : tiled_min_blocks<float, kModelSM, 4, 32>();
-    case 2: return fp64 ? tiled_min_blocks<double, kModelSM, 4, 16>() : tiled_min_blocks<float, kModelSM, 4, 16>();
-    default: return fp64 ? tiled_min_blocks<double, kModelSM, 16, 16>() : tiled_min_blocks<float, kModelSM, 16, 16>();
+    case 0: return fp64 ? tile_ctas<double, kModelSM, 8, 32>() : tile_ctas<float, kModelSM, 8, 32>();
+    case 1: return fp64 ? tile_ctas<double, kModelSM, 4, 32>() : tile_ctas<float, kModelSM, 4, 32>();
+    case 2: return fp64 ? tile_ctas<double, kModelSM, 4, 16>() : tile_ctas<float, kModelSM, 4, 16>();
+    case kTileFP64: return tile_ctas<double, kModelSM, 8, 16>();
+    default: return fp64 ? tile_ctas<double, kModelSM, 16, 16>() : tile_ctas<float, kModelSM, 16, 16>();
     }
 }
 
@@ -316,20 +303,17 @@ static cudaError_t launch_tiled_t(const TMaps& maps, const TMaps& pmaps, const S
                                   const LevelPtrs<S>& past, int lx, int xa, int xn, unsigned* status, double* partials,
                                   bool energy, cudaStream_t stream)
 {
-    constexpr int ND = (MODEL == kModelSM) ? 1 : 2;
-    using G = Geom<S, TY, TZ, ND>;
-    using H = HaloStage<S, TY, TZ, ND>;
     const dim3 block(TZ, TY, 1);
     const dim3 grid(P.nz / TZ, P.ny / TY, (xn + lx - 1) / lx);
     // both step kinds stage their wrapped halo cells where that costs no resident CTA (logging step,
     // us at SM 256^3 / 2HDM 192^3: 1187 / 715 loading them after the plane's wait, 1161 / 687 staged)
     if (energy) {
-        constexpr int SMEM = H::use(true) ? H::SMEM : G::SMEM;
+        constexpr int SMEM = tile_smem<S, MODEL, TY, TZ, true>();
         auto k = tiled_step_kernel<S, MODEL, TY, TZ, true>;
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
         k<<<grid, block, SMEM, stream>>>(maps, pmaps, P, make_kconst<S>(P), now, past, lx, xa, xn, status, partials);
     } else {
-        constexpr int SMEM = H::use(false) ? H::SMEM : G::SMEM;
+        constexpr int SMEM = tile_smem<S, MODEL, TY, TZ, false>();
         auto k = tiled_step_kernel<S, MODEL, TY, TZ, false>;
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
         k<<<grid, block, SMEM, stream>>>(maps, pmaps, P, make_kconst<S>(P), now, past, lx, xa, xn, status, partials);
@@ -343,6 +327,10 @@ cudaError_t launch_tiled_step(const TMaps& maps, const TMaps& pmaps, const StepP
                               bool energy, cudaStream_t stream, int xa, int xn)
 {
     if (xn < 0) xn = P.nx - xa;  // default: every plane from xa on
+    if constexpr (sizeof(S) == 8) {
+        if (variant == kTileFP64)
+            return launch_tiled_t<S, MODEL, 8, 16>(maps, pmaps, P, now, past, lx, xa, xn, status, partials, energy, stream);
+    }
     switch (variant) {
     case 0: return launch_tiled_t<S, MODEL, 8, 32>(maps, pmaps, P, now, past, lx, xa, xn, status, partials, energy, stream);
     case 1: return launch_tiled_t<S, MODEL, 4, 32>(maps, pmaps, P, now, past, lx, xa, xn, status, partials, energy, stream);

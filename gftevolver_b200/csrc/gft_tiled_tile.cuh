@@ -25,6 +25,7 @@
 
 #include "gft_device.cuh"
 #include "gft_launch.h"
+#include "gft_shared_body.cuh"
 #include "gft_step_body.cuh"
 
 namespace gft {
@@ -76,15 +77,6 @@ __device__ __forceinline__ bool mbar_test_wait(unsigned long long* bar, unsigned
         : "r"(smem_u32(bar)), "r"(parity)
         : "memory");
     return ok != 0;
-}
-
-// Shared-memory counter add with acquire-release semantics at CTA scope:
-// returns the previous value.
-__device__ __forceinline__ unsigned atom_add_acq_rel(unsigned* p, unsigned v)
-{
-    unsigned old;
-    asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(smem_u32(p)), "r"(v) : "memory");
-    return old;
 }
 
 constexpr unsigned long long kWaitLimitNs = 2000000000ull;  // 2 s
@@ -175,6 +167,37 @@ struct HaloStage {
         return sizeof(S) == 4 && SMEM <= 227 * 1024 - 16 && per_sm(SMEM, energy) >= per_sm(G::SMEM, energy);
     }
     static constexpr bool kUse = use(false);
+};
+
+template <class S, int TY, int TZ, int ND>
+struct TileAcc;
+
+// The buffers of the values handed from site to site within a tile (gft_shared_body.cuh; SM
+// model), after the halo stage: for the y neighbours, slot y - y0 of the receiving row; for the
+// z neighbours, the receiving row of the tile's first column.  Two planes of each: a plane's are
+// read after its barrier, while faster warps write the next plane's.
+template <class S, int TY, int TZ>
+struct HandBuf {
+    using H = HaloStage<S, TY, TZ, 1>;
+    static constexpr int QUAD = 4 * (int)sizeof(S);
+    static constexpr int YB = 3 * TY * TZ * QUAD, ZB = 3 * TY * QUAD;  // one plane's
+    static constexpr int BYTES = 2 * (YB + ZB);
+    static constexpr int OFFSET = (H::OFFSET + (sizeof(S) == 4 ? H::BYTES : 0) + 15) / 16 * 16;
+    static constexpr int SMEM = OFFSET + BYTES + 128;  // + alignment slack of the dynamic base
+
+    __device__ __forceinline__ static void put(unsigned char* b, int n, int i, const Handed<S>& h)
+    {
+        S* p = reinterpret_cast<S*>(b);
+        st4(p, i, h.fa[0], h.fa[1], h.fa[2], h.sa);
+        st4(p, n + i, h.fb[0], h.fb[1], h.fb[2], h.sb);
+        st4(p, 2 * n + i, h.t.w, h.t.x, h.t.y, h.t.z);
+    }
+    __device__ __forceinline__ static Handed<S> get(const unsigned char* b, int n, int i)
+    {
+        using A = TileAcc<S, TY, TZ, 1>;
+        const Q<S> a = A::lds4(b, i), c = A::lds4(b, n + i);
+        return {{a.w, a.x, a.y}, a.z, {c.w, c.x, c.y}, c.z, A::lds4(b, 2 * n + i)};
+    }
 };
 
 // Reference to a site in a staged plane: buffer base, q/phi cell, theta cell.
@@ -356,7 +379,8 @@ struct RingPhase {
 // The plane ring of one tile (planes x0 .. x0+nloc-1 of columns y0.., z0..):
 // TMA copies, waits, wrapped-halo patches and one CTA barrier per plane.
 // body(i, bm, bc, bp) evolves the tile's sites of plane x0 + i from the staged
-// planes bc (x) and bp (x + 1), and with BACK also bm (x - 1).  Without BACK,
+// planes bc (x) and bp (x + 1), and with BACK also bm (x - 1); close(i) follows the
+// plane's barrier and reads none of them.  Without BACK,
 // start(bc, bp) is called first, on the planes x0 - 1 and x0: what the first sites
 // need of the plane before them.  tid: the thread's index in the CTA
 // (the halo cells and the copy issue are divided by it).  smem: NBUF plane
@@ -367,11 +391,12 @@ struct RingPhase {
 // STAGE: the wrapped halo cells of plane i+4 are copied by cp.async into
 // `stage` (HaloStage) while plane i+1 is computed, instead of prefetched into L2
 // and loaded after the plane's wait.
-template <class S, int TY, int TZ, int ND, class LV, bool STAGE, bool BACK, class Start, class Body>
+template <class S, int TY, int TZ, int ND, class LV, bool STAGE, bool BACK, class Start, class Body, class Close>
 __device__ __forceinline__ bool run_ring(const TMaps& maps, const TMaps& pmaps, const StepParams& P, const LV& now,
                                          int y0, int z0, int x0, int nloc, unsigned char* smem,
                                          unsigned long long* bars, RingPhase& ring, int* s_abort,
-                                         unsigned char* stage, int tid, Start&& start, Body&& body)
+                                         unsigned char* stage, int tid, Start&& start, Body&& body,
+                                         Close&& close)
 {
     using G = Geom<S, TY, TZ, ND, BACK ? 4 : 3>;
     // the plane whose buffer is free once plane i has been computed: i + FREE (relative planes)
@@ -388,24 +413,8 @@ __device__ __forceinline__ bool run_ring(const TMaps& maps, const TMaps& pmaps, 
     auto issue = [&](int p) {
         issue_plane<S, TY, TZ, ND>(maps, smem + slot(p) * G::BUF, &bars[slot(p)], plane_x(p), y0, z0);
     };
-    // Tiles without wrapped halo cells in the FP64 form march without a CTA
-    // barrier per plane (below): its warps wait on long FP64 latencies, and the
-    // FP64 step (one CTA of 8 warps per SM) measured 2 % faster at 256^3.  The
-    // FP32 steps keep the barrier: without it the SM step (two CTAs per SM) was
-    // 3 % slower at 256^3 and the 2HDM step (one CTA per SM) 4 % slower at
-    // 192^3, their warps waiting on copies and past-level loads instead.
-    constexpr bool kFree = sizeof(S) == 8;
-    // After the barriers: per buffer, the warps that are done with the plane in
-    // it (tiles without wrapped halo); then the number of planes issued.
-    unsigned* ctr = reinterpret_cast<unsigned*>(bars + G::NBUF);
-    const unsigned nwarps = (blockDim.x * blockDim.y * blockDim.z) >> 5;
-
     if (tid == 0) {
         for (int p = 0; p < min(G::NBUF, nplanes); p++) issue(p);
-        if constexpr (kFree) {
-            for (int b = 0; b < G::NBUF; b++) ctr[b] = 0u;
-            ctr[G::NBUF] = (unsigned)min(G::NBUF, nplanes);
-        }
     }
     if (tid == 32 % (TY * TZ)) {
         // past level of the first two planes computed (relative planes 1 and 2)
@@ -434,40 +443,17 @@ __device__ __forceinline__ bool run_ring(const TMaps& maps, const TMaps& pmaps, 
         if (!aborted) {
             start(smem, smem + G::BUF);
             __syncthreads();  // plane 0's buffer is free
-            if (tid == 0 && G::NBUF < nplanes) {
-                issue(G::NBUF);
-                if constexpr (kFree) ctr[G::NBUF] = (unsigned)(G::NBUF + 1);
-            }
+            if (tid == 0 && G::NBUF < nplanes) issue(G::NBUF);
         }
     }
 
-    // Tiles with wrapped halo cells: one CTA barrier per plane: after computing
-    // plane i the threads wait for (and patch) plane i+3, which the next site
-    // needs, then synchronise once; that barrier both publishes the patches and
-    // frees a plane's buffer for the next copy.
+    // One CTA barrier per plane: after computing plane i the threads wait for (and patch)
+    // plane i+3, which the next site needs, then synchronise once; that barrier publishes
+    // the patches and what the sites hand over, and frees a plane's buffer for the next copy.
     for (int i = 0; i < nloc && !aborted; i++) {
         body(i, smem + slot(i) * G::BUF, smem + slot(i + 1) * G::BUF, smem + slot(i + 2) * G::BUF);
 
         const int nxt = i + FREE + G::NBUF;  // the plane copied into the buffer freed by this one
-        if (kFree && !wraps) {
-            // No patches to publish: the buffer is free once every warp has
-            // computed plane i, and the last warp to finish it issues the next copy
-            // there (release by each warp's count, acquire by the last),
-            // so a warp waits only for the copy of the plane it needs next and may
-            // run up to a plane ahead of the slowest.
-            __syncwarp();
-            if ((tid & 31) == 0 && nxt < nplanes && atom_add_acq_rel(&ctr[slot(nxt)], 1u) % nwarps == nwarps - 1) {
-                issue(nxt);
-                *reinterpret_cast<volatile unsigned*>(&ctr[G::NBUF]) = (unsigned)(nxt + 1);
-            }
-            if (tid == 32 % (TY * TZ) && i + 3 <= nloc) prefetch_past<ND>(pmaps, plane_x(i + 3), y0, z0);
-            if (i + 3 < nplanes && !mbar_wait_bounded(&bars[slot(i + 3)], parity(i + 3), P.wait_limit_ns))
-                *reinterpret_cast<volatile int*>(s_abort) = 1;
-            // leave the march warp by warp (the next __syncwarp needs every lane)
-            if (__any_sync(0xffffffffu, *reinterpret_cast<volatile int*>(s_abort) != 0)) break;
-            continue;
-        }
-
         // plane i+3 (x+2) for the next site; its copy was issued one plane ago
         bool okn = true;
         if (i + 3 < nplanes) {
@@ -496,18 +482,9 @@ __device__ __forceinline__ bool run_ring(const TMaps& maps, const TMaps& pmaps, 
                 prefetch_wrapped_halo<S, TY, TZ, ND>(P, now, plane_x(i + 4), y0, z0, tid);
         }
         if (tid == 0 && nxt < nplanes) issue(nxt);
+        close(i);
     }
     if constexpr (STAGE) cp_async_wait_all();  // a staged plane not patched (abort) is still in flight
-    if (kFree && !wraps) {
-        // every warp is done with the ring (the next tile refills it); on a failed
-        // wait, the copies of the last NBUF planes issued may still be in flight
-        __syncthreads();
-        aborted = *reinterpret_cast<volatile int*>(s_abort) != 0;
-        if (aborted) {  // no next tile then
-            drain1 = (int)*reinterpret_cast<volatile unsigned*>(&ctr[G::NBUF]);
-            drain0 = max(0, drain1 - G::NBUF);
-        }
-    }
     if (aborted) {
         // drain: wait (bounded) for the copies still in flight into this CTA's buffers
         if (tid == 0)
@@ -548,11 +525,11 @@ template <class S, int MODEL, int TY, int TZ, bool ENERGY, class LV, bool STAGE 
 __device__ __forceinline__ bool run_tile(const TMaps& maps, const TMaps& pmaps, const StepParams& P, const KConst<S>& F,
                                          const LV& now, const LV& past, int y0, int z0, int x0,
                                          int nloc, unsigned char* smem, unsigned long long* bars, RingPhase& ring,
-                                         int* s_abort, double (&obs)[kObsCount], unsigned& warn,
-                                         unsigned char* stage = nullptr)
+                                         int* s_abort, double (&obs)[kObsCount], unsigned& warn)
 {
     constexpr int ND = (MODEL == kModelSM) ? 1 : 2;
     using G = Geom<S, TY, TZ, ND>;
+    using Acc = TileAcc<S, TY, TZ, ND>;
     const int tz = threadIdx.x, ty = threadIdx.y;
     const int tid = ty * TZ + tz;
     // own cells
@@ -564,22 +541,111 @@ __device__ __forceinline__ bool run_tile(const TMaps& maps, const TMaps& pmaps, 
     // Fixed y and z faces freeze whole columns, Fixed x faces the ends of a march
     const bool column_frozen = ((P.fixed_axes & 2) && (y == 0 || y == P.ny - 1)) ||
                                ((P.fixed_axes & 4) && (z == 0 || z == P.nz - 1));
-    return run_ring<S, TY, TZ, ND, LV, STAGE, false>(
-        maps, pmaps, P, now, y0, z0, x0, nloc, smem, bars, ring, s_abort, stage, tid,
-        [&](const unsigned char* bc, const unsigned char* bp) {
-            site_carry<S, ND>(TileAcc<S, TY, TZ, ND>{}, plane_stencil<G::QP, G::HP>(bc, bc, bp, cq0, ch0), carry);
-        },
-        [&](int i, const unsigned char*, const unsigned char* bc, const unsigned char* bp) {
-            const Stencil<TRef> n = plane_stencil<G::QP, G::HP>(bc, bc, bp, cq0, ch0);
-            const int x = x0 + i;
-            const int s = (x * P.ny + y) * P.nz + z;
-            if (column_frozen) return;
-            if ((P.fixed_axes & 1) && (x == 0 || x == P.nx - 1))
-                site_carry<S, ND>(TileAcc<S, TY, TZ, ND>{}, n, carry);  // not evolved; the next site needs its loops
-            else
-                site_step<S, MODEL, ENERGY, kHfNone, true>(P, F, TileAcc<S, TY, TZ, ND>{}, n,
-                                                           PastSite<S, LV>{past, s}, carry, obs, warn, counts(P, x));
-        });
+    auto frozen_at = [&](int x) { return column_frozen || ((P.fixed_axes & 1) && (x == 0 || x == P.nx - 1)); };
+    auto site = [&](int x) { return (x * P.ny + y) * P.nz + z; };
+    auto start = [&](const unsigned char* bc, const unsigned char* bp) {
+        site_carry<S, ND>(Acc{}, plane_stencil<G::QP, G::HP>(bc, bc, bp, cq0, ch0), carry);
+    };
+    unsigned char* stage = smem + HaloStage<S, TY, TZ, ND>::OFFSET;
+    if constexpr (MODEL == kModelSM) {
+        using HB = HandBuf<S, TY, TZ>;
+        OpenSite<S> o;
+        PastValues<S, 1, LV, !ENERGY> pv = {{past, 0}};
+        auto ybuf = [&](int i) { return smem + HB::OFFSET + (i & 1) * HB::YB; };
+        auto zbuf = [&](int i) { return smem + HB::OFFSET + 2 * HB::YB + (i & 1) * HB::ZB; };
+        constexpr int NW = TY * TZ / 32;  // warps of the tile
+        return run_ring<S, TY, TZ, ND, LV, STAGE, false>(
+            maps, pmaps, P, now, y0, z0, x0, nloc, smem, bars, ring, s_abort, stage, tid, start,
+            [&](int i, const unsigned char*, const unsigned char* bc, const unsigned char* bp) {
+                {   // the halo row's and column's lanes, on warps that change with the plane
+                    const int h = (((tid >> 5) + i) % NW) * 32 + (tid & 31);
+                    if (h < TZ + TY) {
+                        const bool row = h < TZ;
+                        const int ly = row ? 0 : h - TZ + 1, lz = row ? h + 1 : 0;
+                        const int cq = ly * G::QP + lz, ch = ly * G::HP + lz + G::TP - 1;
+                        Handed<S> hh;
+                        halo_hand_over<S>(Acc{}, row ? 1 : 2, TRef{bc, cq, ch}, TRef{bp, cq, ch},
+                                          TRef{bc, cq + G::QP, ch + G::HP}, TRef{bc, cq + 1, ch + 1}, hh);
+                        if (row)
+                            HB::put(ybuf(i), TY * TZ, h, hh);
+                        else
+                            HB::put(zbuf(i), TY, h - TZ, hh);
+                    }
+                }
+                Handed<S> hy, hz;
+                site_open<S, ENERGY>(P, F, Acc{}, plane_stencil<G::QP, G::HP>(bc, bc, bp, cq0, ch0), carry, o, hy, hz);
+                if (ty + 1 < TY) HB::put(ybuf(i), TY * TZ, tid + TZ, hy);
+                // the z neighbour's, from the lane below; the first column's come through shared memory
+                const S lz = tz == 0 ? (S)0 : F.ldt[2];
+                Handed<S> hv;
+                auto up = [](S v) { return __shfl_up_sync(0xffffffffu, v, 1, TZ < 32 ? TZ : 32); };
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    hv.fa[k] = up(hz.fa[k]);
+                    hv.fb[k] = up(hz.fb[k]);
+                }
+                hv.sa = up(hz.sa);
+                hv.sb = up(hz.sb);
+                hv.t = {up(hz.t.w), up(hz.t.x), up(hz.t.y), up(hz.t.z)};
+                receive(o, 0, 1, lz, hv);
+                pv.at.s = site(x0 + i);
+                if (!frozen_at(x0 + i)) pv.load();
+            },
+            [&](int i) {
+                const int x = x0 + i;
+                if (frozen_at(x)) return;
+                receive(o, 0, 2, F.ldt[1], HB::get(ybuf(i), TY * TZ, tid));
+                if (tz == 0) receive(o, 0, 1, F.ldt[2], HB::get(zbuf(i), TY, ty));
+                site_close<S, ENERGY>(P, F, o, pv, obs, warn, counts(P, x));
+            });
+    } else {
+        return run_ring<S, TY, TZ, ND, LV, STAGE, false>(
+            maps, pmaps, P, now, y0, z0, x0, nloc, smem, bars, ring, s_abort, stage, tid, start,
+            [&](int i, const unsigned char*, const unsigned char* bc, const unsigned char* bp) {
+                const Stencil<TRef> n = plane_stencil<G::QP, G::HP>(bc, bc, bp, cq0, ch0);
+                const int x = x0 + i;
+                if (column_frozen) return;
+                if (frozen_at(x))
+                    site_carry<S, ND>(Acc{}, n, carry);  // not evolved; the next site needs its loops
+                else
+                    site_step<S, MODEL, ENERGY, kHfNone, true>(P, F, Acc{}, n, PastSite<S, LV>{past, site(x)}, carry,
+                                                               obs, warn, counts(P, x));
+            },
+            [](int) {});
+    }
+}
+
+// Whether a step stages its wrapped halo cells (HaloStage; the SM tile's shared memory has the room).
+template <class S, int MODEL, int TY, int TZ, bool ENERGY>
+constexpr bool tile_stage()
+{
+    if constexpr (MODEL == kModelSM)
+        return sizeof(S) == 4;
+    else
+        return HaloStage<S, TY, TZ, 2>::use(ENERGY);
+}
+
+// Dynamic shared memory of a one-site tile kernel.
+template <class S, int MODEL, int TY, int TZ, bool ENERGY>
+constexpr int tile_smem()
+{
+    if constexpr (MODEL == kModelSM) {
+        static_assert(HandBuf<S, TY, TZ>::SMEM <= 227 * 1024 - 16 - 32 * kObsCount * 8, "shared memory of a tile");
+        return HandBuf<S, TY, TZ>::SMEM;
+    } else {
+        return tile_stage<S, MODEL, TY, TZ, ENERGY>() ? HaloStage<S, TY, TZ, 2>::SMEM : Geom<S, TY, TZ, 2>::SMEM;
+    }
+}
+
+// Resident CTAs per SM that shared memory admits, at most 512 threads: 228 KB per SM, 1 KB
+// reserved per CTA, the logging steps' reduction rows.
+template <class S, int MODEL, int TY, int TZ>
+constexpr int tile_ctas()
+{
+    constexpr int smem = tile_smem<S, MODEL, TY, TZ, true>() + 16 + 32 * kObsCount * 8 + 1024;
+    constexpr int by_smem = (228 * 1024) / smem, by_threads = 512 / (TY * TZ);
+    constexpr int b = by_smem < by_threads ? by_smem : by_threads;
+    return b < 1 ? 1 : b;
 }
 
 }  // namespace tiled

@@ -34,3 +34,28 @@ def test_march_ends_match_oracle(oracle_mod, form, model, nx, march, fixed):
     for a, b in ((g_sc, sc), (g_ve, ve)):
         err = np.max(np.abs(a.astype(np.float64) - b))
         assert err <= (1e-12 * np.max(np.abs(b)) if form == "fp64" else 6e-6)
+
+
+@pytest.mark.parametrize("fixed", [0, 7], ids=["periodic", "fixed"])
+def test_fp64_default_tile_matches_one_thread_per_site(fixed):
+    """The FP64 step's own 8 x 16 tile, which only the automatic choice takes, on a lattice thin in x
+    with enough tiles for it, against the oracle-pinned one-thread-per-site step: every loop and
+    transport that sites hand over within a tile, across its halo row and column and over the wrap.
+    Bar: 1e-12 of the fields after 5 steps, the rows within 1e-12 of the total energy."""
+    from gftevolver_b200 import Evolver, InitialData, LatticeParams
+    p = LatticeParams(model=1, nx=3, ny=384, nz=512, energy_every=2, gauss_every=2, fixed_axes=fixed)
+    ic = InitialData(seed=5, mean=[1.0] * 8, sigma=[0.1] * 8, theta_sigma=0.1, eps_sigma=0.1)
+    out = []
+    for kind in (0, 1):
+        with Evolver(p, form="fp64") as ev:
+            if kind:
+                ev.set_kernel(kind, 0, 32)
+            assert ev.step_kernel_name == ("fast_step_kernel" if kind else "tiled_step_kernel")
+            ev.init_fields(ic)
+            rows = ev.evolve(5)
+            out.append((*ev.download(), rows))
+    for a, b in zip(out[0][:2], out[1][:2]):
+        assert np.max(np.abs(a - b)) <= 1e-12 * np.max(np.abs(b))
+    for a, b in zip(out[0][2], out[1][2]):
+        for k in ("energy", "potential", "gradient", "kinetic", "magnetic", "electric"):
+            assert abs(a[k] - b[k]) <= 1e-12 * abs(b["energy"]), k
