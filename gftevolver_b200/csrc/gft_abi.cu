@@ -89,7 +89,7 @@ struct gft_handle {
                             // sites per thread on plain steps (SM), 4 tiled with each site split
                             // between two threads on plain steps (SM)
     int tile_variant = 0;   // tiled: index into the built tile shapes
-    int march = 32;         // tiled: planes per CTA along x
+    int march = 32;         // tiled: planes per CTA along x (gft_create sets the form's)
     unsigned wait_limit_ns = 0;  // gft_set_wait_limit (0: the 2 s default)
     bool tiled_ready = false;
     TMaps tm[2];   // staged "now" planes (with halo), per level
@@ -292,32 +292,33 @@ bool encode_tiled(const gft_handle* h, const StepParams& P, int tile, TMaps* tm,
     return true;
 }
 
-// Automatic choice (kernel_kind 0), from B200 measurements at 192^3-448^3: the
-// tiled kernel for SM (46 % of HBM against 42 % for one thread per site);
-// one thread per site for 2HDM, whose four staged plane buffers (two doublets)
-// need 130 KB of shared memory and leave one CTA per SM (30 % against 45 %).
-// The automatic choice (kernel kind 0) takes the staged step for the SM model
-// when its tiles fill enough waves of resident CTAs: fewer tiles leave SMs idle
-// while each CTA marches its planes, and one thread per site is faster there
-// (mixed form at 32^3: 14x, 64^3 (0.11 waves): 3.6x; 128^3 (0.86 waves): the
-// staged step 2 % faster, 192^3 (2.9 waves): 15 %.  FP64, one CTA per SM: one
-// thread per site 11 % faster at 128^3 (1.7 waves) and 7.5 % at 160^3 (3.4
-// waves); the staged step 1.6 % faster at 192^3 (5.8 waves) and 7 % at 256^3
-// (13.8 waves)).
-constexpr double kAutoWavesMixed = 0.8, kAutoWavesFP64 = 5.0;
+// Automatic choice (kernel_kind 0): the staged step when its tiles fill enough waves of
+// resident CTAs (fewer leave SMs idle while each CTA marches its planes), else one thread per
+// site.  us per plain step on a B200, staged (the march below) / one thread per site:
+//   SM mixed:   64^3 (0.3 waves) 34 / 21, 96^3 (0.97) 58 / 62, 128^3 (2.4) 133 / 136, 160^3 224 /
+//               257, 192^3 (8) 376 / 439; logging steps 71 / 86 and 170 / 195 at 96^3 and 128^3;
+//   2HDM mixed: 128^3 (2.4 waves) 175 / 163, 144^3 (3.3) 239 / 259, 160^3 (4.7) 303 / 317, 192^3
+//               (8) 512 / 546, logging 659 / 736;
+//   FP64 SM:    128^3 (1.7 waves) 301 / 287, 192^3 (5.8) 823 / 993, 256^3 (13.8) 1936 / 2290.
+constexpr double kAutoWavesSM = 0.9, kAutoWaves2HDM = 3.0, kAutoWavesFP64 = 5.0;
+// Planes per CTA unless the caller sets them.  Mixed form: short enough to balance the last
+// wave, long enough for the start of a march (two more planes staged) not to count: SM 128^3 /
+// 192^3 / 256^3 at 8, 12, 16, 32 planes 133 / 377 / 849, 133 / 376 / 830, 135 / 372 / 857,
+// 135 / 375 / 837 us; 96^3 58 at 12, 72 to 95 at the others.
+constexpr int kAutoMarchMixed = 12, kAutoMarchFP64 = 32;
 
 bool use_tiled(const gft_handle* h, const StepParams& P)
 {
     if (!h->tiled_ready || h->kernel_kind == 1 || h->hf != kHfNone) return false;
-    const bool fp64 = h->cfg.form == GFT_FORM_FP64;
+    const bool fp64 = h->cfg.form == GFT_FORM_FP64, sm = h->cfg.model == GFT_MODEL_SM;
     // the FP64 form: the staged SM step only (kinds 0 and 2)
-    if (fp64 && (h->cfg.model != GFT_MODEL_SM || h->kernel_kind > 2)) return false;
+    if (fp64 && (!sm || h->kernel_kind > 2)) return false;
     if (h->cfg.form != GFT_FORM_MIXED && !fp64) return false;
     if (!tiled_supported(P, h->tile_variant)) return false;
     if (h->kernel_kind != 0) return true;
-    if (h->cfg.model != GFT_MODEL_SM) return false;
-    const long long slots = (long long)h->nsm * tiled_ctas_per_sm(h->tile_variant, fp64);
-    return tiled_blocks(P, h->tile_variant, h->march) >= (fp64 ? kAutoWavesFP64 : kAutoWavesMixed) * (double)slots;
+    const double slots = (double)h->nsm * tiled_ctas_per_sm(h->tile_variant, fp64, sm);
+    return tiled_blocks(P, h->tile_variant, h->march) >=
+           (fp64 ? kAutoWavesFP64 : (sm ? kAutoWavesSM : kAutoWaves2HDM)) * slots;
 }
 
 // Plain steps of the SM mixed form with two sites per thread (kernel kind 3):
@@ -524,6 +525,7 @@ int gft_create(const gft_config* cfg, gft_handle** out)
             carve<double>(h->level_mem[t], h->nsite, h->nsc, h->ld[t], h->hf);
     }
     const StepParams P = make_params(h, 0, false);
+    h->march = cfg->form == GFT_FORM_FP64 ? kAutoMarchFP64 : kAutoMarchMixed;
     if (cfg->form == GFT_FORM_MIXED || (cfg->form == GFT_FORM_FP64 && cfg->model == GFT_MODEL_SM)) {
         // default tile: the largest built shape the lattice divides
         h->tile_variant = 0;

@@ -374,7 +374,7 @@ struct gft_batch {
     std::vector<std::array<LevelPtrs<float>, 2>> lv;
     EnsMaps* d_maps = nullptr;
     int variant = -1;
-    int lx = 32;
+    int lx = 24;  // 16 x 16 tiles, march 16 / 24 / 32 / 64: 405 / 397 / 405 / 441 us per step as below
     int4* d_items = nullptr;
     int nitems = 0;
     int* d_order = nullptr;       // per-CTA tile lists of each group (group-local item indices)
@@ -821,8 +821,11 @@ int gft_batch_create(const gft_config* cfgs, int n, gft_batch** out)
     b->nve = 3 * (5 + (b->hf == kHfSU2 ? 4 : (b->hf == kHfU1 ? 1 : 0)));
     b->neq = config_neq(cfgs[0]);
     b->cfg.assign(cfgs, cfgs + n);
-    for (int v = 0; v < kTiledVariants && b->variant < 0; v++)
-        if (variant_fits(b, v)) b->variant = v;
+    // 256-thread tiles before the smaller ones: a small tile's halo row and column are a larger part
+    // of its work (32 members of 32 to 96 planes an edge, us per step at march 24: 16 x 16 397, 4 x 16
+    // 595; 12 of 32 and 64: 8 x 32 123, 16 x 16 117, 4 x 32 110, 4 x 16 143)
+    for (const int v : {0, 3, 1, 2})
+        if (b->variant < 0 && variant_fits(b, v)) b->variant = v;
     if (b->variant < 0 && b->hf == kHfNone) {
         delete b;
         set_error("gft_batch_create: the members' (ny, nz) share no built tile shape (4 x 16, the smallest, needs ny % 4 == 0 and nz % 16 == 0)");
@@ -882,7 +885,7 @@ int gft_batch_create(const gft_config* cfgs, int n, gft_batch** out)
         *out = b;
         return GFT_OK;
     }
-    int rc = configure(b, b->variant, 32);
+    int rc = configure(b, b->variant, b->lx);
     if (rc != GFT_OK) {
         gft_batch_destroy(b);
         return rc;

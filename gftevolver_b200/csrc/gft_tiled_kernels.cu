@@ -280,14 +280,21 @@ bool tiled_supported(const StepParams& P, int variant)
     return encode_fn() != nullptr && P.nz % tz == 0 && P.ny % ty == 0 && P.nx >= 1;
 }
 
-int tiled_ctas_per_sm(int variant, bool fp64)
+template <int TY, int TZ>
+static int ctas_of(bool fp64, bool sm)
+{
+    if (fp64) return tile_ctas<double, kModelSM, TY, TZ>();
+    return sm ? tile_ctas<float, kModelSM, TY, TZ>() : tile_ctas<float, kModel2HDM, TY, TZ>();
+}
+
+int tiled_ctas_per_sm(int variant, bool fp64, bool sm)
 {
     switch (variant) {
-    case 0: return fp64 ? tile_ctas<double, kModelSM, 8, 32>() : tile_ctas<float, kModelSM, 8, 32>();
-    case 1: return fp64 ? tile_ctas<double, kModelSM, 4, 32>() : tile_ctas<float, kModelSM, 4, 32>();
-    case 2: return fp64 ? tile_ctas<double, kModelSM, 4, 16>() : tile_ctas<float, kModelSM, 4, 16>();
+    case 0: return ctas_of<8, 32>(fp64, sm);
+    case 1: return ctas_of<4, 32>(fp64, sm);
+    case 2: return ctas_of<4, 16>(fp64, sm);
     case kTileFP64: return tile_ctas<double, kModelSM, 8, 16>();
-    default: return fp64 ? tile_ctas<double, kModelSM, 16, 16>() : tile_ctas<float, kModelSM, 16, 16>();
+    default: return ctas_of<16, 16>(fp64, sm);
     }
 }
 
