@@ -27,6 +27,7 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler",
 SOURCES = [
     ("gft_ref_kernels.cu", ["-fmad=false"]),
     ("gft_fast_kernels.cu", []),
+    ("gft_role_kernels.cu", []),
     ("gft_tiled_kernels.cu", []),
     ("gft_aux_kernels.cu", []),
     ("gft_static_observe.cu", []),

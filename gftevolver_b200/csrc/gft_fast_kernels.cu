@@ -43,19 +43,72 @@ struct GlobalAcc {
     __device__ __forceinline__ Q<S> hq(int d, int s) const { return ld4<S>(L.hq[d], s); }
 };
 
-// One thread per site; the kernel below instantiates it with its launch bounds.
-template <class S, int MODEL, int HF, bool ENERGY>
-__device__ __forceinline__ void fast_step_body(StepParams P, KConst<S> F, LevelPtrs<S> now, LevelPtrs<S> past,
-                                               unsigned* status, double* partials)
+constexpr int kStepThreads = 128;
+constexpr int kGaussThreads = 256;  // 32 x 8: 2 % faster than 32 x 4 at 256^3 (624 against 638 us)
+
+// The (z, y) patch of sites a block of T threads covers: bz x by of them, bz * by <= T, thread t at
+// column t % bz, row t / bz.  32 x T/32 wherever z divides into 32; elsewhere the shape that leaves the
+// fewest threads without a site (75 sites along z in three blocks of 32 idle a fifth of them: SM
+// mixed 150 x 100 x 75 in patches of 25 x 5 92 -> 80 us per step, 100^3 84 -> 72).
+struct Patch {
+    int bz, by;
+    int inv;  // t / bz = t * inv >> 16, exact for t < 1024 and bz <= 64
+};
+
+Patch pick_patch(const StepParams& P, int threads)
 {
-    const int z = blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = blockIdx.y * blockDim.y + threadIdx.y;
-    const int x = blockIdx.z;
+    Patch best = {32, threads / 32, 65536 / 32};
+    if (P.nz % 32 == 0) return best;
+    double most = 0.0;
+    for (int bz = 8; bz <= 64; bz++) {
+        const int by = threads / bz;
+        const double cover = (double)((P.nz + bz - 1) / bz) * ((P.ny + by - 1) / by) * threads;
+        const double used = (double)P.nz * P.ny / cover;
+        if (used > most * 1.02) {  // wider rows only where they pay
+            most = used;
+            best = {bz, by, (65536 + bz - 1) / bz};
+        }
+    }
+    return best;
+}
+
+dim3 patch_grid(const StepParams& P, const Patch& p)
+{
+    return dim3((P.nz + p.bz - 1) / p.bz, (P.ny + p.by - 1) / p.by, P.nx);
+}
+
+// The thread's site; false past the patch or the lattice.  ANY: any patch; else 32 x T/32, known
+// to the compiler (the run-time division costs the FP64 2HDM step registers it has not: 1272
+// against 1160 us at 192^3).
+template <int T, bool ANY>
+__device__ __forceinline__ bool patch_site(const StepParams& P, const Patch& p, int& x, int& y, int& z)
+{
+    x = blockIdx.z;
+    if constexpr (ANY) {
+        const int ty = (int)(threadIdx.x * p.inv) >> 16, tz = (int)threadIdx.x - ty * p.bz;
+        z = blockIdx.x * p.bz + tz;
+        y = blockIdx.y * p.by + ty;
+        return ty < p.by && z < P.nz && y < P.ny;
+    } else {
+        z = blockIdx.x * 32 + (threadIdx.x & 31);
+        y = blockIdx.y * (T / 32) + (threadIdx.x >> 5);
+        return z < P.nz && y < P.ny;
+    }
+}
+
+// One thread per site; the kernel below instantiates it with its launch bounds.
+template <class S, int MODEL, int HF, bool ENERGY, bool ANY>
+__device__ __forceinline__ void fast_step_body(StepParams P, KConst<S> F, LevelPtrs<S> now,
+                                               LevelPtrs<S> past, Patch p, unsigned* status,
+                                               double* partials)
+{
+    int x, y, z;
+    const bool in = patch_site<kStepThreads, ANY>(P, p, x, y, z);
     double obs[kObsCount];
 #pragma unroll
     for (int k = 0; k < kObsCount; k++) obs[k] = 0.0;
     unsigned warn = 0;
-    if ((z < P.nz) && (y < P.ny) && !frozen(P, x, y, z)) {  // Fixed faces: not evolved
+    if (in && !frozen(P, x, y, z)) {  // Fixed faces: not evolved
         const Offs o = offsets(P, x, y, z);
         Stencil<int> n;
         n.c = o.c;
@@ -99,29 +152,29 @@ constexpr int fast_min_blocks()
     return HF == kHfSU2 ? 3 : 4;
 }
 
-template <class S, int MODEL, int HF, bool ENERGY>
-__global__ void __launch_bounds__(128, fast_min_blocks<S, MODEL, HF>())
-    fast_step_kernel(StepParams P, KConst<S> F, LevelPtrs<S> now, LevelPtrs<S> past, unsigned* status, double* partials)
+template <class S, int MODEL, int HF, bool ENERGY, bool ANY>
+__global__ void __launch_bounds__(kStepThreads, fast_min_blocks<S, MODEL, HF>())
+    fast_step_kernel(StepParams P, KConst<S> F, LevelPtrs<S> now, LevelPtrs<S> past, Patch p, unsigned* status,
+                     double* partials)
 {
-    fast_step_body<S, MODEL, HF, ENERGY>(P, F, now, past, status, partials);
+    fast_step_body<S, MODEL, HF, ENERGY, ANY>(P, F, now, past, p, status, partials);
 }
 
 // Gauss-law residual after a step (gauss_site in gft_step_body.cuh), one
 // thread per site: every load of a site is independent of the others, which
 // keeps the most loads in flight (a march along x that carries the x - 1 links
 // in registers serialises them and measured slower).
-template <class S, int MODEL, int HF>
-__global__ void __launch_bounds__(256) fast_gauss_kernel(StepParams P, LevelPtrs<S> now, LevelPtrs<S> fut,
+template <class S, int MODEL, int HF, bool ANY>
+__global__ void __launch_bounds__(kGaussThreads) fast_gauss_kernel(StepParams P, LevelPtrs<S> now, LevelPtrs<S> fut, Patch p,
                                                          double* partials)
 {
     constexpr int NG = 2 * hf_neq(HF);
-    const int z = blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = blockIdx.y * blockDim.y + threadIdx.y;
-    const int x = blockIdx.z;
+    int x, y, z;
+    const bool in = patch_site<kGaussThreads, ANY>(P, p, x, y, z);
     double v[NG];
 #pragma unroll
     for (int k = 0; k < NG; k++) v[k] = 0.0;
-    if (z < P.nz && y < P.ny && counts(P, x) && !frozen(P, x, y, z)) {
+    if (in && counts(P, x) && !frozen(P, x, y, z)) {
         const Offs o = offsets(P, x, y, z);
         gauss_site<S, MODEL, HF>(P, now, fut, o.c, o.c + o.m[0], o.c + o.m[1], o.c + o.m[2], v);
     }
@@ -133,27 +186,44 @@ template <class S, int MODEL, int HF>
 void fast_step_launch(const StepParams& P, const LevelPtrs<S>& now, const LevelPtrs<S>& past, unsigned* status,
                       double* partials, bool energy, cudaStream_t stream)
 {
-    const dim3 block(32, 4, 1);
-    const dim3 grid((P.nz + 31) / 32, (P.ny + 3) / 4, P.nx);
-    if (energy)
-        fast_step_kernel<S, MODEL, HF, true><<<grid, block, 0, stream>>>(P, make_kconst<S>(P), now, past, status, partials);
-    else
-        fast_step_kernel<S, MODEL, HF, false><<<grid, block, 0, stream>>>(P, make_kconst<S>(P), now, past, status, partials);
+    const Patch p = pick_patch(P, kStepThreads);
+    const bool any = p.bz != 32;
+    auto k = energy ? (any ? fast_step_kernel<S, MODEL, HF, true, true> : fast_step_kernel<S, MODEL, HF, true, false>)
+                    : (any ? fast_step_kernel<S, MODEL, HF, false, true> : fast_step_kernel<S, MODEL, HF, false, false>);
+    k<<<patch_grid(P, p), kStepThreads, 0, stream>>>(P, make_kconst<S>(P), now, past, p, status, partials);
 }
 
 template <class S, int MODEL, int HF>
 void fast_gauss_launch(const StepParams& P, const LevelPtrs<S>& now, const LevelPtrs<S>& fut, double* partials,
                        cudaStream_t stream)
 {
-    const dim3 block(32, 8, 1);  // 32 x 8: 2 % faster than 32 x 4 at 256^3 (624 against 638 us)
-    const dim3 grid((P.nz + 31) / 32, (P.ny + 7) / 8, P.nx);
-    fast_gauss_kernel<S, MODEL, HF><<<grid, block, 0, stream>>>(P, now, fut, partials);
+    const Patch p = pick_patch(P, kGaussThreads);
+    auto k = p.bz != 32 ? fast_gauss_kernel<S, MODEL, HF, true> : fast_gauss_kernel<S, MODEL, HF, false>;
+    k<<<patch_grid(P, p), kGaussThreads, 0, stream>>>(P, now, fut, p, partials);
 }
 
 }  // namespace
 
-int fast_launch_blocks(const StepParams& P, int /*variant*/) { return ((P.nz + 31) / 32) * ((P.ny + 3) / 4) * P.nx; }
-int fast_gauss_blocks(const StepParams& P) { return ((P.nz + 31) / 32) * ((P.ny + 7) / 8) * P.nx; }
+static int patch_blocks(const StepParams& P, int threads)
+{
+    const dim3 g = patch_grid(P, pick_patch(P, threads));
+    return (int)(g.x * g.y * g.z);
+}
+
+// Small lattices divide a site's update over several warps (gft_role_kernels.cu): up to about one
+// warp of sites per scheduler (592 of them), where one thread per site leaves them waiting on one
+// chain of instructions each.  us per step replayed from a graph, divided / one thread per site:
+//   16^3: SM mixed 2.9 / 4.1, FP64 3.9 / 5.6, 2HDM with the family SU(2) 3.4 / 6.6, FP64 4.1 / 8.4
+//   24^3:          3.6 / 4.4,      4.9 / 6.0,                            4.7 / 6.9,      8.3 / 9.2
+//   32^3:          5.0 / 4.8,      8.7 / 7.3,                            9.6 / 6.9,       17 / 12
+constexpr int kRoleMaxSites = 16384;
+static bool use_roles(const StepParams& P) { return P.nsite <= kRoleMaxSites; }
+
+int fast_launch_blocks(const StepParams& P, int /*variant*/)
+{
+    return use_roles(P) ? role_launch_blocks(P) : patch_blocks(P, kStepThreads);
+}
+int fast_gauss_blocks(const StepParams& P) { return patch_blocks(P, kGaussThreads); }
 
 // P.hf selects the Higgs-family variant (2HDM only); the Gauss kernel writes
 // 2 * gaugeNum partial slots per block.
@@ -161,6 +231,7 @@ template <class S, int MODEL>
 cudaError_t launch_fast_step(const StepParams& P, const LevelPtrs<S>& now, const LevelPtrs<S>& past, unsigned* status,
                              double* partials, bool energy, int /*variant*/, cudaStream_t stream)
 {
+    if (use_roles(P)) return launch_role_step<S, MODEL>(P, now, past, status, partials, energy, stream);
     if constexpr (MODEL == kModel2HDM) {
         if (P.hf == kHfU1)
             fast_step_launch<S, MODEL, kHfU1>(P, now, past, status, partials, energy, stream);

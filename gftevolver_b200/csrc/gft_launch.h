@@ -27,6 +27,12 @@ cudaError_t launch_fast_step(const StepParams& P, const LevelPtrs<S>& now, const
 template <class S, int MODEL>
 cudaError_t launch_fast_gauss(const StepParams& P, const LevelPtrs<S>& now, const LevelPtrs<S>& fut, double* partials,
                               cudaStream_t stream);
+// A site's update divided over the warps of a block (gft_role_kernels.cu), which
+// launch_fast_step takes for small lattices.
+template <class S, int MODEL>
+cudaError_t launch_role_step(const StepParams& P, const LevelPtrs<S>& now, const LevelPtrs<S>& past, unsigned* status,
+                             double* partials, bool energy, cudaStream_t stream);
+int role_launch_blocks(const StepParams& P);
 int fast_launch_blocks(const StepParams& P, int variant);
 int fast_gauss_blocks(const StepParams& P);
 

@@ -362,6 +362,81 @@ __device__ __forceinline__ void warn_range(const C (&th)[3], unsigned& warn)
     }
 }
 
+// dt^2 times a site's own-site scalar terms into D -- the Laplacian's diagonal minus dV/dphi, both
+// multiples of the doublets -- and, on logging steps, its potential energy.
+template <int MODEL, bool ENERGY, class C, int ND>
+__device__ __forceinline__ double site_potential(const StepParams& P, const KConst<C>& F, const Q<C> (&fc)[ND],
+                                                 Q<C> (&D)[ND])
+{
+    double pot_e = 0.0;
+    if (MODEL == kModelSM) {
+        const C fsq = fc[0].w * fc[0].w + fc[0].x * fc[0].x + fc[0].y * fc[0].y + fc[0].z * fc[0].z;
+        const C k = F.diag - F.lambda * (fsq - F.eta_sqr);
+        D[0] = {k * fc[0].w, k * fc[0].x, k * fc[0].y, k * fc[0].z};
+        if (ENERGY) {
+            const double t = (double)fsq - P.eta_sqr;
+            pot_e = 0.25 * P.lambda * t * t;
+        }
+    } else {
+        const Q<C> f1 = fc[0], f2 = fc[ND - 1];
+        const C s1 = f1.w * f1.w + f1.x * f1.x + f1.y * f1.y + f1.z * f1.z;
+        const C s2 = f2.w * f2.w + f2.x * f2.x + f2.y * f2.y + f2.z * f2.z;
+        const C dot = P.break_son ? f1.w * f2.w + f1.x * f2.x + f1.y * f2.y + f1.z * f2.z : (C)0;
+        const C anti = (P.break_son && P.break_uhalfn) ? f1.w * f2.x - f1.x * f2.w + f1.y * f2.z - f1.z * f2.y : (C)0;
+        C a1 = F.diag1 - F.l1x4 * s1 - F.l3x2 * s2;
+        C a2 = F.diag2 - F.l2x4 * s2 - F.l3x2 * s1;
+        const C f1v[4] = {f1.w, f1.x, f1.y, f1.z};
+        const C f2v[4] = {f2.w, f2.x, f2.y, f2.z};
+        C v1[4], v2[4];
+        if (P.break_son) {
+            // single SO(N): (-m12r + 2 l4p5 dot + l6r s1 + l7r s2) f_other + 2 l6r|l7r dot f_self
+            const C bs = F.m12r - F.l4p5x2 * dot - F.l6r * s1 - F.l7r * s2;
+            a1 -= F.l6rx2 * dot;
+            a2 -= F.l7rx2 * dot;
+            if (P.break_uhalfn) {
+                // U(N/2): (m12i + 2 l4m5 anti - 2 l5i dot - l6i s1 - l7i s2) J f_other - 2 l5i anti f_other
+                // - 2 l6i|l7i anti f_self
+                const C cu = F.l5ix2 * dot + F.l6i * s1 + F.l7i * s2 - F.m12i - F.l4m5x2 * anti;
+                const C bo = bs + F.l5ix2 * anti;
+                a1 += F.l6ix2 * anti;
+                a2 += F.l7ix2 * anti;
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const int alt = 1 - 2 * (k % 2);
+                    v1[k] = a1 * f1v[k] + bo * f2v[k] + cu * (C)alt * f2v[k + alt];
+                    v2[k] = a2 * f2v[k] + bo * f1v[k] - cu * (C)alt * f1v[k + alt];
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    v1[k] = a1 * f1v[k] + bs * f2v[k];
+                    v2[k] = a2 * f2v[k] + bs * f1v[k];
+                }
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                v1[k] = a1 * f1v[k];
+                v2[k] = a2 * f2v[k];
+            }
+        }
+        D[0] = {v1[0], v1[1], v1[2], v1[3]};
+        D[ND - 1] = {v2[0], v2[1], v2[2], v2[3]};
+        if (ENERGY) {
+            const double d1 = s1, d2 = s2, dd = dot, da = anti;
+            double v = -P.m1 * d1 - P.m2 * d2 + P.l1 * d1 * d1 + P.l2 * d2 * d2 + P.l3 * d1 * d2;
+            if (P.break_son) {
+                v += -P.m12r * dd + P.l4p5 * dd * dd + P.l6r * d1 * dd + P.l7r * d2 * dd;
+                if (P.break_uhalfn)
+                    v += P.m12i * da + P.l4m5 * da * da - 2.0 * P.l5i * dd * da - P.l6i * d1 * da - P.l7i * d2 * da;
+            }
+            if (P.apply_norm) v += P.energy_offset;
+            pot_e = v;
+        }
+    }
+    return pot_e;
+}
+
 // Scalar leapfrog (Model.cpp:347-356) of one doublet f, from D = dt^2 (Laplacian - dV/dphi):
 // phi(t+dt) = phi + [(phi - phi_past)(1 - damping) + D], one rounding at the end.
 template <bool ENERGY, class C, class S>
@@ -598,78 +673,12 @@ __device__ __forceinline__ void site_step(const StepParams& P, const KConst<S>& 
                          });
     }
 
-    // ---- potential dV/dphi: D starts as dt^2 times the own-site terms, the Laplacian's
-    //      diagonal minus dV/dphi (both multiples of the doublets) ----
+    // ---- potential dV/dphi and the Laplacian's diagonal ----
     Q<C> fc[ND];
 #pragma unroll
     for (int db = 0; db < ND; db++) fc[db] = acc.ph(db, n.c);
     Q<C> D[ND];
-    double pot_e = 0.0;
-    if (MODEL == kModelSM) {
-        const C fsq = fc[0].w * fc[0].w + fc[0].x * fc[0].x + fc[0].y * fc[0].y + fc[0].z * fc[0].z;
-        const C k = F.diag - F.lambda * (fsq - F.eta_sqr);
-        D[0] = {k * fc[0].w, k * fc[0].x, k * fc[0].y, k * fc[0].z};
-        if (ENERGY) {
-            const double t = (double)fsq - P.eta_sqr;
-            pot_e = 0.25 * P.lambda * t * t;
-        }
-    } else {
-        const Q<C> f1 = fc[0], f2 = fc[ND - 1];
-        const C s1 = f1.w * f1.w + f1.x * f1.x + f1.y * f1.y + f1.z * f1.z;
-        const C s2 = f2.w * f2.w + f2.x * f2.x + f2.y * f2.y + f2.z * f2.z;
-        const C dot = P.break_son ? f1.w * f2.w + f1.x * f2.x + f1.y * f2.y + f1.z * f2.z : (C)0;
-        const C anti = (P.break_son && P.break_uhalfn) ? f1.w * f2.x - f1.x * f2.w + f1.y * f2.z - f1.z * f2.y : (C)0;
-        C a1 = F.diag1 - F.l1x4 * s1 - F.l3x2 * s2;
-        C a2 = F.diag2 - F.l2x4 * s2 - F.l3x2 * s1;
-        const C f1v[4] = {f1.w, f1.x, f1.y, f1.z};
-        const C f2v[4] = {f2.w, f2.x, f2.y, f2.z};
-        C v1[4], v2[4];
-        if (P.break_son) {
-            // single SO(N): (-m12r + 2 l4p5 dot + l6r s1 + l7r s2) f_other + 2 l6r|l7r dot f_self
-            const C bs = F.m12r - F.l4p5x2 * dot - F.l6r * s1 - F.l7r * s2;
-            a1 -= F.l6rx2 * dot;
-            a2 -= F.l7rx2 * dot;
-            if (P.break_uhalfn) {
-                // U(N/2): (m12i + 2 l4m5 anti - 2 l5i dot - l6i s1 - l7i s2) J f_other - 2 l5i anti f_other
-                // - 2 l6i|l7i anti f_self
-                const C cu = F.l5ix2 * dot + F.l6i * s1 + F.l7i * s2 - F.m12i - F.l4m5x2 * anti;
-                const C bo = bs + F.l5ix2 * anti;
-                a1 += F.l6ix2 * anti;
-                a2 += F.l7ix2 * anti;
-#pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    const int alt = 1 - 2 * (k % 2);
-                    v1[k] = a1 * f1v[k] + bo * f2v[k] + cu * (C)alt * f2v[k + alt];
-                    v2[k] = a2 * f2v[k] + bo * f1v[k] - cu * (C)alt * f1v[k + alt];
-                }
-            } else {
-#pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    v1[k] = a1 * f1v[k] + bs * f2v[k];
-                    v2[k] = a2 * f2v[k] + bs * f1v[k];
-                }
-            }
-        } else {
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                v1[k] = a1 * f1v[k];
-                v2[k] = a2 * f2v[k];
-            }
-        }
-        D[0] = {v1[0], v1[1], v1[2], v1[3]};
-        D[ND - 1] = {v2[0], v2[1], v2[2], v2[3]};
-        if (ENERGY) {
-            const double d1 = s1, d2 = s2, dd = dot, da = anti;
-            double v = -P.m1 * d1 - P.m2 * d2 + P.l1 * d1 * d1 + P.l2 * d2 * d2 + P.l3 * d1 * d2;
-            if (P.break_son) {
-                v += -P.m12r * dd + P.l4p5 * dd * dd + P.l6r * d1 * dd + P.l7r * d2 * dd;
-                if (P.break_uhalfn)
-                    v += P.m12i * da + P.l4m5 * da * da - 2.0 * P.l5i * dd * da - P.l6i * d1 * da - P.l7i * d2 * da;
-            }
-            if (P.apply_norm) v += P.energy_offset;
-            pot_e = v;
-        }
-    }
+    const double pot_e = site_potential<MODEL, ENERGY>(P, F, fc, D);
 
     // ---- scalar sector: covariant Laplacian D and currents J (four times the reference's, whose
     //      1/4 is in the constants cY, cI and cH; the SU(2) currents join Mg) ----
