@@ -298,9 +298,12 @@ bool encode_tiled(const gft_handle* h, const StepParams& P, int tile, TMaps* tm,
 //   SM mixed:   64^3 (0.3 waves) 34 / 21, 96^3 (0.97) 58 / 62, 128^3 (2.4) 133 / 136, 160^3 224 /
 //               257, 192^3 (8) 376 / 439; logging steps 71 / 86 and 170 / 195 at 96^3 and 128^3;
 //   2HDM mixed: 128^3 (2.4 waves) 175 / 163, 144^3 (3.3) 239 / 259, 160^3 (4.7) 303 / 317, 192^3
-//               (8) 512 / 546, logging 659 / 736;
-//   FP64 SM:    128^3 (1.7 waves) 301 / 287, 192^3 (5.8) 823 / 993, 256^3 (13.8) 1936 / 2290.
-constexpr double kAutoWavesSM = 0.9, kAutoWaves2HDM = 3.0, kAutoWavesFP64 = 5.0;
+//               (8) 510 / 546, logging 660 / 736;
+//   FP64 SM:    128^3 (1.7 waves) 302 / 287, 160^3 (3.4) 574 / 558, 176^3 (4.9) 627 / 827, 192^3
+//               (5.8) 823 / 993, 256^3 (13.8) 1936 / 2290;
+//   FP64 2HDM:  128^3 369 / 348, logging 552 / 581, 144^3 (2.7) 474 / 572, 160^3 650 / 673, logging
+//               1027 / 1127, 192^3 1064 / 1160, logging 1588 / 1938.
+constexpr double kAutoWavesSM = 0.9, kAutoWaves2HDM = 3.0, kAutoWavesFP64SM = 4.0, kAutoWavesFP642HDM = 2.5;
 // Planes per CTA unless the caller sets them.  Mixed form: short enough to balance the last
 // wave, long enough for the start of a march (two more planes staged) not to count: SM 128^3 /
 // 192^3 / 256^3 at 8, 12, 16, 32 planes 133 / 377 / 849, 133 / 376 / 830, 135 / 372 / 857,
@@ -311,14 +314,14 @@ bool use_tiled(const gft_handle* h, const StepParams& P)
 {
     if (!h->tiled_ready || h->kernel_kind == 1 || h->hf != kHfNone) return false;
     const bool fp64 = h->cfg.form == GFT_FORM_FP64, sm = h->cfg.model == GFT_MODEL_SM;
-    // the FP64 form: the staged SM step only (kinds 0 and 2)
-    if (fp64 && (!sm || h->kernel_kind > 2)) return false;
+    // the FP64 form: a tile the caller picks serves the SM model only
+    if (fp64 && ((!sm && h->kernel_kind != 0) || h->kernel_kind > 2)) return false;
     if (h->cfg.form != GFT_FORM_MIXED && !fp64) return false;
     if (!tiled_supported(P, h->tile_variant)) return false;
     if (h->kernel_kind != 0) return true;
     const double slots = (double)h->nsm * tiled_ctas_per_sm(h->tile_variant, fp64, sm);
-    return tiled_blocks(P, h->tile_variant, h->march) >=
-           (fp64 ? kAutoWavesFP64 : (sm ? kAutoWavesSM : kAutoWaves2HDM)) * slots;
+    const double waves = sm ? (fp64 ? kAutoWavesFP64SM : kAutoWavesSM) : (fp64 ? kAutoWavesFP642HDM : kAutoWaves2HDM);
+    return tiled_blocks(P, h->tile_variant, h->march) >= waves * slots;
 }
 
 // Plain steps of the SM mixed form with two sites per thread (kernel kind 3):
@@ -357,9 +360,14 @@ cudaError_t launch_step(gft_handle* h, const StepParams& P, int tn, const LevelP
         return launch_ref_step<S, kModel2HDM>(P, now, past, h->d_status, h->d_part_e, energy, h->stream);
     }
     if constexpr (sizeof(S) == 8) {
-        if (model == GFT_MODEL_SM && use_tiled(h, P))
-            return launch_tiled_step<S, kModelSM>(h->tm[tn], h->tp[1 - tn], P, now, past, h->tile_variant, h->march,
-                                                  h->d_status, h->d_part_e, energy, st ? st : h->stream, xa, xn);
+        if (use_tiled(h, P)) {
+            cudaStream_t s = st ? st : h->stream;
+            if (model == GFT_MODEL_SM)
+                return launch_tiled_step<S, kModelSM>(h->tm[tn], h->tp[1 - tn], P, now, past, h->tile_variant, h->march,
+                                                      h->d_status, h->d_part_e, energy, s, xa, xn);
+            return launch_tiled_step<S, kModel2HDM>(h->tm[tn], h->tp[1 - tn], P, now, past, h->tile_variant, h->march,
+                                                    h->d_status, h->d_part_e, energy, s, xa, xn);
+        }
     }
     if constexpr (sizeof(S) == 4) {
         if (use_tiled(h, P)) {
@@ -526,15 +534,21 @@ int gft_create(const gft_config* cfg, gft_handle** out)
     }
     const StepParams P = make_params(h, 0, false);
     h->march = cfg->form == GFT_FORM_FP64 ? kAutoMarchFP64 : kAutoMarchMixed;
-    if (cfg->form == GFT_FORM_MIXED || (cfg->form == GFT_FORM_FP64 && cfg->model == GFT_MODEL_SM)) {
+    if (cfg->form == GFT_FORM_MIXED || cfg->form == GFT_FORM_FP64) {
         // default tile: the largest built shape the lattice divides
         h->tile_variant = 0;
         while (h->tile_variant < kTiledVariants && !tiled_supported(P, h->tile_variant)) h->tile_variant++;
         // FP64: two CTAs of four warps per SM, where an 8 x 32 tile's staged planes leave one of
-        // eight; its barriers stop half the warps (us per step, 256^3 / 192^3: 1936 / 823 against
-        // 2017 / 866; logging step 2928 against 2802)
-        if (cfg->form == GFT_FORM_FP64 && tiled_supported(P, kTileFP64)) h->tile_variant = kTileFP64;
-        h->tiled_ready = (h->tile_variant < kTiledVariants || h->tile_variant == kTileFP64) && encode_tiled(h, P, h->tile_variant, h->tm, h->tp);
+        // eight; its barriers stop half the warps (SM, us per step, 256^3 / 192^3: 1936 / 823
+        // against 2017 / 866; logging step 2928 against 2802).  The 2HDM is built for it alone.
+        if (cfg->form == GFT_FORM_FP64) {
+            if (tiled_supported(P, kTileFP64))
+                h->tile_variant = kTileFP64;
+            else if (cfg->model != GFT_MODEL_SM)
+                h->tile_variant = kTiledVariants;
+        }
+        h->tiled_ready = (h->tile_variant < kTiledVariants || h->tile_variant == kTileFP64) &&
+                         encode_tiled(h, P, h->tile_variant, h->tm, h->tp);
     }
     int nb = std::max(fast_launch_blocks(P, 0), fast_gauss_blocks(P));
     nb = std::max(nb, ref_launch_blocks(P));
@@ -1155,7 +1169,7 @@ int gft_set_kernel(gft_handle* h, int kind, int tile, int march)
     }
     if (kind >= 2 && h->hf != kHfNone)
         return h->fail(GFT_E_UNSUPPORTED, "gft_set_kernel: the tiled kernel has no Higgs-family field");
-    // the FP64 form of the SM model takes tiles too (kind 2, and kind 0's automatic choice)
+    // the FP64 form of the SM model takes these tiles too (kind 2, and kind 0's automatic choice)
     const bool fp64_sm = h->cfg.form == GFT_FORM_FP64 && h->cfg.model == GFT_MODEL_SM && (kind == 2 || kind == 0);
     if (h->cfg.form != GFT_FORM_MIXED && !fp64_sm) {
         if (kind >= 2)

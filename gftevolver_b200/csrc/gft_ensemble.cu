@@ -95,20 +95,6 @@ __device__ __forceinline__ void tmap_acquire(const TMaps& m)
 // group, y0, z0, x0}; tile i's energy partials go to partials row i.  UNIFORM:
 // the members share ep.common but for their geometry (the per-member fields
 // copied below).
-// Steps stage the wrapped halo sites (run_tile's STAGE) where the staging
-// area leaves the resident CTAs per SM unchanged; the dynamic shared memory
-// then includes it.
-template <int MODEL, int TY, int TZ, bool ENERGY>
-constexpr bool ens_stage()
-{
-    return tile_stage<float, MODEL, TY, TZ, ENERGY>();
-}
-template <int MODEL, int TY, int TZ, bool ENERGY>
-constexpr int ens_smem()
-{
-    return tile_smem<float, MODEL, TY, TZ, ENERGY>();
-}
-
 template <int MODEL, int TY, int TZ, bool ENERGY, bool UNIFORM>
 __global__ void __launch_bounds__(TY * TZ, tile_ctas<float, MODEL, TY, TZ>())
     ensemble_step_kernel(const __grid_constant__ EnsParams ep, const EnsMaps* __restrict__ maps,
@@ -117,7 +103,7 @@ __global__ void __launch_bounds__(TY * TZ, tile_ctas<float, MODEL, TY, TZ>())
                          double* partials)
 {
     constexpr int ND = (MODEL == kModelSM) ? 1 : 2;
-    using G = Geom<float, TY, TZ, ND>;
+    using G = Geom<float, TY, TZ, ND, ring_planes<float, MODEL>()>;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem =
         reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~(uintptr_t)127);
@@ -166,7 +152,7 @@ __global__ void __launch_bounds__(TY * TZ, tile_ctas<float, MODEL, TY, TZ>())
         KConst<float> Fm;
         if constexpr (!UNIFORM) Fm = make_kconst<float>(P);
         const KConst<float>& F = UNIFORM ? ep.fcommon : Fm;
-        const bool ok = run_tile<float, MODEL, TY, TZ, ENERGY, EnsLevel, ens_stage<MODEL, TY, TZ, ENERGY>()>(
+        const bool ok = run_tile<float, MODEL, TY, TZ, ENERGY, EnsLevel>(
             mp.tm[tn], mp.tp[1 - tn], P, F, ep.lv[m][tn], ep.lv[m][1 - tn], w.y, w.z, w.w, min(lx, P.nx - w.w), smem,
             bars, ring, &s_abort, obs, warn);
         if (!ok) {
@@ -231,7 +217,7 @@ __global__ void __launch_bounds__(kFinThreads) ensemble_finalize_kernel(const do
 template <int MODEL, int TY, int TZ, bool ENERGY, bool UNIFORM>
 int resident_ctas()
 {
-    constexpr int SMEM = ens_smem<MODEL, TY, TZ, ENERGY>();
+    constexpr int SMEM = tile_smem<float, MODEL, TY, TZ, ENERGY>();
     static int per_sm = 0;
     if (per_sm == 0) {
         auto k = ensemble_step_kernel<MODEL, TY, TZ, ENERGY, UNIFORM>;
@@ -259,7 +245,8 @@ cudaError_t launch_step_u(const EnsParams& ep, const EnsMaps* maps, const GroupT
 {
     const int grid = std::min(gt.nitems, nsm * resident_ctas<MODEL, TY, TZ, ENERGY, UNIFORM>());
     if (grid < 1) return cudaSuccess;
-    ensemble_step_kernel<MODEL, TY, TZ, ENERGY, UNIFORM><<<grid, dim3(TZ, TY, 1), ens_smem<MODEL, TY, TZ, ENERGY>(), s>>>(
+    constexpr int SMEM = tile_smem<float, MODEL, TY, TZ, ENERGY>();
+    ensemble_step_kernel<MODEL, TY, TZ, ENERGY, UNIFORM><<<grid, dim3(TZ, TY, 1), SMEM, s>>>(
         ep, maps, gt.items, gt.nitems, gt.order, gt.start, gt.nlist, lx, tn, status, partials);
     return cudaGetLastError();
 }

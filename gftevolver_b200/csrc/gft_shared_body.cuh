@@ -1,4 +1,4 @@
-// gft_shared_body.cuh -- the SM site update of the tiled kernels with every loop and
+// gft_shared_body.cuh -- the site update of the tiled kernels with every loop and
 // every transported doublet computed once per tile.
 //
 // A site's lower loops are its back neighbours' upper loops, turned by its own links
@@ -20,8 +20,8 @@
 // cosines too; three turns remain: 1,436 -> 1,265 warp instructions per 32 sites at SM 128^3,
 // the halo row and column (4 % of the work of an 8 x 32 tile) included.  us per step, against
 // every thread computing its own lower loops (site_step with CARRY): SM mixed 256^3 887 -> 835,
-// 128^3 (march 12) 143 -> 133, logging 256^3 1112 -> 1061.  The 2HDM tile has no room in shared
-// memory for a second doublet's values beside two resident CTAs and keeps site_step.
+// 128^3 (march 12) 143 -> 133, logging 256^3 1112 -> 1061; FP64 2HDM 192^3 against one thread per
+// site 1160 -> 1064, logging 1938 -> 1588.  The float 2HDM's tiles keep site_step (hands_over).
 #pragma once
 
 #include "gft_step_body.cuh"
@@ -30,27 +30,27 @@ namespace gft {
 
 // What a site hands to its +e_d neighbour (d = 1, 2; a < b the other two directions): the
 // vector parts of link d's upper loops in the planes with a and b, the sines of F_ad and
-// F_bd, and the doublet transported along link d.  Three quads.
-template <class C>
+// F_bd, and the doublets transported along link d.  2 + ND quads.
+template <class C, int ND>
 struct Handed {
     C fa[3], sa;
     C fb[3], sb;
-    Q<C> t;
+    Q<C> t[ND];
 };
 
 // A site between its two halves.  r[i]: the sum over planes of weight times the vector
 // that link i's lower loops are, before the turn by U_i.
-template <class C>
+template <class C, int ND>
 struct OpenSite {
-    Q<C> U[3], fc, D;
+    Q<C> U[3], fc[ND], D[ND];
     C th[3], Mg[3][3], r[3][3], MgY[3];
     C mag_e, plaq2, plaq1, grad_e;
     double pot_e;
 };
 
 // Adds what the back neighbour of direction d handed over, weight l = dt^2 / dx_d^2.
-template <class C>
-__device__ __forceinline__ void receive(OpenSite<C>& o, int a, int b, C l, const Handed<C>& h)
+template <class C, int ND>
+__device__ __forceinline__ void receive(OpenSite<C, ND>& o, int a, int b, C l, const Handed<C, ND>& h)
 {
 #pragma unroll
     for (int k = 0; k < 3; k++) {
@@ -59,12 +59,14 @@ __device__ __forceinline__ void receive(OpenSite<C>& o, int a, int b, C l, const
     }
     o.MgY[a] += l * h.sa;
     o.MgY[b] += l * h.sb;
-    o.D = qadd_scaled(o.D, l, h.t);
+#pragma unroll
+    for (int db = 0; db < ND; db++) o.D[db] = qadd_scaled(o.D[db], l, h.t[db]);
 }
 
-template <class S, bool ENERGY, class A, class R>
+template <class S, int MODEL, bool ENERGY, class A, class R, int ND>
 __device__ __forceinline__ void site_open(const StepParams& P, const KConst<S>& F, const A& acc, const Stencil<R>& n,
-                                          XCarry<S, 1>& carry, OpenSite<S>& o, Handed<S>& hy, Handed<S>& hz)
+                                          XCarry<S, ND>& carry, OpenSite<S, ND>& o, Handed<S, ND>& hy,
+                                          Handed<S, ND>& hz)
 {
     using C = S;
     const C l[3] = {F.ldt[0], F.ldt[1], F.ldt[2]};
@@ -73,14 +75,13 @@ __device__ __forceinline__ void site_open(const StepParams& P, const KConst<S>& 
         o.U[a] = acc.q(a, n.c);
         o.th[a] = acc.th(a, n.c);
     }
-    o.fc = acc.ph(0, n.c);
 
     // ---- own-site terms and what the x neighbour handed over ----
-    const Q<C> f = o.fc;
-    const C fsq = f.w * f.w + f.x * f.x + f.y * f.y + f.z * f.z;
-    const C kd = F.diag - F.lambda * (fsq - F.eta_sqr);
-    o.D = {kd * f.w, kd * f.x, kd * f.y, kd * f.z};
-    o.D = qadd_scaled(o.D, l[0], carry.t0[0]);
+#pragma unroll
+    for (int db = 0; db < ND; db++) o.fc[db] = acc.ph(db, n.c);
+    o.pot_e = site_potential<MODEL, ENERGY>(P, F, o.fc, o.D);
+#pragma unroll
+    for (int db = 0; db < ND; db++) o.D[db] = qadd_scaled(o.D[db], l[0], carry.t0[db]);
     o.MgY[0] = (C)0;
     o.MgY[1] = -l[0] * carry.s01;
     o.MgY[2] = -l[0] * carry.s02;
@@ -92,11 +93,7 @@ __device__ __forceinline__ void site_open(const StepParams& P, const KConst<S>& 
 #pragma unroll
         for (int i = 0; i < 3; i++) o.Mg[i][k] = (C)0;
     }
-    if (ENERGY) {
-        const double t = (double)fsq - P.eta_sqr;
-        o.pot_e = 0.25 * P.lambda * t * t;
-        o.mag_e = o.plaq2 = o.plaq1 = o.grad_e = (C)0;
-    }
+    if (ENERGY) o.mag_e = o.plaq2 = o.plaq1 = o.grad_e = (C)0;
 
     // ---- upper loops ----
 #pragma unroll
@@ -144,28 +141,31 @@ __device__ __forceinline__ void site_open(const StepParams& P, const KConst<S>& 
     for (int a = 0; a < 3; a++) {
         C sn, cs;
         gsincos(o.th[a], sn, cs);
-        const Q<C> g = acc.ph(0, n.p[a]);
-        o.D = qadd_scaled(o.D, l[a], transport_back(o.U[a], cs, sn, g));
-        const Q<C> u = transport(o.U[a], cs, sn, f);
-        const C up = u.w * g.x - u.x * g.w, lo = u.y * g.z - u.z * g.y;
-        o.MgY[a] += F.cY * (up + lo);
-        o.Mg[a][0] += F.cI * (u.w * g.z - u.x * g.y + u.y * g.x - u.z * g.w);
-        o.Mg[a][1] += F.cI * (-u.w * g.y - u.x * g.z + u.y * g.w + u.z * g.x);
-        o.Mg[a][2] += F.cI * (up - lo);
-        if (ENERGY) {
-            const C e0 = g.w - u.w, e1 = g.x - u.x, e2 = g.y - u.y, e3 = g.z - u.z;
-            o.grad_e += F.e_grad[a] * (e0 * e0 + e1 * e1 + e2 * e2 + e3 * e3);
+#pragma unroll
+        for (int db = 0; db < ND; db++) {
+            const Q<C> g = acc.ph(db, n.p[a]);
+            o.D[db] = qadd_scaled(o.D[db], l[a], transport_back(o.U[a], cs, sn, g));
+            const Q<C> u = transport(o.U[a], cs, sn, o.fc[db]);
+            const C up = u.w * g.x - u.x * g.w, lo = u.y * g.z - u.z * g.y;
+            o.MgY[a] += F.cY * (up + lo);
+            o.Mg[a][0] += F.cI * (u.w * g.z - u.x * g.y + u.y * g.x - u.z * g.w);
+            o.Mg[a][1] += F.cI * (-u.w * g.y - u.x * g.z + u.y * g.w + u.z * g.x);
+            o.Mg[a][2] += F.cI * (up - lo);
+            if (ENERGY) {
+                const C e0 = g.w - u.w, e1 = g.x - u.x, e2 = g.y - u.y, e3 = g.z - u.z;
+                o.grad_e += F.e_grad[a] * (e0 * e0 + e1 * e1 + e2 * e2 + e3 * e3);
+            }
+            if (a == 0) carry.t0[db] = u;
+            if (a == 1) hy.t[db] = u;
+            if (a == 2) hz.t[db] = u;
         }
-        if (a == 0) carry.t0[0] = u;
-        if (a == 1) hy.t = u;
-        if (a == 2) hz.t = u;
     }
 }
 
 // What the site c of a staged plane hands to its +e_d neighbour, d (1 or 2)
 // a run-time value of the lane; p0, p1, p2: the cells of x + e_a.
-template <class S, class A, class R>
-__device__ __forceinline__ void halo_hand_over(const A& acc, int d, R c, R p0, R p1, R p2, Handed<S>& h)
+template <class S, class A, class R, int ND>
+__device__ __forceinline__ void halo_hand_over(const A& acc, int d, R c, R p0, R p1, R p2, Handed<S, ND>& h)
 {
     using C = S;
     const int b = 3 - d;
@@ -180,11 +180,12 @@ __device__ __forceinline__ void halo_hand_over(const A& acc, int d, R c, R p0, R
     h.sb = gsin(acc.th(b, c) + acc.th(d, pb) - acc.th(b, pd) - thd);
     C sn, cs;
     gsincos(thd, sn, cs);
-    h.t = transport(Ud, cs, sn, acc.ph(0, c));
+#pragma unroll
+    for (int db = 0; db < ND; db++) h.t[db] = transport(Ud, cs, sn, acc.ph(db, c));
 }
 
-template <class S, bool ENERGY, class PV>
-__device__ __forceinline__ void site_close(const StepParams& P, const KConst<S>& F, OpenSite<S>& o, const PV& past,
+template <class S, bool ENERGY, int ND, class PV>
+__device__ __forceinline__ void site_close(const StepParams& P, const KConst<S>& F, OpenSite<S, ND>& o, const PV& past,
                                            double (&obs)[kObsCount], unsigned& warn, bool count)
 {
     using C = S;
@@ -192,7 +193,9 @@ __device__ __forceinline__ void site_close(const StepParams& P, const KConst<S>&
 #pragma unroll
     for (int i = 0; i < 3; i++) add_turned(o.Mg[i], (C)1, o.U[i], o.r[i]);
     C kin_e = (C)0, phisq = (C)0, elec_e = (C)0, check = (C)0;
-    leapfrog_doublet<ENERGY>(F, o.fc, past.ph(0), o.D, past.at.L.ph[0], past.at.s, kin_e, phisq, check);
+#pragma unroll
+    for (int db = 0; db < ND; db++)
+        leapfrog_doublet<ENERGY>(F, o.fc[db], past.ph(db), o.D[db], past.at.L.ph[db], past.at.s, kin_e, phisq, check);
     leapfrog_links<ENERGY>(F, o.U, o.th, o.Mg, o.MgY, past, elec_e, warn, check);
     if (!isfinite(check)) warn |= kWarnNonFinite;
     if (!count) {

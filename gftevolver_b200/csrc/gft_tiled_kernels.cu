@@ -21,7 +21,7 @@ __global__ void __launch_bounds__(TY * TZ, tile_ctas<S, MODEL, TY, TZ>())
                       LevelPtrs<S> now, LevelPtrs<S> past, int lx, int xa, int xn, unsigned* status, double* partials)
 {
     constexpr int ND = (MODEL == kModelSM) ? 1 : 2;
-    using G = Geom<S, TY, TZ, ND>;
+    using G = Geom<S, TY, TZ, ND, ring_planes<S, MODEL>()>;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem =
         reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~(uintptr_t)127);
@@ -42,8 +42,7 @@ __global__ void __launch_bounds__(TY * TZ, tile_ctas<S, MODEL, TY, TZ>())
     unsigned warn = 0;
     RingPhase ring = {0u};
     const int x0 = xa + blockIdx.z * lx;  // planes [xa, xa + xn) in chunks of lx
-    constexpr bool STAGE = tile_stage<S, MODEL, TY, TZ, ENERGY>();
-    const bool ok = run_tile<S, MODEL, TY, TZ, ENERGY, LevelPtrs<S>, STAGE>(
+    const bool ok = run_tile<S, MODEL, TY, TZ, ENERGY, LevelPtrs<S>>(
         maps, pmaps, P, F, now, past, blockIdx.y * TY, blockIdx.x * TZ, x0, min(lx, xa + xn - x0), smem, bars, ring,
         &s_abort, obs, warn);
     if (!ok && tid == 0) atomicOr(status, kErrTimeout);
@@ -114,7 +113,7 @@ __global__ void __launch_bounds__(TY * TZ / 2, 2) tiled_pair_kernel(const __grid
     carry.valid = false;
     unsigned warn = 0;
     RingPhase ring = {0u};
-    const bool ok = run_ring<float, TY, TZ, 1, LevelPtrs<float>, H::kUse, true>(
+    const bool ok = run_ring<float, TY, TZ, 1, LevelPtrs<float>, H::kUse, 4>(
         maps, pmaps, P, now, y0, z0, x0, min(lx, xa + xn - x0), smem, bars, ring, &s_abort, smem + H::OFFSET, tid,
         [](const unsigned char*, const unsigned char*) {},
         [&](int i, const unsigned char* bm, const unsigned char* bc, const unsigned char* bp) {
@@ -194,7 +193,7 @@ __global__ void __launch_bounds__(2 * TY * TZ, 3) tiled_split_kernel(const __gri
     carry.valid = false;
     unsigned warn = 0;
     RingPhase ring = {0u};
-    const bool ok = run_ring<float, TY, TZ, 1, LevelPtrs<float>, L::kStage, true>(
+    const bool ok = run_ring<float, TY, TZ, 1, LevelPtrs<float>, L::kStage, 4>(
         maps, pmaps, P, now, y0, z0, x0, min(lx, xa + xn - x0), smem, bars, ring, &s_abort,
         smem + HaloStage<float, TY, TZ, 1, 4>::OFFSET, tid, [](const unsigned char*, const unsigned char*) {},
         [&](int i, const unsigned char* bm, const unsigned char* bc, const unsigned char* bp) {
@@ -293,7 +292,7 @@ int tiled_ctas_per_sm(int variant, bool fp64, bool sm)
     case 0: return ctas_of<8, 32>(fp64, sm);
     case 1: return ctas_of<4, 32>(fp64, sm);
     case 2: return ctas_of<4, 16>(fp64, sm);
-    case kTileFP64: return tile_ctas<double, kModelSM, 8, 16>();
+    case kTileFP64: return sm ? tile_ctas<double, kModelSM, 8, 16>() : tile_ctas<double, kModel2HDM, 8, 16>();
     default: return ctas_of<16, 16>(fp64, sm);
     }
 }
@@ -338,11 +337,15 @@ cudaError_t launch_tiled_step(const TMaps& maps, const TMaps& pmaps, const StepP
         if (variant == kTileFP64)
             return launch_tiled_t<S, MODEL, 8, 16>(maps, pmaps, P, now, past, lx, xa, xn, status, partials, energy, stream);
     }
-    switch (variant) {
-    case 0: return launch_tiled_t<S, MODEL, 8, 32>(maps, pmaps, P, now, past, lx, xa, xn, status, partials, energy, stream);
-    case 1: return launch_tiled_t<S, MODEL, 4, 32>(maps, pmaps, P, now, past, lx, xa, xn, status, partials, energy, stream);
-    case 2: return launch_tiled_t<S, MODEL, 4, 16>(maps, pmaps, P, now, past, lx, xa, xn, status, partials, energy, stream);
-    default: return launch_tiled_t<S, MODEL, 16, 16>(maps, pmaps, P, now, past, lx, xa, xn, status, partials, energy, stream);
+    if constexpr (sizeof(S) == 8 && MODEL == kModel2HDM) {
+        return cudaErrorInvalidValue;  // built for the 8 x 16 tile alone
+    } else {
+        switch (variant) {
+        case 0: return launch_tiled_t<S, MODEL, 8, 32>(maps, pmaps, P, now, past, lx, xa, xn, status, partials, energy, stream);
+        case 1: return launch_tiled_t<S, MODEL, 4, 32>(maps, pmaps, P, now, past, lx, xa, xn, status, partials, energy, stream);
+        case 2: return launch_tiled_t<S, MODEL, 4, 16>(maps, pmaps, P, now, past, lx, xa, xn, status, partials, energy, stream);
+        default: return launch_tiled_t<S, MODEL, 16, 16>(maps, pmaps, P, now, past, lx, xa, xn, status, partials, energy, stream);
+        }
     }
 }
 
@@ -395,6 +398,9 @@ template cudaError_t launch_tiled_step<float, kModelSM>(const TMaps&, const TMap
 template cudaError_t launch_tiled_step<double, kModelSM>(const TMaps&, const TMaps&, const StepParams&,
                                                          const LevelPtrs<double>&, const LevelPtrs<double>&, int, int,
                                                          unsigned*, double*, bool, cudaStream_t, int, int);
+template cudaError_t launch_tiled_step<double, kModel2HDM>(const TMaps&, const TMaps&, const StepParams&,
+                                                           const LevelPtrs<double>&, const LevelPtrs<double>&, int, int,
+                                                           unsigned*, double*, bool, cudaStream_t, int, int);
 template cudaError_t launch_tiled_step<float, kModel2HDM>(const TMaps&, const TMaps&, const StepParams&,
                                                           const LevelPtrs<float>&, const LevelPtrs<float>&, int, int,
                                                           unsigned*, double*, bool, cudaStream_t, int, int);

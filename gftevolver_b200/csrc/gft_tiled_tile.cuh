@@ -172,31 +172,56 @@ struct HaloStage {
 template <class S, int TY, int TZ, int ND>
 struct TileAcc;
 
-// The buffers of the values handed from site to site within a tile (gft_shared_body.cuh; SM
-// model), after the halo stage: for the y neighbours, slot y - y0 of the receiving row; for the
+// Whether a tile's sites hand their loops and transports to one another (gft_shared_body.cuh).
+// Not the float 2HDM's: with the hand-over buffers two CTAs fit an SM only over a ring of two
+// planes, and two doublets' values do not fit 128 registers beside the energy's or the ensemble's
+// list (us per step handed over / not: 192^3 plain 495 / 509, logging 736 / 660; 16 members of
+// 64^3 356 / 338).
+template <class S, int MODEL>
+constexpr bool hands_over()
+{
+    return MODEL == kModelSM || sizeof(S) == 8;
+}
+
+// Plane buffers of the one-site tiles' ring (run_ring): three, or two where only they leave two
+// CTAs per SM (the FP64 2HDM's, with its hand-over buffers).
+template <class S, int MODEL>
+constexpr int ring_planes()
+{
+    return MODEL != kModelSM && hands_over<S, MODEL>() ? 2 : 3;
+}
+
+// The buffers of the values handed from site to site within a tile (gft_shared_body.cuh), after
+// the halo stage: for the y neighbours, slot y - y0 of the receiving row; for the
 // z neighbours, the receiving row of the tile's first column.  Two planes of each: a plane's are
 // read after its barrier, while faster warps write the next plane's.
-template <class S, int TY, int TZ>
+template <class S, int MODEL, int TY, int TZ>
 struct HandBuf {
-    using H = HaloStage<S, TY, TZ, 1>;
+    static constexpr int ND = (MODEL == kModelSM) ? 1 : 2;
+    using H = HaloStage<S, TY, TZ, ND, ring_planes<S, MODEL>()>;
+    using V = Handed<S, ND>;
     static constexpr int QUAD = 4 * (int)sizeof(S);
-    static constexpr int YB = 3 * TY * TZ * QUAD, ZB = 3 * TY * QUAD;  // one plane's
+    static constexpr int YB = (2 + ND) * TY * TZ * QUAD, ZB = (2 + ND) * TY * QUAD;  // one plane's
     static constexpr int BYTES = 2 * (YB + ZB);
     static constexpr int OFFSET = (H::OFFSET + (sizeof(S) == 4 ? H::BYTES : 0) + 15) / 16 * 16;
     static constexpr int SMEM = OFFSET + BYTES + 128;  // + alignment slack of the dynamic base
 
-    __device__ __forceinline__ static void put(unsigned char* b, int n, int i, const Handed<S>& h)
+    __device__ __forceinline__ static void put(unsigned char* b, int n, int i, const V& h)
     {
         S* p = reinterpret_cast<S*>(b);
         st4(p, i, h.fa[0], h.fa[1], h.fa[2], h.sa);
         st4(p, n + i, h.fb[0], h.fb[1], h.fb[2], h.sb);
-        st4(p, 2 * n + i, h.t.w, h.t.x, h.t.y, h.t.z);
+#pragma unroll
+        for (int db = 0; db < ND; db++) st4(p, (2 + db) * n + i, h.t[db].w, h.t[db].x, h.t[db].y, h.t[db].z);
     }
-    __device__ __forceinline__ static Handed<S> get(const unsigned char* b, int n, int i)
+    __device__ __forceinline__ static V get(const unsigned char* b, int n, int i)
     {
-        using A = TileAcc<S, TY, TZ, 1>;
+        using A = TileAcc<S, TY, TZ, ND>;
         const Q<S> a = A::lds4(b, i), c = A::lds4(b, n + i);
-        return {{a.w, a.x, a.y}, a.z, {c.w, c.x, c.y}, c.z, A::lds4(b, 2 * n + i)};
+        V h = {{a.w, a.x, a.y}, a.z, {c.w, c.x, c.y}, c.z, {}};
+#pragma unroll
+        for (int db = 0; db < ND; db++) h.t[db] = A::lds4(b, (2 + db) * n + i);
+        return h;
     }
 };
 
@@ -379,26 +404,32 @@ struct RingPhase {
 // The plane ring of one tile (planes x0 .. x0+nloc-1 of columns y0.., z0..):
 // TMA copies, waits, wrapped-halo patches and one CTA barrier per plane.
 // body(i, bm, bc, bp) evolves the tile's sites of plane x0 + i from the staged
-// planes bc (x) and bp (x + 1), and with BACK also bm (x - 1); close(i) follows the
-// plane's barrier and reads none of them.  Without BACK,
+// planes bc (x) and bp (x + 1), and with NB = 4 also bm (x - 1); close(i) follows the
+// plane's barrier and reads none of them.  With NB < 4,
 // start(bc, bp) is called first, on the planes x0 - 1 and x0: what the first sites
-// need of the plane before them.  tid: the thread's index in the CTA
+// need of the plane before them.
+// NB, the plane buffers: with 3 (or 4) the copy of a plane is in flight while the one
+// before it is computed, and is waited for ahead of the barrier, which publishes its patches.
+// With 2 it is issued into the buffer that the barrier frees and lands during close(i); it is
+// waited for ahead of body, and a tile with wrapped halo cells takes a second barrier to publish them.
+// tid: the thread's index in the CTA
 // (the halo cells and the copy issue are divided by it).  smem: NBUF plane
 // buffers followed by NBUF initialised mbarriers; s_abort: a shared flag that
 // is 0 on entry.  Returns false (on every thread) if a wait gave up; the ring
 // is then drained and must not be reused.  LV: the level pointer struct (its
 // q / th / ph members are read).
-// STAGE: the wrapped halo cells of plane i+4 are copied by cp.async into
-// `stage` (HaloStage) while plane i+1 is computed, instead of prefetched into L2
+// STAGE: the wrapped halo cells of a plane are copied by cp.async into
+// `stage` (HaloStage) a plane ahead (NB = 2: with its copy), instead of prefetched into L2
 // and loaded after the plane's wait.
-template <class S, int TY, int TZ, int ND, class LV, bool STAGE, bool BACK, class Start, class Body, class Close>
+template <class S, int TY, int TZ, int ND, class LV, bool STAGE, int NB, class Start, class Body, class Close>
 __device__ __forceinline__ bool run_ring(const TMaps& maps, const TMaps& pmaps, const StepParams& P, const LV& now,
                                          int y0, int z0, int x0, int nloc, unsigned char* smem,
                                          unsigned long long* bars, RingPhase& ring, int* s_abort,
                                          unsigned char* stage, int tid, Start&& start, Body&& body,
                                          Close&& close)
 {
-    using G = Geom<S, TY, TZ, ND, BACK ? 4 : 3>;
+    using G = Geom<S, TY, TZ, ND, NB>;
+    constexpr bool BACK = NB == 4, LATE = NB == 2;
     // the plane whose buffer is free once plane i has been computed: i + FREE (relative planes)
     constexpr int FREE = BACK ? 0 : 1;
     const int nplanes = nloc + 2;  // planes x0-1 .. x0+nloc
@@ -413,6 +444,21 @@ __device__ __forceinline__ bool run_ring(const TMaps& maps, const TMaps& pmaps, 
     auto issue = [&](int p) {
         issue_plane<S, TY, TZ, ND>(maps, smem + slot(p) * G::BUF, &bars[slot(p)], plane_x(p), y0, z0);
     };
+    auto wait = [&](int p) { return mbar_wait_bounded(&bars[slot(p)], parity(p), P.wait_limit_ns); };
+    auto halo_ahead = [&](int p) {
+        if constexpr (STAGE)
+            stage_wrapped_halo<S, TY, TZ, ND>(P, now, plane_x(p), y0, z0, tid, stage);
+        else
+            prefetch_wrapped_halo<S, TY, TZ, ND>(P, now, plane_x(p), y0, z0, tid);
+    };
+    auto patch = [&](int p) {
+        if constexpr (STAGE)
+            patch_from_stage<S, TY, TZ, ND>(P, smem + slot(p) * G::BUF, y0, z0, tid, stage);
+        else
+            patch_wrapped_halo<S, TY, TZ, ND>(P, now, smem + slot(p) * G::BUF, plane_x(p), y0, z0, tid);
+    };
+
+    constexpr int FIRST = LATE ? 2 : 3;  // planes resident and patched before the first body
     if (tid == 0) {
         for (int p = 0; p < min(G::NBUF, nplanes); p++) issue(p);
     }
@@ -420,17 +466,11 @@ __device__ __forceinline__ bool run_ring(const TMaps& maps, const TMaps& pmaps, 
         // past level of the first two planes computed (relative planes 1 and 2)
         for (int p = 1; p <= 2 && p <= nloc; p++) prefetch_past<ND>(pmaps, plane_x(p), y0, z0);
     }
-    if (wraps && nplanes > 3) {
-        if constexpr (STAGE)
-            stage_wrapped_halo<S, TY, TZ, ND>(P, now, plane_x(3), y0, z0, tid, stage);
-        else
-            prefetch_wrapped_halo<S, TY, TZ, ND>(P, now, plane_x(3), y0, z0, tid);
-    }
+    if (wraps && FIRST < nplanes) halo_ahead(FIRST);
 
-    // planes 0, 1, 2 (x0-1, x0, x0+1) resident and patched before the first site
     bool ok = true;
-    for (int p = 0; p < 3; p++) {  // nplanes >= 3
-        ok = ok && mbar_wait_bounded(&bars[slot(p)], parity(p), P.wait_limit_ns);
+    for (int p = 0; p < FIRST; p++) {  // nplanes >= 3
+        ok = ok && wait(p);
         if (ok && wraps) patch_wrapped_halo<S, TY, TZ, ND>(P, now, smem + slot(p) * G::BUF, plane_x(p), y0, z0, tid);
     }
     if (!ok) *s_abort = 1;
@@ -447,40 +487,37 @@ __device__ __forceinline__ bool run_ring(const TMaps& maps, const TMaps& pmaps, 
         }
     }
 
-    // One CTA barrier per plane: after computing plane i the threads wait for (and patch)
-    // plane i+3, which the next site needs, then synchronise once; that barrier publishes
-    // the patches and what the sites hand over, and frees a plane's buffer for the next copy.
     for (int i = 0; i < nloc && !aborted; i++) {
-        body(i, smem + slot(i) * G::BUF, smem + slot(i + 1) * G::BUF, smem + slot(i + 2) * G::BUF);
-
         const int nxt = i + FREE + G::NBUF;  // the plane copied into the buffer freed by this one
-        // plane i+3 (x+2) for the next site; its copy was issued one plane ago
         bool okn = true;
-        if (i + 3 < nplanes) {
-            okn = mbar_wait_bounded(&bars[slot(i + 3)], parity(i + 3), P.wait_limit_ns);
-            if (okn && wraps) {
-                if constexpr (STAGE)
-                    patch_from_stage<S, TY, TZ, ND>(P, smem + slot(i + 3) * G::BUF, y0, z0, tid, stage);
-                else
-                    patch_wrapped_halo<S, TY, TZ, ND>(P, now, smem + slot(i + 3) * G::BUF, plane_x(i + 3), y0, z0,
-                                                      tid);
+        if constexpr (LATE) {
+            // plane i+2, issued after the last barrier
+            okn = wait(i + 2);
+            if (wraps) {
+                if (okn) patch(i + 2);
+                __syncthreads();
+            }
+            okn = __all_sync(0xffffffffu, okn);  // the body's shuffles need the whole warp
+        }
+        if (okn)
+            body(i, smem + slot(i) * G::BUF, smem + slot(i + 1) * G::BUF, smem + slot(i + 2) * G::BUF);
+        if constexpr (!LATE) {
+            // plane i+3 (x+2) for the next site; its copy was issued one plane ago
+            if (i + 3 < nplanes) {
+                okn = wait(i + 3);
+                if (okn && wraps) patch(i + 3);
             }
         }
         if (!okn) *s_abort = 1;
         __syncthreads();
-        if (*s_abort) {  // planes 0 .. i+2 were waited; the last copy issued was plane nxt-1 <= i+3
+        if (*s_abort) {  // the planes before these were waited for; the last copy issued was plane nxt-1
             aborted = true;
-            drain0 = i + 3;
+            drain0 = LATE ? i + 2 : i + 3;
             drain1 = min(nplanes, nxt);
             break;
         }
         if (tid == 32 % (TY * TZ) && i + 3 <= nloc) prefetch_past<ND>(pmaps, plane_x(i + 3), y0, z0);
-        if (wraps && i + 4 < nplanes) {
-            if constexpr (STAGE)
-                stage_wrapped_halo<S, TY, TZ, ND>(P, now, plane_x(i + 4), y0, z0, tid, stage);
-            else
-                prefetch_wrapped_halo<S, TY, TZ, ND>(P, now, plane_x(i + 4), y0, z0, tid);
-        }
+        if (wraps && i + FIRST + 1 < nplanes) halo_ahead(i + FIRST + 1);
         if (tid == 0 && nxt < nplanes) issue(nxt);
         close(i);
     }
@@ -520,15 +557,27 @@ __device__ __forceinline__ Stencil<TRef> plane_stencil(const unsigned char* bm, 
     return n;
 }
 
+// Whether a step stages its wrapped halo cells: HaloStage holds FP32 records, and the room for
+// them is there beside the hand-over buffers.
+template <class S, int MODEL, int TY, int TZ, bool ENERGY>
+constexpr bool tile_stage()
+{
+    if constexpr (hands_over<S, MODEL>())
+        return sizeof(S) == 4;
+    else
+        return HaloStage<S, TY, TZ, 2>::use(ENERGY);
+}
+
 // Evolves one tile by one step, one site per thread (threads TZ x TY).
-template <class S, int MODEL, int TY, int TZ, bool ENERGY, class LV, bool STAGE = false>
+template <class S, int MODEL, int TY, int TZ, bool ENERGY, class LV>
 __device__ __forceinline__ bool run_tile(const TMaps& maps, const TMaps& pmaps, const StepParams& P, const KConst<S>& F,
                                          const LV& now, const LV& past, int y0, int z0, int x0,
                                          int nloc, unsigned char* smem, unsigned long long* bars, RingPhase& ring,
                                          int* s_abort, double (&obs)[kObsCount], unsigned& warn)
 {
-    constexpr int ND = (MODEL == kModelSM) ? 1 : 2;
-    using G = Geom<S, TY, TZ, ND>;
+    constexpr int ND = (MODEL == kModelSM) ? 1 : 2, NB = ring_planes<S, MODEL>();
+    constexpr bool STAGE = tile_stage<S, MODEL, TY, TZ, ENERGY>();
+    using G = Geom<S, TY, TZ, ND, NB>;
     using Acc = TileAcc<S, TY, TZ, ND>;
     const int tz = threadIdx.x, ty = threadIdx.y;
     const int tid = ty * TZ + tz;
@@ -537,33 +586,32 @@ __device__ __forceinline__ bool run_tile(const TMaps& maps, const TMaps& pmaps, 
     const int ch0 = (ty + 1) * G::HP + (tz + 1) + G::TP - 1;
     const int y = y0 + ty, z = z0 + tz;
     XCarry<S, ND> carry;
-    carry.valid = false;
-    // Fixed y and z faces freeze whole columns, Fixed x faces the ends of a march
+    // Fixed y and z faces freeze whole columns, Fixed x faces the ends of a march: such sites
+    // hand over their loops and transports, and keep their own words
     const bool column_frozen = ((P.fixed_axes & 2) && (y == 0 || y == P.ny - 1)) ||
                                ((P.fixed_axes & 4) && (z == 0 || z == P.nz - 1));
     auto frozen_at = [&](int x) { return column_frozen || ((P.fixed_axes & 1) && (x == 0 || x == P.nx - 1)); };
-    auto site = [&](int x) { return (x * P.ny + y) * P.nz + z; };
     auto start = [&](const unsigned char* bc, const unsigned char* bp) {
         site_carry<S, ND>(Acc{}, plane_stencil<G::QP, G::HP>(bc, bc, bp, cq0, ch0), carry);
     };
-    unsigned char* stage = smem + HaloStage<S, TY, TZ, ND>::OFFSET;
-    if constexpr (MODEL == kModelSM) {
-        using HB = HandBuf<S, TY, TZ>;
-        OpenSite<S> o;
-        PastValues<S, 1, LV, !ENERGY> pv = {{past, 0}};
+    unsigned char* stage = smem + HaloStage<S, TY, TZ, ND, NB>::OFFSET;
+    if constexpr (hands_over<S, MODEL>()) {
+        using HB = HandBuf<S, MODEL, TY, TZ>;
+        OpenSite<S, ND> o;
+        PastValues<S, ND, LV, !ENERGY> pv = {{past, 0}};
         auto ybuf = [&](int i) { return smem + HB::OFFSET + (i & 1) * HB::YB; };
         auto zbuf = [&](int i) { return smem + HB::OFFSET + 2 * HB::YB + (i & 1) * HB::ZB; };
         constexpr int NW = TY * TZ / 32;  // warps of the tile
-        return run_ring<S, TY, TZ, ND, LV, STAGE, false>(
+        return run_ring<S, TY, TZ, ND, LV, STAGE, NB>(
             maps, pmaps, P, now, y0, z0, x0, nloc, smem, bars, ring, s_abort, stage, tid, start,
             [&](int i, const unsigned char*, const unsigned char* bc, const unsigned char* bp) {
-                {   // the halo row's and column's lanes, on warps that change with the plane
+                {  // the halo row's and column's lanes, on warps that change with the plane
                     const int h = (((tid >> 5) + i) % NW) * 32 + (tid & 31);
                     if (h < TZ + TY) {
                         const bool row = h < TZ;
                         const int ly = row ? 0 : h - TZ + 1, lz = row ? h + 1 : 0;
                         const int cq = ly * G::QP + lz, ch = ly * G::HP + lz + G::TP - 1;
-                        Handed<S> hh;
+                        Handed<S, ND> hh;
                         halo_hand_over<S>(Acc{}, row ? 1 : 2, TRef{bc, cq, ch}, TRef{bp, cq, ch},
                                           TRef{bc, cq + G::QP, ch + G::HP}, TRef{bc, cq + 1, ch + 1}, hh);
                         if (row)
@@ -572,12 +620,13 @@ __device__ __forceinline__ bool run_tile(const TMaps& maps, const TMaps& pmaps, 
                             HB::put(zbuf(i), TY, h - TZ, hh);
                     }
                 }
-                Handed<S> hy, hz;
-                site_open<S, ENERGY>(P, F, Acc{}, plane_stencil<G::QP, G::HP>(bc, bc, bp, cq0, ch0), carry, o, hy, hz);
+                Handed<S, ND> hy, hz;
+                site_open<S, MODEL, ENERGY>(P, F, Acc{}, plane_stencil<G::QP, G::HP>(bc, bc, bp, cq0, ch0), carry, o, hy,
+                                            hz);
                 if (ty + 1 < TY) HB::put(ybuf(i), TY * TZ, tid + TZ, hy);
                 // the z neighbour's, from the lane below; the first column's come through shared memory
                 const S lz = tz == 0 ? (S)0 : F.ldt[2];
-                Handed<S> hv;
+                Handed<S, ND> hv;
                 auto up = [](S v) { return __shfl_up_sync(0xffffffffu, v, 1, TZ < 32 ? TZ : 32); };
 #pragma unroll
                 for (int k = 0; k < 3; k++) {
@@ -586,20 +635,25 @@ __device__ __forceinline__ bool run_tile(const TMaps& maps, const TMaps& pmaps, 
                 }
                 hv.sa = up(hz.sa);
                 hv.sb = up(hz.sb);
-                hv.t = {up(hz.t.w), up(hz.t.x), up(hz.t.y), up(hz.t.z)};
+#pragma unroll
+                for (int db = 0; db < ND; db++) hv.t[db] = {up(hz.t[db].w), up(hz.t[db].x), up(hz.t[db].y), up(hz.t[db].z)};
                 receive(o, 0, 1, lz, hv);
-                pv.at.s = site(x0 + i);
-                if (!frozen_at(x0 + i)) pv.load();
+                const int x = x0 + i;
+                pv.at.s = (x * P.ny + y) * P.nz + z;
+                // ahead of the barrier: its wait covers the loads' latency (two doublets of doubles have
+                // no registers for them there)
+                if (ND == 1 && !frozen_at(x)) pv.load();
             },
             [&](int i) {
                 const int x = x0 + i;
                 if (frozen_at(x)) return;
+                if (ND == 2) pv.load();
                 receive(o, 0, 2, F.ldt[1], HB::get(ybuf(i), TY * TZ, tid));
                 if (tz == 0) receive(o, 0, 1, F.ldt[2], HB::get(zbuf(i), TY, ty));
                 site_close<S, ENERGY>(P, F, o, pv, obs, warn, counts(P, x));
             });
     } else {
-        return run_ring<S, TY, TZ, ND, LV, STAGE, false>(
+        return run_ring<S, TY, TZ, ND, LV, STAGE, NB>(
             maps, pmaps, P, now, y0, z0, x0, nloc, smem, bars, ring, s_abort, stage, tid, start,
             [&](int i, const unsigned char*, const unsigned char* bc, const unsigned char* bp) {
                 const Stencil<TRef> n = plane_stencil<G::QP, G::HP>(bc, bc, bp, cq0, ch0);
@@ -608,30 +662,22 @@ __device__ __forceinline__ bool run_tile(const TMaps& maps, const TMaps& pmaps, 
                 if (frozen_at(x))
                     site_carry<S, ND>(Acc{}, n, carry);  // not evolved; the next site needs its loops
                 else
-                    site_step<S, MODEL, ENERGY, kHfNone, true>(P, F, Acc{}, n, PastSite<S, LV>{past, site(x)}, carry,
+                    site_step<S, MODEL, ENERGY, kHfNone, true>(P, F, Acc{}, n,
+                                                               PastSite<S, LV>{past, (x * P.ny + y) * P.nz + z}, carry,
                                                                obs, warn, counts(P, x));
             },
             [](int) {});
     }
 }
 
-// Whether a step stages its wrapped halo cells (HaloStage; the SM tile's shared memory has the room).
-template <class S, int MODEL, int TY, int TZ, bool ENERGY>
-constexpr bool tile_stage()
-{
-    if constexpr (MODEL == kModelSM)
-        return sizeof(S) == 4;
-    else
-        return HaloStage<S, TY, TZ, 2>::use(ENERGY);
-}
-
 // Dynamic shared memory of a one-site tile kernel.
 template <class S, int MODEL, int TY, int TZ, bool ENERGY>
 constexpr int tile_smem()
 {
-    if constexpr (MODEL == kModelSM) {
-        static_assert(HandBuf<S, TY, TZ>::SMEM <= 227 * 1024 - 16 - 32 * kObsCount * 8, "shared memory of a tile");
-        return HandBuf<S, TY, TZ>::SMEM;
+    if constexpr (hands_over<S, MODEL>()) {
+        constexpr int b = HandBuf<S, MODEL, TY, TZ>::SMEM;
+        static_assert(b <= 227 * 1024 - 16 - 32 * kObsCount * 8, "shared memory of a tile");
+        return b;
     } else {
         return tile_stage<S, MODEL, TY, TZ, ENERGY>() ? HaloStage<S, TY, TZ, 2>::SMEM : Geom<S, TY, TZ, 2>::SMEM;
     }
@@ -642,7 +688,9 @@ constexpr int tile_smem()
 template <class S, int MODEL, int TY, int TZ>
 constexpr int tile_ctas()
 {
-    constexpr int smem = tile_smem<S, MODEL, TY, TZ, true>() + 16 + 32 * kObsCount * 8 + 1024;
+    constexpr int plain = tile_smem<S, MODEL, TY, TZ, false>();
+    constexpr int logging = tile_smem<S, MODEL, TY, TZ, true>() + 32 * kObsCount * 8;
+    constexpr int smem = (plain > logging ? plain : logging) + 16 + 1024;
     constexpr int by_smem = (228 * 1024) / smem, by_threads = 512 / (TY * TZ);
     constexpr int b = by_smem < by_threads ? by_smem : by_threads;
     return b < 1 ? 1 : b;

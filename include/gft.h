@@ -273,7 +273,7 @@ int gft_observe_static(const gft_config* cfg, const float* d_scalars, const floa
 /* Step-kernel selection for the throughput forms (no reference counterpart):
  * kind 0 = automatic (the tiled kernel when the lattice divides into a built
  * tile and the tiles fill enough waves of resident CTAs -- 0.9 of a wave for the SM
- * model, 3 for the 2HDM, 5 in the FP64 form of the SM model --, else the
+ * model and 3 for the 2HDM; in the FP64 form, in 8 x 16 tiles, 4 and 2.5 --, else the
  * one-thread-per-site kernel), 1 = one
  * thread per site with neighbours read through L1/L2, 2 = TMA-staged tiles
  * marching along x (mixed form; FP64 form of the SM model), 3 = as 2, with two sites per thread in paired

@@ -59,3 +59,29 @@ def test_fp64_default_tile_matches_one_thread_per_site(fixed):
     for a, b in zip(out[0][2], out[1][2]):
         for k in ("energy", "potential", "gradient", "kinetic", "magnetic", "electric"):
             assert abs(a[k] - b[k]) <= 1e-12 * abs(b["energy"]), k
+
+
+@pytest.mark.parametrize("fixed", [0, 7], ids=["periodic", "fixed"])
+@pytest.mark.parametrize("nx", [1, 2, 5, 34])
+def test_fp64_two_doublets_tile_matches_one_thread_per_site(nx, fixed):
+    """The FP64 2HDM's 8 x 16 tile over its ring of two planes, against the oracle-pinned
+    one-thread-per-site step: marches shorter than the ring, odd ones, and a second march of two
+    planes.  Bars as above."""
+    from gftevolver_b200 import Evolver, InitialData, LatticeParams
+    ny, nz = (768, 512) if nx < 34 else (384, 512)
+    p = LatticeParams(model=2, nx=nx, ny=ny, nz=nz, energy_every=2, gauss_every=2, fixed_axes=fixed)
+    ic = InitialData(seed=5, mean=[0.7] * 8, sigma=[0.1] * 8, theta_sigma=0.1, eps_sigma=0.1)
+    out = []
+    for kind in (0, 1):
+        with Evolver(p, form="fp64") as ev:
+            if kind:
+                ev.set_kernel(kind, 0, 32)
+            assert ev.step_kernel_name == ("fast_step_kernel" if kind else "tiled_step_kernel")
+            ev.init_fields(ic)
+            rows = ev.evolve(5)
+            out.append((*ev.download(), rows))
+    for a, b in zip(out[0][:2], out[1][:2]):
+        assert np.max(np.abs(a - b)) <= 1e-12 * np.max(np.abs(b))
+    for a, b in zip(out[0][2], out[1][2]):
+        for k in ("energy", "potential", "gradient", "kinetic", "magnetic", "electric"):
+            assert abs(a[k] - b[k]) <= 1e-12 * abs(b["energy"]), k
