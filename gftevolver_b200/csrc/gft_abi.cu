@@ -393,7 +393,8 @@ cudaError_t launch_step(gft_handle* h, const StepParams& P, int tn, const LevelP
 // Partial rows the Gauss kernel of this handle's form writes.
 int gauss_blocks(const gft_handle* h, const StepParams& P)
 {
-    return (h->cfg.form == GFT_FORM_REF) ? ref_launch_blocks(P) : fast_gauss_blocks(P);
+    return (h->cfg.form == GFT_FORM_REF) ? ref_launch_blocks(P)
+                                            : fast_gauss_blocks(P, h->cfg.form == GFT_FORM_MIXED);
 }
 
 template <class S>
@@ -550,7 +551,7 @@ int gft_create(const gft_config* cfg, gft_handle** out)
         h->tiled_ready = (h->tile_variant < kTiledVariants || h->tile_variant == kTileFP64) &&
                          encode_tiled(h, P, h->tile_variant, h->tm, h->tp);
     }
-    int nb = std::max(fast_launch_blocks(P, 0), fast_gauss_blocks(P));
+    int nb = std::max(fast_launch_blocks(P, 0), fast_gauss_blocks(P, cfg->form == GFT_FORM_MIXED));
     nb = std::max(nb, ref_launch_blocks(P));
     const size_t pe = (size_t)nb * kObsCount * sizeof(double), pg = (size_t)nb * 2 * h->neq * sizeof(double);
     h->rows_cap = 64;

@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "gft.h"
+#include "gft_gauss_body.cuh"
 #include "gft_launch.h"
 #include "gft_reduce.cuh"
 #include "gft_tiled_tile.cuh"
@@ -168,44 +169,52 @@ __global__ void __launch_bounds__(TY * TZ, tile_ctas<float, MODEL, TY, TZ>())
     if (warn) atomicOr(status, warn);
 }
 
-// Gauss-law residual over the same tiles: CTA (tile, i) takes plane i of the
-// tile's x-chunk, one thread per site (independent loads; a march of the
-// chunk's planes per thread serialises them: 0.948 against 0.866 ms on the
-// 64-member benchmark with 16 x 16 tiles, march 64), and writes partial row
-// tile * gridDim.y + i (zeros past the chunk's end).
-template <int MODEL, int TY, int TZ>
-__global__ void __launch_bounds__(TY * TZ) ensemble_gauss_kernel(const __grid_constant__ EnsParams ep,
-                                                                 const int4* __restrict__ items, int lx, int tn,
-                                                                 double* partials)
+// Gauss-law residual, one thread per site: block i takes sites [items[i].y, items[i].z) of member
+// items[i].x of the group and writes partial row items[i].w.
+constexpr int kGaussThreads = 256;
+
+template <int MODEL>
+__global__ void __launch_bounds__(kGaussThreads)
+    ensemble_gauss_kernel(const __grid_constant__ EnsParams ep, const int4* __restrict__ items, int tn, double* partials)
 {
-    const int it = blockIdx.x, i = blockIdx.y;
-    const int4 w = items[it];
-    const int m = w.x;
-    const StepParams& P = ep.P[m];
-    const int y = w.y + threadIdx.y, z = w.z + threadIdx.x;
-    const int ym = (y == 0) ? P.ny - 1 : y - 1, zm = (z == 0) ? P.nz - 1 : z - 1;
+    const int4 w = items[blockIdx.x];
+    const StepParams& P = ep.P[w.x];
     double v[kGaussSlots];
 #pragma unroll
     for (int k = 0; k < kGaussSlots; k++) v[k] = 0.0;
-    const int x = w.w + i, xm = (x == 0) ? P.nx - 1 : x - 1;
-    if (i < min(lx, P.nx - w.w) && counts(P, x) && !frozen(P, x, y, z)) {
-        gauss_site<float, MODEL>(P, ep.lv[m][tn], ep.lv[m][1 - tn], (x * P.ny + y) * P.nz + z,
-                                 (xm * P.ny + y) * P.nz + z, (x * P.ny + ym) * P.nz + z, (x * P.ny + y) * P.nz + zm,
-                                 v);
+    const int s = w.y + threadIdx.x, row = s / P.nz, z = s - row * P.nz, x = row / P.ny, y = row - x * P.ny;
+    if (s < w.z && counts(P, x) && !frozen(P, x, y, z)) {
+        const int plane = P.ny * P.nz;
+        gauss_site<float, MODEL>(P, ep.lv[w.x][tn], ep.lv[w.x][1 - tn], s, s + (x == 0 ? (P.nx - 1) * plane : -plane),
+                                 s + (y == 0 ? (P.ny - 1) * P.nz : -P.nz), s + (z == 0 ? P.nz - 1 : -1), v);
     }
-    block_reduce_store<kGaussSlots>(v, partials + ((size_t)it * gridDim.y + i) * kGaussSlots, 4);
+    block_reduce_store<kGaussSlots>(v, partials + (size_t)w.w * kGaussSlots, 4);
 }
 
-// One block per member: reduce its tiles' partial rows [first[m] * rpt,
-// first[m+1] * rpt) (rpt rows per tile) into slots [off, off + nslots) of its
-// observables row.
+// The same over planes [items[i].y, items[i].z) of gauss_planes' tiles, every link once
+// (gft_gauss_body.cuh).
+template <int MODEL>
+__global__ void __launch_bounds__(kGaussTileThreads, 2)
+    ensemble_gauss_tile_kernel(const __grid_constant__ EnsParams ep, const int4* __restrict__ items, int tn, double* partials)
+{
+    __shared__ GaussBuf sm;
+    const int4 w = items[blockIdx.x];
+    double v[kGaussSlots];
+#pragma unroll
+    for (int k = 0; k < kGaussSlots; k++) v[k] = 0.0;
+    gauss_planes<MODEL>(ep.P[w.x], ep.lv[w.x][tn], ep.lv[w.x][1 - tn], w.y, w.z, sm, v);
+    block_reduce_store<kGaussSlots>(v, partials + (size_t)w.w * kGaussSlots, 4);
+}
+
+// One block per member: reduce its partial rows [first[m], first[m + 1]) into
+// slots [off, off + nslots) of its observables row.
 __global__ void __launch_bounds__(kFinThreads) ensemble_finalize_kernel(const double* __restrict__ partials,
-                                                                        const int* __restrict__ first, int rpt,
-                                                                        int nslots, int max_from,
-                                                                        const double* scales, int off, double* rows)
+                                                                        const int* __restrict__ first, int nslots,
+                                                                        int max_from, const double* scales, int off,
+                                                                        double* rows)
 {
     const int m = blockIdx.x;
-    const double t = reduce_rows_block(partials, first[m] * rpt, first[m + 1] * rpt, nslots, max_from);
+    const double t = reduce_rows_block(partials, first[m], first[m + 1], nslots, max_from);
     if (threadIdx.x < (unsigned)nslots) {
         const size_t o = (size_t)m * kRowSlotCount + off + threadIdx.x;
         rows[o] = t * scales[o];
@@ -291,15 +300,6 @@ int resident_m(int variant)
     }
 }
 
-template <int MODEL, int TY, int TZ>
-cudaError_t launch_gauss_t(const EnsParams& ep, const int4* items, int nitems, int lx, int rows, int tn,
-                           double* partials, cudaStream_t s)
-{
-    if (nitems < 1) return cudaSuccess;
-    ensemble_gauss_kernel<MODEL, TY, TZ><<<dim3(nitems, rows, 1), dim3(TZ, TY, 1), 0, s>>>(ep, items, lx, tn, partials);
-    return cudaGetLastError();
-}
-
 template <int MODEL>
 cudaError_t launch_step_m(int variant, bool energy, bool uniform, const EnsParams& ep, const EnsMaps* maps,
                           const GroupTiles& gt, int lx, int tn, unsigned* status, double* partials, int nsm,
@@ -317,16 +317,14 @@ cudaError_t launch_step_m(int variant, bool energy, bool uniform, const EnsParam
 #undef GFT_ENS_STEP
 }
 
+// Both kinds of shares of one group: ntile of them in tiles, then nsite of single sites.
 template <int MODEL>
-cudaError_t launch_gauss_m(int variant, const EnsParams& ep, const int4* items, int nitems, int lx, int rows, int tn,
-                           double* partials, cudaStream_t s)
+cudaError_t launch_gauss(const EnsParams& ep, const int4* items, int ntile, int nsite, int tn, double* partials,
+                         cudaStream_t s)
 {
-    switch (variant) {
-    case 0: return launch_gauss_t<MODEL, 8, 32>(ep, items, nitems, lx, rows, tn, partials, s);
-    case 1: return launch_gauss_t<MODEL, 4, 32>(ep, items, nitems, lx, rows, tn, partials, s);
-    case 2: return launch_gauss_t<MODEL, 4, 16>(ep, items, nitems, lx, rows, tn, partials, s);
-    default: return launch_gauss_t<MODEL, 16, 16>(ep, items, nitems, lx, rows, tn, partials, s);
-    }
+    if (ntile > 0) ensemble_gauss_tile_kernel<MODEL><<<ntile, kGaussTileThreads, 0, s>>>(ep, items, tn, partials);
+    if (nsite > 0) ensemble_gauss_kernel<MODEL><<<nsite, kGaussThreads, 0, s>>>(ep, items + ntile, tn, partials);
+    return cudaGetLastError();
 }
 
 constexpr int kMaxGraphPeriod = 256;
@@ -372,8 +370,11 @@ struct gft_batch {
     double* d_part_e = nullptr;
     double* d_part_g = nullptr;
     int part_cap = 0;           // tiles the energy partials hold
-    long long part_cap_g = 0;   // rows the Gauss partials hold (tiles x gauss_rows)
-    int gauss_rows = 32;        // Gauss partial rows per tile: planes of the longest chunk, min(lx, max nx)
+    int part_cap_g = 0;         // rows the Gauss partials hold
+    int4* d_gauss_items = nullptr;  // the Gauss pass's shares, by group; within it those in tiles first
+    int* d_gauss_first = nullptr;   // first partial row of each member (+ end)
+    std::vector<int> group_gauss;   // first share of each group (+ end)
+    std::vector<int> group_tiles;   // how many of its shares are in tiles
     double* d_scale = nullptr;  // [n][kRowSlotCount]
     double* d_rows = nullptr;   // [rows_cap][n][kRowSlotCount]
     int rows_cap = 0;
@@ -501,6 +502,38 @@ void balance_tiles(const std::vector<int4>& items, int i0, int ni, const std::ve
     }
 }
 
+// The Gauss pass's shares of the members, each a partial row: 8 to 32 planes of gauss_planes' tiles;
+// single sites where more than a third of the tiles' sites would lie past the member's edges (nz =
+// 16, say), which costs what the links' reuse gains.  A member's shares depend on its shape alone, so
+// its rows do not on the ensemble's other members.  us per pass over 32 members of 32^3 to 96^3,
+// tiles / sites: SM 325 / 451; 16 of 64^3: SM 142 / 191, 2HDM 228 / 231; 16 of 48^3: 87 / 89.
+void gauss_shares(const gft_batch* b, std::vector<int4>& items, std::vector<int>& first, std::vector<int>& group,
+                  std::vector<int>& tiles)
+{
+    first.assign(b->n + 1, 0);
+    group.assign(b->ngroups() + 1, 0);
+    tiles.assign(b->ngroups(), 0);
+    for (int g = 0; g < b->ngroups(); g++) {
+        std::vector<int4> single;
+        int row = (int)items.size();
+        for (int m = g * kGroup; m < std::min(b->n, (g + 1) * kGroup); m++) {
+            const StepParams P = config_params(b->cfg[m], b->nsite[m], false, 0, false);
+            const long long planes = gauss_tile_planes(P);
+            const bool in_tiles = (double)planes * kGaussTileY * kGaussTileZ <= 1.5 * P.nsite;
+            const long long all = in_tiles ? planes : P.nsite;
+            const long long share = in_tiles ? std::min(32LL, std::max(8LL, planes / 64)) : kGaussThreads;
+            const long long n = (all + share - 1) / share;
+            for (long long i = 0; i < n; i++)
+                (in_tiles ? items : single)
+                    .push_back(make_int4(m - g * kGroup, (int)(all * i / n), (int)(all * (i + 1) / n), row++));
+            first[m + 1] = row;
+        }
+        tiles[g] = (int)items.size() - group[g];
+        items.insert(items.end(), single.begin(), single.end());
+        group[g + 1] = (int)items.size();
+    }
+}
+
 // Tile list, tensor maps and partial buffers for a tile shape and march depth.
 int configure(gft_batch* b, int variant, int lx)
 {
@@ -538,20 +571,30 @@ int configure(gft_batch* b, int variant, int lx)
     if (e == cudaSuccess) e = cudaMemcpy(b->d_items, items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(b->d_first, first.data(), first.size() * sizeof(int), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(b->d_maps, maps.data(), maps.size() * sizeof(EnsMaps), cudaMemcpyHostToDevice);
-    // energy partials: a row per tile; Gauss partials: a row per tile and plane of its chunk
-    int maxnx = 1;
-    for (const auto& c : b->cfg) maxnx = std::max(maxnx, c.nx);
-    const int grows = std::min(lx, maxnx);
-    if (e == cudaSuccess && ((int)items.size() > b->part_cap || (long long)items.size() * grows > b->part_cap_g)) {
+    std::vector<int4> gauss_items;
+    std::vector<int> gauss_first;
+    gauss_shares(b, gauss_items, gauss_first, b->group_gauss, b->group_tiles);
+    cudaFree(b->d_gauss_items);
+    cudaFree(b->d_gauss_first);
+    b->d_gauss_items = nullptr;
+    b->d_gauss_first = nullptr;
+    if (e == cudaSuccess) e = cudaMalloc(&b->d_gauss_items, gauss_items.size() * sizeof(int4));
+    if (e == cudaSuccess) e = cudaMalloc(&b->d_gauss_first, gauss_first.size() * sizeof(int));
+    if (e == cudaSuccess)
+        e = cudaMemcpy(b->d_gauss_items, gauss_items.data(), gauss_items.size() * sizeof(int4), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess)
+        e = cudaMemcpy(b->d_gauss_first, gauss_first.data(), gauss_first.size() * sizeof(int), cudaMemcpyHostToDevice);
+    // energy partials: a row per tile; Gauss partials: a row per share
+    const int rows_g = (int)gauss_items.size();
+    if (e == cudaSuccess && ((int)items.size() > b->part_cap || rows_g > b->part_cap_g)) {
         cudaFree(b->d_part_e);
         cudaFree(b->d_part_g);
         b->d_part_e = b->d_part_g = nullptr;
         e = cudaMalloc(&b->d_part_e, items.size() * kObsCount * sizeof(double));
-        if (e == cudaSuccess) e = cudaMalloc(&b->d_part_g, items.size() * (size_t)grows * kGaussSlots * sizeof(double));
+        if (e == cudaSuccess) e = cudaMalloc(&b->d_part_g, (size_t)rows_g * kGaussSlots * sizeof(double));
         b->part_cap = (e == cudaSuccess) ? (int)items.size() : 0;
-        b->part_cap_g = (e == cudaSuccess) ? (long long)items.size() * grows : 0;
+        b->part_cap_g = (e == cudaSuccess) ? rows_g : 0;
     }
-    b->gauss_rows = grows;
     if (e != cudaSuccess) return b->cuda_fail(e, "gft_batch: configure");
     b->nitems = (int)items.size();
     b->variant = variant;
@@ -611,7 +654,7 @@ cudaError_t issue_step_family(gft_batch* b, int ti, bool e, bool g, double* rows
             *nlaunch += finalize_launches(&job, 1);
         }
         if (err == cudaSuccess && g) {
-            const int nb = fast_gauss_blocks(P);
+            const int nb = fast_gauss_blocks(P, true);
             err = launch_fast_gauss<float, kModel2HDM>(P, b->lv[m][tn], b->lv[m][tp], b->d_part_f, b->stream);
             const FinJob job = {b->d_part_f, nb, 2 * b->neq, b->neq, scale + kObsCount, row + kObsCount};
             if (err == cudaSuccess) err = launch_finalize(&job, 1, b->d_mid, b->stream);
@@ -641,7 +684,7 @@ cudaError_t issue_step(gft_batch* b, int ti, bool e, bool g, double* rows, long 
         (*nlaunch)++;
     }
     if (err == cudaSuccess && e) {
-        ensemble_finalize_kernel<<<b->n, kFinThreads, 0, b->stream>>>(b->d_part_e, b->d_first, 1, kObsCount, kObsCount,
+        ensemble_finalize_kernel<<<b->n, kFinThreads, 0, b->stream>>>(b->d_part_e, b->d_first, kObsCount, kObsCount,
                                                                       b->d_scale, 0, rows);
         err = cudaGetLastError();
         (*nlaunch)++;
@@ -649,17 +692,14 @@ cudaError_t issue_step(gft_batch* b, int ti, bool e, bool g, double* rows, long 
     if (err == cudaSuccess && g) {
         for (int gr = 0; gr < b->ngroups() && err == cudaSuccess; gr++) {
             fill_params(b, gr, ti, false, &ep);
-            const int i0 = b->group_item[gr], ni = b->group_item[gr + 1] - i0;
+            const int g0 = b->group_gauss[gr], nt = b->group_tiles[gr], ns = b->group_gauss[gr + 1] - g0 - nt;
             err = (b->model == GFT_MODEL_SM)
-                      ? launch_gauss_m<kModelSM>(b->variant, ep, b->d_items + i0, ni, b->lx, b->gauss_rows, tn,
-                                                 b->d_part_g + (size_t)i0 * b->gauss_rows * kGaussSlots, b->stream)
-                      : launch_gauss_m<kModel2HDM>(b->variant, ep, b->d_items + i0, ni, b->lx, b->gauss_rows, tn,
-                                                   b->d_part_g + (size_t)i0 * b->gauss_rows * kGaussSlots,
-                                                   b->stream);
-            (*nlaunch)++;
+                      ? launch_gauss<kModelSM>(ep, b->d_gauss_items + g0, nt, ns, tn, b->d_part_g, b->stream)
+                      : launch_gauss<kModel2HDM>(ep, b->d_gauss_items + g0, nt, ns, tn, b->d_part_g, b->stream);
+            *nlaunch += (nt > 0) + (ns > 0);
         }
         if (err == cudaSuccess) {
-            ensemble_finalize_kernel<<<b->n, kFinThreads, 0, b->stream>>>(b->d_part_g, b->d_first, b->gauss_rows, kGaussSlots, 4,
+            ensemble_finalize_kernel<<<b->n, kFinThreads, 0, b->stream>>>(b->d_part_g, b->d_gauss_first, kGaussSlots, 4,
                                                                           b->d_scale, kObsCount, rows);
             err = cudaGetLastError();
             (*nlaunch)++;
@@ -860,7 +900,7 @@ int gft_batch_create(const gft_config* cfgs, int n, gft_batch** out)
         int rows = 0;
         for (int m = 0; m < n; m++) {
             const StepParams P = config_params(b->cfg[m], b->nsite[m], false, 0, false);
-            rows = std::max(rows, std::max(fast_launch_blocks(P, 0), fast_gauss_blocks(P)));
+            rows = std::max(rows, std::max(fast_launch_blocks(P, 0), fast_gauss_blocks(P, true)));
         }
         e = cudaMalloc(&b->d_part_f, (size_t)rows * kMaxSlots * sizeof(double));
         if (e == cudaSuccess) e = cudaMalloc(&b->d_mid, (size_t)kFinMidCapacity * sizeof(double));
@@ -892,6 +932,8 @@ void gft_batch_destroy(gft_batch* b)
     cudaFree(b->d_items);
     cudaFree(b->d_order);
     cudaFree(b->d_start);
+    cudaFree(b->d_gauss_items);
+    cudaFree(b->d_gauss_first);
     cudaFree(b->d_first);
     cudaFree(b->d_part_e);
     cudaFree(b->d_part_g);

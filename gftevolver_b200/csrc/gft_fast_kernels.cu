@@ -7,6 +7,7 @@
 #include "gft_device.cuh"
 #include "gft_launch.h"
 #include "gft_math.cuh"
+#include "gft_gauss_body.cuh"
 #include "gft_step_body.cuh"
 
 namespace gft {
@@ -182,6 +183,23 @@ __global__ void __launch_bounds__(kGaussThreads) fast_gauss_kernel(StepParams P,
     block_reduce_store<NG>(v, partials + (size_t)blk * NG, NG / 2);
 }
 
+// The same over 7 x 32 tiles marching along x, the FP32 fields' links once each
+// (gft_gauss_body.cuh).  Two blocks per SM, each an equal share of all tiles' planes.
+constexpr int kGaussCtas = 2 * 148;
+
+template <int MODEL>
+__global__ void __launch_bounds__(kGaussTileThreads, 2)
+    gauss_tile_kernel(StepParams P, LevelPtrs<float> now, LevelPtrs<float> fut, double* partials)
+{
+    __shared__ GaussBuf sm;
+    double v[kGaussSlots];
+#pragma unroll
+    for (int k = 0; k < kGaussSlots; k++) v[k] = 0.0;
+    const long long w = gauss_tile_planes(P);
+    gauss_planes<MODEL>(P, now, fut, (int)(w * blockIdx.x / gridDim.x), (int)(w * (blockIdx.x + 1) / gridDim.x), sm, v);
+    block_reduce_store<kGaussSlots>(v, partials + (size_t)blockIdx.x * kGaussSlots, 4);
+}
+
 template <class S, int MODEL, int HF>
 void fast_step_launch(const StepParams& P, const LevelPtrs<S>& now, const LevelPtrs<S>& past, unsigned* status,
                       double* partials, bool energy, cudaStream_t stream)
@@ -223,7 +241,22 @@ int fast_launch_blocks(const StepParams& P, int /*variant*/)
 {
     return use_roles(P) ? role_launch_blocks(P) : patch_blocks(P, kStepThreads);
 }
-int fast_gauss_blocks(const StepParams& P) { return patch_blocks(P, kGaussThreads); }
+
+// The mixed form's Gauss pass runs in tiles from 300,000 sites on (its 296 blocks then march five planes or more) where at most a third of the tiles' sites lie past a ragged
+// edge.  us per pass with its reduction, tiles / one thread per site: SM 48^3 17 / 15, 64^3 20 / 21,
+// 100^3 46 / 63, 150 x 100 x 75 50 / 67, 128^3 72 / 103, 256^3 465 / 692; 2HDM 64^3 23 / 21, 96^3 49 / 57,
+// 192^3 280 / 308.  The FP64 form's words would not fit the registers; it keeps one thread per site.
+constexpr int kGaussTileSites = 300000;
+static bool gauss_in_tiles(const StepParams& P, bool fp32)
+{
+    const double padded = (double)gauss_tile_planes(P) * kGaussTileY * kGaussTileZ;
+    return fp32 && P.hf == kHfNone && P.nsite >= kGaussTileSites && padded <= 1.5 * P.nsite;
+}
+
+int fast_gauss_blocks(const StepParams& P, bool fp32)
+{
+    return gauss_in_tiles(P, fp32) ? kGaussCtas : patch_blocks(P, kGaussThreads);
+}
 
 // P.hf selects the Higgs-family variant (2HDM only); the Gauss kernel writes
 // 2 * gaugeNum partial slots per block.
@@ -249,6 +282,12 @@ template <class S, int MODEL>
 cudaError_t launch_fast_gauss(const StepParams& P, const LevelPtrs<S>& now, const LevelPtrs<S>& fut, double* partials,
                               cudaStream_t stream)
 {
+    if constexpr (sizeof(S) == 4) {
+        if (gauss_in_tiles(P, true)) {
+            gauss_tile_kernel<MODEL><<<kGaussCtas, kGaussTileThreads, 0, stream>>>(P, now, fut, partials);
+            return cudaGetLastError();
+        }
+    }
     if constexpr (MODEL == kModel2HDM) {
         if (P.hf == kHfU1)
             fast_gauss_launch<S, MODEL, kHfU1>(P, now, fut, partials, stream);

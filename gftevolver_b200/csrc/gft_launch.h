@@ -34,7 +34,7 @@ cudaError_t launch_role_step(const StepParams& P, const LevelPtrs<S>& now, const
                              double* partials, bool energy, cudaStream_t stream);
 int role_launch_blocks(const StepParams& P);
 int fast_launch_blocks(const StepParams& P, int variant);
-int fast_gauss_blocks(const StepParams& P);
+int fast_gauss_blocks(const StepParams& P, bool fp32);
 
 // Tiled throughput kernel (gft_tiled_kernels.cu): TMA-staged planes, x-march.
 // Tensor maps of the "now" level: quaternions and doublets as {4 nz, ny, nx},
