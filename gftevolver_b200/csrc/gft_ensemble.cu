@@ -850,8 +850,12 @@ int gft_batch_create(const gft_config* cfgs, int n, gft_batch** out)
     b->cfg.assign(cfgs, cfgs + n);
     // 256-thread tiles before the smaller ones: a small tile's halo row and column are a larger part
     // of its work (32 members of 32 to 96 planes an edge, us per step at march 24: 16 x 16 397, 4 x 16
-    // 595; 12 of 32 and 64: 8 x 32 123, 16 x 16 117, 4 x 32 110, 4 x 16 143)
-    for (const int v : {0, 3, 1, 2})
+    // 595; 12 of 32 and 64: 8 x 32 123, 16 x 16 117, 4 x 32 110, 4 x 16 143).  Of those the SM model
+    // takes 16 x 16 first, whose halo is the shorter, the 2HDM 8 x 32, whose rows are (us per step 16 x
+    // 16 / 8 x 32, 16 members of 64^3: SM 264 / 275, logging 332 / 338, 2HDM 345 / 338; 12 of 96^3: SM 610 /
+    // 628, logging 768 / 788, 2HDM 790 / 783; 32 of 32^3: SM 86 / 92, 2HDM 105 / 102).
+    const bool sm = b->model == GFT_MODEL_SM;
+    for (const int v : {sm ? 3 : 0, sm ? 0 : 3, 1, 2})
         if (b->variant < 0 && variant_fits(b, v)) b->variant = v;
     if (b->variant < 0 && b->hf == kHfNone) {
         delete b;
