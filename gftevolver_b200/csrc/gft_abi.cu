@@ -553,6 +553,8 @@ int gft_create(const gft_config* cfg, gft_handle** out)
     }
     int nb = std::max(fast_launch_blocks(P, 0), fast_gauss_blocks(P, cfg->form == GFT_FORM_MIXED));
     nb = std::max(nb, ref_launch_blocks(P));
+    // a lattice one plane thick has more 4 x 16 tiles than 32-wide blocks (nz = 48: three to two)
+    if (h->tiled_ready) nb = std::max(nb, tiled_blocks(P, h->tile_variant, h->march));
     const size_t pe = (size_t)nb * kObsCount * sizeof(double), pg = (size_t)nb * 2 * h->neq * sizeof(double);
     h->rows_cap = 64;
     if ((e = cudaMalloc(&h->d_status, sizeof(unsigned))) != cudaSuccess ||

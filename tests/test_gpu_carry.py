@@ -85,3 +85,23 @@ def test_fp64_two_doublets_tile_matches_one_thread_per_site(nx, fixed):
     for a, b in zip(out[0][2], out[1][2]):
         for k in ("energy", "potential", "gradient", "kinetic", "magnetic", "electric"):
             assert abs(a[k] - b[k]) <= 1e-12 * abs(b["energy"]), k
+
+
+def test_one_plane_of_small_tiles_keeps_every_partial_row():
+    """A lattice one plane thick whose edges admit 4 x 16 tiles only: 1,203 of them, more than the
+    one-thread-per-site step has blocks, each with its row of partial energies.  The rows of the two
+    steps agree as their sums do: 1e-5 of the total energy, the mixed form's bar."""
+    from gftevolver_b200 import Evolver, InitialData, LatticeParams
+    p = LatticeParams(model=1, nx=1, ny=1604, nz=48, energy_every=1)
+    ic = InitialData(seed=5, mean=[1.0] * 8, sigma=[0.1] * 8, theta_sigma=0.1, eps_sigma=0.1)
+    out = []
+    for kind in (0, 1):
+        with Evolver(p, form="mixed") as ev:
+            if kind:
+                ev.set_kernel(kind, 0, 32)
+            assert ev.step_kernel_name == ("fast_step_kernel" if kind else "tiled_step_kernel")
+            ev.init_fields(ic)
+            out.append(ev.evolve(3))
+    for a, b in zip(*out):
+        for k in ("energy", "potential", "gradient", "kinetic", "magnetic", "electric"):
+            assert abs(a[k] - b[k]) <= 1e-5 * abs(b["energy"]), k
