@@ -123,8 +123,8 @@ __device__ __forceinline__ void advance_link(const KConst<S>& F, S* out, int s, 
     e = fma(Un.x, Un.x, e);
     e = fma(Un.y, Un.y, e);
     e = fma(Un.z, Un.z, e);
-    const C a = sqrt1m_minus1(cm) + e * ((C)0.375 * e - (C)0.5);
-    const Q<C> dU = qmul(Q<C>{a, R1, R2, R3}, Un);
+    const C f = e * ((C)0.375 * e - (C)0.5), u0m1 = sqrt1m_minus1(cm), a = fma(f, u0m1, u0m1 + f);
+    const Q<C> dU = qmul(Q<C>{a, fma(f, R1, R1), fma(f, R2, R2), fma(f, R3, R3)}, Un);
     check += a;
     st4(out, s, Un.w + dU.w, Un.x + dU.x, Un.y + dU.y, Un.z + dU.z);
 }

@@ -105,3 +105,23 @@ def test_one_plane_of_small_tiles_keeps_every_partial_row():
     for a, b in zip(*out):
         for k in ("energy", "potential", "gradient", "kinetic", "magnetic", "electric"):
             assert abs(a[k] - b[k]) <= 1e-5 * abs(b["energy"]), k
+
+
+@pytest.mark.parametrize("model,shape,kind", [(1, (16, 16, 16), 0), (1, (40, 40, 40), 0), (1, (8, 24, 96), 2),
+                                              (2, (16, 16, 16), 0), (2, (40, 40, 40), 0)])
+def test_fp64_step_renormalises_links_of_float_words(oracle_mod, model, shape, kind):
+    """FP64 form, links of float words (unit to 6e-8): the step leaves them unit to double rounding,
+    as the reference's renormalisation does.  Bar: |U|^2 - 1 of a link whose four words are each
+    rounded thrice, 8 ulp of 2.2e-16 with the norm's own evaluation."""
+    from gftevolver_b200 import Evolver, LatticeParams
+    op = oracle_mod.Params(model=model, nx=shape[0], ny=shape[1], nz=shape[2])
+    ic = oracle_mod.ICSpec(seed=23, mean=[1.0 if model == 1 else 0.7] * 8, sigma=[0.1] * 8, theta_sigma=0.1,
+                           eps_sigma=0.1)
+    sc, ve = (a.astype(np.float64) for a in oracle_mod.init_fields(op, ic, np.float32))
+    with Evolver(LatticeParams(**op.__dict__), form="fp64") as ev:
+        if kind:
+            ev.set_kernel(kind, 0, 4)
+        ev.upload(sc, ve, 0)
+        ev.evolve(1)
+        new = ev.download()[1][0].reshape(*shape, 3, 5)[..., 1:]  # the step from iteration 0 writes slot 0
+    assert np.max(np.abs(np.sum(new * new, -1) - 1.0)) <= 8 * 2.0 ** -52
