@@ -374,7 +374,7 @@ __device__ __forceinline__ double site_potential(const StepParams& P, const KCon
     double pot_e = 0.0;
     if (MODEL == kModelSM) {
         const C fsq = fc[0].w * fc[0].w + fc[0].x * fc[0].x + fc[0].y * fc[0].y + fc[0].z * fc[0].z;
-        const C k = F.diag - F.lambda * (fsq - F.eta_sqr);
+        const C k = F.diag + (F.rest - F.lambda * (fsq - F.eta_sqr));
         D[0] = {k * fc[0].w, k * fc[0].x, k * fc[0].y, k * fc[0].z};
         if (ENERGY) {
             const double t = (double)fsq - P.eta_sqr;
@@ -386,8 +386,8 @@ __device__ __forceinline__ double site_potential(const StepParams& P, const KCon
         const C s2 = f2.w * f2.w + f2.x * f2.x + f2.y * f2.y + f2.z * f2.z;
         const C dot = P.break_son ? f1.w * f2.w + f1.x * f2.x + f1.y * f2.y + f1.z * f2.z : (C)0;
         const C anti = (P.break_son && P.break_uhalfn) ? f1.w * f2.x - f1.x * f2.w + f1.y * f2.z - f1.z * f2.y : (C)0;
-        C a1 = F.diag1 - F.l1x4 * s1 - F.l3x2 * s2;
-        C a2 = F.diag2 - F.l2x4 * s2 - F.l3x2 * s1;
+        C a1 = F.m1x2 - F.l1x4 * s1 - F.l3x2 * s2;
+        C a2 = F.m2x2 - F.l2x4 * s2 - F.l3x2 * s1;
         const C f1v[4] = {f1.w, f1.x, f1.y, f1.z};
         const C f2v[4] = {f2.w, f2.x, f2.y, f2.z};
         C v1[4], v2[4];
@@ -401,8 +401,8 @@ __device__ __forceinline__ double site_potential(const StepParams& P, const KCon
                 // - 2 l6i|l7i anti f_self
                 const C cu = F.l5ix2 * dot + F.l6i * s1 + F.l7i * s2 - F.m12i - F.l4m5x2 * anti;
                 const C bo = bs + F.l5ix2 * anti;
-                a1 += F.l6ix2 * anti;
-                a2 += F.l7ix2 * anti;
+                a1 = F.diag + (a1 + F.l6ix2 * anti);
+                a2 = F.diag + (a2 + F.l7ix2 * anti);
 #pragma unroll
                 for (int k = 0; k < 4; k++) {
                     const int alt = 1 - 2 * (k % 2);
@@ -410,6 +410,8 @@ __device__ __forceinline__ double site_potential(const StepParams& P, const KCon
                     v2[k] = a2 * f2v[k] + bo * f1v[k] - cu * (C)alt * f1v[k + alt];
                 }
             } else {
+                a1 += F.diag;
+                a2 += F.diag;
 #pragma unroll
                 for (int k = 0; k < 4; k++) {
                     v1[k] = a1 * f1v[k] + bs * f2v[k];
@@ -417,6 +419,8 @@ __device__ __forceinline__ double site_potential(const StepParams& P, const KCon
                 }
             }
         } else {
+            a1 += F.diag;
+            a2 += F.diag;
 #pragma unroll
             for (int k = 0; k < 4; k++) {
                 v1[k] = a1 * f1v[k];
