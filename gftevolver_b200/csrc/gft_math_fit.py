@@ -5,7 +5,7 @@ the kernels evaluate (s = r^2):
   sin r = r + r^3 P(s) on |r| <= pi/2, weighted to the relative error of sin;
   cos r = 1 + s Q(s) on |r| <= pi/2, weighted to the absolute error of cos;
   asin x = x + x^3 A(x^2) on |x| <= 1/4 (float), 1/8 (double), relative error;
-  sqrt(1 - c) - 1 = c (-1/2 + c G(c)) on 0 <= c <= 1/64, relative error.
+  sqrt(1 - c) - 1 = -c/2 + c^2 G(c) on 0 <= c <= 1/64, relative error.
 Prints each polynomial's maximum error and its coefficients, lowest order first.
 """
 from mpmath import lu_solve, matrix, mp, mpf, pi
@@ -67,6 +67,6 @@ if __name__ == "__main__":
             ("sin double", SIN, lambda s: s / (1 + s * SIN(s)), HALF_PI_SQ, 7),
             ("cos double", COS, lambda s: s, HALF_PI_SQ, 7),
             ("asin double", ASIN, lambda s: s / (1 + s * ASIN(s)), mpf(1) / 64, 5),
-            ("sqrt1m double", SQRT, lambda c: c / (mpf(1) / 2 - c * SQRT(c)), mpf(1) / 64, 4)):
+            ("sqrt1m double", SQRT, lambda c: c / (mpf(1) / 2 - c * SQRT(c)), mpf(1) / 64, 5)):
         c, e = remez(f, lambda s, w=w: max(w(s), TINY), b, deg)
         print(f"{name}: error {mp.nstr(e, 3)}, coefficients {[mp.nstr(x, 18, min_fixed=0, max_fixed=0) for x in c]}")
