@@ -10,8 +10,9 @@
 //           error <= 2.5e-10 -- both below float's rounding, and two multiply-adds
 //           shorter each than the Taylor series of equal accuracy (degree 13 / 14);
 //   double: the same forms by the same fit in extended precision, sin of degree 17
-//           (relative error <= 2.8e-19), cos of degree 16 (absolute error <= 4.2e-18):
-//           three and four multiply-adds shorter than the Taylor series of equal use.
+//           (relative error <= 2.8e-19), cos of degree 18 (absolute error <= 6.8e-21; one
+//           degree less leaves no room for -1/2 to be exact, and its rounding counts at every
+//           angle): three multiply-adds shorter each than the Taylor series of equal use.
 // The reduction uses the 1.5*2^p rounding constant (no conversion to integer):
 // it holds for |x| < 1.3e7 (float) / 1.4e15 (double); phases that large do not
 // occur in the evolution (the step kernels flag |theta| > 1e4).
@@ -33,14 +34,15 @@ namespace gft {
 #define GFT_S13 (1.6058939705911306e-10)
 #define GFT_S15 (-7.64299148958033802e-13)
 #define GFT_S17 (2.72117496446829863e-15)
-#define GFT_C2 (-4.99999999999999825e-1)
-#define GFT_C4 (4.16666666666643693e-2)
-#define GFT_C6 (-1.38888888887856523e-3)
-#define GFT_C8 (2.48015872791490212e-5)
-#define GFT_C10 (-2.75573165252276417e-7)
-#define GFT_C12 (2.08765677410145851e-9)
-#define GFT_C14 (-1.14630393689959251e-11)
-#define GFT_C16 (4.61029415573876858e-14)
+#define GFT_C2 (-0.5)
+#define GFT_C4 (4.1666666666666661e-2)
+#define GFT_C6 (-1.38888888888885709e-3)
+#define GFT_C8 (2.48015873014999769e-5)
+#define GFT_C10 (-2.75573192104185647e-7)
+#define GFT_C12 (2.08767557145721576e-9)
+#define GFT_C14 (-1.14706719540102727e-11)
+#define GFT_C16 (4.77690866610973073e-14)
+#define GFT_C18 (-1.51229471791906704e-16)
 
 // Float minimax coefficients on |r| <= pi/2 (gft_math_fit.py): sin r = r + r^3 P(r^2), cos r = 1 + r^2 Q(r^2).
 #define GFT_FS3 (-0.16666659712791443f)
@@ -166,7 +168,8 @@ __device__ __forceinline__ void sincos_poly(double r, double& s, double& c)
     ps = fma(ps, r2, GFT_S5);
     ps = fma(ps, r2, GFT_S3);
     s = fma(ps * r2, r, r);
-    double pc = GFT_C16;
+    double pc = GFT_C18;
+    pc = fma(pc, r2, GFT_C16);
     pc = fma(pc, r2, GFT_C14);
     pc = fma(pc, r2, GFT_C12);
     pc = fma(pc, r2, GFT_C10);

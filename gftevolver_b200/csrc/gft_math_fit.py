@@ -65,7 +65,7 @@ if __name__ == "__main__":
             ("asin float", ASIN, lambda s: s / (1 + s * ASIN(s)), mpf(1) / 16, 3),
             ("sqrt1m float", SQRT, lambda c: c / (mpf(1) / 2 - c * SQRT(c)), mpf(1) / 64, 1),
             ("sin double", SIN, lambda s: s / (1 + s * SIN(s)), HALF_PI_SQ, 7),
-            ("cos double", COS, lambda s: s, HALF_PI_SQ, 7),
+            ("cos double", COS, lambda s: s, HALF_PI_SQ, 8),
             ("asin double", ASIN, lambda s: s / (1 + s * ASIN(s)), mpf(1) / 64, 5),
             ("sqrt1m double", SQRT, lambda c: c / (mpf(1) / 2 - c * SQRT(c)), mpf(1) / 64, 5)):
         c, e = remez(f, lambda s, w=w: max(w(s), TINY), b, deg)

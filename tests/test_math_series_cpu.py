@@ -60,8 +60,9 @@ int main()
     report<float>("sqrt1m_float", 1e-12, 1.0 / 64, true, [](float c) { return sqrt1m_series(c); }, long_sqrt1m);
     report<double>("sqrt1m_double", 1e-12, 1.0 / 64, true, [](double c) { return sqrt1m_series(c); }, long_sqrt1m);
     report<double>("sin_double", 1e-9, 1.5707963267948966, true, [](double r) { return sin_poly(r); }, long_sin);
-    report<double>("cos_double", 1e-9, 1.5707963267948966, false,
-                   [](double r) { double s, c; sincos_poly(r, s, c); return c; }, long_cos);
+    auto cosine = [](double r) { double s, c; sincos_poly(r, s, c); return c; };
+    report<double>("cos_double", 1e-9, 1.5707963267948966, false, cosine, long_cos);
+    report<double>("cos_double_small", 1e-9, 0.3, false, cosine, long_cos);
     report<float>("asin_float", 1e-6, 0.25, true, [](float x) { return asin_series(x); }, long_asin);
     report<double>("asin_double", 1e-9, 0.125, true, [](double x) { return asin_series(x); }, long_asin);
 }
@@ -93,3 +94,10 @@ def test_sines_and_arcsines_round_once_or_twice(errors):
     assert errors["asin_float"] <= 2.0 ** -24 * (1 + 4 / 96)
     assert errors["asin_double"] <= 2.0 ** -53 * (1 + 4 / 384) + 4.5e-19
     assert errors["sin_double"] <= 2.0 ** -53 * (1 + 3 * 0.58) + 2.8e-19
+
+
+def test_cosine_of_a_small_angle_keeps_its_half(errors):
+    """1 + r^2 Q(r^2), |r| <= 0.3: half an ulp of the sum, of r^2 (below 2^-3) times 1/2, and of Q (below
+    1/2) times r^2; nothing of the leading coefficient."""
+    assert errors["cos_double_small"] <= 2.0 ** -54 + 0.5 * 2.0 ** -57 + 0.09 * 2.0 ** -55 + 1e-19
+    assert errors["cos_double"] <= 2.0 ** -53 * (0.5 + 1 + 1.24)
