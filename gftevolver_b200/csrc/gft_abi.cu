@@ -90,6 +90,7 @@ struct gft_handle {
                             // between two threads on plain steps (SM)
     int tile_variant = 0;   // tiled: index into the built tile shapes
     int march = 32;         // tiled: planes per CTA along x (gft_create sets the form's)
+    int auto_tile = -1, auto_march = 32;  // what gft_create chose (-1: no tile), which kind 0 restores
     unsigned wait_limit_ns = 0;  // gft_set_wait_limit (0: the 2 s default)
     bool tiled_ready = false;
     TMaps tm[2];   // staged "now" planes (with halo), per level
@@ -309,6 +310,8 @@ constexpr double kAutoWavesSM = 0.9, kAutoWaves2HDM = 3.0, kAutoWavesFP64SM = 4.
 // 192^3 / 256^3 at 8, 12, 16, 32 planes 133 / 377 / 849, 133 / 376 / 830, 135 / 372 / 857,
 // 135 / 375 / 837 us; 96^3 58 at 12, 72 to 95 at the others.
 constexpr int kAutoMarchMixed = 12, kAutoMarchFP64 = 32;
+// gft_set_kernel's march where a caller names none (with tile 0: the automatic choice of gft_create)
+constexpr int kKernelMarchDefault = 32;
 
 bool use_tiled(const gft_handle* h, const StepParams& P)
 {
@@ -548,9 +551,10 @@ int gft_create(const gft_config* cfg, gft_handle** out)
             else if (cfg->model != GFT_MODEL_SM)
                 h->tile_variant = kTiledVariants;
         }
-        h->tiled_ready = (h->tile_variant < kTiledVariants || h->tile_variant == kTileFP64) &&
-                         encode_tiled(h, P, h->tile_variant, h->tm, h->tp);
+        h->tiled_ready = tiled_supported(P, h->tile_variant) && encode_tiled(h, P, h->tile_variant, h->tm, h->tp);
+        if (h->tiled_ready) h->auto_tile = h->tile_variant;
     }
+    h->auto_march = h->march;
     int nb = std::max(fast_launch_blocks(P, 0), fast_gauss_blocks(P, cfg->form == GFT_FORM_MIXED));
     nb = std::max(nb, ref_launch_blocks(P));
     // a lattice one plane thick has more 4 x 16 tiles than 32-wide blocks (nz = 48: three to two)
@@ -1186,13 +1190,16 @@ int gft_set_kernel(gft_handle* h, int kind, int tile, int march)
     cudaSetDevice(h->cfg.device);
     drop_graph(h);
     const StepParams P = make_params(h, h->time_iter, false);
-    if (!tiled_supported(P, tile)) {
-        if (kind == 0) {  // automatic: the tile shape chosen at creation, or one thread per site
-            h->kernel_kind = 0;
-            return GFT_OK;
-        }
-        return h->fail(GFT_E_UNSUPPORTED, "gft_set_kernel: the lattice shape does not divide into this tile");
+    const bool supported = tiled_supported(P, tile);
+    if (kind == 0 && (!supported || (tile == 0 && march == kKernelMarchDefault))) {
+        // automatic with nothing asked for, or with a tile the lattice does not divide into
+        h->tiled_ready = h->auto_tile >= 0 && encode_tiled(h, P, h->auto_tile, h->tm, h->tp);
+        if (h->tiled_ready) h->tile_variant = h->auto_tile;
+        h->march = h->auto_march;
+        h->kernel_kind = 0;
+        return GFT_OK;
     }
+    if (!supported) return h->fail(GFT_E_UNSUPPORTED, "gft_set_kernel: the lattice shape does not divide into this tile");
     TMaps tm[2], tp[2];
     if (!encode_tiled(h, P, tile, tm, tp))
         return h->fail(GFT_E_UNSUPPORTED, "gft_set_kernel: tensor map encoding failed");

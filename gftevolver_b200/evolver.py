@@ -287,7 +287,8 @@ class Evolver:
         _lib.check(self.lib.gft_set_wait_limit(self.h, int(ns)), self.h)
 
     def set_kernel(self, kind: int = 0, tile: int = 0, march: int = 32) -> None:
-        """Step kernel of the throughput forms: 0 auto, 1 one thread per site, 2 TMA-staged tiles."""
+        """Step kernel of the throughput forms: 0 auto, 1 one thread per site, 2 TMA-staged tiles.
+        With the defaults, the choice of a fresh evolver again; see gft_set_kernel."""
         _lib.check(self.lib.gft_set_kernel(self.h, int(kind), int(tile), int(march)), self.h)
 
     def observe(self) -> dict:

@@ -279,7 +279,9 @@ int gft_observe_static(const gft_config* cfg, const float* d_scalars, const floa
  * marching along x (mixed form; FP64 form of the SM model), 3 = as 2, with two sites per thread in paired
  * FP32 arithmetic on the plain (non-logging) steps (periodic SM model, tiles 0
  * and 3).  tile = tile shape (0: 8 x 32, 1: 4 x 32,
- * 2: 4 x 16, 3: 16 x 16 sites in y x z); march = planes per CTA along x.  Returns
+ * 2: 4 x 16, 3: 16 x 16 sites in y x z); march = planes per CTA along x.  Kind 0 with
+ * tile 0 and march 32 restores the tile and march gft_create chose; with others its
+ * choice is between those tiles and one thread per site.  Returns
  * GFT_E_UNSUPPORTED when the lattice does not divide into the tile or carries a
  * Higgs-family field (one thread per site serves those). */
 int gft_set_kernel(gft_handle* h, int kind, int tile, int march);

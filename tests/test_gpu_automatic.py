@@ -1,0 +1,52 @@
+"""gft_set_kernel with kind 0 and nothing else asked for: a fresh handle's choice again (GPU).
+
+Each lattice is on one side of the automatic rule with the tile and march gft_create chooses and on
+the other with those of the call before: SM mixed 128^3 takes tiles in marches of 12 planes, not of
+32; SM FP64 96 x 96 x 240 would take 4 x 16 tiles in marches of 8, not the 8 x 16 of its own.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("form,model,shape,before,name", [
+    ("mixed", 1, (128, 128, 128), (2, 0, 32), "tiled_step_kernel"),
+    ("mixed", 2, (192, 192, 192), (1, 0, 32), "tiled_step_kernel"),
+    ("mixed", 1, (64, 64, 48), (2, 2, 1), "fast_step_kernel"),
+    ("fp64", 1, (96, 96, 240), (2, 2, 8), "fast_step_kernel"),
+    ("fp64", 1, (3, 384, 512), (2, 3, 32), "tiled_step_kernel"),
+    ("fp64", 2, (3, 768, 512), (1, 0, 32), "tiled_step_kernel"),
+])
+def test_kind_0_restores_the_choice_made_at_creation(form, model, shape, before, name):
+    from gftevolver_b200 import Evolver, InitialData, LatticeParams
+    nx, ny, nz = shape
+    p = LatticeParams(model=model, nx=nx, ny=ny, nz=nz, energy_every=2)
+    ic = InitialData(seed=5, mean=[1.0 if model == 1 else 0.7] * 8, sigma=[0.1] * 8, theta_sigma=0.1, eps_sigma=0.1)
+    out = []
+    for restored in (False, True):
+        with Evolver(p, form=form) as ev:
+            if restored:
+                ev.set_kernel(*before)
+                ev.set_kernel()
+            assert ev.step_kernel_name == name
+            ev.init_fields(ic)
+            rows = ev.evolve(3)
+            out.append((rows, ev.launch_count, *ev.download()))
+    (rows, launches, sc, ve), again = out
+    assert rows == again[0] and launches == again[1]
+    np.testing.assert_array_equal(sc, again[2])
+    np.testing.assert_array_equal(ve, again[3])
+
+
+def test_kind_0_keeps_a_tile_it_is_given():
+    """Asked for a tile or march, kind 0 chooses between it and one thread per site, as before."""
+    from gftevolver_b200 import Evolver, LatticeParams
+    with Evolver(LatticeParams(model=1, nx=64, ny=64, nz=64), form="mixed") as ev:
+        assert ev.step_kernel_name == "fast_step_kernel"
+        ev.set_kernel(0, 2, 8)  # 4 x 16 tiles in marches of 8: 512 of them, under a wave
+        assert ev.step_kernel_name == "fast_step_kernel"
+        ev.set_kernel(0, 0, 2)  # 8 x 32 tiles in marches of 2: 512, 1.7 waves
+        assert ev.step_kernel_name == "tiled_step_kernel"
+        ev.set_kernel()
+        assert ev.step_kernel_name == "fast_step_kernel"
