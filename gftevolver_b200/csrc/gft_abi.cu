@@ -85,7 +85,7 @@ struct gft_handle {
     std::string err;
     size_t dev_bytes = 0;
     // step kernel selection for the throughput forms
-    int kernel_kind = 0;    // 0 auto, 1 global-memory kernel, 2 tiled (TMA) kernel, 3 tiled with two
+    int kernel_kind = 0;    // 0 auto, 1 one thread per site, 2 tiled (TMA) kernel, 3 tiled with two
                             // sites per thread on plain steps (SM), 4 tiled with each site split
                             // between two threads on plain steps (SM)
     int tile_variant = 0;   // tiled: index into the built tile shapes
@@ -347,7 +347,7 @@ int step_blocks(const gft_handle* h, const StepParams& P)
 {
     if (h->cfg.form == GFT_FORM_REF) return ref_launch_blocks(P);
     if (use_tiled(h, P)) return tiled_blocks(P, h->tile_variant, h->march);
-    return fast_launch_blocks(P, 0);
+    return fast_launch_blocks(P, h->kernel_kind != 1);
 }
 
 // `tn` is the index (0 or 1) of the handle level passed as `now`.
@@ -388,9 +388,10 @@ cudaError_t launch_step(gft_handle* h, const StepParams& P, int tn, const LevelP
                                                     h->d_status, h->d_part_e, energy, s, xa, xn);
         }
     }
+    const bool divide = h->kernel_kind != 1;
     if (model == GFT_MODEL_SM)
-        return launch_fast_step<S, kModelSM>(P, now, past, h->d_status, h->d_part_e, energy, 0, h->stream);
-    return launch_fast_step<S, kModel2HDM>(P, now, past, h->d_status, h->d_part_e, energy, 0, h->stream);
+        return launch_fast_step<S, kModelSM>(P, now, past, h->d_status, h->d_part_e, energy, divide, h->stream);
+    return launch_fast_step<S, kModel2HDM>(P, now, past, h->d_status, h->d_part_e, energy, divide, h->stream);
 }
 
 // Partial rows the Gauss kernel of this handle's form writes.
@@ -555,7 +556,8 @@ int gft_create(const gft_config* cfg, gft_handle** out)
         if (h->tiled_ready) h->auto_tile = h->tile_variant;
     }
     h->auto_march = h->march;
-    int nb = std::max(fast_launch_blocks(P, 0), fast_gauss_blocks(P, cfg->form == GFT_FORM_MIXED));
+    int nb = std::max(fast_launch_blocks(P, true), fast_launch_blocks(P, false));
+    nb = std::max(nb, fast_gauss_blocks(P, cfg->form == GFT_FORM_MIXED));
     nb = std::max(nb, ref_launch_blocks(P));
     // a lattice one plane thick has more 4 x 16 tiles than 32-wide blocks (nz = 48: three to two)
     if (h->tiled_ready) nb = std::max(nb, tiled_blocks(P, h->tile_variant, h->march));

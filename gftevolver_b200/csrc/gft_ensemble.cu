@@ -644,11 +644,11 @@ cudaError_t issue_step_family(gft_batch* b, int ti, bool e, bool g, double* rows
         const StepParams P = config_params(b->cfg[m], b->nsite[m], false, ti, e);
         const double* scale = b->d_scale + (size_t)m * kRowSlotCount;
         double* row = rows + (size_t)m * kRowSlotCount;
-        err = launch_fast_step<float, kModel2HDM>(P, b->lv[m][tn], b->lv[m][tp], b->d_status, b->d_part_f, e, 0,
+        err = launch_fast_step<float, kModel2HDM>(P, b->lv[m][tn], b->lv[m][tp], b->d_status, b->d_part_f, e, true,
                                                   b->stream);
         (*nlaunch)++;
         if (err == cudaSuccess && e) {
-            const int nb = fast_launch_blocks(P, 0);
+            const int nb = fast_launch_blocks(P, true);
             const FinJob job = {b->d_part_f, nb, kObsCount, kObsCount, scale, row};
             err = launch_finalize(&job, 1, b->d_mid, b->stream);
             *nlaunch += finalize_launches(&job, 1);
@@ -904,7 +904,7 @@ int gft_batch_create(const gft_config* cfgs, int n, gft_batch** out)
         int rows = 0;
         for (int m = 0; m < n; m++) {
             const StepParams P = config_params(b->cfg[m], b->nsite[m], false, 0, false);
-            rows = std::max(rows, std::max(fast_launch_blocks(P, 0), fast_gauss_blocks(P, true)));
+            rows = std::max(rows, std::max(fast_launch_blocks(P, true), fast_gauss_blocks(P, true)));
         }
         e = cudaMalloc(&b->d_part_f, (size_t)rows * kMaxSlots * sizeof(double));
         if (e == cudaSuccess) e = cudaMalloc(&b->d_mid, (size_t)kFinMidCapacity * sizeof(double));

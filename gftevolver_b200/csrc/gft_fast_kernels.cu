@@ -237,9 +237,9 @@ static int patch_blocks(const StepParams& P, int threads)
 constexpr int kRoleMaxSites = 16384;
 static bool use_roles(const StepParams& P) { return P.nsite <= kRoleMaxSites; }
 
-int fast_launch_blocks(const StepParams& P, int /*variant*/)
+int fast_launch_blocks(const StepParams& P, bool divide)
 {
-    return use_roles(P) ? role_launch_blocks(P) : patch_blocks(P, kStepThreads);
+    return divide && use_roles(P) ? role_launch_blocks(P) : patch_blocks(P, kStepThreads);
 }
 
 // The mixed form's Gauss pass runs in tiles from 300,000 sites on (its 296 blocks then march five planes or more) where at most a third of the tiles' sites lie past a ragged
@@ -262,9 +262,9 @@ int fast_gauss_blocks(const StepParams& P, bool fp32)
 // 2 * gaugeNum partial slots per block.
 template <class S, int MODEL>
 cudaError_t launch_fast_step(const StepParams& P, const LevelPtrs<S>& now, const LevelPtrs<S>& past, unsigned* status,
-                             double* partials, bool energy, int /*variant*/, cudaStream_t stream)
+                             double* partials, bool energy, bool divide, cudaStream_t stream)
 {
-    if (use_roles(P)) return launch_role_step<S, MODEL>(P, now, past, status, partials, energy, stream);
+    if (divide && use_roles(P)) return launch_role_step<S, MODEL>(P, now, past, status, partials, energy, stream);
     if constexpr (MODEL == kModel2HDM) {
         if (P.hf == kHfU1)
             fast_step_launch<S, MODEL, kHfU1>(P, now, past, status, partials, energy, stream);
@@ -303,7 +303,7 @@ cudaError_t launch_fast_gauss(const StepParams& P, const LevelPtrs<S>& now, cons
 
 #define GFT_INSTANTIATE_FAST(S, M)                                                                                   \
     template cudaError_t launch_fast_step<S, M>(const StepParams&, const LevelPtrs<S>&, const LevelPtrs<S>&,         \
-                                                unsigned*, double*, bool, int, cudaStream_t);                         \
+                                                unsigned*, double*, bool, bool, cudaStream_t);                        \
     template cudaError_t launch_fast_gauss<S, M>(const StepParams&, const LevelPtrs<S>&, const LevelPtrs<S>&,        \
                                                  double*, cudaStream_t);
 GFT_INSTANTIATE_FAST(float, kModelSM)

@@ -20,10 +20,11 @@ cudaError_t launch_ref_gauss(const StepParams& P, const LevelPtrs<S>& now, const
 int ref_launch_blocks(const StepParams& P);
 
 // Throughput forms (gft_fast_kernels.cu): FP64 plain form (S = double) and
-// mixed form (S = float).
+// mixed form (S = float).  divide: small lattices may divide a site's update over warps
+// (launch_role_step); else one thread per site whatever the size.
 template <class S, int MODEL>
 cudaError_t launch_fast_step(const StepParams& P, const LevelPtrs<S>& now, const LevelPtrs<S>& past, unsigned* status,
-                             double* partials, bool energy, int variant, cudaStream_t stream);
+                             double* partials, bool energy, bool divide, cudaStream_t stream);
 template <class S, int MODEL>
 cudaError_t launch_fast_gauss(const StepParams& P, const LevelPtrs<S>& now, const LevelPtrs<S>& fut, double* partials,
                               cudaStream_t stream);
@@ -33,7 +34,7 @@ template <class S, int MODEL>
 cudaError_t launch_role_step(const StepParams& P, const LevelPtrs<S>& now, const LevelPtrs<S>& past, unsigned* status,
                              double* partials, bool energy, cudaStream_t stream);
 int role_launch_blocks(const StepParams& P);
-int fast_launch_blocks(const StepParams& P, int variant);
+int fast_launch_blocks(const StepParams& P, bool divide);
 int fast_gauss_blocks(const StepParams& P, bool fp32);
 
 // Tiled throughput kernel (gft_tiled_kernels.cu): TMA-staged planes, x-march.

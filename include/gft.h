@@ -196,8 +196,9 @@ size_t gft_device_bytes(const gft_handle* h);
 double gft_step_kernel_ms(gft_handle* h, int* launches);
 
 /* Name of the step kernel gft_evolve launches for this handle's form, lattice and
- * gft_set_kernel choice ("ref_step_kernel", "fast_step_kernel" or
- * "tiled_step_kernel"; no reference counterpart). */
+ * gft_set_kernel choice: "ref_step_kernel", "tiled_step_kernel" (or "tiled_pair_kernel",
+ * "tiled_split_kernel"), or "fast_step_kernel" for the untiled step, one thread per
+ * site or divided over warps (no reference counterpart). */
 const char* gft_step_kernel_name(const gft_handle* h);
 
 /* Number of kernels gft_evolve has launched on this handle so far (step
@@ -274,8 +275,8 @@ int gft_observe_static(const gft_config* cfg, const float* d_scalars, const floa
  * kind 0 = automatic (the tiled kernel when the lattice divides into a built
  * tile and the tiles fill enough waves of resident CTAs -- 0.9 of a wave for the SM
  * model and 3 for the 2HDM; in the FP64 form, in 8 x 16 tiles, 4 and 2.5 --, else the
- * one-thread-per-site kernel), 1 = one
- * thread per site with neighbours read through L1/L2, 2 = TMA-staged tiles
+ * one-thread-per-site kernel, which up to 16,384 sites divides a site's update over
+ * warps), 1 = one thread per site, whatever the size, with neighbours read through L1/L2, 2 = TMA-staged tiles
  * marching along x (mixed form; FP64 form of the SM model), 3 = as 2, with two sites per thread in paired
  * FP32 arithmetic on the plain (non-logging) steps (periodic SM model, tiles 0
  * and 3).  tile = tile shape (0: 8 x 32, 1: 4 x 32,

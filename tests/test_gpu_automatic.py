@@ -50,3 +50,23 @@ def test_kind_0_keeps_a_tile_it_is_given():
         assert ev.step_kernel_name == "tiled_step_kernel"
         ev.set_kernel()
         assert ev.step_kernel_name == "fast_step_kernel"
+
+
+@pytest.mark.parametrize("form,model,family", [("mixed", 1, 0), ("fp64", 1, 0), ("mixed", 2, 2), ("fp64", 2, 1)])
+def test_kind_1_is_one_thread_per_site_on_small_lattices_too(form, model, family):
+    """Kind 1 on 16,384 sites, which the automatic choice divides over warps, against the same fields
+    twice along x, which are too many for that: the same kernel leaves the same bits, twice."""
+    from gftevolver_b200 import Evolver, InitialData, LatticeParams
+    ic = InitialData(seed=9, mean=[1.0 if model == 1 else 0.7] * 8, sigma=[0.1] * 8, theta_sigma=0.1, eps_sigma=0.1)
+    make = lambda nx: Evolver(LatticeParams(model=model, nx=nx, ny=32, nz=32, higgs_family=family, energy_every=2),  # noqa: E731
+                              form=form)
+    with make(16) as small, make(32) as large:
+        small.init_fields(ic)
+        sc, ve = small.download()
+        large.upload(*(np.concatenate([a, a], 1) for a in (sc, ve)), 0)
+        small.set_kernel(1)
+        small.evolve(3)
+        large.evolve(3)
+        assert large.step_kernel_name == small.step_kernel_name == "fast_step_kernel"
+        for a, b in zip(small.download(), large.download()):
+            np.testing.assert_array_equal(np.concatenate([a, a], 1), b)
