@@ -339,10 +339,15 @@ constexpr int ref_min_blocks()
 {
     return HF == kHfNone ? 7 : 8;
 }
+// The generator links' sines and roots make one block's chain long.  Where seven blocks per SM need a
+// second wave and five fill at most two, or a last wave is less than a quarter full, the SM step takes
+// five (us per step, FP32 storage, seven / five: 48^3, 1,152 blocks, 220 / 194, logging 293 / 261; 264 x 32 x 32,
+// 2,112 blocks, 334 / 309; the other sizes run up to 30 % faster with seven).
+constexpr int kRefFewBlocks = 5;
 
-template <class S, int MODEL, int HF, bool ENERGY>
-__global__ void __launch_bounds__(128, ref_min_blocks<HF>()) ref_step_kernel(StepParams P, LevelPtrs<S> now, LevelPtrs<S> past,
-                                                       unsigned* status, double* partials)
+template <class S, int MODEL, int HF, bool ENERGY, int BLOCKS = ref_min_blocks<HF>()>
+__global__ void __launch_bounds__(128, BLOCKS) ref_step_kernel(StepParams P, LevelPtrs<S> now, LevelPtrs<S> past,
+                                                               unsigned* status, double* partials)
 {
     constexpr int NSC = (MODEL == kModelSM) ? 4 : 8;
     constexpr int NEQ = hf_neq(HF);  // gauge equations per direction
@@ -775,6 +780,15 @@ void ref_step_launch(const StepParams& P, const LevelPtrs<S>& now, const LevelPt
 {
     const dim3 block(32, 4, 1);
     const dim3 grid((P.nz + 31) / 32, (P.ny + 3) / 4, P.nx);
+    if constexpr (MODEL == kModelSM) {
+        const int wave = ref_min_blocks<HF>() * 148, few = kRefFewBlocks * 148, blocks = ref_launch_blocks(P);
+        if (P.gen && blocks > wave && (blocks <= 2 * few || blocks % wave <= wave / 4)) {
+            auto k = energy ? ref_step_kernel<S, MODEL, HF, true, kRefFewBlocks>
+                            : ref_step_kernel<S, MODEL, HF, false, kRefFewBlocks>;
+            k<<<grid, block, 0, stream>>>(P, now, past, status, partials);
+            return;
+        }
+    }
     if (energy)
         ref_step_kernel<S, MODEL, HF, true><<<grid, block, 0, stream>>>(P, now, past, status, partials);
     else
