@@ -69,7 +69,8 @@ def parse():
     ap.add_argument("--kernel", choices=["auto", "global", "tiled", "pair", "split"], default="auto",
                     help="step kernel of the throughput forms")
     ap.add_argument("--tile", type=int, default=0, help="tiled kernel: tile shape index (0: 8x32, 1: 4x32, 2: 4x16, 3: 16x16)")
-    ap.add_argument("--march", type=int, default=32, help="tiled kernel: planes per CTA along x")
+    ap.add_argument("--march", type=int, default=32,
+                    help="tiled kernel: planes per CTA along x (with the other defaults: the library's own choice)")
     ap.add_argument("--precision-table", type=int, default=0,
                     help="steps of a run of every form (mixed, ref32, fp64) against the FP64 form (0: skip)")
     ap.add_argument("--precision-steps", type=int, default=1000,
@@ -531,6 +532,7 @@ def main():
 
     kind = {"auto": 0, "global": 1, "tiled": 2, "pair": 3, "split": 4}[args.kernel]
     kind64 = {"auto": 0, "global": 1, "tiled": 2}[args.fp64_kernel]
+    launch_asked = kind != 0 or args.tile != 0 or args.march != 32  # else the library's own tile and march
 
     def make_runner(form_):
         """N = 1: the whole lattice.  N > 1: this rank's x-slab of an (N * n) x n x n lattice
@@ -547,7 +549,7 @@ def main():
 
     def timed_run(form_, steps, warmup, sampler=None):
         runner, ev = make_runner(form_)
-        if form_ == "mixed" and (kind != 0 or args.tile != 0 or args.march != 32):
+        if form_ == "mixed" and launch_asked:
             ev.set_kernel(kind, args.tile, args.march)
         if form_ == "fp64" and kind64 != 0:
             ev.set_kernel(kind64, args.tile if kind64 == 2 else 0, args.march)
@@ -687,7 +689,8 @@ def main():
                                       if args.exchange == "library" else "after the step, from a callback")
                                    + "), FP64 all-reduce of the analyser rows") if world > 1 else
                                   ("single GPU, one x-slab exchanging with itself" if args.slab else "single GPU"),
-                   "kernel": args.kernel, "tile": args.tile, "march": args.march},
+                   "kernel": args.kernel, "tile": args.tile if launch_asked else "auto",
+                   "march": args.march if launch_asked else "auto"},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": traffic, "peak_kind": peak_kind, "kernel": kernel_name,
                      "bytes_per_site_update": balg, "avg_kernel_ms": kms, "kernel_launches_timed": nk,
