@@ -124,8 +124,7 @@ __device__ __forceinline__ void fast_step_body(StepParams P, KConst<S> F, LevelP
         n.d12 = o.c + o.p[1] + o.m[2];
         n.d20 = o.c + o.p[2] + o.m[0];
         n.d21 = o.c + o.p[2] + o.m[1];
-        XCarry<S, (MODEL == kModelSM) ? 1 : 2> carry;
-        carry.valid = false;
+        XCarry<S, (MODEL == kModelSM) ? 1 : 2> carry;  // of a march; not read here
         site_step<S, MODEL, ENERGY, HF>(P, F, GlobalAcc<S>{now}, n, PastSite<S>{past, o.c}, carry, obs, warn,
                                         counts(P, x));
     }
@@ -242,7 +241,8 @@ int fast_launch_blocks(const StepParams& P, bool divide)
     return divide && use_roles(P) ? role_launch_blocks(P) : patch_blocks(P, kStepThreads);
 }
 
-// The mixed form's Gauss pass runs in tiles from 300,000 sites on (its 296 blocks then march five planes or more) where at most a third of the tiles' sites lie past a ragged
+// The mixed form's Gauss pass runs in tiles from 300,000 sites on (its 296 blocks then march four
+// planes at least, each after one more) where at most a third of the tiles' sites lie past a ragged
 // edge.  us per pass with its reduction, tiles / one thread per site: SM 48^3 17 / 15, 64^3 20 / 21,
 // 100^3 46 / 63, 150 x 100 x 75 50 / 67, 128^3 72 / 103, 256^3 465 / 692; 2HDM 64^3 23 / 21, 96^3 49 / 57,
 // 192^3 280 / 308.  The FP64 form's words would not fit the registers; it keeps one thread per site.

@@ -183,7 +183,6 @@ struct Stencil {
 // the plane x - 1.
 template <class C, int ND>
 struct XCarry {
-    bool valid;
     C s01, s02;
     C v01[3], v02[3];
     Q<C> t0[ND];
@@ -328,7 +327,6 @@ __device__ __forceinline__ void site_carry(const A& acc, const Stencil<R>& n, XC
     gsincos(th0, sn, cs);
 #pragma unroll
     for (int db = 0; db < ND; db++) carry.t0[db] = transport(U0, cs, sn, acc.ph(db, n.c));
-    carry.valid = true;
 }
 
 // asin of the three U(1) increments: the series where all are small, which
@@ -832,7 +830,6 @@ __device__ __forceinline__ void site_step(const StepParams& P, const KConst<S>& 
         su2_advance3(H, RH, ps.L.hq, ps.s, warn, check);
     }
     if (!isfinite(check)) warn |= kWarnNonFinite;
-    if constexpr (CARRY) carry.valid = true;
     if (!count) {
         warn = warn_in;
         return;
