@@ -296,15 +296,29 @@ bool encode_tiled(const gft_handle* h, const StepParams& P, int tile, TMaps* tm,
 // Automatic choice (kernel_kind 0): the staged step when its tiles fill enough waves of
 // resident CTAs (fewer leave SMs idle while each CTA marches its planes), else one thread per
 // site.  us per plain step on a B200, staged (the march below) / one thread per site:
-//   SM mixed:   64^3 (0.3 waves) 34 / 21, 96^3 (0.97) 58 / 62, 128^3 (2.4) 133 / 136, 160^3 224 /
-//               257, 192^3 (8) 376 / 439; logging steps 71 / 86 and 170 / 195 at 96^3 and 128^3;
-//   2HDM mixed: 128^3 (2.4 waves) 175 / 163, 144^3 (3.3) 239 / 259, 160^3 (4.7) 303 / 317, 192^3
-//               (8) 510 / 546, logging 660 / 736;
-//   FP64 SM:    128^3 (1.7 waves) 302 / 287, 160^3 (3.4) 574 / 558, 176^3 (4.9) 627 / 827, 192^3
-//               (5.8) 823 / 993, 256^3 (13.8) 1936 / 2290;
-//   FP64 2HDM:  128^3 369 / 348, logging 552 / 581, 144^3 (2.7) 474 / 572, 160^3 650 / 673, logging
-//               1027 / 1127, 192^3 1064 / 1160, logging 1588 / 1938.
-constexpr double kAutoWavesSM = 0.9, kAutoWaves2HDM = 3.0, kAutoWavesFP64SM = 4.0, kAutoWavesFP642HDM = 2.5;
+//   SM mixed, 8 x 32:    64^3 (0.3 waves) 39 / 23, 96^3 (0.97) 59 / 63, 128^3 (2.4) 134 / 136, 160^3 226 /
+//                        259, 192^3 (8) 376 / 440; logging steps 72 / 85 and 173 / 192 at 96^3 and 128^3;
+//   SM mixed, 16 x 16:   80^3 (0.6) 56 / 39, 112^3 (1.7) 104 / 97, 120 x 128 x 112 (1.9) 110 / 115, 144^3
+//                        (3.3) 179 / 193; logging 132 / 137 and 229 / 285 at 112^3 and 144^3;
+//   SM mixed, 4 x 32:    128 x 132 x 128 (2.5) 148 / 141, 160 x 164 x 160 (4.8) 260 / 265, logging 351 / 379;
+//   2HDM mixed, 8 x 32:  128^3 (2.4) 176 / 164, 160^3 (4.7) 304 / 318, 192^3 (8) 513 / 545, logging 665 / 748;
+//   2HDM mixed, 16 x 16: 112^3 (1.7) 140 / 123, 144^3 (3.3) 240 / 251, 176^3 (6.1) 406 / 453;
+//   FP64 SM, 8 x 16:     128^3 (1.7) 291 / 289, 300 x 96 x 96 (2.4) 376 / 377, logging 609 / 577, 176^3 (4.9)
+//                        631 / 816, 192^3 (5.8) 827 / 953, 256^3 (13.8) 1854 / 2270.  From 2.7 to 4 waves
+//                        the staged step gains 7 to 17 % (160^3 507 / 556) that this line leaves;
+//   FP64 2HDM, 8 x 16:   128^3 (1.7) 372 / 373, logging 549 / 598, 64 x 160 x 160 (1.4) 315 / 292, 144^3 (2.7)
+//                        480 / 568, 160^3 660 / 718, logging 1021 / 1160, 192^3 1076 / 1233, logging 1617 / 1996.
+// The 2HDM's 4 x 32 and 4 x 16 tiles are slower at every size (192 x 196 x 192 576 / 556, 208^3 829 /
+// 748), as are FP64's (SM 4 x 32 there 1268 / 973).  So are the SM's 4 x 16 (208^3 577 / 563), which
+// only lattices that admit no other tile have.
+constexpr double kAutoNever = 1e30;
+double auto_waves(bool fp64, bool sm, int tile)
+{
+    if (fp64) return !sm ? 2.5 : (tile == kTileFP64 || tile == 0 || tile == 3 ? 4.0 : kAutoNever);
+    static const double waves_sm[kTiledVariants] = {0.9, 4.0, 0.9, 2.0};
+    static const double waves_2hdm[kTiledVariants] = {3.0, kAutoNever, kAutoNever, 3.0};
+    return (sm ? waves_sm : waves_2hdm)[tile];
+}
 // Planes per CTA unless the caller sets them.  Mixed form: short enough to balance the last
 // wave, long enough for the start of a march (two more planes staged) not to count: SM 128^3 /
 // 192^3 / 256^3 at 8, 12, 16, 32 planes 133 / 377 / 849, 133 / 376 / 830, 135 / 372 / 857,
@@ -323,8 +337,7 @@ bool use_tiled(const gft_handle* h, const StepParams& P)
     if (!tiled_supported(P, h->tile_variant)) return false;
     if (h->kernel_kind != 0) return true;
     const double slots = (double)h->nsm * tiled_ctas_per_sm(h->tile_variant, fp64, sm);
-    const double waves = sm ? (fp64 ? kAutoWavesFP64SM : kAutoWavesSM) : (fp64 ? kAutoWavesFP642HDM : kAutoWaves2HDM);
-    return tiled_blocks(P, h->tile_variant, h->march) >= waves * slots;
+    return tiled_blocks(P, h->tile_variant, h->march) >= auto_waves(fp64, sm, h->tile_variant) * slots;
 }
 
 // Plain steps of the SM mixed form with two sites per thread (kernel kind 3):
@@ -540,17 +553,15 @@ int gft_create(const gft_config* cfg, gft_handle** out)
     const StepParams P = make_params(h, 0, false);
     h->march = cfg->form == GFT_FORM_FP64 ? kAutoMarchFP64 : kAutoMarchMixed;
     if (cfg->form == GFT_FORM_MIXED || cfg->form == GFT_FORM_FP64) {
-        // default tile: the largest built shape the lattice divides
-        h->tile_variant = 0;
-        while (h->tile_variant < kTiledVariants && !tiled_supported(P, h->tile_variant)) h->tile_variant++;
-        // FP64: two CTAs of four warps per SM, where an 8 x 32 tile's staged planes leave one of
-        // eight; its barriers stop half the warps (SM, us per step, 256^3 / 192^3: 1936 / 823
-        // against 2017 / 866; logging step 2928 against 2802).  The 2HDM is built for it alone.
-        if (cfg->form == GFT_FORM_FP64) {
-            if (tiled_supported(P, kTileFP64))
-                h->tile_variant = kTileFP64;
-            else if (cfg->model != GFT_MODEL_SM)
-                h->tile_variant = kTiledVariants;
+        // The tile: the largest built shape the lattice divides, 8 x 32 before 16 x 16, whose rows are
+        // longer.  FP64: 8 x 16, two CTAs of four warps per SM where an 8 x 32 tile's staged planes leave
+        // one of eight, whose barriers stop all its warps (SM, us per step, 256^3 / 192^3: 1854 / 827
+        // against 2017 / 889; logging step 2985 against 2865).  The 2HDM is built for it alone.
+        const int order[kTiledVariants] = {0, 3, 1, 2};
+        h->tile_variant = kTileFP64;
+        for (int k = 0; k < kTiledVariants && cfg->form == GFT_FORM_MIXED; k++) {
+            h->tile_variant = order[k];
+            if (tiled_supported(P, h->tile_variant)) break;
         }
         h->tiled_ready = tiled_supported(P, h->tile_variant) && encode_tiled(h, P, h->tile_variant, h->tm, h->tp);
         if (h->tiled_ready) h->auto_tile = h->tile_variant;

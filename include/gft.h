@@ -273,8 +273,9 @@ int gft_observe_static(const gft_config* cfg, const float* d_scalars, const floa
 
 /* Step-kernel selection for the throughput forms (no reference counterpart):
  * kind 0 = automatic (the tiled kernel when the lattice divides into a built
- * tile and the tiles fill enough waves of resident CTAs -- 0.9 of a wave for the SM
- * model and 3 for the 2HDM; in the FP64 form, in 8 x 16 tiles, 4 and 2.5 --, else the
+ * tile and the tiles fill enough waves of resident CTAs -- in 8 x 32 tiles 0.9 of a
+ * wave for the SM model and 3 for the 2HDM, more in smaller tiles; in the FP64 form,
+ * in 8 x 16 tiles, 4 and 2.5 --, else the
  * one-thread-per-site kernel, which up to 16,384 sites divides a site's update over
  * warps), 1 = one thread per site, whatever the size, with neighbours read through L1/L2, 2 = TMA-staged tiles
  * marching along x (mixed form; FP64 form of the SM model), 3 = as 2, with two sites per thread in paired

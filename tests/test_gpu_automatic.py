@@ -70,3 +70,34 @@ def test_kind_1_is_one_thread_per_site_on_small_lattices_too(form, model, family
         assert large.step_kernel_name == small.step_kernel_name == "fast_step_kernel"
         for a, b in zip(small.download(), large.download()):
             np.testing.assert_array_equal(np.concatenate([a, a], 1), b)
+
+
+@pytest.mark.parametrize("form,model,shape", [
+    ("mixed", 1, (80, 80, 80)),     # 16 x 16 tiles fill 0.6 of a wave: 56 us a step, one thread per site 39
+    ("mixed", 1, (96, 100, 96)),    # 4 x 32 tiles, one wave: 81 / 64
+    ("mixed", 2, (200, 100, 144)),  # 4 x 16 tiles only: 275 / 240
+    ("fp64", 1, (128, 132, 128)),   # 4 x 32 tiles only: 433 / 298
+])
+def test_lattices_that_tile_badly_run_one_thread_per_site(form, model, shape):
+    from gftevolver_b200 import Evolver, LatticeParams
+    nx, ny, nz = shape
+    with Evolver(LatticeParams(model=model, nx=nx, ny=ny, nz=nz), form=form) as ev:
+        assert ev.step_kernel_name == "fast_step_kernel"
+
+
+@pytest.mark.parametrize("model", [1, 2])
+def test_an_edge_of_16_takes_16_x_16_tiles(model):
+    """z divides into 16 but not 32: 16 x 16 tiles, not 4 x 16, by the partial sums of the energy row,
+    whose order is the tiles'."""
+    from gftevolver_b200 import Evolver, InitialData, LatticeParams
+    p = LatticeParams(model=model, nx=144, ny=144, nz=144, energy_every=1)
+    ic = InitialData(seed=5, mean=[1.0 if model == 1 else 0.7] * 8, sigma=[0.1] * 8, theta_sigma=0.1, eps_sigma=0.1)
+    rows = []
+    for kernel in (None, (2, 3, 12), (2, 2, 12)):
+        with Evolver(p, form="mixed") as ev:
+            if kernel:
+                ev.set_kernel(*kernel)
+            assert ev.step_kernel_name == "tiled_step_kernel"
+            ev.init_fields(ic)
+            rows.append(ev.evolve(1))
+    assert rows[0] == rows[1] != rows[2]
