@@ -48,29 +48,47 @@ constexpr int kStepThreads = 128;
 constexpr int kGaussThreads = 256;  // 32 x 8: 2 % faster than 32 x 4 at 256^3 (624 against 638 us)
 
 // The (z, y) patch of sites a block of T threads covers: bz x by of them, bz * by <= T, thread t at
-// column t % bz, row t / bz.  32 x T/32 wherever z divides into 32; elsewhere the shape that leaves the
-// fewest threads without a site (75 sites along z in three blocks of 32 idle a fifth of them: SM
-// mixed 150 x 100 x 75 in patches of 25 x 5 92 -> 80 us per step, 100^3 84 -> 72).
+// column t % bz, row t / bz.  32 x T/32 unless the shape that leaves the fewest threads without a site
+// puts `gain` times as many to work (75 sites along z in three blocks of 32 idle a fifth of them).  Any
+// other patch costs a run-time division and shorter or misaligned rows.  us per plain step of 600,000
+// sites in the best shape / in 32 x 4, by how many times the threads with a site:
+//   1.25 (nz = 75): SM mixed 45 / 53, 2HDM 59 / 63, FP64 SM 96 / 110; 1.47 (40): 47 / 64, 60 / 75, 102 / 129;
+//   1.14 (130): 49 / 52, 61 / 62;  1.10 (84): 45 / 49, 60 / 58, FP64 SM 101 / 99;
+//   1.04 (56): 47 / 49, 61 / 58, 107 / 99;  1.00 (60): 48 / 47, 61 / 55, 102 / 95.
+// Logging steps hide the cost (84: 2HDM 74 / 81, FP64 193 / 203; 144, 1.07: 74 / 78, 188 / 195), and so does the
+// family SU(2) (84: 93 / 95).  The mixed Gauss pass runs faster in narrow rows at equal use (60: 21.4 /
+// 22.5), the FP64 one slower (28.5 / 26.0).
 struct Patch {
     int bz, by;
     int inv;  // t / bz = t * inv >> 16, exact for t < 1024 and bz <= 64
 };
 
-Patch pick_patch(const StepParams& P, int threads)
+constexpr double kPatchGain = 1.03, kPatchGainPlain = 1.12;
+template <class S, int MODEL, int HF>
+constexpr double step_gain(bool energy)
 {
-    Patch best = {32, threads / 32, 65536 / 32};
-    if (P.nz % 32 == 0) return best;
+    return energy || (sizeof(S) == 4 && (MODEL == kModelSM || HF != kHfNone)) ? kPatchGain : kPatchGainPlain;
+}
+constexpr double gauss_gain(bool fp32) { return fp32 ? 0.99 : 1.12; }
+
+Patch pick_patch(const StepParams& P, int threads, double gain)
+{
+    const Patch rows = {32, threads / 32, 65536 / 32};
+    if (P.nz % 32 == 0) return rows;
+    auto used = [&](int bz, int by) {
+        const double cover = (double)((P.nz + bz - 1) / bz) * ((P.ny + by - 1) / by) * threads;
+        return (double)P.nz * P.ny / cover;
+    };
+    Patch best = rows;
     double most = 0.0;
     for (int bz = 8; bz <= 64; bz++) {
-        const int by = threads / bz;
-        const double cover = (double)((P.nz + bz - 1) / bz) * ((P.ny + by - 1) / by) * threads;
-        const double used = (double)P.nz * P.ny / cover;
-        if (used > most * 1.02) {  // wider rows only where they pay
-            most = used;
-            best = {bz, by, (65536 + bz - 1) / bz};
+        const double u = used(bz, threads / bz);
+        if (u > most * 1.02) {  // wider rows only where they pay
+            most = u;
+            best = {bz, threads / bz, (65536 + bz - 1) / bz};
         }
     }
-    return best;
+    return most > gain * used(rows.bz, rows.by) ? best : rows;
 }
 
 dim3 patch_grid(const StepParams& P, const Patch& p)
@@ -203,7 +221,7 @@ template <class S, int MODEL, int HF>
 void fast_step_launch(const StepParams& P, const LevelPtrs<S>& now, const LevelPtrs<S>& past, unsigned* status,
                       double* partials, bool energy, cudaStream_t stream)
 {
-    const Patch p = pick_patch(P, kStepThreads);
+    const Patch p = pick_patch(P, kStepThreads, step_gain<S, MODEL, HF>(energy));
     const bool any = p.bz != 32;
     auto k = energy ? (any ? fast_step_kernel<S, MODEL, HF, true, true> : fast_step_kernel<S, MODEL, HF, true, false>)
                     : (any ? fast_step_kernel<S, MODEL, HF, false, true> : fast_step_kernel<S, MODEL, HF, false, false>);
@@ -214,16 +232,16 @@ template <class S, int MODEL, int HF>
 void fast_gauss_launch(const StepParams& P, const LevelPtrs<S>& now, const LevelPtrs<S>& fut, double* partials,
                        cudaStream_t stream)
 {
-    const Patch p = pick_patch(P, kGaussThreads);
+    const Patch p = pick_patch(P, kGaussThreads, gauss_gain(sizeof(S) == 4));
     auto k = p.bz != 32 ? fast_gauss_kernel<S, MODEL, HF, true> : fast_gauss_kernel<S, MODEL, HF, false>;
     k<<<patch_grid(P, p), kGaussThreads, 0, stream>>>(P, now, fut, p, partials);
 }
 
 }  // namespace
 
-static int patch_blocks(const StepParams& P, int threads)
+static int patch_blocks(const StepParams& P, int threads, double gain)
 {
-    const dim3 g = patch_grid(P, pick_patch(P, threads));
+    const dim3 g = patch_grid(P, pick_patch(P, threads, gain));
     return (int)(g.x * g.y * g.z);
 }
 
@@ -238,7 +256,7 @@ static bool use_roles(const StepParams& P) { return P.nsite <= kRoleMaxSites; }
 
 int fast_launch_blocks(const StepParams& P, bool divide)
 {
-    return divide && use_roles(P) ? role_launch_blocks(P) : patch_blocks(P, kStepThreads);
+    return divide && use_roles(P) ? role_launch_blocks(P) : patch_blocks(P, kStepThreads, kPatchGain);
 }
 
 // The mixed form's Gauss pass runs in tiles from 300,000 sites on (its 296 blocks then march four
@@ -255,7 +273,7 @@ static bool gauss_in_tiles(const StepParams& P, bool fp32)
 
 int fast_gauss_blocks(const StepParams& P, bool fp32)
 {
-    return gauss_in_tiles(P, fp32) ? kGaussCtas : patch_blocks(P, kGaussThreads);
+    return gauss_in_tiles(P, fp32) ? kGaussCtas : patch_blocks(P, kGaussThreads, gauss_gain(fp32));
 }
 
 // P.hf selects the Higgs-family variant (2HDM only); the Gauss kernel writes

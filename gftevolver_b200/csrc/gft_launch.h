@@ -34,7 +34,7 @@ template <class S, int MODEL>
 cudaError_t launch_role_step(const StepParams& P, const LevelPtrs<S>& now, const LevelPtrs<S>& past, unsigned* status,
                              double* partials, bool energy, cudaStream_t stream);
 int role_launch_blocks(const StepParams& P);
-int fast_launch_blocks(const StepParams& P, bool divide);
+int fast_launch_blocks(const StepParams& P, bool divide);  // of a logging step: its partial rows
 int fast_gauss_blocks(const StepParams& P, bool fp32);
 
 // Tiled throughput kernel (gft_tiled_kernels.cu): TMA-staged planes, x-march.
