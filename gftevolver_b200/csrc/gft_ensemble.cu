@@ -359,7 +359,7 @@ struct gft_batch {
     std::vector<std::array<LevelPtrs<float>, 2>> lv;
     EnsMaps* d_maps = nullptr;
     int variant = -1;
-    int lx = 24;  // 16 x 16 tiles, march 16 / 24 / 32 / 64: 405 / 397 / 405 / 441 us per step as below
+    int lx = 24;  // 16 x 16 tiles, march 16 / 24 / 32 / 64: 373 / 367 / 375 / 409 us per step as below
     int4* d_items = nullptr;
     int nitems = 0;
     int* d_order = nullptr;       // per-CTA tile lists of each group (group-local item indices)
@@ -849,14 +849,21 @@ int gft_batch_create(const gft_config* cfgs, int n, gft_batch** out)
     b->neq = config_neq(cfgs[0]);
     b->cfg.assign(cfgs, cfgs + n);
     // 256-thread tiles before the smaller ones: a small tile's halo row and column are a larger part
-    // of its work (32 members of 32 to 96 planes an edge, us per step at march 24: 16 x 16 397, 4 x 16
-    // 595; 12 of 32 and 64: 8 x 32 123, 16 x 16 117, 4 x 32 110, 4 x 16 143).  Of those the SM model
+    // of its work (32 members of 32 to 96 planes an edge, us per step at march 24: 16 x 16 367, 4 x 16
+    // 551; 12 of 32 and 64: 16 x 16 134, 8 x 32 139, 4 x 32 140, 4 x 16 170).  Of those the SM model
     // takes 16 x 16 first, whose halo is the shorter, the 2HDM 8 x 32, whose rows are (us per step 16 x
-    // 16 / 8 x 32, 16 members of 64^3: SM 264 / 275, logging 332 / 338, 2HDM 345 / 338; 12 of 96^3: SM 610 /
-    // 628, logging 768 / 788, 2HDM 790 / 783; 32 of 32^3: SM 86 / 92, 2HDM 105 / 102).
+    // 16 / 8 x 32, 16 members of 64^3: SM 268 / 278, 2HDM 352 / 346; 12 of 96^3: SM 614 / 633, 2HDM 838 /
+    // 811; 32 of 32^3: SM 88 / 94, 2HDM 107 / 104).  SM members of up to 768 sites a plane take 4 x 16 at
+    // any number of members: 16 x 16 leave one to three tiles each, marching alone (us per step 4 x 16 / 16 x
+    // 16, 16^3: 1 member 34 / 45, 24 36 / 45, 400 319 / 369; 16 x 16 x 48: 34 / 44, 39 / 46, 531 / 532; but 16 x
+    // 16 x 64: 34 / 44, 50 / 46, 200 416 / 295).  A member's tile depends on the shapes alone, not on their number.
     const bool sm = b->model == GFT_MODEL_SM;
-    for (const int v : {sm ? 3 : 0, sm ? 0 : 3, 1, 2})
-        if (b->variant < 0 && variant_fits(b, v)) b->variant = v;
+    const bool narrow = sm && std::all_of(b->cfg.begin(), b->cfg.end(), [](const gft_config& c) {
+                            return (long long)c.ny * c.nz <= 768;
+                        });
+    const int order[] = {2, sm ? 3 : 0, sm ? 0 : 3, 1, 2};
+    for (int k = narrow ? 0 : 1; k < 5 && b->variant < 0; k++)
+        if (variant_fits(b, order[k])) b->variant = order[k];
     if (b->variant < 0 && b->hf == kHfNone) {
         delete b;
         set_error("gft_batch_create: the members' (ny, nz) share no built tile shape (4 x 16, the smallest, needs ny % 4 == 0 and nz % 16 == 0)");
