@@ -321,8 +321,8 @@ double auto_waves(bool fp64, bool sm, int tile)
 }
 // Planes per CTA unless the caller sets them.  Mixed form: short enough to balance the last
 // wave, long enough for the start of a march (two more planes staged) not to count: SM 128^3 /
-// 192^3 / 256^3 at 8, 12, 16, 32 planes 133 / 377 / 849, 133 / 376 / 830, 135 / 372 / 857,
-// 135 / 375 / 837 us; 96^3 58 at 12, 72 to 95 at the others.
+// 192^3 / 256^3 at 8, 12, 16, 32 planes 134 / 380 / 887, 134 / 383 / 855, 136 / 381 / 863,
+// 136 / 387 / 851 us; 96^3 59 at 12, 73 to 95 at the others.
 constexpr int kAutoMarchMixed = 12, kAutoMarchFP64 = 32;
 // gft_set_kernel's march where a caller names none (with tile 0: the automatic choice of gft_create)
 constexpr int kKernelMarchDefault = 32;

@@ -157,10 +157,11 @@ __device__ __forceinline__ void fast_step_body(StepParams P, KConst<S> F, LevelP
 // Resident blocks per SM the launch bounds of an instance ask for: as many as its
 // registers take with no or a few spilled words, since the warps hide the
 // neighbour loads' latency (us per step on a B200, unbounded / bounded):
-//   FP64 SM 256^3: 8 warps per SM 3410, three blocks (168 registers) 2637; four
-//     blocks spill 288 bytes and were 5 % slower than three;
-//   float 2HDM 192^3: 132 registers, three blocks 689; four blocks (128) 576;
-//   float 2HDM with the family SU(2) 96 x 96 x 192: three blocks (168) 243;
+//   FP64 SM 256^3: three blocks (168 registers) 2926 / 2267, logging 3499 / 3471; four spill, and
+//     measured 2146 and 3228 last (5 % slower than three when the bound was set);
+//   FP64 2HDM: two blocks (254 registers), as without a bound;
+//   float 2HDM 192^3: four blocks (128) 646 / 545, logging 756 / 748;
+//   float 2HDM with the family SU(2) 96 x 96 x 192: three blocks (168) 305 / 235, logging 340 / 340;
 //   float SM: 86-100 registers, five blocks either way.
 template <class S, int MODEL, int HF>
 constexpr int fast_min_blocks()
@@ -248,9 +249,9 @@ static int patch_blocks(const StepParams& P, int threads, double gain)
 // Small lattices divide a site's update over several warps (gft_role_kernels.cu): up to about one
 // warp of sites per scheduler (592 of them), where one thread per site leaves them waiting on one
 // chain of instructions each.  us per step replayed from a graph, divided / one thread per site:
-//   16^3: SM mixed 2.9 / 4.1, FP64 3.9 / 5.6, 2HDM with the family SU(2) 3.4 / 6.6, FP64 4.1 / 8.4
-//   24^3:          3.6 / 4.4,      4.9 / 6.0,                            4.7 / 6.9,      8.3 / 9.2
-//   32^3:          5.0 / 4.8,      8.7 / 7.3,                            9.6 / 6.9,       17 / 12
+//   16^3: SM mixed 2.9 / 3.9, FP64 3.7 / 6.1, 2HDM with the family SU(2) 3.3 / 6.1, FP64 4.1 / 8.9
+//   24^3:          3.6 / 4.2,      4.7 / 5.9,                            4.7 / 6.7,      8.2 / 8.9
+//   32^3:          5.0 / 4.7,      8.7 / 7.0,                            9.3 / 6.9,       17 / 12
 constexpr int kRoleMaxSites = 16384;
 static bool use_roles(const StepParams& P) { return P.nsite <= kRoleMaxSites; }
 
@@ -261,9 +262,9 @@ int fast_launch_blocks(const StepParams& P, bool divide)
 
 // The mixed form's Gauss pass runs in tiles from 300,000 sites on (its 296 blocks then march four
 // planes at least, each after one more) where at most a third of the tiles' sites lie past a ragged
-// edge.  us per pass with its reduction, tiles / one thread per site: SM 48^3 17 / 15, 64^3 20 / 21,
-// 100^3 46 / 63, 150 x 100 x 75 50 / 67, 128^3 72 / 103, 256^3 465 / 692; 2HDM 64^3 23 / 21, 96^3 49 / 57,
-// 192^3 280 / 308.  The FP64 form's words would not fit the registers; it keeps one thread per site.
+// edge.  us per pass with its reduction, tiles / one thread per site: SM 48^3 17 / 15, 64^3 21 / 21,
+// 100^3 46 / 63, 150 x 100 x 75 51 / 67, 128^3 72 / 101, 256^3 467 / 723; 2HDM 64^3 22 / 21, 96^3 49 / 56,
+// 192^3 264 / 293.  The FP64 form's words would not fit the registers; it keeps one thread per site.
 constexpr int kGaussTileSites = 300000;
 static bool gauss_in_tiles(const StepParams& P, bool fp32)
 {

@@ -9,9 +9,9 @@
 //
 // The pass was bound by FP64 work: conversions of the FP32 words and the products.  Per site 38
 // words (46 with two doublets) are converted instead of 68 (76), three sines taken instead of six; at SM
-// 256^3 it reads at 5.4 TB/s (each word of both levels once) and takes 465 us with its reduction, 692
-// before.  Two blocks of eight warps per SM have 128 registers, enough to hold the next plane of one
-// doublet; two doublets' next plane is loaded at the end of a plane (2HDM 192^3 280 us, held: 303).
+// 256^3 it reads at 5.4 TB/s (each word of both levels once) and takes 467 us with its reduction, 723
+// one thread per site.  Two blocks of eight warps per SM have 128 registers, enough to hold the next plane of one
+// doublet; two doublets' next plane is loaded at the end of a plane (2HDM 192^3 264 us; held it took 8 % longer).
 // A block of 8 x 32 sites and a ninth warp leaves 96 registers and spills (870 us).
 #pragma once
 

@@ -331,9 +331,9 @@ __device__ __forceinline__ S ref_potential_energy(const StepParams& P, const S* 
 // Resident blocks per SM the launch bounds ask for.  The kernel waits on FP64 and local-memory
 // latencies in rolled loops (unrolled, the code of six pairs of loops misses the instruction
 // cache: 163 -> 211 us per step at SM 64^3), so it runs faster with more warps and some spills
-// (us per step, SM 64^3 / 2HDM 64^3 / 2HDM with the family SU(2) 48^3: unbounded 144 / 190 /
-// 191, five blocks 152 / 176 / 206, seven 145 / 170 / 221, eight 148 / 175 / 175; logging steps
-// unbounded 210 / 258 / 227, seven 193 / 236 / 265, eight 196 / 242 / 210).
+// (us per step, SM 64^3 / 2HDM 64^3 / 2HDM with the family U(1) 48^3 / SU(2) 48^3: unbounded 125 / 154 /
+// 113 / 165, five blocks 120 / 148 / 127 / 169, seven 120 / 147 / 140 / 188, eight 123 / 153 / 114 / 147;
+// logging steps unbounded 160 / 204 / 142 / 193, seven 161 / 205 / 183 / 234, eight 166 / 204 / 143 / 186).
 template <int HF>
 constexpr int ref_min_blocks()
 {

@@ -15,13 +15,15 @@
 // computed by TY + TZ lanes of two of the tile's warps, a different pair each plane
 // (halo_hand_over).
 //
-// The tiled steps are bound by instruction issue.  Per site the lower loops fall from four
-// (two carried) to none, their sines and the two backward transports with their sines and
-// cosines too; three turns remain: 1,436 -> 1,265 warp instructions per 32 sites at SM 128^3,
-// the halo row and column (4 % of the work of an 8 x 32 tile) included.  us per step, against
-// every thread computing its own lower loops (site_step with CARRY): SM mixed 256^3 887 -> 835,
-// 128^3 (march 12) 143 -> 133, logging 256^3 1112 -> 1061; FP64 2HDM 192^3 against one thread per
-// site 1160 -> 1064, logging 1938 -> 1588.  The float 2HDM's tiles keep site_step (hands_over).
+// The mixed form's tiled steps are bound by instruction issue (66 to 74 % of the slots, 16 warps per
+// SM); the FP64 ones wait on chains of FP64 operations with 8 warps per SM (issue 36 to 39 %, FP64
+// pipe 48 %).  Per site the lower loops fall from four (two carried) to none, their sines and the two
+// backward transports with their sines and cosines too; three turns remain: 1,306 warp instructions
+// per 32 sites at SM 128^3, the halo row and column (4 % of the work of an 8 x 32 tile) included.  us
+// per step, against every thread computing its own lower loops (site_step with CARRY): SM mixed 256^3
+// 896 -> 831, 128^3 140 -> 134, logging 256^3 1147 -> 1110; FP64 2HDM 192^3 1090 -> 1076, logging 1600 ->
+// 1617 (one thread per site 1233, 1996); FP64 SM 256^3 1793 -> 1854, logging 2993 -> 2985: there the
+// sines saved no longer pay.  The float 2HDM's tiles keep site_step (hands_over).
 #pragma once
 
 #include "gft_step_body.cuh"

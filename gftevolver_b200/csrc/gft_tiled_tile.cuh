@@ -175,8 +175,8 @@ struct TileAcc;
 // Whether a tile's sites hand their loops and transports to one another (gft_shared_body.cuh).
 // Not the float 2HDM's: with the hand-over buffers two CTAs fit an SM only over a ring of two
 // planes, and two doublets' values do not fit 128 registers beside the energy's or the ensemble's
-// list (us per step handed over / not: 192^3 plain 495 / 509, logging 736 / 660; 16 members of
-// 64^3 356 / 338).
+// list (us per step handed over / not: 192^3 plain 498 / 513, logging 737 / 665; 16 members of
+// 64^3 361 / 346).
 template <class S, int MODEL>
 constexpr bool hands_over()
 {
