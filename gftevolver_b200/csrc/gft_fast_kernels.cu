@@ -56,7 +56,9 @@ constexpr int kGaussThreads = 256;  // 32 x 8: 2 % faster than 32 x 4 at 256^3 (
 //   1.14 (130): 49 / 52, 61 / 62;  1.10 (84): 45 / 49, 60 / 58, FP64 SM 101 / 99;
 //   1.04 (56): 47 / 49, 61 / 58, 107 / 99;  1.00 (60): 48 / 47, 61 / 55, 102 / 95.
 // Logging steps hide the cost (84: 2HDM 74 / 81, FP64 193 / 203; 144, 1.07: 74 / 78, 188 / 195), and so does the
-// family SU(2) (84: 93 / 95).  The mixed Gauss pass runs faster in narrow rows at equal use (60: 21.4 /
+// family SU(2) (84: 93 / 95).  Up to two blocks of 32 x 4 per SM every block runs at once and a step takes
+// one thread's time, which a patch only lengthens (18 x 32 x 40, 288 blocks: SM mixed 4.9 / 4.7, 2HDM 5.2 /
+// 5.0, FP64 SM 8.2 / 7.3; 24 x 32 x 40, 384: 5.0 / 5.5, 5.2 / 5.8, 8.0 / 9.0).  The mixed Gauss pass runs faster in narrow rows at equal use (60: 21.4 /
 // 22.5), the FP64 one slower (28.5 / 26.0).
 struct Patch {
     int bz, by;
@@ -75,6 +77,9 @@ Patch pick_patch(const StepParams& P, int threads, double gain)
 {
     const Patch rows = {32, threads / 32, 65536 / 32};
     if (P.nz % 32 == 0) return rows;
+    if (threads == kStepThreads &&
+        (long long)((P.nz + 31) / 32) * ((P.ny + rows.by - 1) / rows.by) * P.nx <= 2 * 148)
+        return rows;
     auto used = [&](int bz, int by) {
         const double cover = (double)((P.nz + bz - 1) / bz) * ((P.ny + by - 1) / by) * threads;
         return (double)P.nz * P.ny / cover;
