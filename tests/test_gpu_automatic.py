@@ -101,3 +101,20 @@ def test_an_edge_of_16_takes_16_x_16_tiles(model):
             ev.init_fields(ic)
             rows.append(ev.evolve(1))
     assert rows[0] == rows[1] != rows[2]
+
+
+@pytest.mark.parametrize("form", ["mixed", "fp64"])
+@pytest.mark.parametrize("shape,divided", [((16, 32, 32), True), ((17, 32, 32), False)])
+def test_the_divided_step_serves_16384_sites_and_no_more(form, shape, divided):
+    """Which step runs, by its bits: the divided one sums a site's forces in another order."""
+    from gftevolver_b200 import Evolver, InitialData, LatticeParams
+    ic = InitialData(seed=9, mean=[0.7] * 8, sigma=[0.1] * 8, theta_sigma=0.1, eps_sigma=0.1)
+    out = []
+    for kind in (0, 1):
+        with Evolver(LatticeParams(model=2, nx=shape[0], ny=shape[1], nz=shape[2]), form=form) as ev:
+            ev.set_kernel(kind)
+            ev.init_fields(ic)
+            ev.evolve(2)
+            out.append(ev.download())
+    same = all(np.array_equal(a, b) for a, b in zip(*out))
+    assert same != divided
